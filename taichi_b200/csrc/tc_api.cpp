@@ -313,7 +313,7 @@ tc_status tc_spmm(const tc_plan *p, const float *d_X, int ldx, int k, float *d_Y
 {
     if (!p || k < 1 || k > 64 || ldx < k || ldy < k) return fail(TC_ERR_INVALID, "tc_spmm: k must be in [1, 64], ld >= k");
     if ((!d_X && p->N) || (!d_Y && p->M)) return fail(TC_ERR_INVALID, "tc_spmm: null argument");
-    return tc::launch_spmm(p->dev_plan(), d_X, ldx, k, d_Y, ldy, (cudaStream_t)stream);
+    return tc::launch_spmm(p->dev_plan(), p->nnz_csr, p->max_row, d_X, ldx, k, d_Y, ldy, (cudaStream_t)stream);
 }
 
 // Builds a plan from a CSR pattern, partitioning it on the GPU unless

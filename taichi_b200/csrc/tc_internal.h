@@ -175,6 +175,7 @@ struct tc_plan {
     int dia_shapes = 0, num_negs = 0, dense_nnz = 0, zero_elements = 0, sparse_nnz = 0;
     int row_start = 0, row_stop = 0;
     int64_t nnz_input = 0, nnz_csr = 0;
+    int max_row = 0;                     // CSR words of the longest row
     int hybrid = 0;
     // device arrays (one allocation, `dev`)
     void *dev = nullptr;
@@ -262,8 +263,12 @@ bool plan_window(const tc_plan *p, const int *rowptr, const int *cols, std::vect
 size_t window_smem_bytes(const DevPlan &dp);
 tc_status window_prepare(DevPlan &dp);
 tc_status launch_window(const DevPlan &dp, const float *x, float *y, cudaStream_t s);
-tc_status launch_spmm(const DevPlan &dp, const float *X, int ldx, int k, float *Y, int ldy,
-                      cudaStream_t s);
+// nnz_csr, max_row: the plan's CSR words and those of its longest row (they
+// pick the kernel).
+tc_status launch_spmm(const DevPlan &dp, int64_t nnz_csr, int max_row, const float *X, int ldx, int k, float *Y,
+                      int ldy, cudaStream_t s);
+// Multiprocessors of the current device (read once).
+int num_sms();
 
 // GPU partitioner: device CSR in, format (host vectors) out.
 struct PartitionOut {

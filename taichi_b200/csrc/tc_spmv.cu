@@ -448,108 +448,9 @@ __global__ void __launch_bounds__(kBlock, MANY ? kStreamManyMinBlocks
     tile_stream<SIGNED>(p, t, x, y, true);
 }
 
-// SpMM: a warp owns kRPW consecutive rows at a time; lane l holds columns
-// [l*V, l*V+V) of the k right-hand sides, so every X / Y row access is one
-// coalesced warp transaction.  The entries of the kRPW rows are walked in
-// rounds (one entry per row per round) so their X-row loads overlap.
-constexpr int kRPW = 4;
+}  // namespace
 
-template <int V>
-__device__ __forceinline__ void axpy_row(float (&acc)[V], const float *__restrict__ X, long off,
-                                         int c0, int k, float sg)
-{
-    const float *xr = X + off + c0;
-    if (V == 2 && c0 + 1 < k && ((reinterpret_cast<uintptr_t>(xr) & 7) == 0)) {
-        const float2 v = __ldg(reinterpret_cast<const float2 *>(xr));
-        acc[0] += sg * v.x;
-        acc[V - 1] += sg * v.y;
-    } else {
-#pragma unroll
-        for (int v = 0; v < V; ++v)
-            if (c0 + v < k) acc[v] += sg * __ldg(xr + v);
-    }
-}
-
-template <bool SIGNED, int V>
-__global__ void __launch_bounds__(kBlock) spmm_rows_kernel(DevPlan p, const float *__restrict__ X,
-                                                           int ldx, int k, float *__restrict__ Y,
-                                                           int ldy)
-{
-    const int lane = threadIdx.x & 31;
-    const int warp = (blockIdx.x * kBlock + threadIdx.x) >> 5;
-    const int nwarps = (gridDim.x * kBlock) >> 5;
-    const int c0 = lane * V;
-    const bool active = c0 < k;
-    for (long r0l = (long)warp * kRPW; r0l < p.M; r0l += (long)nwarps * kRPW) {
-        const int r0 = (int)r0l;
-        // row pointers of the kRPW rows: lanes 0..nrow hold rowptr[r0 + lane]
-        const int nrow = min(kRPW, p.M - r0);
-        const int rpv = lane <= nrow ? __ldg(p.rowptr + r0 + lane) : 0;
-        int rb[kRPW], re[kRPW];
-#pragma unroll
-        for (int q = 0; q < kRPW; ++q) {
-            rb[q] = __shfl_sync(0xffffffffu, rpv, q);
-            const int e = __shfl_sync(0xffffffffu, rpv, q + 1);
-            re[q] = q < nrow ? e : rb[q];
-        }
-        float acc[kRPW][V];
-#pragma unroll
-        for (int q = 0; q < kRPW; ++q)
-#pragma unroll
-            for (int v = 0; v < V; ++v) acc[q][v] = 0.f;
-        for (int t = 0;; ++t) {
-            bool any = false;
-            int cv[kRPW];
-#pragma unroll
-            for (int q = 0; q < kRPW; ++q) {
-                const int j = rb[q] + t;
-                cv[q] = j < re[q] ? __ldg(p.cols + j) : -1;
-                any |= cv[q] >= 0;
-            }
-            if (!any) break;            // uniform: every lane sees the same rows
-#pragma unroll
-            for (int q = 0; q < kRPW; ++q) {
-                if (cv[q] < 0 || !active) continue;
-                const int col = SIGNED ? (cv[q] >> 1) : cv[q];
-                const float sg = (!SIGNED || (cv[q] & 1)) ? 1.f : -1.f;
-                axpy_row<V>(acc[q], X, (long)col * ldx, c0, k, sg);
-            }
-        }
-        if (p.dia_shapes > 0) {
-#pragma unroll
-            for (int q = 0; q < kRPW; ++q) {
-                const int r = r0 + q;
-                if (q >= nrow || r < p.row_start || r >= p.row_stop || !active) continue;
-                for (int s = 0; s < p.dia_shapes; ++s) {
-                    const int4 sh = __ldg(p.shapes + s);
-                    if (r < sh.x || r >= sh.y) continue;
-                    const int2 dr = __ldg(p.shape_dias + s);
-                    for (int n = dr.x; n < dr.y; ++n) {
-                        const int col = r - sh.x + sh.z + __ldg(p.offsets + n);
-                        if (col >= sh.z && col < sh.z + sh.w)
-                            axpy_row<V>(acc[q], X, (long)col * ldx, c0, k, 1.f);
-                    }
-                }
-            }
-        }
-        if (active) {
-#pragma unroll
-            for (int q = 0; q < kRPW; ++q) {
-                if (q >= nrow) continue;
-                float *yr = Y + (long)(r0 + q) * ldy + c0;
-                if (V == 2 && c0 + 1 < k && ((reinterpret_cast<uintptr_t>(yr) & 7) == 0)) {
-                    *reinterpret_cast<float2 *>(yr) = make_float2(acc[q][0], acc[q][V - 1]);
-                } else {
-#pragma unroll
-                    for (int v = 0; v < V; ++v)
-                        if (c0 + v < k) yr[v] = acc[q][v];
-                }
-            }
-        }
-    }
-}
-
-int g_num_sms = 0;
+static int g_num_sms = 0;
 
 int num_sms()
 {
@@ -561,8 +462,6 @@ int num_sms()
     }
     return g_num_sms;
 }
-
-}  // namespace
 
 size_t stream_smem_bytes(const DevPlan &dp)
 {
@@ -640,23 +539,6 @@ tc_status launch_plan(const tc_plan *p, const float *x, float *y, cudaStream_t s
         return launch_spmv(p->dev_plan(), x, y, s, nullptr, &ws);
     }
     return launch_spmv(p->dev_plan(), x, y, s, nullptr, nullptr);
-}
-
-tc_status launch_spmm(const DevPlan &dp, const float *X, int ldx, int k, float *Y, int ldy,
-                      cudaStream_t s)
-{
-    if (dp.M == 0) return TC_OK;
-    const long warps = (dp.M + kRPW - 1) / kRPW;
-    const int grid = (int)std::min<long>((warps + kBlock / 32 - 1) / (kBlock / 32), num_sms() * 16L);
-    if (k <= 32) {
-        if (dp.hybrid) spmm_rows_kernel<true, 1><<<grid, kBlock, 0, s>>>(dp, X, ldx, k, Y, ldy);
-        else spmm_rows_kernel<false, 1><<<grid, kBlock, 0, s>>>(dp, X, ldx, k, Y, ldy);
-    } else {
-        if (dp.hybrid) spmm_rows_kernel<true, 2><<<grid, kBlock, 0, s>>>(dp, X, ldx, k, Y, ldy);
-        else spmm_rows_kernel<false, 2><<<grid, kBlock, 0, s>>>(dp, X, ldx, k, Y, ldy);
-    }
-    TC_CUDA(cudaGetLastError());
-    return TC_OK;
 }
 
 }  // namespace tc
@@ -787,6 +669,8 @@ tc_status plan_upload(tc_plan *p, const int *csrRow, const int *csrCol, cudaStre
     }
     p->ntiles = (int)tiles.size();
     p->nnz_csr = csrRow[M];
+    p->max_row = 0;
+    for (int i = 0; i < M; ++i) p->max_row = std::max(p->max_row, csrRow[i + 1] - csrRow[i]);
     p->wide_rows = p->ntiles_wide ? tile_nrows(tiles[0]) : kDirectWideRows;
     {   // the most common length of the rows stream tiles hold: skewed slots
         // when it is a multiple of 8 (see vslot), sampled rows
