@@ -98,24 +98,30 @@ using tc::check_params;
 
 extern "C" {
 
-// Validates a host format and builds a plan from it.
-tc_status tc_plan_from_format(int M, int N, const tc_format *f, const tc_params *params,
-                              void *stream, tc_plan **out)
+}  // extern "C"
+
+// A plan with the format's scalars and shape arrays (host arrays, checked
+// against M x N); the CSR remainder is still to be uploaded.
+static tc_status plan_of_shapes(int M, int N, const tc_format *f, const tc_params &prm, tc_plan **out)
 {
-    if (!f || !out || M < 0 || N < 0) return fail(TC_ERR_INVALID, "tc_plan_from_format: bad arguments");
-    *out = nullptr;
-    tc_params prm;
-    tc_params_default(&prm);
-    if (params) prm = *params;
-    TC_CHECK(check_params(prm));
     if (f->dia_shapes < 0 || f->num_negs < 0) return fail(TC_ERR_FORMAT, "negative counts");
     if (f->dia_shapes > 0 && (!f->xStart || !f->yStart || !f->xStop || !f->nDiasPtr || !f->neg_offsets))
         return fail(TC_ERR_FORMAT, "shape arrays missing");
-    if (M > 0 && !f->csrRow && !(f->dia_shapes > 0 && f->zero_elements + f->sparse_nnz == 0))
-        return fail(TC_ERR_FORMAT, "csrRow missing");
     const bool hybrid = f->dia_shapes > 0;
     if (hybrid && N >= (1 << 30)) return fail(TC_ERR_UNSUPPORTED, "N >= 2^30 with signed columns");
-
+    if (hybrid) {
+        for (int s = 0; s < f->dia_shapes; ++s) {
+            int xs = f->xStart[s], xe = f->xStop[s], ys = f->yStart[s];
+            if (xs < 0 || xe > M || xs >= xe || ys < 0 || ys + (xe - xs) > N)
+                return fail(TC_ERR_FORMAT, "shape %d box [%d,%d) x [%d,+%d) outside %d x %d", s, xs,
+                            xe, ys, xe - xs, M, N);
+        }
+        if (f->nDiasPtr[0] != 0 || f->nDiasPtr[f->dia_shapes] != f->num_negs)
+            return fail(TC_ERR_FORMAT, "nDiasPtr does not span neg_offsets");
+        for (int s = 0; s < f->dia_shapes; ++s)
+            if (f->nDiasPtr[s + 1] < f->nDiasPtr[s])
+                return fail(TC_ERR_FORMAT, "nDiasPtr decreases at shape %d", s);
+    }
     tc_plan *p = new (std::nothrow) tc_plan();
     if (!p) return fail(TC_ERR_ALLOC, "host allocation");
     p->M = M; p->N = N; p->params = prm;
@@ -129,43 +135,40 @@ tc_status tc_plan_from_format(int M, int N, const tc_format *f, const tc_params 
         p->h_xStop.assign(f->xStop, f->xStop + f->dia_shapes);
         p->h_nDiasPtr.assign(f->nDiasPtr, f->nDiasPtr + f->dia_shapes + 1);
         p->h_offsets.assign(f->neg_offsets, f->neg_offsets + f->num_negs);
-        for (int s = 0; s < f->dia_shapes; ++s) {
-            int xs = f->xStart[s], xe = f->xStop[s], ys = f->yStart[s];
-            if (xs < 0 || xe > M || xs >= xe || ys < 0 || ys + (xe - xs) > N) {
-                delete p;
-                return fail(TC_ERR_FORMAT, "shape %d box [%d,%d) x [%d,+%d) outside %d x %d", s, xs,
-                            xe, ys, xe - xs, M, N);
-            }
-        }
-        if (f->nDiasPtr[0] != 0 || f->nDiasPtr[f->dia_shapes] != f->num_negs) {
-            delete p;
-            return fail(TC_ERR_FORMAT, "nDiasPtr does not span neg_offsets");
-        }
-        for (int s = 0; s < f->dia_shapes; ++s)
-            if (f->nDiasPtr[s + 1] < f->nDiasPtr[s]) {
-                delete p;
-                return fail(TC_ERR_FORMAT, "nDiasPtr decreases at shape %d", s);
-            }
     }
+    *out = p;
+    return TC_OK;
+}
+
+extern "C" {
+
+// Validates a host format and builds a plan from it.
+tc_status tc_plan_from_format(int M, int N, const tc_format *f, const tc_params *params,
+                              void *stream, tc_plan **out)
+{
+    if (!f || !out || M < 0 || N < 0) return fail(TC_ERR_INVALID, "tc_plan_from_format: bad arguments");
+    *out = nullptr;
+    tc_params prm;
+    tc_params_default(&prm);
+    if (params) prm = *params;
+    TC_CHECK(check_params(prm));
+    if (M > 0 && !f->csrRow && !(f->dia_shapes > 0 && f->zero_elements + f->sparse_nnz == 0))
+        return fail(TC_ERR_FORMAT, "csrRow missing");
     std::vector<int> zero_rp;
     const int *rp = f->csrRow;
     if (!rp) { zero_rp.assign((size_t)M + 1, 0); rp = zero_rp.data(); }
     const int64_t nnz_csr = M > 0 ? rp[M] : 0;
     for (int r = 0; r < M; ++r)
-        if (rp[r + 1] < rp[r]) { delete p; return fail(TC_ERR_FORMAT, "csrRow decreases at row %d", r); }
-    if (rp[0] != 0) { delete p; return fail(TC_ERR_FORMAT, "csrRow[0] != 0"); }
-    const int lim = hybrid ? 2 * N : N;
+        if (rp[r + 1] < rp[r]) return fail(TC_ERR_FORMAT, "csrRow decreases at row %d", r);
+    if (rp[0] != 0) return fail(TC_ERR_FORMAT, "csrRow[0] != 0");
+    const int64_t lim = f->dia_shapes > 0 ? 2LL * N : N;
     for (int64_t j = 0; j < nnz_csr; ++j)
-        if (f->csrCol[j] < 0 || f->csrCol[j] >= lim) {
-            delete p;
+        if (f->csrCol[j] < 0 || f->csrCol[j] >= lim)
             return fail(TC_ERR_FORMAT, "csrCol[%lld] = %d outside the matrix", (long long)j, f->csrCol[j]);
-        }
+    tc_plan *p = nullptr;
+    TC_CHECK(plan_of_shapes(M, N, f, prm, &p));
     p->nnz_input = (int64_t)f->dense_nnz + f->sparse_nnz;
-    if (prm.flags & TC_FLAG_KEEP_HOST) {
-        p->h_rowptr.assign(rp, rp + M + 1);
-        p->h_cols.assign(f->csrCol, f->csrCol + nnz_csr);
-    }
-    tc_status st = tc::plan_upload(p, rp, f->csrCol, (cudaStream_t)stream);
+    tc_status st = tc::plan_upload(p, rp, f->csrCol, nnz_csr, false, (cudaStream_t)stream);
     if (st != TC_OK) { tc_plan_destroy(p); return st; }
     *out = p;
     return TC_OK;
@@ -175,6 +178,7 @@ tc_status tc_plan_destroy(tc_plan *p)
 {
     if (!p) return TC_OK;
     if (p->dev) cudaFree(p->dev);
+    if (p->dev_tiles) cudaFree(p->dev_tiles);
     for (int k = 0; k < TC_HOST_SLOTS; ++k) {
         if (p->d_xbuf[k]) cudaFree(p->d_xbuf[k]);
         if (p->d_ybuf[k]) cudaFree(p->d_ybuf[k]);
@@ -316,6 +320,30 @@ tc_status tc_spmm(const tc_plan *p, const float *d_X, int ldx, int k, float *d_Y
     return tc::launch_spmm(p->dev_plan(), p->nnz_csr, p->max_row, d_X, ldx, k, d_Y, ldy, (cudaStream_t)stream);
 }
 
+}  // extern "C"
+
+namespace {
+
+// A device array freed at the end of the call.
+struct DeviceArray {
+    void *p = nullptr;
+    ~DeviceArray() { if (p) cudaFree(p); }
+    tc_status copy_in(const void *host, size_t bytes, cudaStream_t s)
+    {
+        if (cudaMalloc(&p, std::max<size_t>(bytes, 16)) != cudaSuccess) {
+            (void)cudaGetLastError();
+            p = nullptr;
+            return fail(TC_ERR_ALLOC, "device copy of the input (%zu bytes)", bytes);
+        }
+        if (bytes) TC_CUDA(cudaMemcpyAsync(p, host, bytes, cudaMemcpyHostToDevice, s));
+        return TC_OK;
+    }
+};
+
+}  // namespace
+
+extern "C" {
+
 // Builds a plan from a CSR pattern, partitioning it on the GPU unless
 // TC_FLAG_NO_PARTITION is set.
 tc_status tc_plan_create(int M, int N, int64_t nnz, const int *rowptr, const int *col,
@@ -332,70 +360,54 @@ tc_status tc_plan_create(int M, int N, int64_t nnz, const int *rowptr, const int
     TC_CHECK(check_params(prm));
     cudaStream_t s = (cudaStream_t)stream;
 
-    // host copies of the CSR (the planner needs row pointers on the host)
-    std::vector<int> h_rp((size_t)M + 1), h_col;
-    if (on_device) {
-        TC_CUDA(cudaMemcpyAsync(h_rp.data(), rowptr, sizeof(int) * ((size_t)M + 1), cudaMemcpyDeviceToHost, s));
+    // before any kernel reads nnz columns
+    int ends[2] = {0, (int)nnz};
+    if (!on_device && rowptr) {
+        ends[0] = rowptr[0];
+        ends[1] = rowptr[M];
+    } else if (on_device) {
+        TC_CUDA(cudaMemcpyAsync(ends, rowptr, sizeof(int), cudaMemcpyDeviceToHost, s));
+        TC_CUDA(cudaMemcpyAsync(ends + 1, rowptr + M, sizeof(int), cudaMemcpyDeviceToHost, s));
         TC_CUDA(cudaStreamSynchronize(s));
-    } else {
-        memcpy(h_rp.data(), rowptr, sizeof(int) * ((size_t)M + 1));
     }
-    if (h_rp[0] != 0 || h_rp[M] != nnz) return fail(TC_ERR_FORMAT, "rowptr[0] != 0 or rowptr[M] != nnz");
+    if (ends[0] != 0 || ends[1] != nnz) return fail(TC_ERR_FORMAT, "rowptr[0] != 0 or rowptr[M] != nnz");
 
     if (prm.flags & TC_FLAG_NO_PARTITION) {
-        if (on_device) {
-            h_col.resize((size_t)nnz);
-            if (nnz) TC_CUDA(cudaMemcpy(h_col.data(), col, sizeof(int) * (size_t)nnz, cudaMemcpyDeviceToHost));
-        }
+        std::vector<int> h_rp, h_col;
         tc_format f{};
         f.sparse_nnz = (int)nnz;
-        f.csrRow = h_rp.data();
-        f.csrCol = on_device ? h_col.data() : col;
+        f.csrRow = rowptr;
+        f.csrCol = col;
+        if (on_device) {      // the format's checks run on the host
+            h_rp.resize((size_t)M + 1);
+            h_col.resize((size_t)nnz);
+            TC_CUDA(cudaMemcpyAsync(h_rp.data(), rowptr, sizeof(int) * h_rp.size(), cudaMemcpyDeviceToHost, s));
+            if (nnz) TC_CUDA(cudaMemcpyAsync(h_col.data(), col, sizeof(int) * h_col.size(), cudaMemcpyDeviceToHost, s));
+            TC_CUDA(cudaStreamSynchronize(s));
+            f.csrRow = h_rp.data();
+            f.csrCol = h_col.data();
+        }
         return tc_plan_from_format(M, N, &f, &prm, stream, out);
     }
 
-    // GPU partition from a device copy of the input
-    int *d_rp = nullptr, *d_col = nullptr;
-    float *d_val = nullptr;
-    bool own = !on_device;
-    if (own) {
-        if (cudaMalloc(&d_rp, sizeof(int) * ((size_t)M + 1)) != cudaSuccess ||
-            cudaMalloc(&d_col, sizeof(int) * (size_t)std::max<int64_t>(nnz, 1)) != cudaSuccess)
-            return fail(TC_ERR_ALLOC, "device copy of the input CSR");
-        TC_CUDA(cudaMemcpyAsync(d_rp, rowptr, sizeof(int) * ((size_t)M + 1), cudaMemcpyHostToDevice, s));
-        if (nnz) TC_CUDA(cudaMemcpyAsync(d_col, col, sizeof(int) * (size_t)nnz, cudaMemcpyHostToDevice, s));
-        if (val) {
-            if (cudaMalloc(&d_val, sizeof(float) * (size_t)std::max<int64_t>(nnz, 1)) != cudaSuccess)
-                return fail(TC_ERR_ALLOC, "device copy of the input values");
-            if (nnz) TC_CUDA(cudaMemcpyAsync(d_val, val, sizeof(float) * (size_t)nnz, cudaMemcpyHostToDevice, s));
-        }
-    } else {
-        d_rp = const_cast<int *>(rowptr);
-        d_col = const_cast<int *>(col);
-        d_val = const_cast<float *>(val);
+    // GPU partition from a device copy of the input; the plan is built from
+    // its device arrays (the input's own when nothing was extracted)
+    DeviceArray own_rp, own_col, own_val, out_rp, out_col;
+    const int *d_rp = rowptr, *d_col = col;
+    const float *d_val = val;
+    if (!on_device) {
+        TC_CHECK(own_rp.copy_in(rowptr, sizeof(int) * ((size_t)M + 1), s));
+        TC_CHECK(own_col.copy_in(col, sizeof(int) * (size_t)nnz, s));
+        if (val) TC_CHECK(own_val.copy_in(val, sizeof(float) * (size_t)nnz, s));
+        d_rp = static_cast<int *>(own_rp.p);
+        d_col = static_cast<int *>(own_col.p);
+        d_val = static_cast<float *>(own_val.p);
     }
     tc::PartitionOut po;
-    tc_status st = tc::gpu_partition(M, N, nnz, d_rp, d_col, d_val, prm,
-                                     (prm.flags & TC_FLAG_KEEP_HOST) != 0, false, s, po);
-    std::vector<int> fr, fc;
-    if (st == TC_OK) {
-        if (po.aliases_input) {
-            fr = h_rp;
-            if (on_device) {
-                fc.resize((size_t)nnz);
-                if (nnz) st = cudaMemcpy(fc.data(), col, sizeof(int) * (size_t)nnz, cudaMemcpyDeviceToHost) == cudaSuccess ? TC_OK : fail(TC_ERR_CUDA, "copy of the input columns");
-            }
-        } else {
-            fr.resize((size_t)M + 1);
-            fc.resize((size_t)po.nnz_csr);
-            if (cudaMemcpy(fr.data(), po.d_rowptr, sizeof(int) * ((size_t)M + 1), cudaMemcpyDeviceToHost) != cudaSuccess ||
-                (po.nnz_csr && cudaMemcpy(fc.data(), po.d_cols, sizeof(int) * (size_t)po.nnz_csr, cudaMemcpyDeviceToHost) != cudaSuccess))
-                st = fail(TC_ERR_CUDA, "copy of the partitioned CSR");
-        }
-    }
-    if (po.d_rowptr) cudaFree(po.d_rowptr);
-    if (po.d_cols) cudaFree(po.d_cols);
-    if (own) { cudaFree(d_rp); cudaFree(d_col); if (d_val) cudaFree(d_val); }
+    const tc_status st = tc::gpu_partition(M, N, nnz, d_rp, d_col, d_val, prm,
+                                           (prm.flags & TC_FLAG_KEEP_HOST) != 0, false, s, po);
+    out_rp.p = po.d_rowptr;
+    out_col.p = po.d_cols;
     if (st != TC_OK) return st;
 
     tc_format f{};
@@ -404,10 +416,11 @@ tc_status tc_plan_create(int M, int N, int64_t nnz, const int *rowptr, const int
     f.row_start = po.row_start; f.row_stop = po.row_stop;
     f.xStart = po.xStart.data(); f.yStart = po.yStart.data(); f.xStop = po.xStop.data();
     f.nDiasPtr = po.nDiasPtr.data(); f.neg_offsets = po.offsets.data();
-    f.csrRow = fr.data();
-    f.csrCol = po.aliases_input && !on_device ? col : fc.data();
     tc_plan *p = nullptr;
-    TC_CHECK(tc_plan_from_format(M, N, &f, &prm, stream, &p));
+    TC_CHECK(plan_of_shapes(M, N, &f, prm, &p));
+    const tc_status up = po.aliases_input ? tc::plan_upload(p, d_rp, d_col, nnz, true, s)
+                                          : tc::plan_upload(p, po.d_rowptr, po.d_cols, po.nnz_csr, true, s);
+    if (up != TC_OK) { tc_plan_destroy(p); return up; }
     p->nnz_input = nnz;
     p->partition_ms = po.ms;
     p->thumb_W = po.thumb_W;

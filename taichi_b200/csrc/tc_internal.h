@@ -177,8 +177,8 @@ struct tc_plan {
     int64_t nnz_input = 0, nnz_csr = 0;
     int max_row = 0;                     // CSR words of the longest row
     int hybrid = 0;
-    // device arrays (one allocation, `dev`)
-    void *dev = nullptr;
+    // device arrays: the format (`dev`) and the tiles (`dev_tiles`)
+    void *dev = nullptr, *dev_tiles = nullptr;
     size_t dev_bytes = 0;
     int *d_rowptr = nullptr, *d_cols = nullptr, *d_offsets = nullptr;
     tc::Tile *d_tiles = nullptr;
@@ -218,15 +218,13 @@ struct tc_plan {
 };
 
 namespace tc {
-// Builds the tiles + device format from host arrays of an already formatted
-// matrix (csrRow has M+1 entries).  Shared by every plan constructor.
-tc_status plan_upload(tc_plan *p, const int *csrRow, const int *csrCol,
+// Builds the device format and the tile list of an already formatted matrix
+// (csrRow has M+1 entries, csrCol nnz_csr words; host or device arrays).
+// Shared by every plan constructor.
+tc_status plan_upload(tc_plan *p, const int *csrRow, const int *csrCol, int64_t nnz_csr, bool on_device,
                       cudaStream_t stream);
-// Host tile planner (row-length histogram -> tile kinds).
-// Stream tiles hold at most nnz_csr / min_tiles entries (not below 512), so
-// a small matrix still spreads over the GPU.
-void plan_tiles(const int *rowptr, int M, const tc_params &prm, int min_tiles,
-                std::vector<Tile> &tiles, int *nvec, int *nlong);
+// CTAs of the persistent tile kernel's grid (tile_mode 0 / 1).
+tc_status tiles_grid(const DevPlan &dp, int ctas_per_sm, int *grid);
 // Rows of a wide direct tile: the multiple of 4 that makes two equal tiles
 // per SM (between kDirectRows and kDirectWideRows), so no SM holds twice the
 // rows of another

@@ -1,0 +1,497 @@
+// tc_plan.cu -- from a formatted matrix to a resident plan: the device
+// format, the tile list and what the launches need to know about the rows.
+//
+// Replaces the upload part of taichi_SpMV (TaiChi.cu:1357-1385).  The format
+// comes from host arrays or, after a partition, from device arrays; either
+// way the row statistics and the tile list are computed on the GPU from the
+// plan's own copy of the row pointers, so a partitioned matrix never crosses
+// the host link.  What bounds a build is then the copies of the format (read
+// and written once) and a few round trips of counts to the host.  Measured on
+// the 9-point mesh 2048^2 (25.7 M words): 1 ms from device arrays in place of
+// 85 ms for the copy to the host, the host's passes over the words and rows,
+// and the copy back.
+
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstring>
+
+#include "tc_internal.h"
+#include "tc_scan.cuh"
+
+namespace tc {
+
+int wide_tile_rows(int M, const tc_params &prm, int sms)
+{
+    if ((prm.flags & TC_FLAG_WIDE_FIXED) || sms <= 0) return kDirectWideRows;
+    // two tiles per SM: every SM holds two CTAs of the same size
+    const long per = ((long)M + 2L * sms - 1) / (2L * sms);
+    return (int)std::min<long>(kDirectWideRows, std::max<long>(kDirectRows, (per + 3) & ~3L));
+}
+
+namespace {
+
+// Rows are planned in strips of kStripRows, one warp each; a tile never
+// crosses a strip.  (A strip holds whole multiples of every kind's largest
+// tile, so short rows lose no tile to the cut.)
+constexpr int kStripRows = 2048;
+
+struct RowStats {
+    int max_row;                     // CSR words of the longest row
+    int minus;                       // a word without the addition bit exists
+    int hist[kStreamRowMax + 1];     // sampled rows by length
+};
+
+__global__ void row_stats(const int *__restrict__ rowptr, int M, int step, RowStats *__restrict__ st)
+{
+    __shared__ int hist[kStreamRowMax + 1];
+    for (int i = threadIdx.x; i <= kStreamRowMax; i += blockDim.x) hist[i] = 0;
+    __syncthreads();
+    int most = 0;
+    for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < M; r += (long)gridDim.x * blockDim.x) {
+        const int n = __ldg(rowptr + r + 1) - __ldg(rowptr + r);
+        most = max(most, n);
+        if (n <= kStreamRowMax && r % step == 0) atomicAdd(hist + n, 1);
+    }
+    most = __reduce_max_sync(0xffffffffu, most);
+    if ((threadIdx.x & 31) == 0) atomicMax(&st->max_row, most);
+    __syncthreads();
+    for (int i = threadIdx.x; i <= kStreamRowMax; i += blockDim.x)
+        if (hist[i]) atomicAdd(st->hist + i, hist[i]);
+}
+
+__global__ void word_signs(const int *__restrict__ cols, long nnz, RowStats *__restrict__ st)
+{
+    int all = 1;
+    for (long j = (long)blockIdx.x * blockDim.x + threadIdx.x; j < nnz; j += (long)gridDim.x * blockDim.x)
+        all &= __ldg(cols + j);
+    if (!__all_sync(0xffffffffu, all & 1) && (threadIdx.x & 31) == 0) st->minus = 1;
+}
+
+// The planner's parameters (see tc_params).
+struct TilePrm {
+    int mode, rows_cap, tile_nnz, long_len, spread, max_lanes, strided, no_direct;
+};
+
+// What the tiles of a plan come to, summed over its strips.
+struct TileCounts {
+    int vector, lng, lanes, stream, max_rows, max_nnz;   // max_*: tiles staged in shared memory
+};
+
+// Lanes per row from the mean row length of a run of rows: one lane per row
+// until rows average more than 16 entries, then the smallest power of two
+// giving each lane about 8 entries, capped at max_lanes.  (The CSR words come
+// from shared memory, so a thread walking its own row costs no coalescing.)
+__device__ __forceinline__ int lanes_for(double mean, int max_lanes)
+{
+    if (mean <= 16.0) return 1;
+    int l = 1;
+    while (l < max_lanes && 8.0 * l < mean) l <<= 1;
+    return l;
+}
+
+// The number of leading i in [0, limit) for which ok(i) holds (a warp).
+template <class Ok>
+__device__ __forceinline__ int run_of(int limit, Ok ok)
+{
+    const int lane = threadIdx.x & 31;
+    for (int i = 0; i < limit; i += 32) {
+        const unsigned bad = __ballot_sync(0xffffffffu, !(i + lane < limit && ok(i + lane)));
+        if (bad) return i + __ffs(bad) - 1;
+    }
+    return limit;
+}
+
+// The tiles of one strip per warp (a CTA of 32 threads): counted, and with
+// WRITE written from tiles[first[strip]] on.
+template <bool WRITE>
+__global__ void __launch_bounds__(32) plan_strips(const int *__restrict__ rowptr, int M, TilePrm q,
+                                                  int *__restrict__ count, const int *__restrict__ first,
+                                                  Tile *__restrict__ tiles, TileCounts *__restrict__ sum)
+{
+    __shared__ int rp[kStripRows + 1];
+    const long row0 = (long)blockIdx.x * kStripRows;
+    const int n = (int)min((long)kStripRows, (long)M - row0), lane = threadIdx.x;
+    for (int i = lane; i <= n; i += 32) rp[i] = __ldg(rowptr + row0 + i);
+    __syncwarp();
+    TileCounts c{0, 0, 0, 0, 1, 0};
+    int made = 0;
+    Tile *const out = WRITE ? tiles + first[blockIdx.x] : nullptr;
+    auto len = [&](int r) { return rp[r + 1] - rp[r]; };
+    auto put = [&](int r, int rows, int kind) {
+        const int nz = rp[r + rows] - rp[r];
+        if (WRITE && lane == 0) out[made] = Tile{(int)(row0 + r), rp[r], nz, tile_word(rows, kind)};
+        ++made;
+        c.stream += kind == TILE_STREAM;
+        c.lng += kind == TILE_LONG;
+        if (kind <= TILE_L32 || kind == TILE_MERGE) {
+            ++c.lanes;
+            c.max_rows = max(c.max_rows, rows);
+            c.max_nnz = max(c.max_nnz, nz);
+        }
+    };
+    for (int r = 0; r < n;) {
+        if (len(r) > q.long_len) {
+            put(r, 1, TILE_LONG);
+            ++r;
+            continue;
+        }
+        if (q.mode == 2 && len(r) <= kStreamRowMax) {
+            // stream tile: short rows up to the row and entry caps.  A run
+            // that starts on a multiple of 4 rows and holds many rows runs 4
+            // consecutive rows per thread: read directly from global memory
+            // when they average at most one entry (TILE_DIRECT4), through
+            // shared memory when at most two (TILE_STREAM4); otherwise one
+            // row per thread (TILE_STREAM)
+            const bool a4 = (r & 3) == 0 && !q.strided;
+            const int cap_rows = min(q.rows_cap, a4 ? kDirectRows : kStreamRows);
+            const int cap_nnz = max(1, min(2 * min(q.tile_nnz, 1 << 24), q.spread));
+            int m = run_of(min(cap_rows, n - r), [&](int i) {
+                return len(r + i) <= kStreamRowMax && rp[r + i + 1] - rp[r] <= cap_nnz;
+            });
+            if (m == 0) m = 1;        // a single row longer than cap_nnz but <= kStreamRowMax
+            const int ent = rp[r + m] - rp[r];
+            const bool direct = a4 && m >= 2 * kBlock && ent <= m && !q.no_direct;
+            const bool four = !direct && a4 && m >= 2 * kBlock && ent <= 2 * m;
+            if (!direct) m = min(m, four ? kStream4Rows : kStreamRows);
+            if (r + m < n) {          // end on a multiple of 256 rows (whole row sweeps), else of 4
+                const int cut = (r + m) & ~255;
+                if (cut - r >= 256) m = cut - r;
+                else if (m > 4) m -= (r + m) & 3;
+            }
+            put(r, m, direct ? TILE_DIRECT4 : four ? TILE_STREAM4 : TILE_STREAM);
+            r += m;
+            continue;
+        }
+        // candidate run: up to 1024 rows (merge tiles: tile_rows), stopping
+        // before a long row (stream mode: before a short row too)
+        const int run_cap = q.mode == 0 ? min(q.rows_cap, kStripRows) : 1024;
+        const int m = run_of(min(run_cap, n - r), [&](int i) {
+            return len(r + i) <= q.long_len && !(q.mode == 2 && len(r + i) <= kStreamRowMax);
+        });
+        if (q.mode == 0) {            // merge tile: rows + entries split evenly
+            int rows = m;
+            while (rows > 1 && rp[r + rows] - rp[r] > kStageNnz) rows = (rows + 1) / 2;
+            put(r, rows, TILE_MERGE);
+            r += rows;
+            continue;
+        }
+        int lanes = lanes_for((double)(rp[r + m] - rp[r]) / m, q.max_lanes);
+        int rows = min(min(m, kBlock / lanes * 4), q.rows_cap);
+        while (rows > 1 && rp[r + rows] - rp[r] > kStageNnz) rows = (rows + 1) / 2;   // fits a stage
+        lanes = lanes_for((double)(rp[r + rows] - rp[r]) / rows, q.max_lanes);
+        c.vector += lanes > 1;
+        put(r, rows, 31 - __clz(lanes));
+        r += rows;
+    }
+    if (WRITE || lane) return;
+    count[blockIdx.x] = made;
+    if (c.vector) atomicAdd(&sum->vector, c.vector);
+    if (c.lng) atomicAdd(&sum->lng, c.lng);
+    if (c.lanes) atomicAdd(&sum->lanes, c.lanes);
+    if (c.stream) atomicAdd(&sum->stream, c.stream);
+    atomicMax(&sum->max_rows, c.max_rows);
+    atomicMax(&sum->max_nnz, c.max_nnz);
+}
+
+// Wide direct tiles: `rows` rows each, in row order.
+__global__ void wide_tiles(const int *__restrict__ rowptr, int M, int rows, int ntiles, Tile *__restrict__ tiles)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= ntiles) return;
+    const int r = i * rows, n = min(rows, M - r), z = __ldg(rowptr + r);
+    tiles[i] = Tile{r, z, __ldg(rowptr + r + n) - z, tile_word(n, TILE_DIRECT_WIDE)};
+}
+
+// Sets each tile's diagonal class (see kDiagGeneral / kDiagNone), a warp per
+// tile: the multiply adds the dense-diagonal terms of a classed tile without
+// searching the shapes per row, with the same terms in the same order.
+__global__ void classify_tiles(Tile *__restrict__ tiles, int ntiles, const int4 *__restrict__ shapes,
+                               const int2 *__restrict__ shape_dias, const int *__restrict__ offsets,
+                               int dia_shapes, int row_start, int row_stop)
+{
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (i >= ntiles) return;
+    const int r0 = tiles[i].row0, r1 = r0 + tile_nrows(tiles[i]);
+    int dc = kDiagNone;
+    if (r1 > row_start && r0 < row_stop) {
+        int found = -1;
+        bool two = false;                            // two shapes share rows of the tile
+        for (int s = 0; s < dia_shapes && !two; ++s) {
+            const int4 sh = shapes[s];
+            if (r1 <= sh.x || r0 >= sh.y) continue;
+            two = found >= 0;
+            found = s;
+        }
+        if (two) dc = kDiagGeneral;
+        else if (found >= 0) {
+            const int4 sh = shapes[found];
+            const int2 dr = shape_dias[found];
+            bool in = r0 >= sh.x && r1 <= sh.y && r0 >= row_start && r1 <= row_stop && found + 1 < kDiagNone;
+            for (int d = dr.x + lane; d < dr.y; d += 32)
+                in = in && r0 - sh.x + offsets[d] >= 0 && r1 - 1 - sh.x + offsets[d] < sh.w;
+            dc = __all_sync(0xffffffffu, in) ? found + 1 : kDiagGeneral;
+        }
+    }
+    if (lane == 0) tiles[i].nrows_kind |= dc << kDiagShift;
+}
+
+struct Temp {
+    void *p = nullptr;
+    ~Temp() { if (p) cudaFree(p); }
+};
+
+size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
+
+unsigned blocks_for(long n, int threads)
+{
+    return (unsigned)std::max(1L, std::min((n + threads - 1) / threads, 16L * num_sms()));
+}
+
+}  // namespace
+
+tc_status plan_upload(tc_plan *p, const int *csrRow, const int *csrCol, int64_t nnz_csr, bool on_device,
+                      cudaStream_t stream)
+{
+    const int M = p->M;
+    const tc_params &prm = p->params;
+    p->nnz_csr = nnz_csr;
+    // shape table {xStart, xStop, yStart, Msub} and offset ranges
+    std::vector<int4> shapes(p->dia_shapes);
+    std::vector<int2> sd(p->dia_shapes);
+    p->max_span = 0;
+    for (int s = 0; s < p->dia_shapes; ++s) {
+        shapes[s] = make_int4(p->h_xStart[s], p->h_xStop[s], p->h_yStart[s],
+                              p->h_xStop[s] - p->h_xStart[s]);
+        sd[s] = make_int2(p->h_nDiasPtr[s], p->h_nDiasPtr[s + 1]);
+        if (sd[s].y <= sd[s].x) return fail(TC_ERR_FORMAT, "shape %d has no diagonals", s);
+        for (int n = sd[s].x + 1; n < sd[s].y; ++n)
+            if (p->h_offsets[n] <= p->h_offsets[n - 1])
+                return fail(TC_ERR_FORMAT, "offsets of shape %d are not increasing", s);
+        p->max_span = std::max(p->max_span, p->h_offsets[sd[s].y - 1] - p->h_offsets[sd[s].x]);
+    }
+
+    // window plan: a second tile list for the window kernel (the batch and
+    // served launches keep running `tiles`, with the same terms and order),
+    // planned on the host
+    std::vector<Tile> wtiles;
+    p->nwtiles = 0;
+    if (prm.flags & TC_FLAG_WINDOW) {
+        std::vector<int> hr, hc;
+        const int *wr = csrRow, *wc = csrCol;
+        if (on_device) {
+            hr.resize((size_t)M + 1);
+            hc.resize((size_t)nnz_csr);
+            TC_CUDA(cudaMemcpyAsync(hr.data(), csrRow, sizeof(int) * hr.size(), cudaMemcpyDeviceToHost, stream));
+            if (nnz_csr)
+                TC_CUDA(cudaMemcpyAsync(hc.data(), csrCol, sizeof(int) * hc.size(), cudaMemcpyDeviceToHost, stream));
+            TC_CUDA(cudaStreamSynchronize(stream));
+            wr = hr.data();
+            wc = hc.data();
+        }
+        int wlo = 0, whi = 0, wrows = 0, wnnz = 0;
+        if (plan_window(p, wr, wc, wtiles, &wlo, &whi, &wrows, &wnnz)) {
+            const int w_rp = (wrows + 8 + 3) & ~3, w_cw = (wnnz + 8 + 3) & ~3;
+            const int w_xw = (wrows + whi - wlo + 8 + 3) & ~3;
+            const size_t stage = 4 * (size_t)(w_rp + w_cw + w_xw);
+            const int S = (int)std::min<size_t>(kWinMaxStages, (kWinSmemBudget - 128) / stage);
+            if (S >= 2) {
+                p->nwtiles = (int)wtiles.size();
+                p->wlo = wlo;
+                p->whi = whi;
+                p->w_rp = w_rp;
+                p->w_cw = w_cw;
+                p->w_xw = w_xw;
+                p->w_stages = S;
+                p->w_grid = std::min(p->nwtiles, num_sms());
+            } else {
+                wtiles.clear();
+            }
+        }
+    }
+
+    // the format: row pointers and words, each followed by at least 16 zero
+    // bytes (the kernels' aligned loads run past the last element), the
+    // shapes, the error word, the window tiles
+    const size_t rp_end = sizeof(int) * ((size_t)M + 1);
+    const size_t o_cols = align256(rp_end + 16), cols_end = o_cols + sizeof(int) * (size_t)nnz_csr;
+    const size_t o_sh = align256(cols_end + 16);
+    const size_t o_sd = align256(o_sh + sizeof(int4) * shapes.size());
+    const size_t o_off = align256(o_sd + sizeof(int2) * sd.size());
+    const size_t o_err = align256(o_off + sizeof(int) * (size_t)p->num_negs + 16);
+    const size_t o_wt = align256(o_err + 16);
+    const size_t total = align256(o_wt + sizeof(Tile) * wtiles.size());
+    char *base = nullptr;
+    cudaError_t e = cudaMalloc(&base, total);
+    if (e != cudaSuccess)
+        return fail(TC_ERR_ALLOC, "cudaMalloc(%zu) for the plan: %s", total, cudaGetErrorString(e));
+    p->dev = base;
+    p->dev_bytes = total;
+    p->d_rowptr = reinterpret_cast<int *>(base);
+    p->d_cols = reinterpret_cast<int *>(base + o_cols);
+    p->d_shapes = reinterpret_cast<int4 *>(base + o_sh);
+    p->d_shape_dias = reinterpret_cast<int2 *>(base + o_sd);
+    p->d_offsets = reinterpret_cast<int *>(base + o_off);
+    p->d_err = reinterpret_cast<int *>(base + o_err);
+    p->d_wtiles = p->nwtiles ? reinterpret_cast<Tile *>(base + o_wt) : nullptr;
+    const cudaMemcpyKind in = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+    TC_CUDA(cudaMemsetAsync(base + rp_end, 0, o_cols - rp_end, stream));
+    TC_CUDA(cudaMemsetAsync(base + cols_end, 0, o_sh - cols_end, stream));
+    TC_CUDA(cudaMemsetAsync(base + o_off, 0, o_wt - o_off, stream));
+    TC_CUDA(cudaMemcpyAsync(p->d_rowptr, csrRow, rp_end, in, stream));
+    if (nnz_csr) TC_CUDA(cudaMemcpyAsync(p->d_cols, csrCol, sizeof(int) * (size_t)nnz_csr, in, stream));
+    if (!shapes.empty()) {
+        TC_CUDA(cudaMemcpyAsync(p->d_shapes, shapes.data(), sizeof(int4) * shapes.size(),
+                                cudaMemcpyHostToDevice, stream));
+        TC_CUDA(cudaMemcpyAsync(p->d_shape_dias, sd.data(), sizeof(int2) * sd.size(),
+                                cudaMemcpyHostToDevice, stream));
+        TC_CUDA(cudaMemcpyAsync(p->d_offsets, p->h_offsets.data(), sizeof(int) * p->num_negs,
+                                cudaMemcpyHostToDevice, stream));
+    }
+    if (p->nwtiles)
+        TC_CUDA(cudaMemcpyAsync(p->d_wtiles, wtiles.data(), sizeof(Tile) * wtiles.size(),
+                                cudaMemcpyHostToDevice, stream));
+
+    // row statistics, and the tiles per strip unless the tiles are wide
+    const int strips = (int)(((long)M + kStripRows - 1) / kStripRows);
+    const size_t o_sum = align256(sizeof(RowStats)), o_cnt = align256(o_sum + sizeof(TileCounts));
+    const size_t o_first = align256(o_cnt + sizeof(int) * ((size_t)strips + 1));
+    const size_t o_tmp = align256(o_first + sizeof(int) * ((size_t)strips + 1));
+    Temp tmp;
+    e = cudaMalloc(&tmp.p, o_tmp + sizeof(int) * scan_tmp_ints(strips));
+    if (e != cudaSuccess) {
+        tmp.p = nullptr;
+        return fail(TC_ERR_ALLOC, "planner scratch: %s", cudaGetErrorString(e));
+    }
+    char *t = static_cast<char *>(tmp.p);
+    RowStats *d_st = reinterpret_cast<RowStats *>(t);
+    TileCounts *d_sum = reinterpret_cast<TileCounts *>(t + o_sum);
+    int *d_cnt = reinterpret_cast<int *>(t + o_cnt), *d_first = reinterpret_cast<int *>(t + o_first);
+    int *d_tmp = reinterpret_cast<int *>(t + o_tmp);
+    TC_CUDA(cudaMemsetAsync(t, 0, o_first, stream));
+    const int step = std::max(1, M / 65536);
+    if (M) row_stats<<<blocks_for(M, 256), 256, 0, stream>>>(p->d_rowptr, M, step, d_st);
+    if (p->hybrid && nnz_csr)
+        word_signs<<<blocks_for(nnz_csr, 256), 256, 0, stream>>>(p->d_cols, nnz_csr, d_st);
+    const int min_tiles = 4 * num_sms();
+    TilePrm q;
+    q.mode = prm.tile_mode;
+    q.rows_cap = std::max(1, std::min(prm.tile_rows, kMaxTileRows));
+    q.tile_nnz = prm.tile_nnz;
+    q.long_len = std::max(1, std::min(prm.tile_nnz, kStageNnz));
+    // stream tiles hold at most nnz_csr / min_tiles entries (not below 512),
+    // so a small matrix still spreads over the GPU
+    q.spread = (int)std::min<int64_t>(kStreamNnz, std::max<int64_t>(512, nnz_csr / std::max(1, min_tiles)));
+    q.max_lanes = prm.max_lanes;
+    q.strided = (prm.flags & TC_FLAG_ROWS_STRIDED) != 0;
+    q.no_direct = (prm.flags & TC_FLAG_NO_DIRECT) != 0;
+    if (M) {
+        plan_strips<false><<<strips, 32, 0, stream>>>(p->d_rowptr, M, q, d_cnt, nullptr, nullptr, d_sum);
+        TC_CUDA(cudaGetLastError());
+        TC_CHECK(exclusive_scan(d_cnt, d_first, strips, d_tmp, stream));
+    }
+    RowStats st{};
+    TileCounts sum{};
+    int made = 0;
+    TC_CUDA(cudaMemcpyAsync(&st, d_st, sizeof st, cudaMemcpyDeviceToHost, stream));
+    TC_CUDA(cudaMemcpyAsync(&sum, d_sum, sizeof sum, cudaMemcpyDeviceToHost, stream));
+    if (M) TC_CUDA(cudaMemcpyAsync(&made, d_first + strips, sizeof made, cudaMemcpyDeviceToHost, stream));
+    TC_CUDA(cudaStreamSynchronize(stream));   // host arrays may be freed after return
+    p->max_row = st.max_row;
+    p->all_pos = !st.minus;                   // a hybrid plan with no holes: every word adds its term
+    // rows of at most one entry on average and none long: the whole matrix as
+    // wide direct tiles (a 1024-thread CTA each)
+    const bool wide = prm.tile_mode == 2 && prm.tile_rows >= kDirectRows &&
+                      !(prm.flags & (TC_FLAG_NO_DIRECT | TC_FLAG_NO_WIDE | TC_FLAG_ROWS_STRIDED)) &&
+                      M >= kDirectWideRows && nnz_csr <= M && st.max_row <= kStreamRowMax;
+    p->wide_rows = wide ? wide_tile_rows(M, prm, num_sms()) : kDirectWideRows;
+    p->ntiles = wide ? (M + p->wide_rows - 1) / p->wide_rows : made;
+    p->ntiles_wide = wide ? p->ntiles : 0;
+    p->ntiles_vector = wide ? 0 : sum.vector;
+    p->ntiles_long = wide ? 0 : sum.lng;
+    p->ntiles_lanes = wide ? 0 : sum.lanes;
+    p->ntiles_stream = wide ? 0 : sum.stream;
+    // shared-memory stage sizes (ints, multiples of 4) from the largest tile
+    p->stage_rp = (std::max(1, wide ? 1 : sum.max_rows) + 1 + 8 + 3) & ~3;
+    p->stage_cw = ((wide ? 0 : sum.max_nnz) + 8 + 3) & ~3;
+    {   // the most common length of the rows stream tiles hold: skewed slots
+        // when it is a multiple of 8 (see vslot), sampled rows
+        const int *h = st.hist;
+        const int mode = (int)(std::max_element(h + 1, h + kStreamRowMax + 1) - h);
+        p->stream_skew = h[mode] > 0 && mode % 8 == 0;
+        // the rows kernel loads W words of a row together: the least of 4, 6, 8
+        // that holds 90 % of the rows whole
+        int64_t tot = 0, upto = 0;
+        for (int L = 0; L <= kStreamRowMax; ++L) tot += h[L];
+        p->rows_w = 8;
+        for (int L = 0, w = 4; L <= 8 && tot > 0; ++L) {
+            upto += h[L];
+            if (L == w) {
+                if (upto * 10 >= tot * 9) {
+                    p->rows_w = w;
+                    break;
+                }
+                w += 2;
+            }
+        }
+    }
+
+    e = cudaMalloc(&p->dev_tiles, align256(sizeof(Tile) * (size_t)std::max(p->ntiles, 1)));
+    if (e != cudaSuccess) {
+        p->dev_tiles = nullptr;
+        return fail(TC_ERR_ALLOC, "%d tiles: %s", p->ntiles, cudaGetErrorString(e));
+    }
+    p->dev_bytes += align256(sizeof(Tile) * (size_t)std::max(p->ntiles, 1));
+    p->d_tiles = static_cast<Tile *>(p->dev_tiles);
+    if (wide)
+        wide_tiles<<<(unsigned)((p->ntiles + 255) / 256), 256, 0, stream>>>(p->d_rowptr, M, p->wide_rows, p->ntiles,
+                                                                          p->d_tiles);
+    else if (M)
+        plan_strips<true><<<strips, 32, 0, stream>>>(p->d_rowptr, M, q, nullptr, d_first, p->d_tiles, nullptr);
+    for (int k = 0; k < 2; ++k) {
+        Tile *list = k ? p->d_wtiles : p->d_tiles;
+        const int n = k ? p->nwtiles : p->ntiles;
+        if (n) classify_tiles<<<(unsigned)((n + 7L) / 8), 256, 0, stream>>>(
+            list, n, p->d_shapes, p->d_shape_dias, p->d_offsets, p->dia_shapes, p->row_start, p->row_stop);
+    }
+    TC_CUDA(cudaGetLastError());
+    // wide plans of few tiles: each tile's first word travels in the launch
+    // parameters, for the word prefetch or the staged words
+    const bool bounds = wide && p->ntiles <= kWideBoundTiles && M % kDirectWideRows == 0 &&
+                        (prm.flags & TC_FLAG_WIDE_BOUNDS);
+    const bool starts = wide && p->ntiles <= kWideParamTiles &&
+                        !(prm.flags & (TC_FLAG_NO_PREFETCH | TC_FLAG_NO_PARAM_STARTS));
+    p->h_wide_nz.clear();
+    p->h_wide_z.clear();
+    if (bounds || starts) {
+        std::vector<Tile> ht(p->ntiles);
+        TC_CUDA(cudaMemcpyAsync(ht.data(), p->d_tiles, sizeof(Tile) * ht.size(), cudaMemcpyDeviceToHost, stream));
+        TC_CUDA(cudaStreamSynchronize(stream));
+        std::vector<int> nz;
+        for (const Tile &w : ht) nz.push_back(w.nz0);
+        nz.push_back((int)nnz_csr);
+        if (starts) p->h_wide_z = nz;
+        if (bounds) p->h_wide_nz = nz;
+    }
+    p->grid = 1;
+    if (prm.tile_mode != 2) {   // persistent grid: CTAs per SM from occupancy at this stage size
+        DevPlan dp = p->dev_plan();
+        TC_CHECK(tiles_grid(dp, prm.ctas_per_sm, &p->grid));
+    }
+    if (p->nwtiles) {
+        DevPlan dp = p->dev_plan();
+        TC_CHECK(window_prepare(dp));
+    }
+    if (prm.flags & TC_FLAG_KEEP_HOST) {
+        p->h_rowptr.resize((size_t)M + 1);
+        p->h_cols.resize((size_t)nnz_csr);
+        TC_CUDA(cudaMemcpyAsync(p->h_rowptr.data(), p->d_rowptr, rp_end, cudaMemcpyDeviceToHost, stream));
+        if (nnz_csr)
+            TC_CUDA(cudaMemcpyAsync(p->h_cols.data(), p->d_cols, sizeof(int) * (size_t)nnz_csr,
+                                    cudaMemcpyDeviceToHost, stream));
+    }
+    TC_CUDA(cudaStreamSynchronize(stream));
+    return TC_OK;
+}
+
+}  // namespace tc

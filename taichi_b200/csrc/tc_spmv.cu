@@ -1,10 +1,10 @@
-// tc_spmv.cu -- the multiply: tile planner, device format upload, and the
-// value-free hybrid SpMV / SpMM kernels for sm_100a.
+// tc_spmv.cu -- the multiply: the value-free hybrid SpMV kernels for sm_100a
+// and their launch.
 //
 // Replaces taichi_SpMV's dispatch and kernels (TaiChi.cu:965-1329).  The
 // reference launches one of four CSR-vector kernels with a single vector
 // width per matrix (TPV = sqrt of the mean row length) and a volatile
-// shared-memory reduction.  Here the host planner cuts the rows into tiles
+// shared-memory reduction.  Here the planner (tc_plan.cu) cuts the rows into tiles
 // and gives each tile its own lanes-per-row from that tile's row lengths (a
 // CTA per row above a length limit); the kernel walks the tile list, keeps
 // kRPT rows' loads in flight per lane group, adds the dense-diagonal terms in
@@ -22,119 +22,6 @@
 #include "tc_tma.cuh"
 
 namespace tc {
-
-// ------------------------------------------------------------------ planner
-// Lanes per row from the mean row length of a run of rows: one lane per row
-// until rows average more than 16 entries, then the smallest power of two
-// giving each lane about 8 entries, capped at max_lanes.  (The CSR words come
-// from shared memory, so a thread walking its own row costs no coalescing.)
-static int lanes_for(double mean, int max_lanes)
-{
-    if (mean <= 16.0) return 1;
-    int l = 1;
-    while (l < max_lanes && 8.0 * l < mean) l <<= 1;
-    return l;
-}
-
-static int kind_of(int lanes)
-{
-    int k = 0;
-    while ((1 << k) < lanes) ++k;
-    return k;
-}
-
-int wide_tile_rows(int M, const tc_params &prm, int sms)
-{
-    if ((prm.flags & TC_FLAG_WIDE_FIXED) || sms <= 0) return kDirectWideRows;
-    // two tiles per SM: every SM holds two CTAs of the same size
-    const long per = ((long)M + 2L * sms - 1) / (2L * sms);
-    return (int)std::min<long>(kDirectWideRows, std::max<long>(kDirectRows, (per + 3) & ~3L));
-}
-
-void plan_tiles(const int *rp, int M, const tc_params &prm, int min_tiles, std::vector<Tile> &tiles,
-                int *nvec, int *nlong)
-{
-    const int spread = (int)std::min<int64_t>(kStreamNnz, std::max<int64_t>(512, (int64_t)rp[M] / std::max(1, min_tiles)));
-    const int long_len = std::max(1, std::min(prm.tile_nnz, kStageNnz));
-    const int rows_cap = std::max(1, std::min(prm.tile_rows, kMaxTileRows));
-    tiles.clear();
-    *nvec = *nlong = 0;
-    if (prm.tile_mode == 2 && prm.tile_rows >= kDirectRows &&
-        !(prm.flags & (TC_FLAG_NO_DIRECT | TC_FLAG_NO_WIDE | TC_FLAG_ROWS_STRIDED)) && M >= kDirectWideRows &&
-        rp[M] <= M) {
-        // rows of at most one entry on average and none long: the whole
-        // matrix as wide direct tiles (one 1024-thread CTA per 4096 rows)
-        bool short_rows = true;
-        for (int i = 0; i < M && short_rows; ++i) short_rows = rp[i + 1] - rp[i] <= kStreamRowMax;
-        if (short_rows) {
-            const int R = wide_tile_rows(M, prm, min_tiles / 4);
-            for (int r = 0; r < M; r += R) {
-                const int n = std::min(R, M - r);
-                tiles.push_back(Tile{r, rp[r], rp[r + n] - rp[r], tile_word(n, TILE_DIRECT_WIDE)});
-            }
-            return;
-        }
-    }
-    int r = 0;
-    while (r < M) {
-        if (rp[r + 1] - rp[r] > long_len) {
-            tiles.push_back(Tile{r, rp[r], rp[r + 1] - rp[r], tile_word(1, TILE_LONG)});
-            ++*nlong;
-            ++r;
-            continue;
-        }
-        if (prm.tile_mode == 2 && rp[r + 1] - rp[r] <= kStreamRowMax) {
-            // stream tile: short rows up to the row and entry caps.  A run
-            // that starts on a multiple of 4 rows and holds many rows runs 4
-            // consecutive rows per thread: read directly from global memory
-            // when they average at most one entry (TILE_DIRECT4), through
-            // shared memory when at most two (TILE_STREAM4); otherwise one
-            // row per thread (TILE_STREAM)
-            const bool a4 = (r & 3) == 0 && !(prm.flags & TC_FLAG_ROWS_STRIDED);
-            const int cap_rows = std::min(rows_cap, a4 ? kDirectRows : kStreamRows);
-            const int cap_nnz = std::max(1, std::min(2 * prm.tile_nnz, spread));
-            int n = 0;
-            while (r + n < M && n < cap_rows && rp[r + n + 1] - rp[r + n] <= kStreamRowMax &&
-                   rp[r + n + 1] - rp[r] <= cap_nnz)
-                ++n;
-            if (n == 0) n = 1;        // a single row longer than cap_nnz but <= kStreamRowMax
-            const int ent = rp[r + n] - rp[r];
-            const bool direct = a4 && n >= 2 * kBlock && ent <= n && !(prm.flags & TC_FLAG_NO_DIRECT);
-            const bool four = !direct && a4 && n >= 2 * kBlock && ent <= 2 * n;
-            if (!direct) n = std::min(n, four ? kStream4Rows : kStreamRows);
-            if (r + n < M) {          // end on a multiple of 256 rows (whole row sweeps), else of 4
-                const int cut = (r + n) & ~255;
-                if (cut - r >= 256) n = cut - r;
-                else if (n > 4) n -= (r + n) & 3;
-            }
-            const int kind = direct ? TILE_DIRECT4 : four ? TILE_STREAM4 : TILE_STREAM;
-            tiles.push_back(Tile{r, rp[r], rp[r + n] - rp[r], tile_word(n, kind)});
-            r += n;
-            continue;
-        }
-        // candidate run: up to 1024 rows (merge tiles: tile_rows), stopping
-        // before a long row (stream mode: before a short row too)
-        const int run_cap = prm.tile_mode == 0 ? std::min(rows_cap, kMergeRows) : 1024;
-        int n = 0;
-        while (r + n < M && n < run_cap && rp[r + n + 1] - rp[r + n] <= long_len &&
-               !(prm.tile_mode == 2 && rp[r + n + 1] - rp[r + n] <= kStreamRowMax))
-            ++n;
-        if (prm.tile_mode == 0) {          // merge tile: rows + entries split evenly
-            int rows = n;
-            while (rows > 1 && rp[r + rows] - rp[r] > kStageNnz) rows = (rows + 1) / 2;
-            tiles.push_back(Tile{r, rp[r], rp[r + rows] - rp[r], tile_word(rows, TILE_MERGE)});
-            r += rows;
-            continue;
-        }
-        int lanes = lanes_for((double)(rp[r + n] - rp[r]) / n, prm.max_lanes);
-        int rows = std::min(std::min(n, tile_rows_for(lanes)), rows_cap);
-        while (rows > 1 && rp[r + rows] - rp[r] > kStageNnz) rows = (rows + 1) / 2;   // fits a stage
-        lanes = lanes_for((double)(rp[r + rows] - rp[r]) / rows, prm.max_lanes);
-        if (lanes > 1) ++*nvec;
-        tiles.push_back(Tile{r, rp[r], rp[r + rows] - rp[r], tile_word(rows, kind_of(lanes))});
-        r += rows;
-    }
-}
 
 // ------------------------------------------------------------------ kernels
 namespace {
@@ -468,6 +355,18 @@ size_t stream_smem_bytes(const DevPlan &dp)
     return 16 + 2 * sizeof(int) * (size_t)(dp.stage_rp + dp.stage_cw);
 }
 
+tc_status tiles_grid(const DevPlan &dp, int ctas_per_sm, int *grid)
+{
+    const size_t smem = stream_smem_bytes(dp);
+    int per_sm = 0;
+    TC_CHECK(ensure_smem((const void *)spmv_tiles_kernel<false>, smem));
+    TC_CHECK(ensure_smem((const void *)spmv_tiles_kernel<true>, smem));
+    TC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, spmv_tiles_kernel<true>, kBlock, smem));
+    const int cps = std::max(1, std::min(per_sm, ctas_per_sm));
+    *grid = std::max(1, std::min(dp.ntiles, cps * num_sms()));
+    return TC_OK;
+}
+
 template <bool SIGNED>
 static tc_status launch_tiles(const DevPlan &dp, const WideBounds *wb, const WideStarts *ws, const float *x,
                               float *y, cudaStream_t s)
@@ -543,7 +442,6 @@ tc_status launch_plan(const tc_plan *p, const float *x, float *y, cudaStream_t s
 
 }  // namespace tc
 
-// ------------------------------------------------------------- plan upload
 tc::DevPlan tc_plan::dev_plan() const
 {
     tc::DevPlan d{};
@@ -619,214 +517,3 @@ int64_t tc_plan::spmv_bytes() const
     return 4LL * (M + 1) + 4LL * nnz_csr + 4LL * N + 4LL * M + 20LL * dia_shapes +
            4LL * num_negs;
 }
-
-namespace tc {
-
-static size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
-
-// Diagonal class of rows [r0, r1) (see kDiagGeneral / kDiagNone): the
-// multiply adds the dense-diagonal terms of such a tile without searching the
-// shapes per row, with the same terms in the same order as diag_row.
-static int diag_class(const tc_plan *p, int r0, int r1)
-{
-    if (p->dia_shapes == 0 || r1 <= p->row_start || r0 >= p->row_stop) return kDiagNone;
-    int found = -1;
-    for (int s = 0; s < p->dia_shapes; ++s) {
-        if (r1 <= p->h_xStart[s] || r0 >= p->h_xStop[s]) continue;
-        if (found >= 0) return kDiagGeneral;        // two shapes share rows of the tile
-        found = s;
-    }
-    if (found < 0) return kDiagNone;
-    const int xs = p->h_xStart[found], xe = p->h_xStop[found], msub = xe - xs;
-    if (r0 < xs || r1 > xe || r0 < p->row_start || r1 > p->row_stop) return kDiagGeneral;
-    for (int n = p->h_nDiasPtr[found]; n < p->h_nDiasPtr[found + 1]; ++n) {
-        const int off = p->h_offsets[n];
-        if (r0 - xs + off < 0 || r1 - 1 - xs + off >= msub) return kDiagGeneral;
-    }
-    return found + 1 < kDiagNone ? found + 1 : kDiagGeneral;
-}
-
-tc_status plan_upload(tc_plan *p, const int *csrRow, const int *csrCol, cudaStream_t stream)
-{
-    const int M = p->M;
-    std::vector<Tile> tiles;
-    plan_tiles(csrRow, M, p->params, 4 * num_sms(), tiles, &p->ntiles_vector, &p->ntiles_long);
-    p->ntiles_lanes = 0;
-    p->ntiles_wide = 0;
-    p->ntiles_stream = 0;
-    for (const Tile &t : tiles) {
-        p->ntiles_wide += tile_kind(t) == TILE_DIRECT_WIDE;
-        p->ntiles_stream += tile_kind(t) == TILE_STREAM;
-    }
-    // the direct kernel finds a wide tile's rows from its index
-    for (size_t i = 0; i < tiles.size() && p->ntiles_wide; ++i)
-        if (tiles[i].row0 != (int)i * tile_nrows(tiles[0]) || tile_kind(tiles[i]) != TILE_DIRECT_WIDE)
-            return fail(TC_ERR_FORMAT, "wide tile %d out of order", (int)i);
-    for (const Tile &t : tiles) {
-        p->ntiles_lanes += tile_kind(t) <= TILE_L32 || tile_kind(t) == TILE_MERGE;
-        if (tile_nrows(t) < 1 || tile_nrows(t) > kMaxTileNrows)
-            return fail(TC_ERR_FORMAT, "tile of %d rows", tile_nrows(t));
-    }
-    p->ntiles = (int)tiles.size();
-    p->nnz_csr = csrRow[M];
-    p->max_row = 0;
-    for (int i = 0; i < M; ++i) p->max_row = std::max(p->max_row, csrRow[i + 1] - csrRow[i]);
-    p->wide_rows = p->ntiles_wide ? tile_nrows(tiles[0]) : kDirectWideRows;
-    {   // the most common length of the rows stream tiles hold: skewed slots
-        // when it is a multiple of 8 (see vslot), sampled rows
-        std::vector<int> h(kStreamRowMax + 1, 0);
-        const int step = std::max(1, M / 65536);
-        for (int r = 0; r < M; r += step) {
-            const int L = csrRow[r + 1] - csrRow[r];
-            if (L <= kStreamRowMax) ++h[L];
-        }
-        const int mode = (int)(std::max_element(h.begin() + 1, h.end()) - h.begin());
-        p->stream_skew = h[mode] > 0 && mode % 8 == 0;
-        // a hybrid plan with no holes: every word adds its term
-        p->all_pos = 1;
-        if (p->hybrid)
-            for (int64_t j = 0; j < csrRow[M] && p->all_pos; ++j) p->all_pos = csrCol[j] & 1;
-        // the rows kernel loads W words of a row together: the least of 4, 6, 8
-        // that holds 90 % of the rows whole
-        int64_t tot = 0, upto = 0;
-        for (int L = 0; L <= kStreamRowMax; ++L) tot += h[L];
-        p->rows_w = 8;
-        for (int L = 0, w = 4; L <= 8 && tot > 0; ++L) {
-            upto += h[L];
-            if (L == w) {
-                if (upto * 10 >= tot * 9) {
-                    p->rows_w = w;
-                    break;
-                }
-                w += 2;
-            }
-        }
-    }
-    p->h_wide_nz.clear();
-    if (p->ntiles_wide == p->ntiles && p->ntiles > 0 && p->ntiles <= kWideBoundTiles &&
-        M % kDirectWideRows == 0 && (p->params.flags & TC_FLAG_WIDE_BOUNDS)) {
-        for (const Tile &t : tiles) p->h_wide_nz.push_back(t.nz0);
-        p->h_wide_nz.push_back(csrRow[M]);
-    }
-    // wide plans of few tiles: each tile's first word travels in the launch
-    // parameters, for the word prefetch
-    p->h_wide_z.clear();
-    if (p->ntiles_wide == p->ntiles && p->ntiles > 0 && p->ntiles <= kWideParamTiles &&
-        !(p->params.flags & (TC_FLAG_NO_PREFETCH | TC_FLAG_NO_PARAM_STARTS))) {
-        for (const Tile &t : tiles) p->h_wide_z.push_back(t.nz0);
-        p->h_wide_z.push_back(csrRow[M]);
-    }
-    // shared-memory stage sizes (ints, multiples of 4) from the largest tile
-    int max_rows = 1, max_nnz = 0;
-    for (const Tile &t : tiles)
-        if (tile_kind(t) != TILE_LONG && tile_kind(t) < TILE_STREAM) {
-            max_rows = std::max(max_rows, tile_nrows(t));
-            max_nnz = std::max(max_nnz, t.nnz);
-        }
-    p->stage_rp = (max_rows + 1 + 8 + 3) & ~3;
-    p->stage_cw = (max_nnz + 8 + 3) & ~3;
-
-    // shape table {xStart, xStop, yStart, Msub} and offset ranges
-    std::vector<int4> shapes(p->dia_shapes);
-    std::vector<int2> sd(p->dia_shapes);
-    p->max_span = 0;
-    for (int s = 0; s < p->dia_shapes; ++s) {
-        shapes[s] = make_int4(p->h_xStart[s], p->h_xStop[s], p->h_yStart[s],
-                              p->h_xStop[s] - p->h_xStart[s]);
-        sd[s] = make_int2(p->h_nDiasPtr[s], p->h_nDiasPtr[s + 1]);
-        if (sd[s].y <= sd[s].x) return fail(TC_ERR_FORMAT, "shape %d has no diagonals", s);
-        for (int n = sd[s].x + 1; n < sd[s].y; ++n)
-            if (p->h_offsets[n] <= p->h_offsets[n - 1])
-                return fail(TC_ERR_FORMAT, "offsets of shape %d are not increasing", s);
-        p->max_span = std::max(p->max_span, p->h_offsets[sd[s].y - 1] - p->h_offsets[sd[s].x]);
-    }
-    for (Tile &t : tiles) t.nrows_kind |= diag_class(p, t.row0, t.row0 + tile_nrows(t)) << kDiagShift;
-
-    // window plan: a second tile list for the window kernel (the batch and
-    // served launches keep running `tiles`, with the same terms and order)
-    std::vector<Tile> wtiles;
-    p->nwtiles = 0;
-    {
-        int wlo = 0, whi = 0, wrows = 0, wnnz = 0;
-        if (plan_window(p, csrRow, csrCol, wtiles, &wlo, &whi, &wrows, &wnnz)) {
-            const int w_rp = (wrows + 8 + 3) & ~3, w_cw = (wnnz + 8 + 3) & ~3;
-            const int w_xw = (wrows + whi - wlo + 8 + 3) & ~3;
-            const size_t stage = 4 * (size_t)(w_rp + w_cw + w_xw);
-            const int S = (int)std::min<size_t>(kWinMaxStages, (kWinSmemBudget - 128) / stage);
-            if (S >= 2) {
-                p->nwtiles = (int)wtiles.size();
-                p->wlo = wlo;
-                p->whi = whi;
-                p->w_rp = w_rp;
-                p->w_cw = w_cw;
-                p->w_xw = w_xw;
-                p->w_stages = S;
-                p->w_grid = std::min(p->nwtiles, num_sms());
-                for (Tile &t : wtiles) t.nrows_kind |= diag_class(p, t.row0, t.row0 + tile_nrows(t)) << kDiagShift;
-            } else {
-                wtiles.clear();
-            }
-        }
-    }
-
-    size_t o_rp = 0;
-    size_t o_cols = align256(o_rp + sizeof(int) * ((size_t)M + 1) + 16);
-    size_t o_tiles = align256(o_cols + sizeof(int) * (size_t)p->nnz_csr + 16);
-    size_t o_sh = align256(o_tiles + sizeof(Tile) * tiles.size());
-    size_t o_sd = align256(o_sh + sizeof(int4) * shapes.size());
-    size_t o_off = align256(o_sd + sizeof(int2) * sd.size());
-    size_t o_err = align256(o_off + sizeof(int) * (size_t)p->num_negs + 16);
-    size_t o_wt = align256(o_err + 16);
-    size_t total = align256(o_wt + sizeof(Tile) * wtiles.size());
-    char *base = nullptr;
-    cudaError_t e = cudaMalloc(&base, total);
-    if (e != cudaSuccess)
-        return fail(TC_ERR_ALLOC, "cudaMalloc(%zu) for the plan: %s", total, cudaGetErrorString(e));
-    p->dev = base;
-    p->dev_bytes = total;
-    p->d_rowptr = reinterpret_cast<int *>(base + o_rp);
-    p->d_cols = reinterpret_cast<int *>(base + o_cols);
-    p->d_tiles = reinterpret_cast<Tile *>(base + o_tiles);
-    p->d_shapes = reinterpret_cast<int4 *>(base + o_sh);
-    p->d_shape_dias = reinterpret_cast<int2 *>(base + o_sd);
-    p->d_offsets = reinterpret_cast<int *>(base + o_off);
-    p->d_err = reinterpret_cast<int *>(base + o_err);
-    p->d_wtiles = p->nwtiles ? reinterpret_cast<Tile *>(base + o_wt) : nullptr;
-    {   // persistent grid: CTAs per SM from occupancy at this stage size
-        DevPlan tmp = p->dev_plan();
-        const size_t smem = stream_smem_bytes(tmp);
-        int per_sm = 0;
-        TC_CHECK(ensure_smem((const void *)spmv_tiles_kernel<false>, smem));
-        TC_CHECK(ensure_smem((const void *)spmv_tiles_kernel<true>, smem));
-        TC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, spmv_tiles_kernel<true>, kBlock, smem));
-        const int cps = std::max(1, std::min(per_sm, p->params.ctas_per_sm));
-        p->grid = std::max(1, std::min(p->ntiles, cps * num_sms()));
-    }
-    TC_CUDA(cudaMemsetAsync(base, 0, total, stream));
-    TC_CUDA(cudaMemcpyAsync(p->d_rowptr, csrRow, sizeof(int) * ((size_t)M + 1),
-                            cudaMemcpyHostToDevice, stream));
-    if (p->nnz_csr)
-        TC_CUDA(cudaMemcpyAsync(p->d_cols, csrCol, sizeof(int) * (size_t)p->nnz_csr,
-                                cudaMemcpyHostToDevice, stream));
-    if (!tiles.empty())
-        TC_CUDA(cudaMemcpyAsync(p->d_tiles, tiles.data(), sizeof(Tile) * tiles.size(),
-                                cudaMemcpyHostToDevice, stream));
-    if (p->nwtiles) {
-        TC_CUDA(cudaMemcpyAsync(p->d_wtiles, wtiles.data(), sizeof(Tile) * wtiles.size(),
-                                cudaMemcpyHostToDevice, stream));
-        DevPlan dp = p->dev_plan();
-        TC_CHECK(window_prepare(dp));
-    }
-    if (!shapes.empty()) {
-        TC_CUDA(cudaMemcpyAsync(p->d_shapes, shapes.data(), sizeof(int4) * shapes.size(),
-                                cudaMemcpyHostToDevice, stream));
-        TC_CUDA(cudaMemcpyAsync(p->d_shape_dias, sd.data(), sizeof(int2) * sd.size(),
-                                cudaMemcpyHostToDevice, stream));
-        TC_CUDA(cudaMemcpyAsync(p->d_offsets, p->h_offsets.data(), sizeof(int) * p->num_negs,
-                                cudaMemcpyHostToDevice, stream));
-    }
-    TC_CUDA(cudaStreamSynchronize(stream));   // host arrays may be freed after return
-    return TC_OK;
-}
-
-}  // namespace tc
