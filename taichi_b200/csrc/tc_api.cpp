@@ -178,12 +178,12 @@ tc_status tc_plan_destroy(tc_plan *p)
 {
     if (!p) return TC_OK;
     if (p->dev) cudaFree(p->dev);
-    if (p->dev_tiles) cudaFree(p->dev_tiles);
     for (int k = 0; k < TC_HOST_SLOTS; ++k) {
         if (p->d_xbuf[k]) cudaFree(p->d_xbuf[k]);
         if (p->d_ybuf[k]) cudaFree(p->d_ybuf[k]);
     }
     delete p;
+    tc::plan_gone();
     return TC_OK;
 }
 
@@ -322,25 +322,12 @@ tc_status tc_spmm(const tc_plan *p, const float *d_X, int ldx, int k, float *d_Y
 
 }  // extern "C"
 
-namespace {
-
-// A device array freed at the end of the call.
-struct DeviceArray {
-    void *p = nullptr;
-    ~DeviceArray() { if (p) cudaFree(p); }
-    tc_status copy_in(const void *host, size_t bytes, cudaStream_t s)
-    {
-        if (cudaMalloc(&p, std::max<size_t>(bytes, 16)) != cudaSuccess) {
-            (void)cudaGetLastError();
-            p = nullptr;
-            return fail(TC_ERR_ALLOC, "device copy of the input (%zu bytes)", bytes);
-        }
-        if (bytes) TC_CUDA(cudaMemcpyAsync(p, host, bytes, cudaMemcpyHostToDevice, s));
-        return TC_OK;
-    }
-};
-
-}  // namespace
+static tc_status copy_in(tc::Scratch &a, const void *host, size_t bytes, cudaStream_t s)
+{
+    TC_CHECK(a.alloc(bytes, s));
+    if (bytes) TC_CUDA(cudaMemcpyAsync(a.p, host, bytes, cudaMemcpyHostToDevice, s));
+    return TC_OK;
+}
 
 extern "C" {
 
@@ -392,23 +379,20 @@ tc_status tc_plan_create(int M, int N, int64_t nnz, const int *rowptr, const int
 
     // GPU partition from a device copy of the input; the plan is built from
     // its device arrays (the input's own when nothing was extracted)
-    DeviceArray own_rp, own_col, own_val, out_rp, out_col;
+    tc::Scratch own_rp, own_col, own_val;
     const int *d_rp = rowptr, *d_col = col;
     const float *d_val = val;
     if (!on_device) {
-        TC_CHECK(own_rp.copy_in(rowptr, sizeof(int) * ((size_t)M + 1), s));
-        TC_CHECK(own_col.copy_in(col, sizeof(int) * (size_t)nnz, s));
-        if (val) TC_CHECK(own_val.copy_in(val, sizeof(float) * (size_t)nnz, s));
+        TC_CHECK(copy_in(own_rp, rowptr, sizeof(int) * ((size_t)M + 1), s));
+        TC_CHECK(copy_in(own_col, col, sizeof(int) * (size_t)nnz, s));
+        if (val) TC_CHECK(copy_in(own_val, val, sizeof(float) * (size_t)nnz, s));
         d_rp = static_cast<int *>(own_rp.p);
         d_col = static_cast<int *>(own_col.p);
         d_val = static_cast<float *>(own_val.p);
     }
     tc::PartitionOut po;
-    const tc_status st = tc::gpu_partition(M, N, nnz, d_rp, d_col, d_val, prm,
-                                           (prm.flags & TC_FLAG_KEEP_HOST) != 0, false, s, po);
-    out_rp.p = po.d_rowptr;
-    out_col.p = po.d_cols;
-    if (st != TC_OK) return st;
+    TC_CHECK(tc::gpu_partition(M, N, nnz, d_rp, d_col, d_val, prm, (prm.flags & TC_FLAG_KEEP_HOST) != 0, false, s,
+                               po));
 
     tc_format f{};
     f.dia_shapes = po.dia_shapes; f.num_negs = po.num_negs; f.dense_nnz = po.dense_nnz;
@@ -419,7 +403,7 @@ tc_status tc_plan_create(int M, int N, int64_t nnz, const int *rowptr, const int
     tc_plan *p = nullptr;
     TC_CHECK(plan_of_shapes(M, N, &f, prm, &p));
     const tc_status up = po.aliases_input ? tc::plan_upload(p, d_rp, d_col, nnz, true, s)
-                                          : tc::plan_upload(p, po.d_rowptr, po.d_cols, po.nnz_csr, true, s);
+                                          : tc::plan_upload(p, po.d_rowptr.as<int>(), po.d_cols.as<int>(), po.nnz_csr, true, s);
     if (up != TC_OK) { tc_plan_destroy(p); return up; }
     p->nnz_input = nnz;
     p->partition_ms = po.ms;

@@ -153,18 +153,19 @@ tc_status coo_to_csr_device(int M, int N, bool symmetric, const MtxEntry *h_entr
                             int **d_rowptr, int **d_col, float **d_val, int64_t *nnz_out)
 {
     (void)N;
-    Buf ent, keyA, keyB, idxA, idxB, hist, tmp, rp, cl, vl;
+    Scratch ent, keyA, keyB, idxA, idxB, hist, tmp;
+    Buf rp, cl, vl;                                  // handed to the caller
     const long nrec = 2 * n;
     if (nrec > 0x7fffffffL) return fail(TC_ERR_UNSUPPORTED, "more than 2^30 file entries");
-    TC_CHECK(ent.alloc(sizeof(MtxEntry) * (size_t)n));
-    TC_CHECK(keyA.alloc(sizeof(unsigned) * (size_t)nrec));
-    TC_CHECK(keyB.alloc(sizeof(unsigned) * (size_t)nrec));
-    TC_CHECK(idxA.alloc(sizeof(unsigned) * (size_t)nrec));
-    TC_CHECK(idxB.alloc(sizeof(unsigned) * (size_t)nrec));
+    TC_CHECK(ent.alloc(sizeof(MtxEntry) * (size_t)n, s));
+    TC_CHECK(keyA.alloc(sizeof(unsigned) * (size_t)nrec, s));
+    TC_CHECK(keyB.alloc(sizeof(unsigned) * (size_t)nrec, s));
+    TC_CHECK(idxA.alloc(sizeof(unsigned) * (size_t)nrec, s));
+    TC_CHECK(idxB.alloc(sizeof(unsigned) * (size_t)nrec, s));
     const long blocks = std::max(1L, cdivl(nrec, kSortTile));
     const long nh = blocks * kRadix;
-    TC_CHECK(hist.alloc(sizeof(unsigned) * (size_t)(nh + 1)));
-    TC_CHECK(tmp.alloc(sizeof(int) * scan_tmp_ints(std::max<long>(nh, (long)M + 1))));
+    TC_CHECK(hist.alloc(sizeof(unsigned) * (size_t)(nh + 1), s));
+    TC_CHECK(tmp.alloc(sizeof(int) * scan_tmp_ints(std::max<long>(nh, (long)M + 1)), s));
     TC_CHECK(rp.alloc(sizeof(int) * ((size_t)M + 2)));
     if (n) TC_CUDA(cudaMemcpyAsync(ent.p, h_entries, sizeof(MtxEntry) * (size_t)n, cudaMemcpyHostToDevice, s));
     if (n) {

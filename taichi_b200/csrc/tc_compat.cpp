@@ -235,8 +235,6 @@ void partition_shapes(char *sdf_name, int M, int N, int nnz, int *&csrRow, int *
     cudaFree(d_rp); cudaFree(d_col); cudaFree(d_val);
     if (st != TC_OK) {
         printf("CUDA Runtime Error: %s\n", tc_last_error());
-        if (po.d_rowptr) cudaFree(po.d_rowptr);
-        if (po.d_cols) cudaFree(po.d_cols);
         return;
     }
     // the reference's FLT_MAX marks on claimed entries (TaiChi.cu:866)
@@ -263,11 +261,9 @@ void partition_shapes(char *sdf_name, int M, int N, int nnz, int *&csrRow, int *
     } else if (po.nnz_csr > 0) {
         t->csrRow = (int *)malloc(sizeof(int) * ((size_t)M + 1));
         t->csrCol = (int *)malloc(sizeof(int) * (size_t)po.nnz_csr);
-        cudaMemcpy(t->csrRow, po.d_rowptr, sizeof(int) * ((size_t)M + 1), cudaMemcpyDeviceToHost);
-        cudaMemcpy(t->csrCol, po.d_cols, sizeof(int) * (size_t)po.nnz_csr, cudaMemcpyDeviceToHost);
+        cudaMemcpy(t->csrRow, po.d_rowptr.p, sizeof(int) * ((size_t)M + 1), cudaMemcpyDeviceToHost);
+        cudaMemcpy(t->csrCol, po.d_cols.p, sizeof(int) * (size_t)po.nnz_csr, cudaMemcpyDeviceToHost);
     }
-    if (po.d_rowptr) cudaFree(po.d_rowptr);
-    if (po.d_cols) cudaFree(po.d_cols);
     printf("getSdf:%.4f partition_dense:%.4f partition_sparse:%.4f ms\n", po.ms, t1 - t0 - po.ms, 0.0);
 }
 

@@ -42,6 +42,29 @@ tc_status check_params(const tc_params &p);
         if (s_ != TC_OK) return s_;                                                \
     } while (0)
 
+// ------------------------------------------------------- scratch memory
+// A device array of a build, from the library's memory pool (tc_pool.cpp):
+// allocated and freed in the order of `stream`.
+struct Scratch {
+    void *p = nullptr;
+    cudaStream_t s = nullptr;
+    bool pooled = false;
+    Scratch() = default;
+    Scratch(const Scratch &) = delete;
+    Scratch &operator=(const Scratch &) = delete;
+    ~Scratch();
+    tc_status alloc(size_t bytes, cudaStream_t stream);
+    void release();
+    template <class T> T *as() const { return static_cast<T *>(p); }
+};
+// Plans alive in the process (the pool is trimmed when the last one goes).
+void plan_born();
+void plan_gone();
+// Id of the CUDA context current on this thread (0 when there is none yet or
+// the driver entry points are unavailable).  Read through the driver's entry
+// points, so the library does not link libcuda itself.
+unsigned long long current_context_id();
+
 // ------------------------------------------------------------- tile plan
 // A multiply tile is a run of consecutive rows processed by one CTA.  Kinds
 // TILE_L1..TILE_L32 give 1..32 lanes to each row; TILE_MERGE splits the
@@ -169,6 +192,9 @@ struct tc_plan_impl;
 
 // Opaque plan (the public tc_plan).
 struct tc_plan {
+    tc_plan() { tc::plan_born(); }
+    tc_plan(const tc_plan &) = delete;
+    tc_plan &operator=(const tc_plan &) = delete;
     int M = 0, N = 0;
     tc_params params{};
     // format scalars (TaiChi_new)
@@ -177,8 +203,8 @@ struct tc_plan {
     int64_t nnz_input = 0, nnz_csr = 0;
     int max_row = 0;                     // CSR words of the longest row
     int hybrid = 0;
-    // device arrays: the format (`dev`) and the tiles (`dev_tiles`)
-    void *dev = nullptr, *dev_tiles = nullptr;
+    // device arrays (one allocation, `dev`)
+    void *dev = nullptr;
     size_t dev_bytes = 0;
     int *d_rowptr = nullptr, *d_cols = nullptr, *d_offsets = nullptr;
     tc::Tile *d_tiles = nullptr;
@@ -273,8 +299,8 @@ struct PartitionOut {
     int dia_shapes = 0, num_negs = 0, dense_nnz = 0, zero_elements = 0, sparse_nnz = 0;
     int row_start = 0, row_stop = 0;
     std::vector<int> xStart, yStart, xStop, nDiasPtr, offsets;
-    // device CSR remainder (allocated here with cudaMalloc; caller frees)
-    int *d_rowptr = nullptr, *d_cols = nullptr;
+    // device CSR remainder (unused when aliases_input)
+    Scratch d_rowptr, d_cols;
     int64_t nnz_csr = 0;
     bool aliases_input = false;      // dense_nnz == 0: the input CSR is the format
     int thumb_W = 0, thumb_H = 0, ncontours = 0;

@@ -24,7 +24,6 @@
 //  5. assembly     per row: holes (shape, diagonal, row order) then unclaimed
 //                  entries in CSR order, with the sign bit.
 
-#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -32,7 +31,6 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
-#include <mutex>
 #include <vector>
 
 #include "tc_ctxcache.h"
@@ -41,23 +39,6 @@
 
 namespace tc {
 namespace {
-
-// ---------------------------------------------------------------- buffers
-struct DevBuf {
-    void *p = nullptr;
-    DevBuf() = default;
-    DevBuf(const DevBuf &) = delete;
-    DevBuf &operator=(const DevBuf &) = delete;
-    ~DevBuf() { if (p) cudaFree(p); }
-    tc_status alloc(size_t bytes)
-    {
-        if (p) { cudaFree(p); p = nullptr; }
-        cudaError_t e = cudaMalloc(&p, std::max<size_t>(bytes, 16));
-        if (e != cudaSuccess) return fail(TC_ERR_ALLOC, "cudaMalloc(%zu): %s", bytes, cudaGetErrorString(e));
-        return TC_OK;
-    }
-    template <class T> T *as() const { return reinterpret_cast<T *>(p); }
-};
 
 // ------------------------------------------------------------- bit images
 // An H x W binary image is stored as H rows of WW = ceil(W/32) uint32 words;
@@ -739,13 +720,13 @@ struct ContourList {
 static tc_status contours_on_device(const Img &img, cudaStream_t s, ContourList &out)
 {
     const int n = img.H * img.W;
-    DevBuf lab, flags, order, parent, tmp, bord, flag;
-    TC_CHECK(lab.alloc(sizeof(int) * ((size_t)n + 1)));
-    TC_CHECK(flags.alloc(sizeof(int) * ((size_t)n + 1)));
-    TC_CHECK(order.alloc(sizeof(int) * ((size_t)n + 1)));
-    TC_CHECK(parent.alloc(sizeof(int) * ((size_t)n + 1)));
-    TC_CHECK(tmp.alloc(sizeof(int) * scan_tmp_ints(n)));
-    TC_CHECK(flag.alloc(sizeof(int)));
+    Scratch lab, flags, order, parent, tmp, bord, flag;
+    TC_CHECK(lab.alloc(sizeof(int) * ((size_t)n + 1), s));
+    TC_CHECK(flags.alloc(sizeof(int) * ((size_t)n + 1), s));
+    TC_CHECK(order.alloc(sizeof(int) * ((size_t)n + 1), s));
+    TC_CHECK(parent.alloc(sizeof(int) * ((size_t)n + 1), s));
+    TC_CHECK(tmp.alloc(sizeof(int) * scan_tmp_ints(n), s));
+    TC_CHECK(flag.alloc(sizeof(int), s));
     TC_CUDA(cudaMemsetAsync(flags.p, 0, sizeof(int) * ((size_t)n + 1), s));
     TC_CUDA(cudaMemsetAsync(flag.p, 0, sizeof(int), s));
     const int T = 256;
@@ -756,8 +737,8 @@ static tc_status contours_on_device(const Img &img, cudaStream_t s, ContourList 
     TC_CUDA(cudaGetLastError());
     // discovery order = raster order of the start pixels
     {
-        DevBuf ones;
-        TC_CHECK(ones.alloc(sizeof(int) * ((size_t)n + 1)));
+        Scratch ones;
+        TC_CHECK(ones.alloc(sizeof(int) * ((size_t)n + 1), s));
         nonzero01<<<cdiv(n + 1, T), T, 0, s>>>(flags.as<int>(), ones.as<int>(), n);
         TC_CUDA(cudaGetLastError());
         TC_CHECK(exclusive_scan(ones.as<int>(), order.as<int>(), n, tmp.as<int>(), s));
@@ -765,7 +746,7 @@ static tc_status contours_on_device(const Img &img, cudaStream_t s, ContourList 
     int nb = 0;
     TC_CUDA(cudaMemcpyAsync(&nb, order.as<int>() + n, sizeof(int), cudaMemcpyDeviceToHost, s));
     TC_CUDA(cudaStreamSynchronize(s));
-    TC_CHECK(bord.alloc(sizeof(Border) * (size_t)std::max(nb, 1)));
+    TC_CHECK(bord.alloc(sizeof(Border) * (size_t)std::max(nb, 1), s));
     border_compact<<<cdiv(n, T), T, 0, s>>>(flags.as<int>(), order.as<int>(), parent.as<int>(), n,
                                             bord.as<Border>());
     trace_kernel<<<cdiv(std::max(nb, 1), 64), 64, 0, s>>>(img, bord.as<Border>(), nb, flag.as<int>());
@@ -833,9 +814,9 @@ static tc_status getsdf_device(int M, int N, const int *d_rowptr, const int *d_c
     const int pN = N / W;
     const int WW = (W + 31) / 32;
     const size_t nw = (size_t)H * WW;
-    DevBuf imgs, flag;
-    TC_CHECK(imgs.alloc(sizeof(unsigned) * nw * 8));
-    TC_CHECK(flag.alloc(sizeof(int)));
+    Scratch imgs, flag;
+    TC_CHECK(imgs.alloc(sizeof(unsigned) * nw * 8, s));
+    TC_CHECK(flag.alloc(sizeof(int), s));
     TC_CUDA(cudaMemsetAsync(imgs.p, 0, sizeof(unsigned) * nw * 8, s));
     TC_CUDA(cudaMemsetAsync(flag.p, 0, sizeof(int), s));
     auto img = [&](int k) { return Img{imgs.as<unsigned>() + k * nw, H, W, WW}; };
@@ -873,9 +854,9 @@ static tc_status getsdf_device(int M, int N, const int *d_rowptr, const int *d_c
         out.widths.push_back(area / std::sqrt(dx * dx + dy * dy));
     }
     if (keep_stages) {
-        DevBuf bytes;
+        Scratch bytes;
         const size_t px = (size_t)H * W;
-        TC_CHECK(bytes.alloc(px * 5));
+        TC_CHECK(bytes.alloc(px * 5, s));
         for (int k = 0; k < 5; ++k)
             unpack_kernel<<<cdiv((long)px, 256), 256, 0, s>>>(img(k), bytes.as<unsigned char>() + k * px);
         out.stages.resize(px * 5);
@@ -893,7 +874,7 @@ struct ShapeResult {
     long nnz = 0;
     std::vector<int> offs, start, end, nzero;
     std::vector<long> hole_off;      // offset of each diagonal's holes in `holes`
-    DevBuf holes;                    // local hole rows, ascending per diagonal
+    Scratch holes;                    // local hole rows, ascending per diagonal
 };
 
 static int g_sms = 0;
@@ -920,8 +901,8 @@ static tc_status process_shape(const int *d_rowptr, const int *d_col, unsigned c
     ShapeBox sb{x, y, a, b, w, nd};
     const int T = 256;
     const int grid = std::max(1, std::min(cdiv(b, T), sm_count() * 8));
-    DevBuf cnt, didx, rowcnt, dup;
-    TC_CHECK(cnt.alloc(sizeof(unsigned) * nd));
+    Scratch cnt, didx, rowcnt, dup;
+    TC_CHECK(cnt.alloc(sizeof(unsigned) * nd, s));
     TC_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(unsigned) * nd, s));
     const size_t hsm = nd <= 8192 ? sizeof(unsigned) * nd : 0;
     band_hist<<<grid, T, hsm, s>>>(d_rowptr, d_col, d_claim, sb, cnt.as<unsigned>());
@@ -945,9 +926,9 @@ static tc_status process_shape(const int *d_rowptr, const int *d_col, unsigned c
         }
     }
     if (R.neg == 0) return TC_OK;
-    TC_CHECK(didx.alloc(sizeof(int) * nd));
-    TC_CHECK(rowcnt.alloc(sizeof(int) * (size_t)R.neg * b));
-    TC_CHECK(dup.alloc(sizeof(int)));
+    TC_CHECK(didx.alloc(sizeof(int) * nd, s));
+    TC_CHECK(rowcnt.alloc(sizeof(int) * (size_t)R.neg * b, s));
+    TC_CHECK(dup.alloc(sizeof(int), s));
     TC_CUDA(cudaMemcpyAsync(didx.p, dense_idx.data(), sizeof(int) * nd, cudaMemcpyHostToDevice, s));
     TC_CUDA(cudaMemsetAsync(rowcnt.p, 0, sizeof(int) * (size_t)R.neg * b, s));
     TC_CUDA(cudaMemsetAsync(dup.p, 0, sizeof(int), s));
@@ -958,13 +939,13 @@ static tc_status process_shape(const int *d_rowptr, const int *d_col, unsigned c
     TC_CUDA(cudaMemcpyAsync(&hdup, dup.p, sizeof(int), cudaMemcpyDeviceToHost, s));
     long total = 0;
     for (int d = 0; d < R.neg; ++d) { R.hole_off.push_back(total); total += std::max(R.nzero[d], 0); }
-    TC_CHECK(R.holes.alloc(sizeof(int) * (size_t)std::max(total, 1L)));
+    TC_CHECK(R.holes.alloc(sizeof(int) * (size_t)std::max(total, 1L), s));
     int maxlen = 0;
     for (int d = 0; d < R.neg; ++d) maxlen = std::max(maxlen, R.end[d] - R.start[d]);
-    DevBuf flags, pos, tmp;
-    TC_CHECK(flags.alloc(sizeof(int) * ((size_t)maxlen + 1)));
-    TC_CHECK(pos.alloc(sizeof(int) * ((size_t)maxlen + 1)));
-    TC_CHECK(tmp.alloc(sizeof(int) * scan_tmp_ints(maxlen)));
+    Scratch flags, pos, tmp;
+    TC_CHECK(flags.alloc(sizeof(int) * ((size_t)maxlen + 1), s));
+    TC_CHECK(pos.alloc(sizeof(int) * ((size_t)maxlen + 1), s));
+    TC_CHECK(tmp.alloc(sizeof(int) * scan_tmp_ints(maxlen), s));
     TC_CUDA(cudaStreamSynchronize(s));
     for (int d = 0; d < R.neg; ++d) {
         const int len = R.end[d] - R.start[d];
@@ -990,11 +971,10 @@ tc_status gpu_partition(int M, int N, int64_t nnz, const int *d_rowptr, const in
                         bool want_claimed, cudaStream_t s, PartitionOut &out)
 {
     auto t0 = std::chrono::steady_clock::now();
-    out = PartitionOut();
     if (M < 0 || N < 0 || nnz < 0) return fail(TC_ERR_INVALID, "negative sizes");
-    DevBuf claim, bad;
-    TC_CHECK(claim.alloc((size_t)std::max<int64_t>(nnz, 1)));
-    TC_CHECK(bad.alloc(sizeof(int)));
+    Scratch claim, bad;
+    TC_CHECK(claim.alloc((size_t)std::max<int64_t>(nnz, 1), s));
+    TC_CHECK(bad.alloc(sizeof(int), s));
     const int T = 256;
     TC_CUDA(cudaMemsetAsync(bad.p, 0, sizeof(int), s));
     validate_csr<<<std::max(1, std::min(cdiv(std::max<long>(nnz, M), T), sm_count() * 16)), T, 0, s>>>(
@@ -1057,13 +1037,13 @@ tc_status gpu_partition(int M, int N, int64_t nnz, const int *d_rowptr, const in
         out.nnz_csr = nnz;
     } else {
         // TaiChi.cu:495-612: per row, holes then unclaimed entries
-        DevBuf zc, uf, sp, cnt, tmp, fill;
-        TC_CHECK(zc.alloc(sizeof(int) * ((size_t)M + 1)));
-        TC_CHECK(uf.alloc(sizeof(int) * ((size_t)nnz + 1)));
-        TC_CHECK(sp.alloc(sizeof(int) * ((size_t)nnz + 1)));
-        TC_CHECK(cnt.alloc(sizeof(int) * ((size_t)M + 1)));
-        TC_CHECK(tmp.alloc(sizeof(int) * scan_tmp_ints(std::max<long>(nnz, M))));
-        TC_CHECK(fill.alloc(sizeof(int) * ((size_t)M + 1)));
+        Scratch zc, uf, sp, cnt, tmp, fill;
+        TC_CHECK(zc.alloc(sizeof(int) * ((size_t)M + 1), s));
+        TC_CHECK(uf.alloc(sizeof(int) * ((size_t)nnz + 1), s));
+        TC_CHECK(sp.alloc(sizeof(int) * ((size_t)nnz + 1), s));
+        TC_CHECK(cnt.alloc(sizeof(int) * ((size_t)M + 1), s));
+        TC_CHECK(tmp.alloc(sizeof(int) * scan_tmp_ints(std::max<long>(nnz, M)), s));
+        TC_CHECK(fill.alloc(sizeof(int) * ((size_t)M + 1), s));
         TC_CUDA(cudaMemsetAsync(zc.p, 0, sizeof(int) * ((size_t)M + 1), s));
         TC_CUDA(cudaMemsetAsync(fill.p, 0, sizeof(int) * ((size_t)M + 1), s));
         for (int i = 0; i < ns; ++i) {
@@ -1079,13 +1059,15 @@ tc_status gpu_partition(int M, int N, int64_t nnz, const int *d_rowptr, const in
         TC_CHECK(exclusive_scan(uf.as<int>(), sp.as<int>(), nnz, tmp.as<int>(), s));
         row_totals<<<cdiv((long)M + 1, T), T, 0, s>>>(d_rowptr, sp.as<int>(), zc.as<int>(), M, cnt.as<int>());
         TC_CUDA(cudaGetLastError());
-        TC_CUDA(cudaMalloc(&out.d_rowptr, sizeof(int) * ((size_t)M + 1) + 16));
-        TC_CHECK(exclusive_scan(cnt.as<int>(), out.d_rowptr, M, tmp.as<int>(), s));
+        TC_CHECK(out.d_rowptr.alloc(sizeof(int) * ((size_t)M + 1) + 16, s));
+        int *const rp_out = out.d_rowptr.as<int>();
+        TC_CHECK(exclusive_scan(cnt.as<int>(), rp_out, M, tmp.as<int>(), s));
         int total = 0;
-        TC_CUDA(cudaMemcpyAsync(&total, out.d_rowptr + M, sizeof(int), cudaMemcpyDeviceToHost, s));
+        TC_CUDA(cudaMemcpyAsync(&total, rp_out + M, sizeof(int), cudaMemcpyDeviceToHost, s));
         TC_CUDA(cudaStreamSynchronize(s));
         out.nnz_csr = total;
-        TC_CUDA(cudaMalloc(&out.d_cols, sizeof(int) * (size_t)std::max(total, 1) + 16));
+        TC_CHECK(out.d_cols.alloc(sizeof(int) * (size_t)std::max(total, 1) + 16, s));
+        int *const cols_out = out.d_cols.as<int>();
         for (int i = 0; i < ns; ++i) {
             const ShapeResult &S = shapes[i];
             if (S.nnz <= 0) continue;
@@ -1093,11 +1075,11 @@ tc_status gpu_partition(int M, int N, int64_t nnz, const int *d_rowptr, const in
                 if (S.nzero[d] > 0)
                     hole_scatter<<<cdiv(S.nzero[d], T), T, 0, s>>>(
                         S.holes.as<int>() + S.hole_off[d], S.nzero[d], S.xStart, S.yStart, S.offs[d],
-                        out.d_rowptr, fill.as<int>(), out.d_cols);
+                        rp_out, fill.as<int>(), cols_out);
         }
         sparse_scatter<<<std::max(1, std::min(cdiv(M, T), sm_count() * 8)), T, 0, s>>>(
-            d_rowptr, d_col, claim.as<unsigned char>(), sp.as<int>(), out.d_rowptr, zc.as<int>(), M,
-            out.d_cols);
+            d_rowptr, d_col, claim.as<unsigned char>(), sp.as<int>(), rp_out, zc.as<int>(), M,
+            cols_out);
         TC_CUDA(cudaGetLastError());
     }
     if (want_claimed && nnz) {
@@ -1114,11 +1096,11 @@ tc_status gpu_one_shape(int M, int64_t nnz, const int *h_rowptr, const int *h_co
                         int x, int y, int a, int b, double density, OneShape &o)
 {
     cudaStream_t s = 0;
-    DevBuf rp, cl, va, claim;
-    TC_CHECK(rp.alloc(sizeof(int) * ((size_t)M + 1)));
-    TC_CHECK(cl.alloc(sizeof(int) * (size_t)std::max<int64_t>(nnz, 1)));
-    TC_CHECK(va.alloc(sizeof(float) * (size_t)std::max<int64_t>(nnz, 1)));
-    TC_CHECK(claim.alloc((size_t)std::max<int64_t>(nnz, 1)));
+    Scratch rp, cl, va, claim;
+    TC_CHECK(rp.alloc(sizeof(int) * ((size_t)M + 1), s));
+    TC_CHECK(cl.alloc(sizeof(int) * (size_t)std::max<int64_t>(nnz, 1), s));
+    TC_CHECK(va.alloc(sizeof(float) * (size_t)std::max<int64_t>(nnz, 1), s));
+    TC_CHECK(claim.alloc((size_t)std::max<int64_t>(nnz, 1), s));
     TC_CUDA(cudaMemcpy(rp.p, h_rowptr, sizeof(int) * ((size_t)M + 1), cudaMemcpyHostToDevice));
     if (nnz) {
         TC_CUDA(cudaMemcpy(cl.p, h_col, sizeof(int) * (size_t)nnz, cudaMemcpyHostToDevice));
@@ -1175,9 +1157,10 @@ extern "C" tc_status tc_trace_contours(const unsigned char *img, int H, int W, i
     if (!img || H <= 0 || W <= 0 || !ncontours) return fail(TC_ERR_INVALID, "tc_trace_contours: bad arguments");
     if ((long)H * W > (1L << 26)) return fail(TC_ERR_UNSUPPORTED, "image too large");
     const int WW = (W + 31) / 32;
-    tc::DevBuf bytes, bits;
-    TC_CHECK(bytes.alloc((size_t)H * W));
-    TC_CHECK(bits.alloc(sizeof(unsigned) * (size_t)H * WW));
+    cudaStream_t s = nullptr;
+    tc::Scratch bytes, bits;
+    TC_CHECK(bytes.alloc((size_t)H * W, s));
+    TC_CHECK(bits.alloc(sizeof(unsigned) * (size_t)H * WW, s));
     TC_CUDA(cudaMemcpy(bytes.p, img, (size_t)H * W, cudaMemcpyHostToDevice));
     tc::Img im{bits.as<unsigned>(), H, W, WW};
     tc::pack_kernel<<<tc::cdiv((long)H * WW, 256), 256>>>(bytes.as<unsigned char>(), im);
@@ -1217,34 +1200,6 @@ constexpr int kNoAllocWords = 8 * kNoAllocMaxH * (kNoAllocMaxW / 32);
 static __device__ __align__(256) unsigned g_thumb_scratch[kNoAllocWords + 64];
 
 ContextAddressCache<> g_noalloc_cache;
-
-// Id of the CUDA context current on this thread (0 when there is none yet or
-// the driver entry points are unavailable).  Read through the driver's entry
-// points, so the library does not link libcuda itself.
-unsigned long long current_context_id()
-{
-    using GetCurrent = CUresult (*)(CUcontext *);
-    using GetId = CUresult (*)(CUcontext, unsigned long long *);
-    static GetCurrent get_current = nullptr;
-    static GetId get_id = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void *a = nullptr, *b = nullptr;
-        cudaDriverEntryPointQueryResult qa, qb;
-        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &a, cudaEnableDefault, &qa) == cudaSuccess &&
-            cudaGetDriverEntryPoint("cuCtxGetId", &b, cudaEnableDefault, &qb) == cudaSuccess &&
-            qa == cudaDriverEntryPointSuccess && qb == cudaDriverEntryPointSuccess) {
-            get_current = reinterpret_cast<GetCurrent>(a);
-            get_id = reinterpret_cast<GetId>(b);
-        }
-        (void)cudaGetLastError();
-    });
-    if (!get_current || !get_id) return 0;
-    CUcontext ctx = nullptr;
-    unsigned long long id = 0;
-    if (get_current(&ctx) != CUDA_SUCCESS || !ctx || get_id(ctx, &id) != CUDA_SUCCESS) return 0;
-    return id;
-}
 
 // Device address of g_thumb_scratch in the current context: looked up once
 // per device and context (the host-side name is not a device address, and a
@@ -1360,9 +1315,9 @@ void getSdf(std::string path, int M, int N, int nnz, int *&csrRowIndexHostPtr, i
         report(tc::fail(TC_ERR_INVALID, "bad arguments"));
         return;
     }
-    tc::DevBuf drp, dcol;
-    tc_status st = drp.alloc(sizeof(int) * ((size_t)M + 1));
-    if (st == TC_OK) st = dcol.alloc(sizeof(int) * (size_t)std::max(nnz, 1));
+    tc::Scratch drp, dcol;
+    tc_status st = drp.alloc(sizeof(int) * ((size_t)M + 1), nullptr);
+    if (st == TC_OK) st = dcol.alloc(sizeof(int) * (size_t)std::max(nnz, 1), nullptr);
     if (st == TC_OK && cudaMemcpy(drp.p, csrRowIndexHostPtr, sizeof(int) * ((size_t)M + 1),
                                   cudaMemcpyHostToDevice) != cudaSuccess)
         st = tc::fail(TC_ERR_CUDA, "row pointer upload");

@@ -3,8 +3,7 @@
 //
 // Replaces the upload part of taichi_SpMV (TaiChi.cu:1357-1385).  The format
 // comes from host arrays or, after a partition, from device arrays; either
-// way the row statistics and the tile list are computed on the GPU from the
-// plan's own copy of the row pointers, so a partitioned matrix never crosses
+// way the row statistics and the tile list are computed on the GPU, so a partitioned matrix never crosses
 // the host link.  What bounds a build is then the copies of the format (read
 // and written once) and a few round trips of counts to the host.  Measured on
 // the 9-point mesh 2048^2 (25.7 M words): 1 ms from device arrays in place of
@@ -236,11 +235,6 @@ __global__ void classify_tiles(Tile *__restrict__ tiles, int ntiles, const int4 
     if (lane == 0) tiles[i].nrows_kind |= dc << kDiagShift;
 }
 
-struct Temp {
-    void *p = nullptr;
-    ~Temp() { if (p) cudaFree(p); }
-};
-
 size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
 unsigned blocks_for(long n, int threads)
@@ -310,69 +304,34 @@ tc_status plan_upload(tc_plan *p, const int *csrRow, const int *csrCol, int64_t 
         }
     }
 
-    // the format: row pointers and words, each followed by at least 16 zero
-    // bytes (the kernels' aligned loads run past the last element), the
-    // shapes, the error word, the window tiles
-    const size_t rp_end = sizeof(int) * ((size_t)M + 1);
-    const size_t o_cols = align256(rp_end + 16), cols_end = o_cols + sizeof(int) * (size_t)nnz_csr;
-    const size_t o_sh = align256(cols_end + 16);
-    const size_t o_sd = align256(o_sh + sizeof(int4) * shapes.size());
-    const size_t o_off = align256(o_sd + sizeof(int2) * sd.size());
-    const size_t o_err = align256(o_off + sizeof(int) * (size_t)p->num_negs + 16);
-    const size_t o_wt = align256(o_err + 16);
-    const size_t total = align256(o_wt + sizeof(Tile) * wtiles.size());
-    char *base = nullptr;
-    cudaError_t e = cudaMalloc(&base, total);
-    if (e != cudaSuccess)
-        return fail(TC_ERR_ALLOC, "cudaMalloc(%zu) for the plan: %s", total, cudaGetErrorString(e));
-    p->dev = base;
-    p->dev_bytes = total;
-    p->d_rowptr = reinterpret_cast<int *>(base);
-    p->d_cols = reinterpret_cast<int *>(base + o_cols);
-    p->d_shapes = reinterpret_cast<int4 *>(base + o_sh);
-    p->d_shape_dias = reinterpret_cast<int2 *>(base + o_sd);
-    p->d_offsets = reinterpret_cast<int *>(base + o_off);
-    p->d_err = reinterpret_cast<int *>(base + o_err);
-    p->d_wtiles = p->nwtiles ? reinterpret_cast<Tile *>(base + o_wt) : nullptr;
-    const cudaMemcpyKind in = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-    TC_CUDA(cudaMemsetAsync(base + rp_end, 0, o_cols - rp_end, stream));
-    TC_CUDA(cudaMemsetAsync(base + cols_end, 0, o_sh - cols_end, stream));
-    TC_CUDA(cudaMemsetAsync(base + o_off, 0, o_wt - o_off, stream));
-    TC_CUDA(cudaMemcpyAsync(p->d_rowptr, csrRow, rp_end, in, stream));
-    if (nnz_csr) TC_CUDA(cudaMemcpyAsync(p->d_cols, csrCol, sizeof(int) * (size_t)nnz_csr, in, stream));
-    if (!shapes.empty()) {
-        TC_CUDA(cudaMemcpyAsync(p->d_shapes, shapes.data(), sizeof(int4) * shapes.size(),
-                                cudaMemcpyHostToDevice, stream));
-        TC_CUDA(cudaMemcpyAsync(p->d_shape_dias, sd.data(), sizeof(int2) * sd.size(),
-                                cudaMemcpyHostToDevice, stream));
-        TC_CUDA(cudaMemcpyAsync(p->d_offsets, p->h_offsets.data(), sizeof(int) * p->num_negs,
-                                cudaMemcpyHostToDevice, stream));
+    Scratch up_rp, up_col;                    // host arrays go through device scratch
+    if (!on_device) {
+        TC_CHECK(up_rp.alloc(sizeof(int) * ((size_t)M + 1), stream));
+        TC_CHECK(up_col.alloc(sizeof(int) * (size_t)nnz_csr, stream));
+        TC_CUDA(cudaMemcpyAsync(up_rp.p, csrRow, sizeof(int) * ((size_t)M + 1), cudaMemcpyHostToDevice, stream));
+        if (nnz_csr)
+            TC_CUDA(cudaMemcpyAsync(up_col.p, csrCol, sizeof(int) * (size_t)nnz_csr, cudaMemcpyHostToDevice, stream));
+        csrRow = up_rp.as<int>();
+        csrCol = up_col.as<int>();
     }
-    if (p->nwtiles)
-        TC_CUDA(cudaMemcpyAsync(p->d_wtiles, wtiles.data(), sizeof(Tile) * wtiles.size(),
-                                cudaMemcpyHostToDevice, stream));
 
     // row statistics, and the tiles per strip unless the tiles are wide
     const int strips = (int)(((long)M + kStripRows - 1) / kStripRows);
     const size_t o_sum = align256(sizeof(RowStats)), o_cnt = align256(o_sum + sizeof(TileCounts));
     const size_t o_first = align256(o_cnt + sizeof(int) * ((size_t)strips + 1));
     const size_t o_tmp = align256(o_first + sizeof(int) * ((size_t)strips + 1));
-    Temp tmp;
-    e = cudaMalloc(&tmp.p, o_tmp + sizeof(int) * scan_tmp_ints(strips));
-    if (e != cudaSuccess) {
-        tmp.p = nullptr;
-        return fail(TC_ERR_ALLOC, "planner scratch: %s", cudaGetErrorString(e));
-    }
-    char *t = static_cast<char *>(tmp.p);
+    Scratch tmp;
+    TC_CHECK(tmp.alloc(o_tmp + sizeof(int) * scan_tmp_ints(strips), stream));
+    char *t = tmp.as<char>();
     RowStats *d_st = reinterpret_cast<RowStats *>(t);
     TileCounts *d_sum = reinterpret_cast<TileCounts *>(t + o_sum);
     int *d_cnt = reinterpret_cast<int *>(t + o_cnt), *d_first = reinterpret_cast<int *>(t + o_first);
     int *d_tmp = reinterpret_cast<int *>(t + o_tmp);
     TC_CUDA(cudaMemsetAsync(t, 0, o_first, stream));
     const int step = std::max(1, M / 65536);
-    if (M) row_stats<<<blocks_for(M, 256), 256, 0, stream>>>(p->d_rowptr, M, step, d_st);
+    if (M) row_stats<<<blocks_for(M, 256), 256, 0, stream>>>(csrRow, M, step, d_st);
     if (p->hybrid && nnz_csr)
-        word_signs<<<blocks_for(nnz_csr, 256), 256, 0, stream>>>(p->d_cols, nnz_csr, d_st);
+        word_signs<<<blocks_for(nnz_csr, 256), 256, 0, stream>>>(csrCol, nnz_csr, d_st);
     const int min_tiles = 4 * num_sms();
     TilePrm q;
     q.mode = prm.tile_mode;
@@ -386,7 +345,7 @@ tc_status plan_upload(tc_plan *p, const int *csrRow, const int *csrCol, int64_t 
     q.strided = (prm.flags & TC_FLAG_ROWS_STRIDED) != 0;
     q.no_direct = (prm.flags & TC_FLAG_NO_DIRECT) != 0;
     if (M) {
-        plan_strips<false><<<strips, 32, 0, stream>>>(p->d_rowptr, M, q, d_cnt, nullptr, nullptr, d_sum);
+        plan_strips<false><<<strips, 32, 0, stream>>>(csrRow, M, q, d_cnt, nullptr, nullptr, d_sum);
         TC_CUDA(cudaGetLastError());
         TC_CHECK(exclusive_scan(d_cnt, d_first, strips, d_tmp, stream));
     }
@@ -396,7 +355,7 @@ tc_status plan_upload(tc_plan *p, const int *csrRow, const int *csrCol, int64_t 
     TC_CUDA(cudaMemcpyAsync(&st, d_st, sizeof st, cudaMemcpyDeviceToHost, stream));
     TC_CUDA(cudaMemcpyAsync(&sum, d_sum, sizeof sum, cudaMemcpyDeviceToHost, stream));
     if (M) TC_CUDA(cudaMemcpyAsync(&made, d_first + strips, sizeof made, cudaMemcpyDeviceToHost, stream));
-    TC_CUDA(cudaStreamSynchronize(stream));   // host arrays may be freed after return
+    TC_CUDA(cudaStreamSynchronize(stream));
     p->max_row = st.max_row;
     p->all_pos = !st.minus;                   // a hybrid plan with no holes: every word adds its term
     // rows of at most one entry on average and none long: the whole matrix as
@@ -436,13 +395,50 @@ tc_status plan_upload(tc_plan *p, const int *csrRow, const int *csrCol, int64_t 
         }
     }
 
-    e = cudaMalloc(&p->dev_tiles, align256(sizeof(Tile) * (size_t)std::max(p->ntiles, 1)));
-    if (e != cudaSuccess) {
-        p->dev_tiles = nullptr;
-        return fail(TC_ERR_ALLOC, "%d tiles: %s", p->ntiles, cudaGetErrorString(e));
+    // the format: row pointers and words, each followed by at least 16 zero
+    // bytes (the kernels' aligned loads run past the last element), the
+    // shapes, the error word, the tiles
+    const size_t rp_end = sizeof(int) * ((size_t)M + 1);
+    const size_t o_cols = align256(rp_end + 16), cols_end = o_cols + sizeof(int) * (size_t)nnz_csr;
+    const size_t o_sh = align256(cols_end + 16);
+    const size_t o_sd = align256(o_sh + sizeof(int4) * shapes.size());
+    const size_t o_off = align256(o_sd + sizeof(int2) * sd.size());
+    const size_t o_err = align256(o_off + sizeof(int) * (size_t)p->num_negs + 16);
+    const size_t o_tiles = align256(o_err + 16);
+    const size_t o_wt = align256(o_tiles + sizeof(Tile) * (size_t)p->ntiles);
+    const size_t total = align256(o_wt + sizeof(Tile) * wtiles.size());
+    char *base = nullptr;
+    const cudaError_t e = cudaMalloc(&base, total);
+    if (e != cudaSuccess)
+        return fail(TC_ERR_ALLOC, "cudaMalloc(%zu) for the plan: %s", total, cudaGetErrorString(e));
+    p->dev = base;
+    p->dev_bytes = total;
+    p->d_rowptr = reinterpret_cast<int *>(base);
+    p->d_cols = reinterpret_cast<int *>(base + o_cols);
+    p->d_shapes = reinterpret_cast<int4 *>(base + o_sh);
+    p->d_shape_dias = reinterpret_cast<int2 *>(base + o_sd);
+    p->d_offsets = reinterpret_cast<int *>(base + o_off);
+    p->d_err = reinterpret_cast<int *>(base + o_err);
+    p->d_tiles = reinterpret_cast<Tile *>(base + o_tiles);
+    p->d_wtiles = p->nwtiles ? reinterpret_cast<Tile *>(base + o_wt) : nullptr;
+    TC_CUDA(cudaMemsetAsync(base + rp_end, 0, o_cols - rp_end, stream));
+    TC_CUDA(cudaMemsetAsync(base + cols_end, 0, o_sh - cols_end, stream));
+    TC_CUDA(cudaMemsetAsync(base + o_off, 0, o_tiles - o_off, stream));
+    TC_CUDA(cudaMemcpyAsync(p->d_rowptr, csrRow, rp_end, cudaMemcpyDeviceToDevice, stream));
+    if (nnz_csr)
+        TC_CUDA(cudaMemcpyAsync(p->d_cols, csrCol, sizeof(int) * (size_t)nnz_csr, cudaMemcpyDeviceToDevice, stream));
+    if (!shapes.empty()) {
+        TC_CUDA(cudaMemcpyAsync(p->d_shapes, shapes.data(), sizeof(int4) * shapes.size(),
+                                cudaMemcpyHostToDevice, stream));
+        TC_CUDA(cudaMemcpyAsync(p->d_shape_dias, sd.data(), sizeof(int2) * sd.size(),
+                                cudaMemcpyHostToDevice, stream));
+        TC_CUDA(cudaMemcpyAsync(p->d_offsets, p->h_offsets.data(), sizeof(int) * p->num_negs,
+                                cudaMemcpyHostToDevice, stream));
     }
-    p->dev_bytes += align256(sizeof(Tile) * (size_t)std::max(p->ntiles, 1));
-    p->d_tiles = static_cast<Tile *>(p->dev_tiles);
+    if (p->nwtiles)
+        TC_CUDA(cudaMemcpyAsync(p->d_wtiles, wtiles.data(), sizeof(Tile) * wtiles.size(),
+                                cudaMemcpyHostToDevice, stream));
+
     if (wide)
         wide_tiles<<<(unsigned)((p->ntiles + 255) / 256), 256, 0, stream>>>(p->d_rowptr, M, p->wide_rows, p->ntiles,
                                                                           p->d_tiles);
