@@ -500,7 +500,7 @@ __device__ __forceinline__ bool is_unclaimed(float v)
 __global__ void claim_init(const float *__restrict__ val, unsigned char *__restrict__ claimed, long nnz)
 {
     const long j = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < nnz) claimed[j] = val ? (is_unclaimed(val[j]) ? 0 : 1) : 0;
+    if (j < nnz) claimed[j] = is_unclaimed(val[j]) ? 0 : 1;
 }
 
 struct ShapeBox {
@@ -541,106 +541,154 @@ __global__ void band_hist(const int *__restrict__ rowptr, const int *__restrict_
     }
 }
 
-// Claims the entries of the dense diagonals (TaiChi.cu:848-874) and counts,
-// per dense diagonal and local row, the entries found (for the hole rows).
+// Claims the entries of the dense diagonals (TaiChi.cu:848-874) with the
+// shape's mark, one thread per row of the box, and notes the diagonals each
+// row has an entry on: bit d & 31 of found[(d >> 5) * b + local row].  The
+// row's words belong to its thread alone.  *dup: a row met a diagonal twice.
 __global__ void band_claim(const int *__restrict__ rowptr, const int *__restrict__ col,
                            unsigned char *__restrict__ claimed, ShapeBox sb,
-                           const int *__restrict__ dense_idx, int *__restrict__ rowcnt,
-                           int *__restrict__ dup)
+                           const int *__restrict__ dense_idx, unsigned char mark,
+                           unsigned *__restrict__ found, int *__restrict__ dup)
 {
     const int dof = sb.y - sb.x;
     for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x + sb.x; r < (long)sb.x + sb.b;
          r += (long)gridDim.x * blockDim.x) {
         const int b = __ldg(rowptr + r), e = __ldg(rowptr + r + 1);
         const long lo = r + dof - sb.w + 1, hi = r + dof + sb.w - 1;
+        unsigned bits = 0;
+        int at = 0;                                  // the word that `bits` goes to
+        auto flush = [&] {
+            if (!bits) return;
+            unsigned *const f = found + (long)at * sb.b + (r - sb.x);
+            const unsigned old = *f;
+            if (old & bits) *dup = 1;
+            *f = old | bits;
+            bits = 0;
+        };
         for (int j = b; j < e; ++j) {
             const int c = __ldg(col + j);
             if (c < sb.y || c >= sb.y + sb.a || c < lo || c > hi || claimed[j]) continue;
             const int d = dense_idx[c - r - dof + sb.w - 1];
             if (d < 0) continue;
-            claimed[j] = 1;
-            const int old = atomicAdd(rowcnt + (long)d * sb.b + (r - sb.x), 1);
-            if (old) *dup = 1;
+            claimed[j] = mark;
+            if (d >> 5 != at) {
+                flush();
+                at = d >> 5;
+            }
+            if (bits >> (d & 31) & 1u) *dup = 1;
+            bits |= 1u << (d & 31);
         }
+        flush();
     }
 }
 
-// hole flag of local row r of dense diagonal d: no entry counted there.
-__global__ void hole_flags(const int *__restrict__ rowcnt, int b, int start, int len,
-                           int *__restrict__ flags)
+// Found bits to hole bits, in place: diagonal d has a hole in every local
+// row of [start[d], end[d]) without an entry on it.
+__global__ void hole_bits(unsigned *__restrict__ bits, int b, int neg, const int2 *__restrict__ range)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < len) flags[i] = rowcnt[start + i] == 0;
-    if (i == len) flags[len] = 0;
+    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int words = (neg + 31) >> 5;
+    if (i >= (long)words * b) return;
+    const int w = (int)(i / b), r = (int)(i % b);
+    unsigned in = 0;
+    for (int d = 32 * w; d < min(neg, 32 * w + 32); ++d) {
+        const int2 se = __ldg(range + d);
+        if (r >= se.x && r < se.y) in |= 1u << (d & 31);
+    }
+    bits[i] = in & ~bits[i];
 }
 
 // Duplicate entries: the reference's row walk (TaiChi.cu:809-827) consumes one
 // listed entry per row once the row reaches it; a row is a hole when no entry
-// is pending.  Sequential per diagonal (only runs when duplicates exist).
-__global__ void hole_flags_dups(const int *__restrict__ rowcnt, int start, int len,
-                                int *__restrict__ flags)
+// is pending, and at most keep[d] holes are kept.  The entries per diagonal
+// and row, then a sequential walk per diagonal (only run when duplicates
+// exist).
+__global__ void dup_counts(const int *__restrict__ rowptr, const int *__restrict__ col,
+                           const unsigned char *__restrict__ claimed, ShapeBox sb,
+                           const int *__restrict__ dense_idx, unsigned char mark, int *__restrict__ rowcnt)
 {
-    if (threadIdx.x || blockIdx.x) return;
-    long pending = 0;
-    for (int i = 0; i < len; ++i) {
-        pending += rowcnt[start + i];
-        if (pending > 0) { flags[i] = 0; --pending; }
-        else flags[i] = 1;
-    }
-    flags[len] = 0;
+    const int dof = sb.y - sb.x;
+    for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x + sb.x; r < (long)sb.x + sb.b;
+         r += (long)gridDim.x * blockDim.x)
+        for (int j = __ldg(rowptr + r); j < __ldg(rowptr + r + 1); ++j)
+            if (claimed[j] == mark)                  // an entry of this shape
+                rowcnt[(long)dense_idx[__ldg(col + j) - r - dof + sb.w - 1] * sb.b + (r - sb.x)] += 1;
 }
 
-__global__ void hole_compact(const int *__restrict__ flags, const int *__restrict__ pos, int len,
-                             int start, int keep, int *__restrict__ out)
+__global__ void dup_holes(const int *__restrict__ rowcnt, int b, int neg, const int2 *__restrict__ range,
+                          const int *__restrict__ keep, unsigned *__restrict__ bits)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < len && flags[i] && pos[i] < keep) out[pos[i]] = start + i;
+    const int d = blockIdx.x * blockDim.x + threadIdx.x;
+    if (d >= neg) return;
+    unsigned *const w = bits + (long)(d >> 5) * b;
+    const unsigned bit = 1u << (d & 31);
+    long pending = 0;
+    int made = 0;
+    for (int r = 0; r < b; ++r) {
+        bool hole = false;
+        if (r >= range[d].x && r < range[d].y) {
+            pending += rowcnt[(long)d * b + r];
+            if (pending > 0) --pending;
+            else hole = made++ < keep[d];
+        }
+        if (hole) atomicOr(w + r, bit);              // a word holds 32 diagonals
+        else atomicAnd(w + r, ~bit);
+    }
+}
+
+// Any mark to 1, so that the marks can be given out again.
+__global__ void settle_marks(unsigned char *__restrict__ claimed, long nnz)
+{
+    const long j = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (j < nnz && claimed[j]) claimed[j] = 1;
 }
 
 // --------------------------------------------------------------- assembly
-__global__ void unclaimed_flags(const unsigned char *__restrict__ claimed, long nnz, int *__restrict__ f)
-{
-    const long j = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < nnz) f[j] = !claimed[j];
-    if (j == nnz) f[nnz] = 0;
-}
+// A shape with dense diagonals, for the assembly: rows [x, x + b), columns
+// from y, `neg` diagonals from offset index `off0` on, hole bits as in
+// hole_bits().
+struct HoleShape {
+    int x, y, b, neg, off0;
+    const unsigned *bits;
+};
 
-__global__ void hole_row_count(const int *__restrict__ holes, int n, int xStart, int *__restrict__ zc)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) atomicAdd(zc + xStart + holes[i], 1);
-}
-
-__global__ void row_totals(const int *__restrict__ rowptr, const int *__restrict__ sp,
-                           const int *__restrict__ zc, int M, int *__restrict__ cnt)
-{
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < M) cnt[r] = zc[r] + sp[rowptr[r + 1]] - sp[rowptr[r]];
-    if (r == M) cnt[M] = 0;
-}
-
-// Holes of one dense diagonal: at most one per row, so rows are distinct.
-__global__ void hole_scatter(const int *__restrict__ holes, int n, int xStart, int yStart, int off,
-                             const int *__restrict__ rp_out, int *__restrict__ fill,
-                             int *__restrict__ cols)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int rs = holes[i], r = xStart + rs;
-    cols[rp_out[r] + fill[r]] = (yStart + rs + off) << 1;
-    fill[r] += 1;
-}
-
-__global__ void sparse_scatter(const int *__restrict__ rowptr, const int *__restrict__ col,
-                               const unsigned char *__restrict__ claimed, const int *__restrict__ sp,
-                               const int *__restrict__ rp_out, const int *__restrict__ zc, int M,
-                               int *__restrict__ cols)
+// Row lengths of the remainder: the row's holes and its unclaimed entries.
+__global__ void remainder_counts(const int *__restrict__ rowptr, const unsigned char *__restrict__ claimed,
+                                 const HoleShape *__restrict__ shapes, int nshapes, int M, int *__restrict__ cnt)
 {
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < M; r += gridDim.x * blockDim.x) {
-        const int b = rowptr[r], e = rowptr[r + 1];
-        const int base = rp_out[r] + zc[r] - sp[b];
-        for (int j = b; j < e; ++j)
-            if (!claimed[j]) cols[base + sp[j]] = (col[j] << 1) + 1;
+        int n = 0;
+        for (int s = 0; s < nshapes; ++s) {
+            const HoleShape h = shapes[s];
+            if (r < h.x || r >= h.x + h.b) continue;
+            for (int w = 0; w < (h.neg + 31) >> 5; ++w) n += __popc(__ldg(h.bits + (long)w * h.b + (r - h.x)));
+        }
+        const int e = __ldg(rowptr + r + 1);
+        for (int j = __ldg(rowptr + r); j < e; ++j) n += !__ldg(claimed + j);
+        cnt[r] = n;
+    }
+}
+
+// The remainder's words: per row its holes (shape order, offset order), then
+// its unclaimed entries (CSR order).
+__global__ void remainder_words(const int *__restrict__ rowptr, const int *__restrict__ col,
+                                const unsigned char *__restrict__ claimed, const HoleShape *__restrict__ shapes,
+                                int nshapes, const int *__restrict__ offs, int M,
+                                const int *__restrict__ rp_out, int *__restrict__ cols)
+{
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < M; r += gridDim.x * blockDim.x) {
+        int at = __ldg(rp_out + r);
+        for (int s = 0; s < nshapes; ++s) {
+            const HoleShape h = shapes[s];
+            if (r < h.x || r >= h.x + h.b) continue;
+            const int rs = r - h.x;
+            for (int w = 0; w < (h.neg + 31) >> 5; ++w)
+                for (unsigned m = __ldg(h.bits + (long)w * h.b + rs); m; m &= m - 1)
+                    cols[at++] = (h.y + rs + __ldg(offs + h.off0 + 32 * w + __ffs(m) - 1)) << 1;
+        }
+        const int e = __ldg(rowptr + r + 1);
+        for (int j = __ldg(rowptr + r); j < e; ++j)
+            if (!__ldg(claimed + j)) cols[at++] = (__ldg(col + j) << 1) + 1;
     }
 }
 
@@ -867,14 +915,18 @@ static tc_status getsdf_device(int M, int N, const int *d_rowptr, const int *d_c
 }
 
 // ======================================================================
-// One shape: dense diagonals, holes, claims (TaiChi.cu:677-879)
+// Shapes: dense diagonals, claims, holes (TaiChi.cu:677-879)
 // ======================================================================
 struct ShapeResult {
-    int xStart = 0, yStart = 0, Msub = 0, Nsub = 0, width = 0, neg = 0;
+    ShapeBox box{};
+    int neg = 0;                     // dense diagonals
     long nnz = 0;
+    int cnt0 = 0;                    // its counts' place in the shared histogram
     std::vector<int> offs, start, end, nzero;
-    std::vector<long> hole_off;      // offset of each diagonal's holes in `holes`
-    Scratch holes;                    // local hole rows, ascending per diagonal
+    std::vector<int> dense_idx;      // of each candidate diagonal, -1: not dense
+    unsigned char mark = 0;          // of its entries among the claims
+    Scratch tab;                     // device: dense_idx, ranges {start, end}, nzero, dup flag
+    Scratch bits;                    // hole bits (see hole_bits)
 };
 
 static int g_sms = 0;
@@ -889,78 +941,143 @@ static int sm_count()
     return g_sms;
 }
 
-static tc_status process_shape(const int *d_rowptr, const int *d_col, unsigned char *d_claim, int x,
-                               int y, int a, int b, double density, cudaStream_t s, ShapeResult &R)
+static int box_grid(const ShapeBox &sb) { return std::max(1, std::min(cdiv(sb.b, 256), sm_count() * 8)); }
+
+// The box of a shape; nd <= 0 or b <= 0: no diagonal can be dense.
+static ShapeBox shape_box(int x, int y, int a, int b)
 {
-    R.xStart = x; R.yStart = y; R.Msub = b; R.Nsub = a;
-    const int small = b < a ? b : a;
-    const int w = band_width(small);
-    R.width = w;
-    const int nd = 2 * w - 1;
-    if (nd <= 0 || b <= 0) return TC_OK;
-    ShapeBox sb{x, y, a, b, w, nd};
-    const int T = 256;
-    const int grid = std::max(1, std::min(cdiv(b, T), sm_count() * 8));
-    Scratch cnt, didx, rowcnt, dup;
-    TC_CHECK(cnt.alloc(sizeof(unsigned) * nd, s));
-    TC_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(unsigned) * nd, s));
-    const size_t hsm = nd <= 8192 ? sizeof(unsigned) * nd : 0;
-    band_hist<<<grid, T, hsm, s>>>(d_rowptr, d_col, d_claim, sb, cnt.as<unsigned>());
-    TC_CUDA(cudaGetLastError());
-    std::vector<unsigned> hc(nd);
-    TC_CUDA(cudaMemcpyAsync(hc.data(), cnt.p, sizeof(unsigned) * nd, cudaMemcpyDeviceToHost, s));
-    TC_CUDA(cudaStreamSynchronize(s));
-    std::vector<int> dense_idx(nd, -1);
-    for (int n = 0; n < nd; ++n) {
-        const int off = n - w + 1;
+    const int w = band_width(b < a ? b : a);
+    return ShapeBox{x, y, a, b, w, 2 * w - 1};
+}
+
+// Which diagonals are dense (TaiChi.cu:740-760), from the box's counts.
+static void dense_diagonals(const unsigned *cnt, double density, ShapeResult &R)
+{
+    const ShapeBox &sb = R.box;
+    R.dense_idx.assign(sb.nd, -1);
+    for (int n = 0; n < sb.nd; ++n) {
+        const int off = n - sb.w + 1;
         int st, en;
-        start_end(b, a, w, off, n, st, en);
-        const float dens = (float)hc[n] / (float)(en - st);
+        start_end(sb.b, sb.a, sb.w, off, n, st, en);
+        const float dens = (float)cnt[n] / (float)(en - st);
         if ((double)dens >= density) {           // TaiChi.cu:756-757
-            dense_idx[n] = R.neg++;
+            R.dense_idx[n] = R.neg++;
             R.offs.push_back(off);
             R.start.push_back(st);
             R.end.push_back(en);
-            R.nzero.push_back(en - st - (int)hc[n]);
-            R.nnz += hc[n];
+            R.nzero.push_back(en - st - (int)cnt[n]);
+            R.nnz += cnt[n];
         }
     }
-    if (R.neg == 0) return TC_OK;
-    TC_CHECK(didx.alloc(sizeof(int) * nd, s));
-    TC_CHECK(rowcnt.alloc(sizeof(int) * (size_t)R.neg * b, s));
-    TC_CHECK(dup.alloc(sizeof(int), s));
-    TC_CUDA(cudaMemcpyAsync(didx.p, dense_idx.data(), sizeof(int) * nd, cudaMemcpyHostToDevice, s));
-    TC_CUDA(cudaMemsetAsync(rowcnt.p, 0, sizeof(int) * (size_t)R.neg * b, s));
-    TC_CUDA(cudaMemsetAsync(dup.p, 0, sizeof(int), s));
-    band_claim<<<grid, T, 0, s>>>(d_rowptr, d_col, d_claim, sb, didx.as<int>(), rowcnt.as<int>(),
-                                  dup.as<int>());
-    TC_CUDA(cudaGetLastError());
-    int hdup = 0;
-    TC_CUDA(cudaMemcpyAsync(&hdup, dup.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-    long total = 0;
-    for (int d = 0; d < R.neg; ++d) { R.hole_off.push_back(total); total += std::max(R.nzero[d], 0); }
-    TC_CHECK(R.holes.alloc(sizeof(int) * (size_t)std::max(total, 1L), s));
-    int maxlen = 0;
-    for (int d = 0; d < R.neg; ++d) maxlen = std::max(maxlen, R.end[d] - R.start[d]);
-    Scratch flags, pos, tmp;
-    TC_CHECK(flags.alloc(sizeof(int) * ((size_t)maxlen + 1), s));
-    TC_CHECK(pos.alloc(sizeof(int) * ((size_t)maxlen + 1), s));
-    TC_CHECK(tmp.alloc(sizeof(int) * scan_tmp_ints(maxlen), s));
-    TC_CUDA(cudaStreamSynchronize(s));
+}
+
+// Where the parts of ShapeResult::tab start (ints).
+static size_t tab_range(const ShapeResult &R) { return ((size_t)R.box.nd + 1) & ~(size_t)1; }
+static size_t tab_keep(const ShapeResult &R) { return tab_range(R) + 2 * (size_t)R.neg; }
+static size_t tab_dup(const ShapeResult &R) { return tab_keep(R) + (size_t)R.neg; }
+
+// Claims the shape's dense entries and finds its holes, taking the entries
+// for free of duplicates (R.tab's dup flag says whether they were).
+static tc_status claim_shape(const int *d_rowptr, const int *d_col, unsigned char *d_claim, cudaStream_t s,
+                             ShapeResult &R)
+{
+    const ShapeBox &sb = R.box;
+    std::vector<int> tab(tab_dup(R) + 1, 0);
+    std::copy(R.dense_idx.begin(), R.dense_idx.end(), tab.begin());
     for (int d = 0; d < R.neg; ++d) {
-        const int len = R.end[d] - R.start[d];
-        if (R.nzero[d] <= 0 || len <= 0) continue;
-        const int *rc = rowcnt.as<int>() + (size_t)d * b;
-        if (hdup) hole_flags_dups<<<1, 1, 0, s>>>(rc, R.start[d], len, flags.as<int>());
-        else hole_flags<<<cdiv(len + 1, T), T, 0, s>>>(rc, b, R.start[d], len, flags.as<int>());
-        TC_CUDA(cudaGetLastError());
-        TC_CHECK(exclusive_scan(flags.as<int>(), pos.as<int>(), len, tmp.as<int>(), s));
-        hole_compact<<<cdiv(len, T), T, 0, s>>>(flags.as<int>(), pos.as<int>(), len, R.start[d],
-                                                R.nzero[d], R.holes.as<int>() + R.hole_off[d]);
-        TC_CUDA(cudaGetLastError());
+        tab[tab_range(R) + 2 * d] = R.start[d];
+        tab[tab_range(R) + 2 * d + 1] = R.end[d];
+        tab[tab_keep(R) + d] = R.nzero[d];
     }
-    TC_CUDA(cudaStreamSynchronize(s));
+    const size_t words = (size_t)((R.neg + 31) / 32) * sb.b;
+    TC_CHECK(R.tab.alloc(sizeof(int) * tab.size(), s));
+    TC_CHECK(R.bits.alloc(sizeof(unsigned) * words, s));
+    TC_CUDA(cudaMemcpyAsync(R.tab.p, tab.data(), sizeof(int) * tab.size(), cudaMemcpyHostToDevice, s));
+    TC_CUDA(cudaMemsetAsync(R.bits.p, 0, sizeof(unsigned) * words, s));
+    int *const t = R.tab.as<int>();
+    band_claim<<<box_grid(sb), 256, 0, s>>>(d_rowptr, d_col, d_claim, sb, t, R.mark, R.bits.as<unsigned>(),
+                                            t + tab_dup(R));
+    hole_bits<<<cdiv((long)words, 256), 256, 0, s>>>(R.bits.as<unsigned>(), sb.b, R.neg,
+                                                     reinterpret_cast<const int2 *>(t + tab_range(R)));
+    TC_CUDA(cudaGetLastError());
     return TC_OK;
+}
+
+// Redoes the holes of a shape whose rows hold duplicate entries, if it does.
+static tc_status settle_duplicates(const int *d_rowptr, const int *d_col, const unsigned char *d_claim,
+                                   cudaStream_t s, ShapeResult &R)
+{
+    int *const t = R.tab.as<int>();
+    int dup = 0;
+    TC_CUDA(cudaMemcpyAsync(&dup, t + tab_dup(R), sizeof(int), cudaMemcpyDeviceToHost, s));
+    TC_CUDA(cudaStreamSynchronize(s));
+    if (!dup) return TC_OK;
+    Scratch rowcnt;
+    const size_t bytes = sizeof(int) * (size_t)R.neg * R.box.b;
+    TC_CHECK(rowcnt.alloc(bytes, s));
+    TC_CUDA(cudaMemsetAsync(rowcnt.p, 0, bytes, s));
+    dup_counts<<<box_grid(R.box), 256, 0, s>>>(d_rowptr, d_col, d_claim, R.box, t, R.mark, rowcnt.as<int>());
+    dup_holes<<<cdiv(R.neg, 32), 32, 0, s>>>(rowcnt.as<int>(), R.box.b, R.neg,
+                                            reinterpret_cast<const int2 *>(t + tab_range(R)), t + tab_keep(R),
+                                            R.bits.as<unsigned>());
+    TC_CUDA(cudaGetLastError());
+    return TC_OK;
+}
+
+static tc_status launch_hist(const int *d_rowptr, const int *d_col, const unsigned char *d_claim,
+                             const ShapeBox &sb, unsigned *cnt, cudaStream_t s)
+{
+    const size_t hsm = sb.nd <= 8192 ? sizeof(unsigned) * sb.nd : 0;
+    band_hist<<<box_grid(sb), 256, hsm, s>>>(d_rowptr, d_col, d_claim, sb, cnt);
+    TC_CUDA(cudaGetLastError());
+    return TC_OK;
+}
+
+// The shapes in order (TaiChi.cu:361-421).  A shape's counts see the claims
+// of the shapes before it, so they are taken for up to kHistAhead shapes at
+// once and taken again for the rest after a shape that claims.
+constexpr int kHistAhead = 32;
+constexpr int kMarks = 250;          // marks 2 .. 251; 1: claimed earlier
+
+static tc_status process_shapes(const int *d_rowptr, const int *d_col, unsigned char *d_claim, int64_t nnz,
+                                double density, cudaStream_t s, std::vector<ShapeResult> &shapes)
+{
+    const size_t n = shapes.size();
+    Scratch cnt;
+    std::vector<unsigned> hc;
+    std::vector<ShapeResult *> open;             // claimed since the marks were last settled
+    auto settle = [&](bool marks) -> tc_status {
+        for (ShapeResult *R : open) TC_CHECK(settle_duplicates(d_rowptr, d_col, d_claim, s, *R));
+        open.clear();
+        if (marks && nnz) settle_marks<<<cdiv(nnz, 256), 256, 0, s>>>(d_claim, nnz);
+        return TC_OK;
+    };
+    for (size_t i = 0; i < n;) {
+        const size_t stop = std::min(n, i + kHistAhead);
+        int total = 0;
+        for (size_t k = i; k < stop; ++k) {
+            shapes[k].cnt0 = total;
+            total += shapes[k].box.nd;
+        }
+        TC_CHECK(cnt.alloc(sizeof(unsigned) * (size_t)total, s));
+        TC_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(unsigned) * (size_t)total, s));
+        for (size_t k = i; k < stop; ++k)
+            TC_CHECK(launch_hist(d_rowptr, d_col, d_claim, shapes[k].box, cnt.as<unsigned>() + shapes[k].cnt0, s));
+        hc.resize(total);
+        TC_CUDA(cudaMemcpyAsync(hc.data(), cnt.p, sizeof(unsigned) * (size_t)total, cudaMemcpyDeviceToHost, s));
+        TC_CUDA(cudaStreamSynchronize(s));
+        for (bool claimed = false; i < stop && !claimed; ++i) {
+            ShapeResult &R = shapes[i];
+            dense_diagonals(hc.data() + R.cnt0, density, R);
+            if (R.neg == 0) continue;
+            if (open.size() == kMarks) TC_CHECK(settle(true));
+            R.mark = (unsigned char)(2 + open.size());
+            TC_CHECK(claim_shape(d_rowptr, d_col, d_claim, s, R));
+            open.push_back(&R);
+            claimed = true;
+        }
+    }
+    return settle(false);
 }
 
 // ======================================================================
@@ -984,7 +1101,8 @@ tc_status gpu_partition(int M, int N, int64_t nnz, const int *d_rowptr, const in
     TC_CUDA(cudaStreamSynchronize(s));
     if (hbad) return fail(TC_ERR_FORMAT, "invalid CSR input (code %d: 1 rowptr decreases, 2 column "
                                          "outside [0, N), 4 rowptr[0]/rowptr[M] wrong)", hbad);
-    if (nnz) claim_init<<<cdiv(nnz, T), T, 0, s>>>(d_val, claim.as<unsigned char>(), nnz);
+    if (nnz && d_val) claim_init<<<cdiv(nnz, T), T, 0, s>>>(d_val, claim.as<unsigned char>(), nnz);
+    else TC_CUDA(cudaMemsetAsync(claim.p, 0, (size_t)std::max<int64_t>(nnz, 1), s));
     TC_CUDA(cudaGetLastError());
 
     SdfOut sdf;
@@ -995,33 +1113,36 @@ tc_status gpu_partition(int M, int N, int64_t nnz, const int *d_rowptr, const in
     out.stages.swap(sdf.stages);
     out.ncontours = sdf.ncontours;
 
-    const int ns = (int)sdf.corners.size() / 4;
-    std::vector<ShapeResult> shapes(ns);
-    long dense = 0;
-    for (int i = 0; i < ns; ++i) {     // TaiChi.cu:361-421, in shape order
-        const int x1 = sdf.corners[4 * i], y1 = sdf.corners[4 * i + 1];
-        const int a1 = sdf.corners[4 * i + 2] - x1, b1 = sdf.corners[4 * i + 3] - y1;
+    std::vector<ShapeBox> boxes;
+    for (size_t i = 0; i + 3 < sdf.corners.size(); i += 4) {     // TaiChi.cu:361-421, in shape order
+        const int x1 = sdf.corners[i], y1 = sdf.corners[i + 1];
         int x, y, a, b;
-        shape_size(M, N, sdf.mF, x1, y1, a1, b1, x, y, a, b);
+        shape_size(M, N, sdf.mF, x1, y1, sdf.corners[i + 2] - x1, sdf.corners[i + 3] - y1, x, y, a, b);
         if (a < prm.min_shape_side || b < prm.min_shape_side) continue;
-        TC_CHECK(process_shape(d_rowptr, d_col, claim.as<unsigned char>(), x, y, a, b, prm.density,
-                               s, shapes[i]));
-        if (shapes[i].nnz > 0) {
-            out.dia_shapes++;
-            out.num_negs += shapes[i].neg;
-            dense += shapes[i].nnz;
-        }
+        const ShapeBox sb = shape_box(x, y, a, b);
+        if (sb.nd > 0 && sb.b > 0) boxes.push_back(sb);
     }
+    std::vector<ShapeResult> shapes(boxes.size());
+    for (size_t i = 0; i < boxes.size(); ++i) shapes[i].box = boxes[i];
+    TC_CHECK(process_shapes(d_rowptr, d_col, claim.as<unsigned char>(), nnz, prm.density, s, shapes));
+    long dense = 0;
+    for (const ShapeResult &S : shapes)
+        if (S.nnz > 0) {
+            out.dia_shapes++;
+            out.num_negs += S.neg;
+            dense += S.nnz;
+        }
     out.dense_nnz = (int)dense;
     out.sparse_nnz = (int)(nnz - dense);
     long zeros = 0;
     out.nDiasPtr.push_back(0);
-    for (int i = 0; i < ns; ++i) {
-        const ShapeResult &S = shapes[i];
+    std::vector<HoleShape> hs;
+    for (const ShapeResult &S : shapes) {
         if (S.nnz <= 0) continue;
-        out.xStart.push_back(S.xStart);
-        out.yStart.push_back(S.yStart);
-        out.xStop.push_back(S.xStart + S.Msub);
+        hs.push_back(HoleShape{S.box.x, S.box.y, S.box.b, S.neg, out.nDiasPtr.back(), S.bits.as<unsigned>()});
+        out.xStart.push_back(S.box.x);
+        out.yStart.push_back(S.box.y);
+        out.xStop.push_back(S.box.x + S.box.b);
         out.nDiasPtr.push_back(out.nDiasPtr.back() + S.neg);
         for (int d = 0; d < S.neg; ++d) { out.offsets.push_back(S.offs[d]); zeros += S.nzero[d]; }
     }
@@ -1037,50 +1158,33 @@ tc_status gpu_partition(int M, int N, int64_t nnz, const int *d_rowptr, const in
         out.nnz_csr = nnz;
     } else {
         // TaiChi.cu:495-612: per row, holes then unclaimed entries
-        Scratch zc, uf, sp, cnt, tmp, fill;
-        TC_CHECK(zc.alloc(sizeof(int) * ((size_t)M + 1), s));
-        TC_CHECK(uf.alloc(sizeof(int) * ((size_t)nnz + 1), s));
-        TC_CHECK(sp.alloc(sizeof(int) * ((size_t)nnz + 1), s));
+        Scratch tab, cnt, tmp;
+        const size_t o_off = sizeof(HoleShape) * hs.size();
+        TC_CHECK(tab.alloc(o_off + sizeof(int) * out.offsets.size(), s));
         TC_CHECK(cnt.alloc(sizeof(int) * ((size_t)M + 1), s));
-        TC_CHECK(tmp.alloc(sizeof(int) * scan_tmp_ints(std::max<long>(nnz, M)), s));
-        TC_CHECK(fill.alloc(sizeof(int) * ((size_t)M + 1), s));
-        TC_CUDA(cudaMemsetAsync(zc.p, 0, sizeof(int) * ((size_t)M + 1), s));
-        TC_CUDA(cudaMemsetAsync(fill.p, 0, sizeof(int) * ((size_t)M + 1), s));
-        for (int i = 0; i < ns; ++i) {
-            const ShapeResult &S = shapes[i];
-            if (S.nnz <= 0) continue;
-            for (int d = 0; d < S.neg; ++d)
-                if (S.nzero[d] > 0)
-                    hole_row_count<<<cdiv(S.nzero[d], T), T, 0, s>>>(S.holes.as<int>() + S.hole_off[d],
-                                                                     S.nzero[d], S.xStart, zc.as<int>());
-        }
-        unclaimed_flags<<<cdiv(nnz + 1, T), T, 0, s>>>(claim.as<unsigned char>(), nnz, uf.as<int>());
-        TC_CUDA(cudaGetLastError());
-        TC_CHECK(exclusive_scan(uf.as<int>(), sp.as<int>(), nnz, tmp.as<int>(), s));
-        row_totals<<<cdiv((long)M + 1, T), T, 0, s>>>(d_rowptr, sp.as<int>(), zc.as<int>(), M, cnt.as<int>());
-        TC_CUDA(cudaGetLastError());
-        TC_CHECK(out.d_rowptr.alloc(sizeof(int) * ((size_t)M + 1) + 16, s));
+        TC_CHECK(tmp.alloc(sizeof(int) * scan_tmp_ints(M), s));
+        TC_CHECK(out.d_rowptr.alloc(sizeof(int) * ((size_t)M + 1), s));
+        const HoleShape *const d_hs = tab.as<HoleShape>();
+        const int *const d_offs = reinterpret_cast<const int *>(tab.as<char>() + o_off);
+        TC_CUDA(cudaMemcpyAsync(tab.p, hs.data(), o_off, cudaMemcpyHostToDevice, s));
+        TC_CUDA(cudaMemcpyAsync(tab.as<char>() + o_off, out.offsets.data(), sizeof(int) * out.offsets.size(),
+                                cudaMemcpyHostToDevice, s));
         int *const rp_out = out.d_rowptr.as<int>();
+        const int grid = std::max(1, std::min(cdiv(M, T), sm_count() * 8));
+        TC_CUDA(cudaMemsetAsync(cnt.as<int>() + M, 0, sizeof(int), s));          // the scan's trailing 0
+        remainder_counts<<<grid, T, 0, s>>>(d_rowptr, claim.as<unsigned char>(), d_hs, (int)hs.size(), M,
+                                            cnt.as<int>());
+        TC_CUDA(cudaGetLastError());
         TC_CHECK(exclusive_scan(cnt.as<int>(), rp_out, M, tmp.as<int>(), s));
         int total = 0;
         TC_CUDA(cudaMemcpyAsync(&total, rp_out + M, sizeof(int), cudaMemcpyDeviceToHost, s));
         TC_CUDA(cudaStreamSynchronize(s));
         out.nnz_csr = total;
-        TC_CHECK(out.d_cols.alloc(sizeof(int) * (size_t)std::max(total, 1) + 16, s));
-        int *const cols_out = out.d_cols.as<int>();
-        for (int i = 0; i < ns; ++i) {
-            const ShapeResult &S = shapes[i];
-            if (S.nnz <= 0) continue;
-            for (int d = 0; d < S.neg; ++d)
-                if (S.nzero[d] > 0)
-                    hole_scatter<<<cdiv(S.nzero[d], T), T, 0, s>>>(
-                        S.holes.as<int>() + S.hole_off[d], S.nzero[d], S.xStart, S.yStart, S.offs[d],
-                        rp_out, fill.as<int>(), cols_out);
-        }
-        sparse_scatter<<<std::max(1, std::min(cdiv(M, T), sm_count() * 8)), T, 0, s>>>(
-            d_rowptr, d_col, claim.as<unsigned char>(), sp.as<int>(), rp_out, zc.as<int>(), M,
-            cols_out);
+        TC_CHECK(out.d_cols.alloc(sizeof(int) * (size_t)total, s));
+        remainder_words<<<grid, T, 0, s>>>(d_rowptr, d_col, claim.as<unsigned char>(), d_hs, (int)hs.size(), d_offs,
+                                           M, rp_out, out.d_cols.as<int>());
         TC_CUDA(cudaGetLastError());
+        TC_CUDA(cudaStreamSynchronize(s));
     }
     if (want_claimed && nnz) {
         out.claimed.resize((size_t)nnz);
@@ -1107,16 +1211,20 @@ tc_status gpu_one_shape(int M, int64_t nnz, const int *h_rowptr, const int *h_co
         TC_CUDA(cudaMemcpy(va.p, h_val, sizeof(float) * (size_t)nnz, cudaMemcpyHostToDevice));
         claim_init<<<cdiv(nnz, 256), 256, 0, s>>>(va.as<float>(), claim.as<unsigned char>(), nnz);
     }
-    ShapeResult R;
-    TC_CHECK(process_shape(rp.as<int>(), cl.as<int>(), claim.as<unsigned char>(), x, y, a, b, density, s, R));
-    o.width = R.width; o.neg = R.neg; o.nnz = R.nnz;
+    std::vector<ShapeResult> one(1);
+    ShapeResult &R = one[0];
+    R.box = shape_box(x, y, a, b);
+    if (R.box.nd > 0 && b > 0)
+        TC_CHECK(process_shapes(rp.as<int>(), cl.as<int>(), claim.as<unsigned char>(), nnz, density, s, one));
+    o.width = R.box.w; o.neg = R.neg; o.nnz = R.nnz;
     o.offs = R.offs; o.start = R.start; o.end = R.end; o.nzero = R.nzero;
     o.holes.assign(R.neg, std::vector<int>());
-    for (int d = 0; d < R.neg; ++d) {
-        o.holes[d].resize(std::max(R.nzero[d], 0));
-        if (R.nzero[d] > 0)
-            TC_CUDA(cudaMemcpy(o.holes[d].data(), R.holes.as<int>() + R.hole_off[d],
-                               sizeof(int) * R.nzero[d], cudaMemcpyDeviceToHost));
+    if (R.neg > 0) {
+        std::vector<unsigned> bits((size_t)((R.neg + 31) / 32) * b);
+        TC_CUDA(cudaMemcpy(bits.data(), R.bits.p, sizeof(unsigned) * bits.size(), cudaMemcpyDeviceToHost));
+        for (int d = 0; d < R.neg; ++d)
+            for (int r = 0; r < b; ++r)
+                if (bits[(size_t)(d / 32) * b + r] >> (d & 31) & 1u) o.holes[d].push_back(r);
     }
     if (nnz && R.neg > 0) {
         std::vector<unsigned char> c((size_t)nnz);
