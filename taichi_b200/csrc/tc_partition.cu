@@ -6,10 +6,11 @@
 //
 //  1. raster       512 x W thumbnail of the pattern (getSdf_GPU1), one CTA per
 //                  thumbnail row, bits in shared memory.
-//  2. morphology   hole fill (imfill), 30x1 and 1x30 openings, subtraction and
-//                  the eye(5) opening, on bit-packed rows in one CTA, with
-//                  OpenCV's conventions (non-reflected element, anchor at the
-//                  centre, erosion sees 1 and dilation 0 outside the image).
+//  2. morphology   hole fill (imfill) by union-find over runs of zeros; 30x1
+//                  and 1x30 openings, subtraction and the eye(5) opening on
+//                  bit-packed rows in one CTA, with OpenCV's conventions
+//                  (non-reflected element, anchor at the centre, erosion sees
+//                  1 and dilation 0 outside the image).
 //  3. contours     findContours(RETR_CCOMP, CHAIN_APPROX_NONE): union-find
 //                  labelling of 8-connected ones and 4-connected zeros gives
 //                  every border's start pixel (Suzuki & Abe: the first pixel of
@@ -107,28 +108,178 @@ __global__ void raster_kernel(const int *__restrict__ rowptr, const int *__restr
     for (int k = threadIdx.x; k < img.WW; k += blockDim.x) img.w[px * img.WW + k] = srow[k];
 }
 
+// ------------------------------------------------------- connected regions
+// Union-find over runs.  A node is a maximal run of equal pixels within one
+// word of a row, named 1 + the index of its first pixel; node 0 is the zero
+// frame around the image.  Links always point to a smaller name, so a
+// region's root names its first pixel in raster order.  Joining runs instead
+// of pixels is what makes it cheap: a word of equal pixels is one node, zero
+// runs on the image border start out linked to the frame, and vertical
+// neighbours join once per overlap.  Hole filling of the 9-point mesh's
+// thumbnail (512 x 512, noisy): 2.5 ms as alternating row and column closures
+// in one CTA, 0.14 ms this way; labelling the opened image: 190 us per pixel,
+// 100 us per run.
+__device__ __forceinline__ int uf_find(int *L, int a)
+{
+    int b = __ldcg(L + a);
+    while (b != a) { a = b; b = __ldcg(L + a); }
+    return a;
+}
+
+__device__ void uf_union(int *L, int a, int b, int *flag)
+{
+    for (int it = 0; it < (1 << 24); ++it) {
+        a = uf_find(L, a);
+        b = uf_find(L, b);
+        if (a == b) return;
+        if (a < b) {
+            const int old = atomicMin(L + b, a);
+            if (old == b) return;
+            b = old;
+        } else {
+            const int old = atomicMin(L + a, b);
+            if (old == a) return;
+            a = old;
+        }
+    }
+    *flag = 2;   // no progress (cannot happen): reported, never waited on
+}
+
+// First bit of the run of set bits of v that holds bit p.
+__device__ __forceinline__ int run_start(unsigned v, int p)
+{
+    return 32 - __clz(~v & ((1u << p) - 1u));
+}
+__device__ __forceinline__ unsigned run_starts(unsigned v) { return v & ~(v << 1); }
+// The run of set bits of v that starts at bit p, as a mask.
+__device__ __forceinline__ unsigned run_mask(unsigned v, int p)
+{
+    const unsigned past = ~(v >> p);                 // first clear bit above p ends the run
+    const int n = past ? __ffs(past) - 1 : 32;
+    return (n >= 32 ? 0xffffffffu : (1u << n) - 1u) << p;
+}
+// Bits of word k inside the image.
+__device__ __forceinline__ unsigned word_mask(const Img &img, int k)
+{
+    return k == img.WW - 1 ? img.lastmask() : 0xffffffffu;
+}
+
+// Names every run of zeros, and with ONES every run of ones: itself, or the
+// frame for a zero run that touches the image border.
+template <bool ONES>
+__global__ void regions_init(Img img, int *__restrict__ L)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) L[0] = 0;
+    if (i >= img.H * img.WW) return;
+    const int y = i / img.WW, k = i % img.WW;
+    const unsigned in = word_mask(img, k), v = img.w[i] & in, z = ~v & in;
+    const int name = 1 + y * img.W + 32 * k;
+    const bool edge_row = y == 0 || y == img.H - 1;
+    for (unsigned m = run_starts(z); m; m &= m - 1) {
+        const int p = __ffs(m) - 1;
+        const bool edge = edge_row || (k == 0 && p == 0) ||
+                          (k == img.WW - 1 && (run_mask(z, p) & ~(in >> 1)));   // holds the last column
+        L[name + p] = edge ? 0 : name + p;
+    }
+    if (ONES)
+        for (unsigned m = run_starts(v); m; m &= m - 1) {
+            const int p = __ffs(m) - 1;
+            L[name + p] = name + p;
+        }
+}
+
+// Joins neighbouring runs: zeros 4-connected, ones 8-connected.
+template <bool ONES>
+__global__ void regions_join(Img img, int *L, int *flag)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= img.H * img.WW) return;
+    const int WW = img.WW, W = img.W, y = i / WW, k = i % WW;
+    const unsigned in = word_mask(img, k), v = img.w[i] & in, z = ~v & in;
+    const int name = 1 + y * W + 32 * k;
+    const unsigned pv = k > 0 ? img.w[i - 1] : 0u;           // word to the left (whole)
+    const unsigned uv = y > 0 ? img.w[i - WW] & in : 0u, uz = y > 0 ? ~uv & in : 0u;
+    if (k > 0 && (z & 1u) && !(pv >> 31)) uf_union(L, name, name - 32 + run_start(~pv, 31), flag);
+    for (unsigned m = run_starts(z & uz); m; m &= m - 1) {
+        const int p = __ffs(m) - 1;
+        uf_union(L, name + run_start(z, p), name - W + run_start(uz, p), flag);
+    }
+    if (!ONES) return;
+    if (k > 0 && (v & 1u) && (pv >> 31)) uf_union(L, name, name - 32 + run_start(pv, 31), flag);
+    if (y == 0) return;
+    const unsigned ul = k > 0 ? img.w[i - WW - 1] : 0u, ur = k < WW - 1 ? img.w[i - WW + 1] & word_mask(img, k + 1) : 0u;
+    for (unsigned m = run_starts(v); m; m &= m - 1) {
+        const int p = __ffs(m) - 1;
+        const unsigned run = run_mask(v, p), near = run | (run << 1) | (run >> 1);
+        for (unsigned t = run_starts(uv & near); t; t &= t - 1)
+            uf_union(L, name + p, name - W + run_start(uv, __ffs(t) - 1), flag);
+        if (p == 0 && (ul >> 31)) uf_union(L, name, name - W - 32 + run_start(ul, 31), flag);
+        if ((run >> 31) && (ur & 1u)) uf_union(L, name + p, name - W + 32, flag);
+    }
+}
+
+// imfill (morohutils.cu:73-83): F = B | (zeros of B that are not 4-connected
+// to the zero frame around the image).
+__global__ void fill_holes(Img B, int *L, Img F)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= B.H * B.WW) return;
+    const int y = i / B.WW, k = i % B.WW;
+    const unsigned in = word_mask(B, k), z = ~B.w[i] & in;
+    unsigned f = B.w[i] & in;
+    for (unsigned m = run_starts(z); m; m &= m - 1) {
+        const int p = __ffs(m) - 1;
+        if (uf_find(L, 1 + y * B.W + 32 * k + p) != 0) f |= run_mask(z, p);
+    }
+    F.w[i] = f;
+}
+
 // --------------------------------------------------------------- morphology
-// All stages in one CTA; images live wherever the pointers say (shared memory
-// for thumbnails up to 32 KB per image, else global memory).
+// The openings in one CTA (65 us for a 512 x 512 thumbnail, most of it the
+// vertical lines' 30 shared-memory reads a word; the horizontal ones take 5
+// steps in registers); images live wherever the pointers say (shared
+// memory for thumbnails up to 50 KB per image, else global memory).
+
+// AND (erode) or OR over the L pixels x - a .. x - a + L - 1 of a row for the
+// 32 pixels x of word k, a = L / 2; outside the image the neutral value.
+// L <= 32: by doubling on three words in registers.
+__device__ __forceinline__ unsigned line_h(const Img &src, int y, int k, int L, bool erode)
+{
+    const unsigned fill = erode ? 0xffffffffu : 0u;
+    const int a = L / 2;
+    if (L > 32) {
+        unsigned v = fill;
+        for (int d = -a; d < L - a; ++d) {
+            const unsigned t = src.shifted(y, k, d, fill);
+            v = erode ? v & t : v | t;
+        }
+        return v;
+    }
+    unsigned lo = src.get(y, k - 1, fill), mid = src.get(y, k, fill), hi = src.get(y, k + 1, fill);
+    if (!erode) { lo = ~lo; mid = ~mid; hi = ~hi; }          // OR of pixels = not AND of their complements
+    for (int m = 1; m < L;) {                                // windows of m pixels from each pixel on
+        const int s = min(m, L - m);
+        lo &= __funnelshift_r(lo, mid, s);
+        mid &= __funnelshift_r(mid, hi, s);
+        hi &= __funnelshift_r(hi, 0xffffffffu, s);
+        m += s;
+    }
+    const unsigned v = a ? __funnelshift_r(lo, mid, 32 - a) : mid;
+    return erode ? v : ~v;
+}
 
 __device__ void erode_dilate_h(const Img &src, Img &tmp, Img &dst, int L)
 {
-    const int a = L / 2;
     const int n = src.H * src.WW;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         const int y = i / src.WW, k = i % src.WW;
-        unsigned v = 0xffffffffu;
-        for (int d = -a; d < L - a; ++d) v &= src.shifted(y, k, d, 0xffffffffu);
-        if (k == src.WW - 1) v &= src.lastmask();
-        tmp.w[i] = v;
+        tmp.w[i] = line_h(src, y, k, L, true) & word_mask(src, k);
     }
     __syncthreads();
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         const int y = i / src.WW, k = i % src.WW;
-        unsigned v = 0;
-        for (int d = -a; d < L - a; ++d) v |= tmp.shifted(y, k, d, 0u);
-        if (k == src.WW - 1) v &= src.lastmask();
-        dst.w[i] = v;
+        dst.w[i] = line_h(tmp, y, k, L, false) & word_mask(src, k);
     }
     __syncthreads();
 }
@@ -138,18 +289,16 @@ __device__ void erode_dilate_v(const Img &src, Img &tmp, Img &dst, int L)
     const int a = L / 2;
     const int n = src.H * src.WW;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const int y = i / src.WW, k = i % src.WW;
+        const int y = i / src.WW;
         unsigned v = 0xffffffffu;
-        for (int d = -a; d < L - a; ++d) v &= src.get(y + d, k, 0xffffffffu);
-        if (k == src.WW - 1) v &= src.lastmask();
+        for (int r = max(y - a, 0); r < min(y + L - a, src.H); ++r) v &= src.w[i + (r - y) * src.WW];
         tmp.w[i] = v;
     }
     __syncthreads();
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const int y = i / src.WW, k = i % src.WW;
+        const int y = i / src.WW;
         unsigned v = 0;
-        for (int d = -a; d < L - a; ++d) v |= tmp.get(y + d, k, 0u);
-        if (k == src.WW - 1) v &= src.lastmask();
+        for (int r = max(y - a, 0); r < min(y + L - a, src.H); ++r) v |= tmp.w[i + (r - y) * src.WW];
         dst.w[i] = v;
     }
     __syncthreads();
@@ -177,127 +326,63 @@ __device__ void erode_dilate_eye(const Img &src, Img &tmp, Img &dst, int K)
     __syncthreads();
 }
 
-// Kogge-Stone fill of `g` through the set bits of `z` toward the MSB / LSB.
-__device__ __forceinline__ unsigned fill_up(unsigned g, unsigned z)
-{
-    g |= z & (g << 1); z &= z << 1;
-    g |= z & (g << 2); z &= z << 2;
-    g |= z & (g << 4); z &= z << 4;
-    g |= z & (g << 8); z &= z << 8;
-    g |= z & (g << 16);
-    return g;
-}
-__device__ __forceinline__ unsigned fill_down(unsigned g, unsigned z)
-{
-    g |= z & (g >> 1); z &= z >> 1;
-    g |= z & (g >> 2); z &= z >> 2;
-    g |= z & (g >> 4); z &= z >> 4;
-    g |= z & (g >> 8); z &= z >> 8;
-    g |= z & (g >> 16);
-    return g;
-}
-
-// imfill (morohutils.cu:73-83): F = B | (zeros of B that a 4-connected flood
-// from a zero frame around the image cannot reach).  R grows monotonically;
-// alternating full row and full column closures converge.
-__device__ void hole_fill(const Img &B, Img &Z, Img &R, Img &F, int *flag)
-{
-    const int H = B.H, WW = B.WW, n = H * WW;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const int y = i / WW, k = i % WW;
-        unsigned z = ~B.w[i];
-        if (k == WW - 1) z &= B.lastmask();
-        Z.w[i] = z;
-        unsigned r = 0;
-        if (y == 0 || y == H - 1) r = z;
-        if (k == 0) r |= z & 1u;
-        if (k == WW - 1) {
-            const int lb = (B.W - 1) & 31;
-            r |= z & (1u << lb);
-        }
-        R.w[i] = r;
-    }
-    __syncthreads();
-    for (int iter = 0;; ++iter) {
-        int changed = 0;
-        // rows: left-to-right then right-to-left closure with carries
-        for (int y = threadIdx.x; y < H; y += blockDim.x) {
-            unsigned carry = 0;
-            for (int k = 0; k < WW; ++k) {
-                const unsigned z = Z.w[y * WW + k], r0 = R.w[y * WW + k];
-                unsigned g = fill_up(r0 | (carry & z & 1u), z);
-                carry = g >> 31;
-                if (g != r0) { R.w[y * WW + k] = g; changed = 1; }
-            }
-            carry = 0;
-            for (int k = WW - 1; k >= 0; --k) {
-                const unsigned z = Z.w[y * WW + k], r0 = R.w[y * WW + k];
-                unsigned g = fill_down(r0 | ((carry << 31) & z & 0x80000000u), z);
-                carry = g & 1u;
-                if (g != r0) { R.w[y * WW + k] = g; changed = 1; }
-            }
-        }
-        __syncthreads();
-        // columns: top-down then bottom-up closure, 32 columns per thread
-        for (int k = threadIdx.x; k < WW; k += blockDim.x) {
-            unsigned prev = R.w[k];
-            for (int y = 1; y < H; ++y) {
-                const unsigned r0 = R.w[y * WW + k];
-                const unsigned g = r0 | (prev & Z.w[y * WW + k]);
-                if (g != r0) { R.w[y * WW + k] = g; changed = 1; }
-                prev = g;
-            }
-            prev = R.w[(H - 1) * WW + k];
-            for (int y = H - 2; y >= 0; --y) {
-                const unsigned r0 = R.w[y * WW + k];
-                const unsigned g = r0 | (prev & Z.w[y * WW + k]);
-                if (g != r0) { R.w[y * WW + k] = g; changed = 1; }
-                prev = g;
-            }
-        }
-        if (!__syncthreads_or(changed)) break;
-        if (iter > 4 * H * WW * 32) { if (threadIdx.x == 0) *flag = 1; break; }   // cannot happen
-    }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) F.w[i] = B.w[i] | (Z.w[i] & ~R.w[i]);
-    __syncthreads();
-}
-
 struct MorphArgs {
-    Img B;                    // raster ("rev" image: set where the matrix has entries)
-    Img F, O2, D, E;          // filled, open-open, subtracted, eye-opened
-    Img T1, T2, T3;           // scratch
+    Img B, F;                 // raster ("rev" image: set where the matrix has entries), filled
+    Img O2, D, E;             // open-open, subtracted, eye-opened
+    Img T1, T2;               // scratch
     int open_len, eye;
     int use_smem;
-    int *flag;
 };
 
 __global__ void __launch_bounds__(1024) morph_kernel(MorphArgs a)
 {
     extern __shared__ unsigned sm[];
     const int n = a.B.H * a.B.WW;
-    Img B = a.B, F = a.F, O2 = a.O2, D = a.D, E = a.E, T1 = a.T1, T2 = a.T2, T3 = a.T3;
+    Img F = a.F, O2 = a.O2, E = a.E, T1 = a.T1, T2 = a.T2;
     if (a.use_smem) {   // work on shared copies; results are written back
-        B.w = sm; T1.w = sm + n; T2.w = sm + 2 * n; T3.w = sm + 3 * n;
-        for (int i = threadIdx.x; i < n; i += blockDim.x) B.w[i] = a.B.w[i];
+        F.w = sm; T1.w = sm + n; T2.w = sm + 2 * n; O2.w = E.w = sm + 3 * n;
+        for (int i = threadIdx.x; i < n; i += blockDim.x) F.w[i] = a.F.w[i];
         __syncthreads();
     }
-    // F = imfill(B)                (T1 = zeros, T2 = reached)
-    Img Fw = a.use_smem ? T3 : F;
-    hole_fill(B, T1, T2, Fw, a.flag);
-    if (a.use_smem) for (int i = threadIdx.x; i < n; i += blockDim.x) F.w[i] = Fw.w[i];
-    // O1 = open 30x1 (F)  -> T1 ; O2 = open 1x30 (O1) -> T3
-    erode_dilate_h(Fw, T2, T1, a.open_len);
-    Img O2w = a.use_smem ? T3 : O2;
-    erode_dilate_v(T1, T2, O2w, a.open_len);
-    if (a.use_smem) for (int i = threadIdx.x; i < n; i += blockDim.x) O2.w[i] = O2w.w[i];
+    // O1 = open 30x1 (F) -> T1 ; O2 = open 1x30 (O1)
+    erode_dilate_h(F, T2, T1, a.open_len);
+    erode_dilate_v(T1, T2, O2, a.open_len);
     // D = B - O2 (saturating) -> T1
-    for (int i = threadIdx.x; i < n; i += blockDim.x) T1.w[i] = B.w[i] & ~O2w.w[i];
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const unsigned o = O2.w[i], d = a.B.w[i] & ~o;
+        if (a.use_smem) a.O2.w[i] = o;
+        T1.w[i] = d;
+        a.D.w[i] = d;
+    }
     __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) D.w[i] = T1.w[i];
     // E = open eye(5) (D)
-    Img Ew = a.use_smem ? T3 : E;
-    erode_dilate_eye(T1, T2, Ew, a.eye);
-    if (a.use_smem) for (int i = threadIdx.x; i < n; i += blockDim.x) E.w[i] = Ew.w[i];
+    erode_dilate_eye(T1, T2, E, a.eye);
+    if (a.use_smem) for (int i = threadIdx.x; i < n; i += blockDim.x) a.E.w[i] = E.w[i];
+}
+
+// Raster of the CSR to the five stage images in `a` (a.B .. a.E), with L
+// (H * W + 1 ints) and *flag as scratch of the hole filling; *flag stays 0
+// unless a union gave up.
+tc_status thumbnail_stages(const int *d_rowptr, const int *d_col, int M, int pM, int pN, MorphArgs &a, int *L,
+                           int *flag, cudaStream_t s)
+{
+    const int H = a.B.H, WW = a.B.WW, n = H * WW, T = 128;
+    raster_kernel<<<H, 512, sizeof(unsigned) * WW, s>>>(d_rowptr, d_col, M, pM, pN, a.B);
+    regions_init<false><<<(n + T - 1) / T, T, 0, s>>>(a.B, L);
+    regions_join<false><<<(n + T - 1) / T, T, 0, s>>>(a.B, L, flag);
+    fill_holes<<<(n + T - 1) / T, T, 0, s>>>(a.B, L, a.F);
+    TC_CUDA(cudaGetLastError());
+    const size_t smem = sizeof(unsigned) * (size_t)n * 4;
+    a.use_smem = smem <= 200 * 1024;
+    if (a.use_smem) {   // raise (never lower) the kernel's shared-memory limit
+        cudaFuncAttributes fa;
+        TC_CUDA(cudaFuncGetAttributes(&fa, morph_kernel));
+        if ((size_t)fa.maxDynamicSharedSizeBytes < smem)
+            TC_CUDA(cudaFuncSetAttribute(morph_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    }
+    morph_kernel<<<1, 1024, a.use_smem ? smem : 0, s>>>(a);
+    TC_CUDA(cudaGetLastError());
+    return TC_OK;
 }
 
 // Bytes (nonzero = set) -> bits, and bits -> 0/255 bytes.
@@ -323,171 +408,192 @@ __global__ void unpack_kernel(Img img, unsigned char *__restrict__ out)
 }
 
 // ----------------------------------------------------------------- contours
-// Labels: index 0 is the zero frame around the image, pixel (y,x) is 1+y*W+x.
-__device__ __forceinline__ int uf_find(int *L, int a)
-{
-    int b = __ldcg(L + a);
-    while (b != a) { a = b; b = __ldcg(L + a); }
-    return a;
-}
-
-__device__ void uf_union(int *L, int a, int b, int *flag)
-{
-    for (int it = 0; it < (1 << 24); ++it) {
-        a = uf_find(L, a);
-        b = uf_find(L, b);
-        if (a == b) return;
-        if (a < b) {
-            const int old = atomicMin(L + b, a);
-            if (old == b) return;
-            b = old;
-        } else {
-            const int old = atomicMin(L + a, b);
-            if (old == a) return;
-            a = old;
-        }
-    }
-    *flag = 2;   // no progress (cannot happen): reported, never waited on
-}
-
-__global__ void ccl_init(int *L, int n)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i <= n) L[i] = i;
-}
-
-// ones: 8-connected; zeros: 4-connected, and zeros on the image border join
-// the frame (OpenCV pads the image with a zero frame).
-__global__ void ccl_union(Img img, int *L, int *flag)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int W = img.W, H = img.H;
-    if (i >= H * W) return;
-    const int y = i / W, x = i % W, me = i + 1;
-    const int v = img.pix(y, x);
-    if (v) {
-        if (x > 0 && img.pix(y, x - 1)) uf_union(L, me, me - 1, flag);
-        if (y > 0) {
-            if (img.pix(y - 1, x)) uf_union(L, me, me - W, flag);
-            if (x > 0 && img.pix(y - 1, x - 1)) uf_union(L, me, me - W - 1, flag);
-            if (x + 1 < W && img.pix(y - 1, x + 1)) uf_union(L, me, me - W + 1, flag);
-        }
-    } else {
-        if (x > 0 && !img.pix(y, x - 1)) uf_union(L, me, me - 1, flag);
-        if (y > 0 && !img.pix(y - 1, x)) uf_union(L, me, me - W, flag);
-        if (x == 0 || y == 0 || x == W - 1 || y == H - 1) uf_union(L, me, 0, flag);
-    }
-}
-
-__global__ void ccl_flatten(int *L, int n)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i <= n) L[i] = uf_find(L, i);
-}
-
-// Border start flags: 1 = outer border (first pixel of a component of ones),
-// 2 = hole border (pixel left of the first pixel of an enclosed zero region).
-__global__ void border_starts(Img img, const int *L, int *flags, int *parent_pix)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int W = img.W;
-    if (i >= img.H * W) return;
-    const int y = i / W, x = i % W;
-    if (img.pix(y, x)) {
-        if (L[i + 1] == i + 1) flags[i] = 1;
-    } else if (L[i + 1] == i + 1 && x > 0) {
-        flags[i - 1] = 2;
-        parent_pix[i - 1] = L[i] - 1;        // first pixel of the enclosing ones
-    }
-}
-
 struct Border {
     int start;      // pixel index y*W+x
     int hole;       // 0 outer, 1 hole
     int parent;     // hole: start pixel of the enclosing outer border
     int len;        // points of the traced contour
     int mid;        // pixel index of point len/2
+    int unused;
     long long area2;   // twice the signed area of the contour polygon (shoelace sum)
 };
 
-__global__ void nonzero01(const int *__restrict__ f, int *__restrict__ o, int n)
+// Border starts of a word: the roots of ones (an outer border starts at a
+// region's first pixel) and of zeros that are not the frame's (a hole's
+// border starts at the pixel left of its first one).  Returns the word's
+// outer starts; *holes: the first pixels of its holes.
+__device__ __forceinline__ unsigned border_bits(const Img &img, int *L, int i, unsigned *holes)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) o[i] = f[i] != 0;
-    if (i == n) o[n] = 0;
+    const int y = i / img.WW, k = i % img.WW;
+    const unsigned in = word_mask(img, k), v = img.w[i] & in, z = ~v & in;
+    const int name = 1 + y * img.W + 32 * k;
+    unsigned o = 0, h = 0;
+    for (unsigned m = run_starts(v); m; m &= m - 1) {
+        const int p = __ffs(m) - 1;
+        if (__ldcg(L + name + p) == name + p) o |= 1u << p;
+    }
+    for (unsigned m = run_starts(z); m; m &= m - 1) {
+        const int p = __ffs(m) - 1;
+        if (__ldcg(L + name + p) == name + p) h |= 1u << p;
+    }
+    *holes = h;
+    return o;
 }
 
-__global__ void border_compact(const int *flags, const int *order, const int *parent_pix, int n,
-                               Border *out)
+__global__ void border_count(Img img, int *L, int *__restrict__ cnt)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, n = img.H * img.WW;
+    if (i == n) cnt[n] = 0;
+    if (i >= n) return;
+    unsigned h;
+    const unsigned o = border_bits(img, L, i, &h);
+    cnt[i] = __popc(o) + __popc(h);
+}
+
+// The borders in discovery order, which is the raster order of their starts.
+// (A hole's border starts one pixel before its first zero, but no other start
+// lies between the two: the pixel is a one that is not its region's first.)
+__global__ void border_write(Img img, int *L, const int *__restrict__ at, Border *__restrict__ out)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || !flags[i]) return;
-    Border b;
-    b.start = i;
-    b.hole = flags[i] == 2;
-    b.parent = b.hole ? parent_pix[i] : -1;
-    b.len = 0;
-    b.mid = i;
-    b.area2 = 0;
-    out[order[i]] = b;
+    if (i >= img.H * img.WW) return;
+    unsigned h;
+    const unsigned o = border_bits(img, L, i, &h);
+    const int y = i / img.WW, k = i % img.WW, first = y * img.W + 32 * k;
+    int slot = at[i];
+    for (unsigned m = o | h; m; m &= m - 1) {
+        const int p = __ffs(m) - 1;
+        Border b;
+        b.hole = h >> p & 1u;
+        b.start = first + p - b.hole;
+        b.parent = -1;
+        if (b.hole) {                                // the region of the one to its left
+            const int lk = p ? k : k - 1, lp = (p + 31) & 31;
+            b.parent = uf_find(L, 1 + y * img.W + 32 * lk + run_start(img.w[y * img.WW + lk], lp)) - 1;
+        }
+        b.len = 0;
+        b.mid = b.start;
+        b.unused = 0;
+        b.area2 = 0;
+        out[slot++] = b;
+    }
 }
 
 // Directions: 0 = +x, counter-clockwise on screen (y grows downward).
 __constant__ int c_dx[8] = {1, 1, 0, -1, -1, -1, 0, 1};
 __constant__ int c_dy[8] = {0, -1, -1, -1, 0, 1, 1, 1};
 
-// Follows one border (Suzuki & Abe steps 3.1-3.5).  With want < 0 returns the
-// number of points; otherwise returns the pixel index of point `want`.
-// area2 (optional, with want < 0): the shoelace sum over the closed polygon
-// of the points, sum of x_i y_{i+1} - x_{i+1} y_i (twice the signed area).
-__device__ long follow(const Img &img, int sy, int sx, int hole, long want, long cap, int *flag,
-                       long long *area2 = nullptr)
+// Three pixels (y, x - 1 .. x + 1): bits 0 .. 2.  From the image in global
+// memory, or from a copy in shared memory with a zero row above and below and
+// a zero word left and right.
+struct GlobalPixels {
+    Img img;
+    __device__ __forceinline__ unsigned three(int y, int x) const
+    {
+        const int k = (x - 1) >> 5;
+        return __funnelshift_r(img.get(y, k, 0u), img.get(y, k + 1, 0u), (x - 1) & 31) & 7u;
+    }
+};
+struct SharedPixels {
+    const unsigned *w;
+    int stride;
+    __device__ __forceinline__ unsigned three(int y, int x) const
+    {
+        const unsigned *r = w + (y + 1) * stride + ((x + 31) >> 5);
+        return __funnelshift_r(r[0], r[1], (x + 31) & 31) & 7u;
+    }
+};
+
+// A position on a border and the direction it was entered from (Suzuki & Abe
+// steps 3.1-3.5).
+struct Walk {
+    int y, x, s;
+    // bit d: the neighbour in direction d is set
+    template <class P>
+    static __device__ __forceinline__ unsigned around(const P &px, int y, int x)
+    {
+        const unsigned u = px.three(y - 1, x), m = px.three(y, x), d = px.three(y + 1, x);
+        return (m >> 2) | (u & 4u) >> 1 | (u & 2u) << 1 | (u & 1u) << 3 | (m & 1u) << 4 | d << 5;
+    }
+    // To the first set neighbour counter-clockwise after direction s (there
+    // is one: the pixel the walk came from).
+    template <class P>
+    __device__ __forceinline__ void step(const P &px)
+    {
+        const unsigned a = around(px, y, x);
+        const int from = (s + 1) & 7;
+        const unsigned turned = ((a | a << 8) >> from) & 0xffu;
+        const int k = turned ? (from + __ffs(turned) - 1) & 7 : s;
+        // dx = 1, 1, 0, -1, -1, -1, 0, 1 and dy = 0, -1, -1, -1, 0, 1, 1, 1, two bits each (value + 1)
+        x += (int)(0x901au >> (2 * k) & 3u) - 1;
+        y += (int)(0xa901u >> (2 * k) & 3u) - 1;
+        s = (k + 4) & 7;
+    }
+};
+
+// Follows one border: its length, middle point and polygon area.  A second
+// walk goes at half the pace, so that it stands on point len / 2 when the
+// first one is round.
+template <class P>
+__device__ void follow(const P &px, int W, long cap, Border &b, int *flag)
 {
-    const int W = img.W;
-    int s = hole ? 0 : 4;
-    const int s0 = s;
+    const int sy = b.start / W, sx = b.start % W;
+    const int s0 = b.hole ? 0 : 4;
+    const unsigned a = Walk::around(px, sy, sx);
+    int s = s0;
     bool found = false;
-    do {
+    for (int t = 0; t < 8 && !found; ++t) {          // clockwise from the outside pixel
         s = (s - 1) & 7;
-        if (img.pix(sy + c_dy[s], sx + c_dx[s])) { found = true; break; }
-    } while (s != s0);
-    if (!found) return want < 0 ? 1 : (long)sy * W + sx;
+        found = a >> s & 1u;
+    }
+    b.len = 1;
+    b.mid = b.start;
+    if (!found) return;                              // a single pixel
     const int ly = sy + c_dy[s], lx = sx + c_dx[s];
-    int cy = sy, cx = sx;
-    for (long n = 0; n < cap; ++n) {
-        if (n == want) return (long)cy * W + cx;
-        int k = s, ny, nx;
-        for (int t = 0; t < 8; ++t) {
-            ++k;
-            ny = cy + c_dy[k & 7];
-            nx = cx + c_dx[k & 7];
-            if (img.pix(ny, nx)) break;
+    Walk fast{sy, sx, s}, slow = fast;
+    long long area = 0;
+    for (long n = 1; n <= cap; ++n) {
+        const int cy = fast.y, cx = fast.x;
+        fast.step(px);
+        if (!(n & 1)) slow.step(px);
+        area += (long long)cx * fast.y - (long long)fast.x * cy;
+        if (fast.y == sy && fast.x == sx && cy == ly && cx == lx) {
+            b.len = (int)n;
+            b.mid = slow.y * W + slow.x;
+            b.area2 = area;
+            return;
         }
-        s = k & 7;
-        if (area2) *area2 += (long long)cx * ny - (long long)nx * cy;
-        if (ny == sy && nx == sx && cy == ly && cx == lx) return want < 0 ? n + 1 : -1;
-        cy = ny;
-        cx = nx;
-        s = (s + 4) & 7;
     }
     *flag = 3;   // longer than any border can be: reported
-    return want < 0 ? cap : -1;
 }
 
-__global__ void trace_kernel(Img img, Border *bs, int nb, int *flag)
+// One thread per border: bound by the longest border, each of whose steps
+// waits on the one before.  A step waits on the image alone (two or three words
+// of three rows), so the image is copied to shared memory when it fits
+// (`shared`): a 512 x 512 thumbnail takes 35 KB.  Two walks at once, from
+// shared memory, with the eight neighbours from three reads: 210 us where one
+// pixel test at a time and a second round for the middle took 787.
+constexpr int kTraceBlock = 256;
+
+__global__ void __launch_bounds__(kTraceBlock) trace_kernel(Img img, Border *__restrict__ bs,
+                                                            const int *__restrict__ count, int shared, int *flag)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nb) return;
-    Border b = bs[i];
-    const int y = b.start / img.W, x = b.start % img.W;
+    extern __shared__ unsigned sp[];
+    const int nb = *count;
+    if ((int)(blockIdx.x * blockDim.x) >= nb) return;
+    const int stride = img.WW + 3;                   // a word each side, and one more for the last pair
+    if (shared) {
+        const int n = stride * (img.H + 2);
+        for (int i = threadIdx.x; i < n; i += blockDim.x) sp[i] = img.get(i / stride - 1, i % stride - 1, 0u);
+        __syncthreads();
+    }
     const long cap = 8L * img.H * img.W + 16;
-    long long a2 = 0;
-    const long len = follow(img, y, x, b.hole, -1, cap, flag, &a2);
-    b.len = (int)len;
-    b.area2 = a2;
-    const long m = follow(img, y, x, b.hole, len / 2, cap, flag);
-    b.mid = m < 0 ? b.start : (int)m;
-    bs[i] = b;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nb; i += gridDim.x * blockDim.x) {
+        Border b = bs[i];
+        if (shared) follow(SharedPixels{sp, stride}, img.W, cap, b, flag);
+        else follow(GlobalPixels{img}, img.W, cap, b, flag);
+        bs[i] = b;
+    }
 }
 
 // ------------------------------------------------------------------ shapes
@@ -767,43 +873,44 @@ struct ContourList {
 
 static tc_status contours_on_device(const Img &img, cudaStream_t s, ContourList &out)
 {
-    const int n = img.H * img.W;
-    Scratch lab, flags, order, parent, tmp, bord, flag;
-    TC_CHECK(lab.alloc(sizeof(int) * ((size_t)n + 1), s));
-    TC_CHECK(flags.alloc(sizeof(int) * ((size_t)n + 1), s));
-    TC_CHECK(order.alloc(sizeof(int) * ((size_t)n + 1), s));
-    TC_CHECK(parent.alloc(sizeof(int) * ((size_t)n + 1), s));
+    const int n = img.H * img.WW, T = 128;
+    const long px = (long)img.H * img.W;
+    // no two border starts are neighbours in a row (an outer one and a hole's
+    // first pixel would share a corner with a one above)
+    const long most = (long)img.H * ((img.W + 1) / 2);
+    Scratch lab, cnt, tmp, bord, flag;
+    TC_CHECK(lab.alloc(sizeof(int) * ((size_t)px + 1), s));
+    TC_CHECK(cnt.alloc(sizeof(int) * 2 * ((size_t)n + 1), s));
     TC_CHECK(tmp.alloc(sizeof(int) * scan_tmp_ints(n), s));
+    TC_CHECK(bord.alloc(sizeof(Border) * (size_t)most, s));
     TC_CHECK(flag.alloc(sizeof(int), s));
-    TC_CUDA(cudaMemsetAsync(flags.p, 0, sizeof(int) * ((size_t)n + 1), s));
+    int *const L = lab.as<int>(), *const at = cnt.as<int>() + n + 1;
     TC_CUDA(cudaMemsetAsync(flag.p, 0, sizeof(int), s));
-    const int T = 256;
-    ccl_init<<<cdiv(n + 1, T), T, 0, s>>>(lab.as<int>(), n);
-    ccl_union<<<cdiv(n, T), T, 0, s>>>(img, lab.as<int>(), flag.as<int>());
-    ccl_flatten<<<cdiv(n + 1, T), T, 0, s>>>(lab.as<int>(), n);
-    border_starts<<<cdiv(n, T), T, 0, s>>>(img, lab.as<int>(), flags.as<int>(), parent.as<int>());
+    regions_init<true><<<cdiv(n, T), T, 0, s>>>(img, L);
+    regions_join<true><<<cdiv(n, T), T, 0, s>>>(img, L, flag.as<int>());
+    border_count<<<cdiv(n + 1, T), T, 0, s>>>(img, L, cnt.as<int>());
     TC_CUDA(cudaGetLastError());
-    // discovery order = raster order of the start pixels
-    {
-        Scratch ones;
-        TC_CHECK(ones.alloc(sizeof(int) * ((size_t)n + 1), s));
-        nonzero01<<<cdiv(n + 1, T), T, 0, s>>>(flags.as<int>(), ones.as<int>(), n);
-        TC_CUDA(cudaGetLastError());
-        TC_CHECK(exclusive_scan(ones.as<int>(), order.as<int>(), n, tmp.as<int>(), s));
-    }
-    int nb = 0;
-    TC_CUDA(cudaMemcpyAsync(&nb, order.as<int>() + n, sizeof(int), cudaMemcpyDeviceToHost, s));
-    TC_CUDA(cudaStreamSynchronize(s));
-    TC_CHECK(bord.alloc(sizeof(Border) * (size_t)std::max(nb, 1), s));
-    border_compact<<<cdiv(n, T), T, 0, s>>>(flags.as<int>(), order.as<int>(), parent.as<int>(), n,
-                                            bord.as<Border>());
-    trace_kernel<<<cdiv(std::max(nb, 1), 64), 64, 0, s>>>(img, bord.as<Border>(), nb, flag.as<int>());
+    TC_CHECK(exclusive_scan(cnt.as<int>(), at, n, tmp.as<int>(), s));
+    border_write<<<cdiv(n, T), T, 0, s>>>(img, L, at, bord.as<Border>());
+    const size_t smem = sizeof(unsigned) * (size_t)(img.WW + 3) * (img.H + 2);
+    const int shared = smem <= 200 * 1024;
+    if (shared) TC_CHECK(ensure_smem((const void *)trace_kernel, smem));
+    const int grid = (int)std::min<long>((most + kTraceBlock - 1) / kTraceBlock, num_sms());
+    trace_kernel<<<grid, kTraceBlock, shared ? smem : 0, s>>>(img, bord.as<Border>(), at + n, shared, flag.as<int>());
     TC_CUDA(cudaGetLastError());
-    std::vector<Border> hb(nb);
-    int hflag = 0;
-    if (nb) TC_CUDA(cudaMemcpyAsync(hb.data(), bord.p, sizeof(Border) * nb, cudaMemcpyDeviceToHost, s));
+    int nb = 0, hflag = 0;
+    std::vector<Border> hb((size_t)std::min(most, 2048L));   // usually all of them, in one round trip
+    TC_CUDA(cudaMemcpyAsync(&nb, at + n, sizeof(int), cudaMemcpyDeviceToHost, s));
     TC_CUDA(cudaMemcpyAsync(&hflag, flag.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    TC_CUDA(cudaMemcpyAsync(hb.data(), bord.p, sizeof(Border) * hb.size(), cudaMemcpyDeviceToHost, s));
     TC_CUDA(cudaStreamSynchronize(s));
+    const size_t have = hb.size();
+    hb.resize(nb);
+    if ((size_t)nb > have) {
+        TC_CUDA(cudaMemcpyAsync(hb.data() + have, bord.as<Border>() + have, sizeof(Border) * (nb - have),
+                                cudaMemcpyDeviceToHost, s));
+        TC_CUDA(cudaStreamSynchronize(s));
+    }
     if (hflag) return fail(TC_ERR_UNSUPPORTED, "contour labelling gave up (code %d)", hflag);
     // OpenCV order: outer borders newest first, each followed by its holes
     // newest first.  hb is in discovery order.
@@ -862,31 +969,24 @@ static tc_status getsdf_device(int M, int N, const int *d_rowptr, const int *d_c
     const int pN = N / W;
     const int WW = (W + 31) / 32;
     const size_t nw = (size_t)H * WW;
-    Scratch imgs, flag;
-    TC_CHECK(imgs.alloc(sizeof(unsigned) * nw * 8, s));
+    Scratch imgs, lab, flag;
+    TC_CHECK(imgs.alloc(sizeof(unsigned) * nw * 7, s));
+    TC_CHECK(lab.alloc(sizeof(int) * ((size_t)H * W + 1), s));
     TC_CHECK(flag.alloc(sizeof(int), s));
-    TC_CUDA(cudaMemsetAsync(imgs.p, 0, sizeof(unsigned) * nw * 8, s));
     TC_CUDA(cudaMemsetAsync(flag.p, 0, sizeof(int), s));
     auto img = [&](int k) { return Img{imgs.as<unsigned>() + k * nw, H, W, WW}; };
     MorphArgs a;
     a.B = img(0); a.F = img(1); a.O2 = img(2); a.D = img(3); a.E = img(4);
-    a.T1 = img(5); a.T2 = img(6); a.T3 = img(7);
+    a.T1 = img(5); a.T2 = img(6);
     a.open_len = p.open_len;
     a.eye = p.eye_size;
-    a.flag = flag.as<int>();
-    raster_kernel<<<H, 256, sizeof(unsigned) * WW, s>>>(d_rowptr, d_col, M, pM, pN, a.B);
-    TC_CUDA(cudaGetLastError());
-    const size_t smem = sizeof(unsigned) * nw * 4;
-    a.use_smem = smem <= 200 * 1024;
-    if (a.use_smem) TC_CHECK(ensure_smem((const void *)morph_kernel, smem));
-    morph_kernel<<<1, 1024, a.use_smem ? smem : 0, s>>>(a);
-    TC_CUDA(cudaGetLastError());
+    TC_CHECK(thumbnail_stages(d_rowptr, d_col, M, pM, pN, a, lab.as<int>(), flag.as<int>(), s));
     ContourList cl;
     TC_CHECK(contours_on_device(a.E, s, cl));
     int hflag = 0;
     TC_CUDA(cudaMemcpyAsync(&hflag, flag.p, sizeof(int), cudaMemcpyDeviceToHost, s));
     TC_CUDA(cudaStreamSynchronize(s));
-    if (hflag) return fail(TC_ERR_UNSUPPORTED, "hole fill did not converge");
+    if (hflag) return fail(TC_ERR_UNSUPPORTED, "hole fill gave up (code %d)", hflag);
     out.mF = H;
     out.W = W;
     out.ncontours = (int)cl.lens.size();
@@ -1369,30 +1469,23 @@ extern "C" tc_status tc_thumbnail_noalloc(int M, int N, const int *d_rowptr, con
     TC_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), s));
     tc::MorphArgs a;
     a.B = img(0); a.F = img(1); a.O2 = img(2); a.D = img(3); a.E = img(4);
-    a.T1 = img(5); a.T2 = img(6); a.T3 = img(7);
+    a.T1 = img(5); a.T2 = img(6);
     a.open_len = p.open_len;
     a.eye = p.eye_size;
-    a.flag = flag;
-    tc::raster_kernel<<<H, 256, sizeof(unsigned) * WW, s>>>(d_rowptr, d_col, M, pM, pN, a.B);
-    TC_CUDA(cudaGetLastError());
-    const size_t smem = sizeof(unsigned) * nw * 4;
-    a.use_smem = smem <= 200 * 1024;
-    if (a.use_smem) {   // raise (never lower) the kernel's shared-memory limit
-        cudaFuncAttributes fa;
-        TC_CUDA(cudaFuncGetAttributes(&fa, tc::morph_kernel));
-        if ((size_t)fa.maxDynamicSharedSizeBytes < smem)
-            TC_CUDA(cudaFuncSetAttribute(tc::morph_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    }
-    tc::morph_kernel<<<1, 1024, a.use_smem ? smem : 0, s>>>(a);
-    TC_CUDA(cudaGetLastError());
+    // the hole filling's H x W + 1 region names live in the output (5 H x W
+    // bytes, written last), from its first 4-byte boundary on; those of a tiny
+    // thumbnail, which would not fit there, behind the images
     const size_t px = (size_t)H * W;
+    int *const names = px < 16 ? reinterpret_cast<int *>(scratch + 7 * nw)
+                               : reinterpret_cast<int *>((reinterpret_cast<uintptr_t>(d_stages) + 3) & ~(uintptr_t)3);
+    TC_CHECK(tc::thumbnail_stages(d_rowptr, d_col, M, pM, pN, a, names, flag, s));
     for (int k = 0; k < 5; ++k)
         tc::unpack_kernel<<<tc::cdiv((long)px, 256), 256, 0, s>>>(img(k), d_stages + k * px);
     TC_CUDA(cudaGetLastError());
     int hflag = 0;
     TC_CUDA(cudaMemcpyAsync(&hflag, flag, sizeof(int), cudaMemcpyDeviceToHost, s));
     TC_CUDA(cudaStreamSynchronize(s));
-    if (hflag) return tc::fail(TC_ERR_UNSUPPORTED, "hole fill did not converge");
+    if (hflag) return tc::fail(TC_ERR_UNSUPPORTED, "hole fill gave up (code %d)", hflag);
     *W_out = W;
     return TC_OK;
 }
