@@ -168,7 +168,7 @@ typedef struct tc_plan_info {
 
 /* tc_plan_info.kernel */
 #define TC_KERNEL_TILES   0   /* persistent grid over staged tiles (tile_mode 0 / 1) */
-#define TC_KERNEL_GRID    1   /* one CTA per tile, every tile kind              */
+#define TC_KERNEL_GRID    1   /* (earlier builds: lane tiles, one CTA each)      */
 #define TC_KERNEL_LEAN    2   /* one CTA per tile: stream, direct and long tiles */
 #define TC_KERNEL_WIDE    3   /* wide direct tiles, one 1024-thread CTA each     */
 #define TC_KERNEL_STREAM  4   /* stream tiles only                              */

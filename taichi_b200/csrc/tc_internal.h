@@ -70,7 +70,8 @@ unsigned long long current_context_id();
 // TILE_L1..TILE_L32 give 1..32 lanes to each row; TILE_MERGE splits the
 // tile's rows and entries evenly over the threads; TILE_STREAM gathers every
 // entry's x term into shared memory with coalesced word loads, then sums each
-// row there; TILE_LONG gives one row a whole CTA.
+// row there (TILE_MIXED: rows of more than kStreamRowMax entries by a warp);
+// TILE_LONG gives one row a whole CTA.
 enum TileKind : int {
     TILE_L1 = 0, TILE_L2 = 1, TILE_L4 = 2, TILE_L8 = 3, TILE_L16 = 4, TILE_L32 = 5,
     TILE_LONG = 6,
@@ -79,7 +80,8 @@ enum TileKind : int {
     TILE_STREAM4 = 9,  // the same with 4 consecutive rows per thread (row0 % 4 == 0)
     TILE_DIRECT4 = 10,    // 4 consecutive rows per thread straight from global memory
     TILE_DIRECT_WIDE = 11, // the same over up to 4096 rows (a 1024-thread CTA)
-    TILE_WINDOW = 12      // rows summed from a staged x window (the window kernel's tiles)
+    TILE_WINDOW = 12,     // rows summed from a staged x window (the window kernel's tiles)
+    TILE_MIXED = 13       // a stream tile with rows of more than kStreamRowMax entries (a warp each)
 };
 
 struct Tile {          // 16 bytes, read once per CTA
@@ -107,7 +109,7 @@ constexpr int kMaxTileRows = 1 << 20; // planner limit on rows per tile
 constexpr int kStageNnz = 8192;       // CSR words of a tile staged in shared memory
 constexpr int kStreamNnz = 4096;      // most entries of a TILE_STREAM tile
 constexpr int kStreamRows = 256;      // most rows of a TILE_STREAM tile (1 per thread)
-constexpr int kStreamRowMax = 128;    // longer rows leave stream tiles for lane tiles
+constexpr int kStreamRowMax = 128;    // longer rows of a stream tile are summed by a warp (TILE_MIXED)
 constexpr int kStream4Rows = 1024;    // most rows of a TILE_STREAM4 tile (a run of 4 per thread)
 constexpr int kDirectRows = 1024;     // most rows of a direct tile (TILE_DIRECT4)
 constexpr int kDirectWideBlock = 1024; // threads of the direct kernel's CTAs
@@ -159,8 +161,7 @@ struct DevPlan {
     int pdl;                // launch with programmatic stream serialization
     int stage_rp, stage_cw; // ints per shared-memory stage (row pointers, CSR words)
     int grid;               // persistent grid size
-    int per_tile;           // one CTA per tile (stream plans): 1, or 2 when only stream,
-                            // direct and long tiles occur (the lean kernel), 3 when
+    int per_tile;           // one CTA per tile (stream plans): 2 (the lean kernel), 3 when
                             // every tile is a wide direct tile (the direct kernel), or 4
                             // when every tile is a stream tile (the stream kernel)
     int *err;               // device error word (1: a bounded wait gave up)
@@ -211,7 +212,6 @@ struct tc_plan {
     int4 *d_shapes = nullptr;
     int2 *d_shape_dias = nullptr;
     int ntiles = 0, ntiles_vector = 0, ntiles_long = 0;
-    int ntiles_lanes = 0;                // lane and merge tiles (TILE_L1..L32, TILE_MERGE)
     int ntiles_wide = 0;                 // TILE_DIRECT_WIDE tiles (all or none)
     int ntiles_stream = 0;               // TILE_STREAM tiles
     int max_span = 0;

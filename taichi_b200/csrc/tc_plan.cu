@@ -74,7 +74,7 @@ struct TilePrm {
 
 // What the tiles of a plan come to, summed over its strips.
 struct TileCounts {
-    int vector, lng, lanes, stream, max_rows, max_nnz;   // max_*: tiles staged in shared memory
+    int vector, lng, stream, max_rows, max_nnz;   // max_*: tiles staged in shared memory
 };
 
 // Lanes per row from the mean row length of a run of rows: one lane per row
@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(32) plan_strips(const int *__restrict__ rowptr
     const int n = (int)min((long)kStripRows, (long)M - row0), lane = threadIdx.x;
     for (int i = lane; i <= n; i += 32) rp[i] = __ldg(rowptr + row0 + i);
     __syncwarp();
-    TileCounts c{0, 0, 0, 0, 1, 0};
+    TileCounts c{0, 0, 0, 1, 0};
     int made = 0;
     Tile *const out = WRITE ? tiles + first[blockIdx.x] : nullptr;
     auto len = [&](int r) { return rp[r + 1] - rp[r]; };
@@ -124,7 +124,6 @@ __global__ void __launch_bounds__(32) plan_strips(const int *__restrict__ rowptr
         c.stream += kind == TILE_STREAM;
         c.lng += kind == TILE_LONG;
         if (kind <= TILE_L32 || kind == TILE_MERGE) {
-            ++c.lanes;
             c.max_rows = max(c.max_rows, rows);
             c.max_nnz = max(c.max_nnz, nz);
         }
@@ -135,39 +134,40 @@ __global__ void __launch_bounds__(32) plan_strips(const int *__restrict__ rowptr
             ++r;
             continue;
         }
-        if (q.mode == 2 && len(r) <= kStreamRowMax) {
-            // stream tile: short rows up to the row and entry caps.  A run
-            // that starts on a multiple of 4 rows and holds many rows runs 4
+        if (q.mode == 2) {
+            // stream tile: rows up to the row and entry caps.  A run that
+            // starts on a multiple of 4 rows and holds many rows runs 4
             // consecutive rows per thread: read directly from global memory
             // when they average at most one entry (TILE_DIRECT4), through
             // shared memory when at most two (TILE_STREAM4); otherwise one
-            // row per thread (TILE_STREAM)
+            // row per thread (TILE_STREAM; TILE_MIXED when it holds a row of
+            // more than kStreamRowMax entries)
             const bool a4 = (r & 3) == 0 && !q.strided;
             const int cap_rows = min(q.rows_cap, a4 ? kDirectRows : kStreamRows);
             const int cap_nnz = max(1, min(2 * min(q.tile_nnz, 1 << 24), q.spread));
             int m = run_of(min(cap_rows, n - r), [&](int i) {
-                return len(r + i) <= kStreamRowMax && rp[r + i + 1] - rp[r] <= cap_nnz;
+                return len(r + i) <= q.long_len && rp[r + i + 1] - rp[r] <= cap_nnz;
             });
-            if (m == 0) m = 1;        // a single row longer than cap_nnz but <= kStreamRowMax
+            if (m == 0) m = 1;        // a single row longer than cap_nnz
+            const int small = run_of(m, [&](int i) { return len(r + i) <= kStreamRowMax; });
+            if (small >= 2 * kBlock) m = small;       // direct and four-row tiles hold short rows only
             const int ent = rp[r + m] - rp[r];
-            const bool direct = a4 && m >= 2 * kBlock && ent <= m && !q.no_direct;
-            const bool four = !direct && a4 && m >= 2 * kBlock && ent <= 2 * m;
+            const bool direct = a4 && small >= 2 * kBlock && ent <= m && !q.no_direct;
+            const bool four = !direct && a4 && small >= 2 * kBlock && ent <= 2 * m;
             if (!direct) m = min(m, four ? kStream4Rows : kStreamRows);
             if (r + m < n) {          // end on a multiple of 256 rows (whole row sweeps), else of 4
                 const int cut = (r + m) & ~255;
                 if (cut - r >= 256) m = cut - r;
                 else if (m > 4) m -= (r + m) & 3;
             }
-            put(r, m, direct ? TILE_DIRECT4 : four ? TILE_STREAM4 : TILE_STREAM);
+            put(r, m, direct ? TILE_DIRECT4 : four ? TILE_STREAM4 : small < m ? TILE_MIXED : TILE_STREAM);
             r += m;
             continue;
         }
         // candidate run: up to 1024 rows (merge tiles: tile_rows), stopping
-        // before a long row (stream mode: before a short row too)
+        // before a long row
         const int run_cap = q.mode == 0 ? min(q.rows_cap, kStripRows) : 1024;
-        const int m = run_of(min(run_cap, n - r), [&](int i) {
-            return len(r + i) <= q.long_len && !(q.mode == 2 && len(r + i) <= kStreamRowMax);
-        });
+        const int m = run_of(min(run_cap, n - r), [&](int i) { return len(r + i) <= q.long_len; });
         if (q.mode == 0) {            // merge tile: rows + entries split evenly
             int rows = m;
             while (rows > 1 && rp[r + rows] - rp[r] > kStageNnz) rows = (rows + 1) / 2;
@@ -187,7 +187,6 @@ __global__ void __launch_bounds__(32) plan_strips(const int *__restrict__ rowptr
     count[blockIdx.x] = made;
     if (c.vector) atomicAdd(&sum->vector, c.vector);
     if (c.lng) atomicAdd(&sum->lng, c.lng);
-    if (c.lanes) atomicAdd(&sum->lanes, c.lanes);
     if (c.stream) atomicAdd(&sum->stream, c.stream);
     atomicMax(&sum->max_rows, c.max_rows);
     atomicMax(&sum->max_nnz, c.max_nnz);
@@ -337,7 +336,7 @@ tc_status plan_upload(tc_plan *p, const int *csrRow, const int *csrCol, int64_t 
     q.mode = prm.tile_mode;
     q.rows_cap = std::max(1, std::min(prm.tile_rows, kMaxTileRows));
     q.tile_nnz = prm.tile_nnz;
-    q.long_len = std::max(1, std::min(prm.tile_nnz, kStageNnz));
+    q.long_len = std::max(1, std::min(prm.tile_nnz, q.mode == 2 ? kStreamNnz : kStageNnz));
     // stream tiles hold at most nnz_csr / min_tiles entries (not below 512),
     // so a small matrix still spreads over the GPU
     q.spread = (int)std::min<int64_t>(kStreamNnz, std::max<int64_t>(512, nnz_csr / std::max(1, min_tiles)));
@@ -368,7 +367,6 @@ tc_status plan_upload(tc_plan *p, const int *csrRow, const int *csrCol, int64_t 
     p->ntiles_wide = wide ? p->ntiles : 0;
     p->ntiles_vector = wide ? 0 : sum.vector;
     p->ntiles_long = wide ? 0 : sum.lng;
-    p->ntiles_lanes = wide ? 0 : sum.lanes;
     p->ntiles_stream = wide ? 0 : sum.stream;
     // shared-memory stage sizes (ints, multiples of 4) from the largest tile
     p->stage_rp = (std::max(1, wide ? 1 : sum.max_rows) + 1 + 8 + 3) & ~3;

@@ -269,22 +269,17 @@ __global__ void __launch_bounds__(kBlock, kRowsMinBlocks)
     if (r < p.M) y[r] = acc;
 }
 
-// The multiply of a stream plan: one CTA per tile, no shared-memory stages
-// (stream tiles read their CSR words as coalesced int4s; lane and long tiles
-// read global memory directly).  LEAN: the plan holds only stream and long
-// tiles, so the kernel carries no lane-tile code and fits more CTAs per SM.
-template <bool SIGNED, bool LEAN>
-__global__ void __launch_bounds__(kBlock, LEAN ? (SIGNED ? kLeanMinBlocksSigned : kLeanMinBlocks) : 1)
+// The multiply of a stream plan (any of its tile kinds): one CTA per tile, no
+// shared-memory stages (stream tiles read their CSR words as coalesced int4s;
+// direct and long tiles read global memory directly).
+template <bool SIGNED>
+__global__ void __launch_bounds__(kBlock, SIGNED ? kLeanMinBlocksSigned : kLeanMinBlocks)
     spmv_grid_kernel(DevPlan p, const float *__restrict__ x, float *__restrict__ y)
 {
     allow_next_grid();
     const Tile t = p.tiles[blockIdx.x];
     if (threadIdx.x == 0) prefetch_x_window(x, p.N, t.row0, tile_nrows(t));
-    if (LEAN) {
-        run_lean_tile<SIGNED>(p, t, x, y, true);
-    } else {
-        run_tile<SIGNED>(p, t, x, y, true);
-    }
+    run_lean_tile<SIGNED>(p, t, x, y, true);
 }
 
 // The whole-tile wide kernel with the tiles' word bounds in the launch
@@ -405,8 +400,7 @@ static tc_status launch_tiles(const DevPlan &dp, const WideBounds *wb, const Wid
     else if (dp.per_tile == 4 && dp.ntiles > kLeanMinBlocks * num_sms())
         TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_stream_kernel<SIGNED, true>, dp, x, y));
     else if (dp.per_tile == 4) TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_stream_kernel<SIGNED, false>, dp, x, y));
-    else if (dp.per_tile == 2) TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_grid_kernel<SIGNED, true>, dp, x, y));
-    else if (dp.per_tile) TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_grid_kernel<SIGNED, false>, dp, x, y));
+    else if (dp.per_tile) TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_grid_kernel<SIGNED>, dp, x, y));
     else TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_tiles_kernel<SIGNED>, dp, x, y));
     return TC_OK;
 }
@@ -466,8 +460,7 @@ tc::DevPlan tc_plan::dev_plan() const
     d.per_tile = params.tile_mode != 2 ? 0
                : ntiles == 0 ? 2
                : ntiles_wide == ntiles ? 3
-               : ntiles_stream == ntiles ? 4
-               : ntiles_lanes == 0 ? 2 : 1;
+               : ntiles_stream == ntiles ? 4 : 2;
     d.err = d_err;
     d.wide_rows = wide_rows;
     d.skew = stream_skew;

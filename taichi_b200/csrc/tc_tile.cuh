@@ -430,7 +430,8 @@ __device__ void tile_merge(const DevPlan &p, const Tile &t, const Src &src,
 // gathers stay inside x and their slots are never read.  Then each row's
 // dense-diagonal terms (offset order) and entries (stored order) are added
 // by one thread: the order of tile_rows_seq, so a matrix gets the same y from
-// every one-lane tile kind.  TILE_STREAM strides single rows over the CTA;
+// every one-lane tile kind; in a TILE_MIXED tile a row of more than
+// kStreamRowMax entries is left to its warp.  TILE_STREAM strides single rows over the CTA;
 // TILE_STREAM4 gives each thread runs of 4 consecutive rows (int4
 // row-pointer loads, float4 y stores) for tiles of many short rows.  The
 // first round's CSR words and the row pointers are immutable plan data, read
@@ -548,40 +549,61 @@ __device__ __forceinline__ float diag_tile_row(const DevPlan &p, const float *__
     return acc;
 }
 
-template <bool SIGNED>
+// The dense-diagonal terms of row r that lane `lane` of a warp owns (offsets
+// lane, lane + 32, ... of each shape holding the row).
+__device__ __forceinline__ float diag_lane(const DevPlan &p, const float *__restrict__ x, int r, int lane)
+{
+    float acc = 0.f;
+    if (r < p.row_start || r >= p.row_stop) return acc;
+    for (int s = 0; s < p.dia_shapes; ++s) {
+        const int4 sh = __ldg(p.shapes + s);
+        if (r < sh.x || r >= sh.y) continue;
+        const int2 dr = __ldg(p.shape_dias + s);
+        for (int d = dr.x + lane; d < dr.y; d += 32) {
+            const int c = r - sh.x + sh.z + __ldg(p.offsets + d);
+            if (c >= sh.z && c < sh.z + sh.w) acc += ldx(x + c);
+        }
+    }
+    return acc;
+}
+
+template <bool SIGNED, bool MIXED = false>
 __device__ void tile_stream(const DevPlan &p, const Tile &t, const float *__restrict__ x,
                             float *__restrict__ y, bool wait)
 {
     float *const vals = tile_smem().vals;
-    constexpr int RQ = kStreamRows / kBlock;
-    const int tid = threadIdx.x, nr = tile_nrows(t), row0 = t.row0, dc = tile_dclass(t);
+    static_assert(kStreamRows == kBlock, "one row per thread");
+    const int rl = threadIdx.x, nr = tile_nrows(t), row0 = t.row0, dc = tile_dclass(t);
     StreamWords sw;
     stream_words_first(p, t, sw);
     const int base = t.nz0 - sw.lead;                           // rowptr value of vals[0]
-    int rb[RQ], re[RQ];
-#pragma unroll
-    for (int k = 0; k < RQ; ++k) {
-        const int rl = tid + k * kBlock;
-        const bool ok = rl < nr;
-        rb[k] = ok ? __ldg(p.rowptr + row0 + rl) - base : 0;
-        re[k] = ok ? __ldg(p.rowptr + row0 + rl + 1) - base : 0;
-    }
+    const int b = rl < nr ? __ldg(p.rowptr + row0 + rl) - base : 0;
+    const int e = rl < nr ? __ldg(p.rowptr + row0 + rl + 1) - base : 0;
     if (wait) wait_prior_grid(x, y);
     stream_gather<SIGNED>(x, vals, sw, p.skew);
     // (Loading the rows' diagonal terms while the gathers are in flight
     // measured slower on the mesh: into registers 69.5 against 65.6 us; as
     // the tile's x segment staged in shared memory 58.3 against 52.5 us.)
-#pragma unroll
-    for (int k = 0; k < RQ; ++k) {
-        const int rl = tid + k * kBlock;
-        if (rl < nr) {
-            float acc = diag_tile_row(p, x, dc, row0 + rl);
-            if (p.skew) {
-                for (int j = rb[k]; j < re[k]; ++j) acc += vals[vslot(j)];
-            } else {
-                for (int j = rb[k]; j < re[k]; ++j) acc += vals[j];
-            }
-            y[row0 + rl] = acc;
+    if (rl < nr && (!MIXED || e - b <= kStreamRowMax)) {
+        float acc = diag_tile_row(p, x, dc, row0 + rl);
+        if (p.skew) {
+            for (int j = b; j < e; ++j) acc += vals[vslot(j)];
+        } else {
+            for (int j = b; j < e; ++j) acc += vals[j];
+        }
+        y[row0 + rl] = acc;
+    }
+    if (MIXED) {
+        const int lane = threadIdx.x & 31;
+        for (unsigned m = __ballot_sync(0xffffffffu, e - b > kStreamRowMax); m; m &= m - 1) {
+            const int src = __ffs(m) - 1;
+            const int lb = __shfl_sync(0xffffffffu, b, src), le = __shfl_sync(0xffffffffu, e, src);
+            const int r = row0 + (rl & ~31) + src;
+            float acc = SIGNED ? diag_lane(p, x, r, lane) : 0.f;
+#pragma unroll 4
+            for (int j = lb + lane; j < le; j += 32) acc += vals[p.skew ? vslot(j) : j];
+            acc = warp_sum(acc);
+            if (lane == 0) y[r] = acc;
         }
     }
     __syncthreads();                                            // vals is reused by the next tile
@@ -907,6 +929,7 @@ __device__ __forceinline__ void run_tile_src(const DevPlan &p, const Tile &t, co
     switch (tile_kind(t)) {
     case TILE_MERGE: tile_merge<SIGNED>(p, t, src, x, y, wait); break;
     case TILE_STREAM: tile_stream<SIGNED>(p, t, x, y, wait); break;
+    case TILE_MIXED: tile_stream<SIGNED, true>(p, t, x, y, wait); break;
     case TILE_STREAM4: tile_stream4<SIGNED>(p, t, x, y, wait); break;
     case TILE_DIRECT4:
     case TILE_DIRECT_WIDE: tile_direct<SIGNED>(p, t, x, y, wait); break;
@@ -929,6 +952,7 @@ __device__ __forceinline__ void run_lean_tile(const DevPlan &p, const Tile &t, c
     switch (tile_kind(t)) {
     case TILE_STREAM4: tile_stream4<SIGNED>(p, t, x, y, wait); break;
     case TILE_STREAM: tile_stream<SIGNED>(p, t, x, y, wait); break;
+    case TILE_MIXED: tile_stream<SIGNED, true>(p, t, x, y, wait); break;
     case TILE_DIRECT4:
     case TILE_DIRECT_WIDE: tile_direct<SIGNED>(p, t, x, y, wait); break;
     default: long_row<SIGNED>(p, t, x, y, wait); break;
