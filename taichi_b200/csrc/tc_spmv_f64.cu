@@ -3,101 +3,244 @@
 // TaiChi.h:62-64, which turns x, y and the kernels' accumulators into double;
 // the pattern and the hybrid format are unchanged).
 //
-// One 256-thread CTA per tile of the plan's own tile list.  Tiles of short
-// rows (stream, direct and one-lane kinds) give each thread whole rows; the
-// other kinds (lane, merge tiles) give each warp a row at a time, its lanes
-// striding the row's offsets and words, combined by a butterfly; a long row
-// (TILE_LONG) gets the whole CTA.  A row adds its dense-diagonal terms in
-// offset order, then its CSR words in stored order (signed words of a hybrid
-// plan subtract the holes).  The kernel is launched without programmatic
-// dependent launch, so x and y follow plain stream order.
+// A row belongs to a group of 2^lg lanes: its dense-diagonal terms in offset
+// order, then its CSR words in stored order, each dealt out to the lanes in
+// turn, three or four words of a lane in flight together, joined by a
+// butterfly.  Plans of short rows run kBlock >> lg consecutive rows a CTA
+// straight from the row pointers; plans with rows of more than kShortRow words
+// run a CTA per tile of the plan's list (whose words are bounded), leaving a
+// row that is long for its tile to a warp and a one-row tile to the whole CTA.  The launch may overlap the end of
+// the kernel before it, as in FP32: x is read and y written after
+// griddepcontrol.wait only, with coherent loads.
+//
+// What bounds it: bytes (8 per x and y value), and the latency of row pointer
+// -> word -> x.  Rows of a few words strided over a tile's CTA, one dependent
+// word and gather after the other, which this replaces, ran at 35 % of the
+// copy rate.  Measured per multiply (us, before -> now):
+//   9-point mesh 1531^2 (hybrid, 6 words a row)      45.1 -> 30.0
+//   banded 700,001 x 32                             107.5 -> 35.9
+//   banded 65,536 x 18                                8.3 -> 5.8
+//   R-MAT scale 20 (0.6 words a row)                 22.9 -> 7.1
+//   15 diagonals of 900,000 rows with holes          31.5 -> 17.2
+//   power-law R-MAT scale 20 / 18 / 16          82 / 30 / 17 -> 73 / 23 / 12
 
 #include <cuda_runtime.h>
 
 #include "tc_internal.h"
+#include "tc_tile.cuh"
 
 namespace tc {
 namespace {
 
-constexpr int kF64Block = 256;
+constexpr int kF64Blocks = 8;     // resident CTAs per SM
+constexpr int kShortRow = 128;    // plans with longer rows go by tiles
+constexpr int kLaneWords = 8;     // in a tile: words of a lane on average, at most,
+constexpr int kLaneMost = 32;     // and words of a lane past which its row is left to the warp
+constexpr int kLongTile = 1024;   // a one-row tile of more words by the whole CTA
+constexpr int kAheadWords = 1 << 14;   // most words of a later CTA prefetched into L2
 
-template <bool SIGNED>
-__device__ __forceinline__ double gather64(const double *__restrict__ x, int c)
+__device__ __forceinline__ double ldx64(const double *p)
 {
-    if (SIGNED) {
-        const double v = x[c >> 1];
-        return (c & 1) ? v : -v;
-    }
-    return x[c];
+    double v;
+    asm("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+
+__device__ __forceinline__ void wait_prior64(const double *__restrict__ &x, double *__restrict__ &y)
+{
+    asm volatile("griddepcontrol.wait;" : "+l"(x), "+l"(y)::"memory");
+}
+
+// Words j, j + by, ... (W of them, before e), and their terms added to acc.
+template <int W>
+__device__ __forceinline__ void load_words(const DevPlan &p, int j, int e, int by, int (&c)[W])
+{
+#pragma unroll
+    for (int w = 0; w < W; ++w) c[w] = j + w * by < e ? __ldg(p.cols + j + w * by) : 0;
+}
+
+template <bool SIGNED, int W>
+__device__ __forceinline__ void add_words(const double *__restrict__ x, int j, int e, int by, const int (&c)[W],
+                                          double &acc)
+{
+    double v[W];                  // a slot past the row loads x[0] and is not added
+#pragma unroll
+    for (int w = 0; w < W; ++w) v[w] = ldx64(x + (SIGNED ? c[w] >> 1 : c[w]));
+#pragma unroll
+    for (int w = 0; w < W; ++w)
+        if (j + w * by < e) acc += SIGNED && !(c[w] & 1) ? -v[w] : v[w];
 }
 
 // The dense-diagonal terms of row r that lane `lane` of `lanes` owns
 // (offsets lane, lane + lanes, ... of each shape holding the row).
-__device__ double diag_terms64(const DevPlan &p, const double *__restrict__ x, int r, int lane, int lanes)
+__device__ __forceinline__ double diag_terms64(const DevPlan &p, const double *__restrict__ x, int r, int lane,
+                                               int lanes)
 {
     double acc = 0.0;
-    if (r < p.row_start || r >= p.row_stop) return acc;
+    if (p.dn > 0) {               // one shape of few offsets: from the launch parameters
+#pragma unroll
+        for (int i = 0; i < kPlanDiags; i += 4) {
+            if (i >= p.dn) break;
+            double d[4];
+            bool in[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                in[u] = i + u < p.dn && r >= p.d_lo[i + u] && r < p.d_hi[i + u] && ((i + u) & (lanes - 1)) == lane;
+                d[u] = ldx64(x + (in[u] ? r + p.d_col[i + u] : 0));
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (in[u]) acc += d[u];
+        }
+        return acc;
+    }
+    if (!p.dgen || r < p.row_start || r >= p.row_stop) return acc;
     for (int s = 0; s < p.dia_shapes; ++s) {
-        const int4 sh = p.shapes[s];
+        const int4 sh = __ldg(p.shapes + s);
         if (r < sh.x || r >= sh.y) continue;
-        const int2 dr = p.shape_dias[s];
+        const int2 dr = __ldg(p.shape_dias + s);
         const int cb = r - sh.x + sh.z;
-        for (int d = dr.x + lane; d < dr.y; d += lanes) {
-            const int c = cb + p.offsets[d];
-            if (c >= sh.z && c < sh.z + sh.w) acc += x[c];
+        for (int d = dr.x + lane; d < dr.y; d += 4 * lanes) {
+            double v[4];
+            bool in[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int c = d + u * lanes < dr.y ? cb + __ldg(p.offsets + d + u * lanes) : -1;
+                in[u] = c >= sh.z && c < sh.z + sh.w;
+                v[u] = ldx64(x + (in[u] ? c : 0));
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (in[u]) acc += v[u];
         }
     }
     return acc;
 }
 
-__device__ __forceinline__ double warp_sum64(double v)
+// Sum over the aligned group of `lanes` lanes (a power of two).
+__device__ __forceinline__ double group_sum(double v, int lanes)
 {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    for (int o = lanes >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
 
-template <bool SIGNED>
-__global__ void __launch_bounds__(kF64Block) spmv_f64_kernel(DevPlan p, const double *__restrict__ x,
-                                                            double *__restrict__ y)
+// Short rows: kBlock >> LG rows a CTA.
+template <bool SIGNED, int LG>
+__global__ void __launch_bounds__(kBlock, kF64Blocks)
+    f64_rows_kernel(DevPlan p, int ahead, const double *__restrict__ x, double *__restrict__ y)
 {
-    __shared__ double red[kF64Block / 32];
+    constexpr int G = 1 << LG, R = kBlock >> LG, W = LG ? 4 : 3;
+    allow_next_grid();
+    const int row0 = blockIdx.x * R, group = threadIdx.x >> LG, lane = threadIdx.x & (G - 1);
+    const bool ok = group < p.M - row0;
+    const int r = row0 + group;
+    if (threadIdx.x == 0 && (long)row0 + (long)ahead * R < p.M) {
+        const int ra = row0 + ahead * R, rb = ra + min(R, p.M - ra);
+        const int za = __ldg(p.rowptr + ra), zb = __ldg(p.rowptr + rb);
+        prefetch_rows_ahead(p, ra, rb, za, min(zb, za + kAheadWords));
+    }
+    const int b = ok ? __ldg(p.rowptr + r) + lane : 0, e = ok ? __ldg(p.rowptr + r + 1) : 0;
+    int c[W];
+    load_words(p, b, e, G, c);
+    wait_prior64(x, y);
+    double acc = SIGNED && ok ? diag_terms64(p, x, r, lane, G) : 0.0;
+    add_words<SIGNED>(x, b, e, G, c, acc);
+    for (int j = b + W * G; j < e; j += W * G) {
+        load_words(p, j, e, G, c);
+        add_words<SIGNED>(x, j, e, G, c, acc);
+    }
+    acc = group_sum(acc, G);
+    if (ok && lane == 0) y[r] = acc;
+}
+
+// A lane's share of the words [b, e): every by-th from b on.
+template <bool SIGNED>
+__device__ __forceinline__ void sum_words64(const DevPlan &p, const double *__restrict__ x, int b, int e, int by,
+                                            double &acc)
+{
+    for (int j = b; j < e; j += 4 * by) {
+        int c[4];
+        load_words(p, j, e, by, c);
+        add_words<SIGNED>(x, j, e, by, c, acc);
+    }
+}
+
+// Any plan: a CTA per tile.
+template <bool SIGNED>
+__global__ void __launch_bounds__(kBlock, kF64Blocks)
+    f64_tiles_kernel(DevPlan p, const double *__restrict__ x, double *__restrict__ y)
+{
+    __shared__ double red[kBlock / 32];
+    allow_next_grid();
     const Tile t = p.tiles[blockIdx.x];
-    const int nr = tile_nrows(t), kind = tile_kind(t);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (kind == TILE_LONG) {
-        const int r = t.row0;
-        double acc = diag_terms64(p, x, r, threadIdx.x, kF64Block);
-        for (int j = p.rowptr[r] + threadIdx.x; j < p.rowptr[r + 1]; j += kF64Block)
-            acc += gather64<SIGNED>(x, p.cols[j]);
-        acc = warp_sum64(acc);
+    const int nr = tile_nrows(t), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    wait_prior64(x, y);
+    if (nr == 1 && t.nnz > kLongTile) {
+        double acc = SIGNED ? diag_terms64(p, x, t.row0, threadIdx.x, kBlock) : 0.0;
+        sum_words64<SIGNED>(p, x, t.nz0 + threadIdx.x, t.nz0 + t.nnz, kBlock, acc);
+        acc = group_sum(acc, 32);
         if (lane == 0) red[warp] = acc;
         __syncthreads();
-        if (warp == 0) {
-            double v = lane < kF64Block / 32 ? red[lane] : 0.0;
-            v = warp_sum64(v);
-            if (lane == 0) y[r] = v;
+        if (threadIdx.x == 0) {
+            for (int i = 1; i < kBlock / 32; ++i) acc += red[i];
+            y[t.row0] = acc;
         }
         return;
     }
-    const bool thread_rows = kind == TILE_L1 || kind == TILE_STREAM || kind == TILE_STREAM4 ||
-                             kind == TILE_DIRECT4 || kind == TILE_DIRECT_WIDE;
-    if (thread_rows) {
-        for (int rl = threadIdx.x; rl < nr; rl += kF64Block) {
-            const int r = t.row0 + rl;
-            double acc = diag_terms64(p, x, r, 0, 1);
-            for (int j = p.rowptr[r]; j < p.rowptr[r + 1]; ++j) acc += gather64<SIGNED>(x, p.cols[j]);
-            y[r] = acc;
+    int lg = 0;                   // lanes per row: about kLaneWords words each
+    while (lg < 5 && t.nnz > (long)nr * (kLaneWords << lg)) ++lg;
+    const int G = 1 << lg, gl = lane & (G - 1);
+    for (int base = 0; base < nr; base += kBlock >> lg) {
+        const int rl = base + (threadIdx.x >> lg), r = t.row0 + rl;
+        const bool ok = rl < nr;
+        const int b = ok ? __ldg(p.rowptr + r) : 0, e = ok ? __ldg(p.rowptr + r + 1) : 0;
+        const bool own = e - b <= kLaneMost << lg;
+        double acc = SIGNED && ok && own ? diag_terms64(p, x, r, gl, G) : 0.0;
+        if (own) sum_words64<SIGNED>(p, x, b + gl, e, G, acc);
+        acc = group_sum(acc, G);
+        if (ok && own && gl == 0) y[r] = acc;
+        for (unsigned mid = __ballot_sync(0xffffffffu, !own && gl == 0); mid; mid &= mid - 1) {
+            const int src = __ffs(mid) - 1;       // a row for the whole warp
+            const int mr = __shfl_sync(0xffffffffu, r, src);
+            const int mb = __shfl_sync(0xffffffffu, b, src), me = __shfl_sync(0xffffffffu, e, src);
+            double a = SIGNED ? diag_terms64(p, x, mr, lane, 32) : 0.0;
+            sum_words64<SIGNED>(p, x, mb + lane, me, 32, a);
+            a = group_sum(a, 32);
+            if (lane == 0) y[mr] = a;
         }
-        return;
     }
-    for (int rl = warp; rl < nr; rl += kF64Block / 32) {      // lane and merge tiles: a warp per row
-        const int r = t.row0 + rl;
-        double acc = diag_terms64(p, x, r, lane, 32);
-        for (int j = p.rowptr[r] + lane; j < p.rowptr[r + 1]; j += 32) acc += gather64<SIGNED>(x, p.cols[j]);
-        acc = warp_sum64(acc);
-        if (lane == 0) y[r] = acc;
+}
+
+template <bool SIGNED>
+tc_status launch_f64(const DevPlan &dp, int64_t nnz_csr, int max_row, const double *x, double *y, cudaStream_t s)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(kBlock);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = dp.pdl ? 1 : 0;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const int ahead = kF64Blocks * num_sms();
+    auto grid = [&](int lg) { return dim3((unsigned)(((long)dp.M + (kBlock >> lg) - 1) / (kBlock >> lg))); };
+    if (max_row > kShortRow) {
+        cfg.gridDim = dim3(dp.ntiles);
+        TC_CUDA(cudaLaunchKernelEx(&cfg, f64_tiles_kernel<SIGNED>, dp, x, y));
+    } else if (nnz_csr <= 8LL * dp.M) {
+        // a thread a row while a warp's words of consecutive rows share lines;
+        // above, lanes enough for 4 words or fewer each (18 words: 4.9 us at 8
+        // lanes in place of 8.3 at one; 32 words: 36 in place of 107)
+        cfg.gridDim = grid(0);
+        TC_CUDA(cudaLaunchKernelEx(&cfg, f64_rows_kernel<SIGNED, 0>, dp, ahead, x, y));
+    } else if (nnz_csr <= 16LL * dp.M) {
+        cfg.gridDim = grid(2);
+        TC_CUDA(cudaLaunchKernelEx(&cfg, f64_rows_kernel<SIGNED, 2>, dp, ahead, x, y));
+    } else {
+        cfg.gridDim = grid(3);
+        TC_CUDA(cudaLaunchKernelEx(&cfg, f64_rows_kernel<SIGNED, 3>, dp, ahead, x, y));
     }
+    return TC_OK;
 }
 
 }  // namespace
@@ -110,8 +253,10 @@ tc_status tc_spmv_f64(const tc_plan *p, const double *d_x, double *d_y, void *st
     const DevPlan dp = p->dev_plan();
     if (dp.M == 0 || dp.ntiles == 0) return TC_OK;
     cudaStream_t s = (cudaStream_t)stream;
-    if (dp.hybrid) spmv_f64_kernel<true><<<dp.ntiles, kF64Block, 0, s>>>(dp, d_x, d_y);
-    else spmv_f64_kernel<false><<<dp.ntiles, kF64Block, 0, s>>>(dp, d_x, d_y);
-    TC_CUDA(cudaGetLastError());
-    return TC_OK;
+    if (dp.N == 0) {      // no terms, and no x for the unconditional loads
+        TC_CUDA(cudaMemsetAsync(d_y, 0, sizeof(double) * (size_t)dp.M, s));
+        return TC_OK;
+    }
+    return dp.hybrid ? launch_f64<true>(dp, p->nnz_csr, p->max_row, d_x, d_y, s)
+                     : launch_f64<false>(dp, p->nnz_csr, p->max_row, d_x, d_y, s);
 }
