@@ -1,24 +1,25 @@
 // tc_batch.cu -- many resident plans multiplied in one launch.
 //
-// The batch flattens the tile lists of all its plans into one work list of
-// (plan, tile) pairs -- the plain plans' tiles first, then the hybrid plans'
-// -- and runs it with one CTA per work item: one launch for the plain part and
-// one for the hybrid part, so each runs tile code of one word kind only.  The
-// item's plan descriptor is read once into shared memory.  A CTA per item
-// keeps the most independent tiles in flight per SM; a
-// persistent grid that walks items in turn serialises each tile's load ->
-// gather -> sum chain per CTA and measured slower.  When every plan holds
-// only stream, direct and long tiles the lean kernels (no lane-tile code,
-// more CTAs per SM) run.  Every tile runs the same device code as the
-// single-plan kernel, so each matrix's y is bit-identical alone and inside a
-// batch.  The launches are captured once in a CUDA graph and replayed
-// (tc_batch_graph_launch).
+// The batch flattens the tile lists of all its plans into one work list, an
+// item per tile, and runs it with one CTA per item in one launch (captured
+// once in a CUDA graph and replayed by tc_batch_graph_launch).  An item holds
+// all that its CTA needs to start -- tile, plan arrays, x and y -- so its
+// words and row pointers are one load away; an item that named a plan and a
+// tile, with the plan descriptor copied to shared memory first, put four
+// loads and a barrier before them.  Small plans bring the tiles planned for
+// batches (tc_plan::d_btiles): a plan alone spreads its entries over the GPU,
+// a batch has the other plans for that and does better with whole tiles.
+// When every plan holds only stream, direct and long tiles the lean kernel
+// (no lane-tile code, more CTAs per SM) runs.  Every tile runs the same
+// device code as the single-plan kernel, so each matrix's y is bit-identical
+// alone and inside a batch.  Measured on 256 matrices of 1e3 to 2e5 rows
+// (92 M entries, 471 MB): 280 us with the longer chain, a launch per word
+// kind and the plans' own tiles, XXX us now.
 
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <new>
-#include <numeric>
 
 #include "tc_internal.h"
 #include "tc_tile.cuh"
@@ -26,27 +27,53 @@
 namespace tc {
 namespace {
 
-struct BatchItem {
-    int plan;
-    int tile;
-    int part;          // quarter of a wide direct tile, else 0
+// One CTA's work: 64 bytes, read as four int4s by every thread of the CTA.
+struct alignas(64) BatchItem {
+    const int *rowptr, *cols;
+    const float *x;
+    float *y;
+    Tile tile;
+    int N;
+    int plan;          // index of its descriptor
+    int part;          // part of a wide direct tile, else 0
+    int hybrid_skew;   // bit 0: hybrid plan, bit 1: skewed slots
 };
+static_assert(sizeof(BatchItem) == 64, "read as four int4s");
 
-// Work items of plain plans (SIGNED = false) or of hybrid plans (true): the
-// work list holds the plain plans' items first, and each half runs under
-// its own kernel so that neither tile code raises the other's registers.
-template <bool SIGNED, bool LEAN>
-__global__ void __launch_bounds__(kBlock, LEAN ? kItemMinBlocks : 1)
-    batch_kernel(const DevPlan *__restrict__ plans, const BatchItem *__restrict__ items, int nitems,
-                 const float *const *xs, float *const *ys)
+// LEAN: no lane-tile code; B: resident CTAs per SM it is compiled for.
+template <bool LEAN, int B>
+__global__ void __launch_bounds__(kBlock, B)
+    batch_kernel(const DevPlan *__restrict__ plans, const BatchItem *__restrict__ items)
 {
-    __shared__ DevPlan sp;                     // the item's plan, read by every thread
-    if ((int)blockIdx.x >= nitems) return;     // the grid has one CTA per item
-    const BatchItem it = items[blockIdx.x];
-    if (threadIdx.x == 0) sp = plans[it.plan];
-    __syncthreads();
-    const Tile t = sp.tiles[it.tile];
-    run_tile_part<SIGNED, LEAN>(sp, t, it.part, xs[it.plan], ys[it.plan], true);
+    union {
+        BatchItem it;
+        int4 q[4];
+    } u;
+    const int4 *src = reinterpret_cast<const int4 *>(items + blockIdx.x);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) u.q[k] = __ldg(src + k);
+    const BatchItem &it = u.it;
+    DevPlan p;                     // the fields the tile code reads
+    p.rowptr = it.rowptr;
+    p.cols = it.cols;
+    p.N = it.N;
+    p.skew = it.hybrid_skew >> 1;
+    p.dia_shapes = 0;
+    if (!(it.hybrid_skew & 1)) {
+        run_tile_part<false, LEAN>(p, it.tile, it.part, it.x, it.y, true);
+        return;
+    }
+    const DevPlan *g = plans + it.plan;
+    p.shapes = g->shapes;
+    p.shape_dias = g->shape_dias;
+    p.offsets = g->offsets;
+    p.dia_shapes = g->dia_shapes;
+    p.row_start = g->row_start;
+    p.row_stop = g->row_stop;
+    p.dn = g->dn;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) p.d_col[k] = g->d_col[k];
+    run_tile_part<true, LEAN>(p, it.tile, it.part, it.x, it.y, true);
 }
 
 }  // namespace
@@ -55,15 +82,10 @@ __global__ void __launch_bounds__(kBlock, LEAN ? kItemMinBlocks : 1)
 struct tc_batch {
     int n = 0;
     int nitems = 0;
-    int nplain = 0;      // items of plain plans (the first ones of the list)
-    int grid = 0;
     bool lean = false;
-    size_t smem = 0;
     void *dev = nullptr;
     tc::DevPlan *d_plans = nullptr;
     tc::BatchItem *d_items = nullptr;
-    const float **d_x = nullptr;
-    float **d_y = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
 };
@@ -79,49 +101,43 @@ tc_status tc_batch_create(int n, tc_plan *const *plans, const float *const *d_x,
     *out = nullptr;
     std::vector<tc::DevPlan> dps(n);
     std::vector<tc::BatchItem> items;
+    std::vector<tc::Tile> tiles;
     bool lean = true;
     for (int i = 0; i < n; ++i) {
-        if (!plans[i]) return fail(TC_ERR_INVALID, "plan %d is null", i);
-        dps[i] = plans[i]->dev_plan();
-        lean = lean && dps[i].per_tile >= 2;
+        const tc_plan *p = plans[i];
+        if (!p) return fail(TC_ERR_INVALID, "plan %d is null", i);
+        const tc::DevPlan &dp = dps[i] = p->dev_plan();
+        lean = lean && dp.per_tile >= 2;
+        tiles.resize(p->nbtiles);
+        if (p->nbtiles)
+            TC_CUDA(cudaMemcpy(tiles.data(), p->d_btiles, sizeof(tc::Tile) * tiles.size(), cudaMemcpyDeviceToHost));
+        for (const tc::Tile &t : tiles)
+            for (int k = 0; k < tc::tile_parts(dp.per_tile, tc::tile_nrows(t)); ++k)
+                items.push_back(tc::BatchItem{dp.rowptr, dp.cols, d_x[i], d_y[i], t, dp.N, i, k,
+                                              (dp.hybrid ? 1 : 0) | (dp.skew ? 2 : 0)});
     }
-    for (int pass = 0; pass < 2; ++pass)     // plain plans' items, then hybrid plans'
-        for (int i = 0; i < n; ++i)
-            if (dps[i].hybrid == pass)
-                for (int t = 0; t < dps[i].ntiles; ++t)
-                    for (int k = 0; k < tc::tile_parts(dps[i].per_tile); ++k)
-                        items.push_back(tc::BatchItem{i, t, k});
     tc_batch *b = new (std::nothrow) tc_batch();
     if (!b) return fail(TC_ERR_ALLOC, "host allocation");
     b->lean = lean;
     b->n = n;
     b->nitems = (int)items.size();
-    b->nplain = 0;
-    for (const tc::BatchItem &it : items) b->nplain += dps[it.plan].hybrid == 0;
-    b->smem = 0;
-    size_t o_pl = 0;
-    size_t o_it = (sizeof(tc::DevPlan) * n + 255) & ~(size_t)255;
-    size_t o_x = o_it + ((sizeof(tc::BatchItem) * items.size() + 255) & ~(size_t)255);
-    size_t o_y = o_x + ((sizeof(void *) * n + 255) & ~(size_t)255);
-    size_t total = o_y + sizeof(void *) * n + 256;
+    const size_t o_it = (sizeof(tc::DevPlan) * n + 255) & ~(size_t)255;
     char *base = nullptr;
-    if (cudaMalloc(&base, total) != cudaSuccess) { delete b; return fail(TC_ERR_ALLOC, "batch tables"); }
+    if (cudaMalloc(&base, o_it + sizeof(tc::BatchItem) * items.size() + 256) != cudaSuccess) {
+        delete b;
+        return fail(TC_ERR_ALLOC, "batch tables");
+    }
     b->dev = base;
-    b->d_plans = reinterpret_cast<tc::DevPlan *>(base + o_pl);
+    b->d_plans = reinterpret_cast<tc::DevPlan *>(base);
     b->d_items = reinterpret_cast<tc::BatchItem *>(base + o_it);
-    b->d_x = reinterpret_cast<const float **>(base + o_x);
-    b->d_y = reinterpret_cast<float **>(base + o_y);
     cudaError_t e = cudaMemcpy(b->d_plans, dps.data(), sizeof(tc::DevPlan) * n, cudaMemcpyHostToDevice);
     if (e == cudaSuccess && !items.empty())
         e = cudaMemcpy(b->d_items, items.data(), sizeof(tc::BatchItem) * items.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(b->d_x, d_x, sizeof(void *) * n, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(b->d_y, d_y, sizeof(void *) * n, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         cudaFree(base);
         delete b;
         return fail(TC_ERR_CUDA, "tc_batch_create: %s", cudaGetErrorString(e));
     }
-    b->grid = std::max(1, b->nitems);                   // one CTA per work item
     *out = b;
     return TC_OK;
 }
@@ -131,15 +147,11 @@ tc_status tc_batch_run(tc_batch *b, void *stream)
     if (!b) return fail(TC_ERR_INVALID, "null batch");
     if (b->nitems == 0) return TC_OK;
     cudaStream_t s = (cudaStream_t)stream;
-    const int np = b->nplain, nh = b->nitems - b->nplain;   // one CTA per item
-    const tc::BatchItem *hi = b->d_items + np;
-    if (b->lean) {
-        if (np) tc::batch_kernel<false, true><<<np, tc::kBlock, 0, s>>>(b->d_plans, b->d_items, np, b->d_x, b->d_y);
-        if (nh) tc::batch_kernel<true, true><<<nh, tc::kBlock, 0, s>>>(b->d_plans, hi, nh, b->d_x, b->d_y);
-    } else {
-        if (np) tc::batch_kernel<false, false><<<np, tc::kBlock, 0, s>>>(b->d_plans, b->d_items, np, b->d_x, b->d_y);
-        if (nh) tc::batch_kernel<true, false><<<nh, tc::kBlock, 0, s>>>(b->d_plans, hi, nh, b->d_x, b->d_y);
-    }
+    constexpr int few = tc::kItemFewBlocks, many = tc::kItemManyBlocks;
+    if (!b->lean) tc::batch_kernel<false, 1><<<b->nitems, tc::kBlock, 0, s>>>(b->d_plans, b->d_items);
+    else if (b->nitems <= 2 * few * tc::num_sms())
+        tc::batch_kernel<true, few><<<b->nitems, tc::kBlock, 0, s>>>(b->d_plans, b->d_items);
+    else tc::batch_kernel<true, many><<<b->nitems, tc::kBlock, 0, s>>>(b->d_plans, b->d_items);
     TC_CUDA(cudaGetLastError());
     return TC_OK;
 }

@@ -214,6 +214,10 @@ struct tc_plan {
     int ntiles = 0, ntiles_vector = 0, ntiles_long = 0;
     int ntiles_wide = 0;                 // TILE_DIRECT_WIDE tiles (all or none)
     int ntiles_stream = 0;               // TILE_STREAM tiles
+    // the tiles that batch and served launches run (d_tiles when the plan's
+    // own tiles are as large as they get)
+    tc::Tile *d_btiles = nullptr;
+    int nbtiles = 0;
     int max_span = 0;
     int stage_rp = 8, stage_cw = 8, grid = 1;
     int *d_err = nullptr;
@@ -271,9 +275,11 @@ constexpr int kStreamManyMinBlocks = 8;
 // The rows kernel: 8 CTAs per SM (32 registers) with one strip of rows per
 // CTA, 4 with two.
 constexpr int kRowsMinBlocks = 8;
-// The same for the batch and served kernels, which read the plan descriptor
-// from memory instead of the parameter bank (48 registers).
-constexpr int kItemMinBlocks = 5;
+// The same for the batch and served kernels: 6 CTAs per SM for a batch of one
+// or two waves, 8 (32 registers) for more, and for served launches.  Batches
+// of 256 / 64 / 17 matrices at 5, 6 and 8 CTAs: 174 / 157 / 151, 48 / 44 / 43
+// and 10.4 / 8.7 / 10.3 us.
+constexpr int kItemFewBlocks = 6, kItemManyBlocks = 8;
 // Launch of the multiply kernel for one plan.
 // wb: the tiles' word bounds of a wide plan (nullptr: the kernels that read
 // them from the tile list).  launch_plan passes the plan's own.

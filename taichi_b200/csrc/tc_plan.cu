@@ -316,15 +316,16 @@ tc_status plan_upload(tc_plan *p, const int *csrRow, const int *csrCol, int64_t 
 
     // row statistics, and the tiles per strip unless the tiles are wide
     const int strips = (int)(((long)M + kStripRows - 1) / kStripRows);
-    const size_t o_sum = align256(sizeof(RowStats)), o_cnt = align256(o_sum + sizeof(TileCounts));
-    const size_t o_first = align256(o_cnt + sizeof(int) * ((size_t)strips + 1));
-    const size_t o_tmp = align256(o_first + sizeof(int) * ((size_t)strips + 1));
+    const size_t o_sum = align256(sizeof(RowStats)), o_cnt = align256(o_sum + 2 * sizeof(TileCounts));
+    const size_t o_first = align256(o_cnt + sizeof(int) * 2 * ((size_t)strips + 1));
+    const size_t o_tmp = align256(o_first + sizeof(int) * 2 * ((size_t)strips + 1));
     Scratch tmp;
     TC_CHECK(tmp.alloc(o_tmp + sizeof(int) * scan_tmp_ints(strips), stream));
     char *t = tmp.as<char>();
     RowStats *d_st = reinterpret_cast<RowStats *>(t);
     TileCounts *d_sum = reinterpret_cast<TileCounts *>(t + o_sum);
     int *d_cnt = reinterpret_cast<int *>(t + o_cnt), *d_first = reinterpret_cast<int *>(t + o_first);
+    int *d_bcnt = d_cnt + strips + 1, *d_bfirst = d_first + strips + 1;
     int *d_tmp = reinterpret_cast<int *>(t + o_tmp);
     TC_CUDA(cudaMemsetAsync(t, 0, o_first, stream));
     const int step = std::max(1, M / 65536);
@@ -343,17 +344,23 @@ tc_status plan_upload(tc_plan *p, const int *csrRow, const int *csrCol, int64_t 
     q.max_lanes = prm.max_lanes;
     q.strided = (prm.flags & TC_FLAG_ROWS_STRIDED) != 0;
     q.no_direct = (prm.flags & TC_FLAG_NO_DIRECT) != 0;
+    TilePrm bq = q;                           // the tiles of batch and served launches
+    bq.spread = kStreamNnz;
+    const bool second = prm.tile_mode == 2 && q.spread < kStreamNnz;
     if (M) {
         plan_strips<false><<<strips, 32, 0, stream>>>(csrRow, M, q, d_cnt, nullptr, nullptr, d_sum);
+        if (second) plan_strips<false><<<strips, 32, 0, stream>>>(csrRow, M, bq, d_bcnt, nullptr, nullptr, d_sum + 1);
         TC_CUDA(cudaGetLastError());
         TC_CHECK(exclusive_scan(d_cnt, d_first, strips, d_tmp, stream));
+        if (second) TC_CHECK(exclusive_scan(d_bcnt, d_bfirst, strips, d_tmp, stream));
     }
     RowStats st{};
     TileCounts sum{};
-    int made = 0;
+    int made = 0, bmade = 0;
     TC_CUDA(cudaMemcpyAsync(&st, d_st, sizeof st, cudaMemcpyDeviceToHost, stream));
     TC_CUDA(cudaMemcpyAsync(&sum, d_sum, sizeof sum, cudaMemcpyDeviceToHost, stream));
     if (M) TC_CUDA(cudaMemcpyAsync(&made, d_first + strips, sizeof made, cudaMemcpyDeviceToHost, stream));
+    if (M && second) TC_CUDA(cudaMemcpyAsync(&bmade, d_bfirst + strips, sizeof bmade, cudaMemcpyDeviceToHost, stream));
     TC_CUDA(cudaStreamSynchronize(stream));
     p->max_row = st.max_row;
     p->all_pos = !st.minus;                   // a hybrid plan with no holes: every word adds its term
@@ -364,6 +371,8 @@ tc_status plan_upload(tc_plan *p, const int *csrRow, const int *csrCol, int64_t 
                       M >= kDirectWideRows && nnz_csr <= M && st.max_row <= kStreamRowMax;
     p->wide_rows = wide ? wide_tile_rows(M, prm, num_sms()) : kDirectWideRows;
     p->ntiles = wide ? (M + p->wide_rows - 1) / p->wide_rows : made;
+    const bool own = wide || !second;         // batches run the plan's own tiles
+    p->nbtiles = own ? p->ntiles : bmade;
     p->ntiles_wide = wide ? p->ntiles : 0;
     p->ntiles_vector = wide ? 0 : sum.vector;
     p->ntiles_long = wide ? 0 : sum.lng;
@@ -403,7 +412,8 @@ tc_status plan_upload(tc_plan *p, const int *csrRow, const int *csrCol, int64_t 
     const size_t o_off = align256(o_sd + sizeof(int2) * sd.size());
     const size_t o_err = align256(o_off + sizeof(int) * (size_t)p->num_negs + 16);
     const size_t o_tiles = align256(o_err + 16);
-    const size_t o_wt = align256(o_tiles + sizeof(Tile) * (size_t)p->ntiles);
+    const size_t o_bt = align256(o_tiles + sizeof(Tile) * (size_t)p->ntiles);
+    const size_t o_wt = align256(o_bt + sizeof(Tile) * (size_t)(own ? 0 : p->nbtiles));
     const size_t total = align256(o_wt + sizeof(Tile) * wtiles.size());
     char *base = nullptr;
     const cudaError_t e = cudaMalloc(&base, total);
@@ -418,6 +428,7 @@ tc_status plan_upload(tc_plan *p, const int *csrRow, const int *csrCol, int64_t 
     p->d_offsets = reinterpret_cast<int *>(base + o_off);
     p->d_err = reinterpret_cast<int *>(base + o_err);
     p->d_tiles = reinterpret_cast<Tile *>(base + o_tiles);
+    p->d_btiles = own ? p->d_tiles : reinterpret_cast<Tile *>(base + o_bt);
     p->d_wtiles = p->nwtiles ? reinterpret_cast<Tile *>(base + o_wt) : nullptr;
     TC_CUDA(cudaMemsetAsync(base + rp_end, 0, o_cols - rp_end, stream));
     TC_CUDA(cudaMemsetAsync(base + cols_end, 0, o_sh - cols_end, stream));
@@ -442,9 +453,10 @@ tc_status plan_upload(tc_plan *p, const int *csrRow, const int *csrCol, int64_t 
                                                                           p->d_tiles);
     else if (M)
         plan_strips<true><<<strips, 32, 0, stream>>>(p->d_rowptr, M, q, nullptr, d_first, p->d_tiles, nullptr);
-    for (int k = 0; k < 2; ++k) {
-        Tile *list = k ? p->d_wtiles : p->d_tiles;
-        const int n = k ? p->nwtiles : p->ntiles;
+    if (!own) plan_strips<true><<<strips, 32, 0, stream>>>(p->d_rowptr, M, bq, nullptr, d_bfirst, p->d_btiles, nullptr);
+    for (int k = 0; k < 3; ++k) {
+        Tile *list = k == 0 ? p->d_tiles : k == 1 ? p->d_wtiles : p->d_btiles;
+        const int n = k == 0 ? p->ntiles : k == 1 ? p->nwtiles : own ? 0 : p->nbtiles;
         if (n) classify_tiles<<<(unsigned)((n + 7L) / 8), 256, 0, stream>>>(
             list, n, p->d_shapes, p->d_shape_dias, p->d_offsets, p->dia_shapes, p->row_start, p->row_stop);
     }

@@ -60,7 +60,7 @@ struct BatchArgs {
 // word kind (plain or hybrid), so one launch serves every request of the
 // batch.  LEAN: every admitted plan holds only stream, direct and long tiles.
 template <bool LEAN>
-__global__ void __launch_bounds__(kBlock, LEAN ? kItemMinBlocks : 1)
+__global__ void __launch_bounds__(kBlock, LEAN ? kItemManyBlocks : 1)
     serve_kernel(const DevPlan *__restrict__ plans, const __grid_constant__ BatchArgs b)
 {
     __shared__ DevPlan sp;
@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(kBlock, LEAN ? kItemMinBlocks : 1)
         sitem = g - sr.tile_begin;
     }
     __syncthreads();
-    const int parts = tile_parts(sp.per_tile);
+    const int parts = tile_parts(sp.per_tile, sp.wide_rows);
     const Tile t = sp.tiles[sitem / parts];
     if (sp.hybrid) run_tile_part<true, LEAN>(sp, t, sitem % parts, sr.x, sr.y, false);
     else run_tile_part<false, LEAN>(sp, t, sitem % parts, sr.x, sr.y, false);
@@ -207,7 +207,8 @@ tc_status launch_batch(tc_server *sv, tc_server::Ctx &c, std::deque<uint64_t> &p
             order.emplace_back(tk, 1);
         } else {
             args.r[args.n] = tc::ReqDesc{s.matrix, tiles, dx, dy};
-            tiles += p->ntiles * tc::tile_parts(p->dev_plan().per_tile);
+            const tc::DevPlan dp = p->dev_plan();
+            tiles += p->ntiles * tc::tile_parts(dp.per_tile, dp.wide_rows);
             ++args.n;
             order.emplace_back(tk, 0);
         }

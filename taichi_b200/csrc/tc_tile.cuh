@@ -969,10 +969,13 @@ __device__ __forceinline__ void run_tile(const DevPlan &p, const Tile &t, const 
 }
 
 // Work items of the batch and served launches (256-thread CTAs): a wide
-// direct tile is four items, part k holding its rows [1024 k, 1024 k + 1024)
-// (every thread one run, all loads of the item in flight); any other tile is
-// one item (part 0).
-__host__ __device__ inline int tile_parts(int per_tile) { return per_tile == 3 ? kDirectWideRows / kDirectRows : 1; }
+// direct tile is an item per kDirectRows rows, part k holding its rows
+// [1024 k, 1024 k + 1024) (every thread one run, all loads of the item in
+// flight); any other tile is one item (part 0).
+__host__ __device__ inline int tile_parts(int per_tile, int wide_rows)
+{
+    return per_tile == 3 ? (wide_rows + kDirectRows - 1) / kDirectRows : 1;
+}
 
 template <bool SIGNED, bool LEAN>
 __device__ __forceinline__ void run_tile_part(const DevPlan &p, const Tile &t, int part,
