@@ -206,7 +206,7 @@ tc_status tc_plan_info_get(const tc_plan *p, tc_plan_info *i)
     i->window_hi = p->whi;
     {
         const tc::DevPlan d = p->dev_plan();
-        i->kernel = d.nwtiles > 0 ? TC_KERNEL_WINDOW : d.per_tile == 4 && d.rows ? TC_KERNEL_ROWS
+        i->kernel = d.nwtiles > 0 ? TC_KERNEL_WINDOW : d.rows ? TC_KERNEL_ROWS
                   : d.per_tile == 0 ? TC_KERNEL_TILES : d.per_tile == 2 ? TC_KERNEL_LEAN : d.per_tile == 3 ? TC_KERNEL_WIDE : TC_KERNEL_STREAM;
     }
     return TC_OK;
@@ -316,7 +316,7 @@ tc_status tc_spmm(const tc_plan *p, const float *d_X, int ldx, int k, float *d_Y
 {
     if (!p || k < 1 || k > 64 || ldx < k || ldy < k) return fail(TC_ERR_INVALID, "tc_spmm: k must be in [1, 64], ld >= k");
     if ((!d_X && p->N) || (!d_Y && p->M)) return fail(TC_ERR_INVALID, "tc_spmm: null argument");
-    return tc::launch_spmm(p->dev_plan(), p->nnz_csr, p->max_row, d_X, ldx, k, d_Y, ldy, (cudaStream_t)stream);
+    return tc::launch_spmm(p->dev_plan(), p->diags, p->nnz_csr, p->max_row, d_X, ldx, k, d_Y, ldy, (cudaStream_t)stream);
 }
 
 }  // extern "C"

@@ -70,9 +70,7 @@ __global__ void __launch_bounds__(kBlock, B)
     p.dia_shapes = g->dia_shapes;
     p.row_start = g->row_start;
     p.row_stop = g->row_stop;
-    p.dn = g->dn;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) p.d_col[k] = g->d_col[k];
+    p.dn = 0;                      // offsets from the shape arrays (the descriptor's would be indexed in local memory)
     run_tile_part<true, LEAN>(p, it.tile, it.part, it.x, it.y, true);
 }
 

@@ -113,7 +113,7 @@ constexpr int kStreamRowMax = 128;    // longer rows of a stream tile are summed
 constexpr int kStream4Rows = 1024;    // most rows of a TILE_STREAM4 tile (a run of 4 per thread)
 constexpr int kDirectRows = 1024;     // most rows of a direct tile (TILE_DIRECT4)
 constexpr int kDirectWideBlock = 1024; // threads of the direct kernel's CTAs
-constexpr int kPlanDiags = 8;         // dense diagonals a plan can carry in its launch parameters
+constexpr int kPlanDiags = 4;         // dense diagonals a plan's descriptor carries
 // The rows kernel by default: stream plans whose rows average at most this
 // many CSR words.  Measured per multiply against stream tiles: mesh (6.1
 // words, hybrid) 39.4 against 45.7 µs; banded plain matrices of 9 words
@@ -148,6 +148,23 @@ constexpr int kWinMaxStages = 4;      // pipeline depth (stages of one CTA)
 constexpr int kWinSmemBudget = 200 * 1024;   // shared memory of the stages
 constexpr double kWinCover = 0.95;    // share of the in-halo accesses the window range holds
 
+// The dense diagonals of a plan with one shape of at most kMaxDiags offsets
+// (n of them, in offset order; otherwise n = 0), for the kernels that walk
+// whole rows: a second launch parameter, so that the others' stays small.
+// Offset i adds x[r + col[i]] to the rows r of [lo[i], hi[i]); every offset
+// reaches the rows of [in.x, in.y).
+constexpr int kMaxDiags = 32;
+struct PlanDiags {
+    int n;
+    int2 in;
+    int lo[kMaxDiags], hi[kMaxDiags], col[kMaxDiags];
+};
+struct NoDiags {};                    // plain plans
+template <bool SIGNED>
+struct DiagsOf { using type = NoDiags; };
+template <>
+struct DiagsOf<true> { using type = PlanDiags; };
+
 // Everything a multiply kernel needs about one plan (passed by value).
 struct DevPlan {
     const int *rowptr;      // M+1
@@ -167,14 +184,14 @@ struct DevPlan {
     int *err;               // device error word (1: a bounded wait gave up)
     int wide_rows;          // rows of each wide direct tile (the last may have fewer)
     // plans whose dense part is one shape of at most kPlanDiags offsets
-    // (dn of them, in offset order): offset i adds x[r + d_col[i]] to the rows
-    // r of [d_lo[i], d_hi[i]) and no other row has a diagonal term.  dn = 0:
+    // (dn of them; see PlanDiags, whose first kPlanDiags they are).  dn = 0:
     // no dense part, or more than one shape / more offsets (dgen = 1: the
     // per-row shape search, diag_row)
     int dn, dgen;
     int d_lo[kPlanDiags], d_hi[kPlanDiags], d_col[kPlanDiags];
+    int2 d_in;              // the rows that every offset reaches
     int rows;               // stream plan run by the rows kernel (one row per thread)
-    int rows_w;             // the rows kernel's words loaded together (4, 6 or 8: from the usual row length)
+    int rows_w;             // the rows kernel's words loaded together (2, 4, 6 or 8: from the usual row length)
     int pos;                // hybrid plan whose words are all additions (no holes)
     int ahead;              // stream / rows kernels: CTA b prefetches the operands of CTA b + ahead
     int prefetch;           // wide kernel: each CTA prefetches its tile's CSR words into L2
@@ -244,6 +261,8 @@ struct tc_plan {
     float *d_xbuf[TC_HOST_SLOTS] = {}, *d_ybuf[TC_HOST_SLOTS] = {};
 
     tc::DevPlan dev_plan() const;
+    tc::PlanDiags diags{};               // set by plan_upload
+    void set_diags();
     int64_t spmv_bytes() const;
 };
 
@@ -283,7 +302,7 @@ constexpr int kItemFewBlocks = 6, kItemManyBlocks = 8;
 // Launch of the multiply kernel for one plan.
 // wb: the tiles' word bounds of a wide plan (nullptr: the kernels that read
 // them from the tile list).  launch_plan passes the plan's own.
-tc_status launch_spmv(const DevPlan &dp, const float *x, float *y, cudaStream_t s,
+tc_status launch_spmv(const DevPlan &dp, const PlanDiags &dg, const float *x, float *y, cudaStream_t s,
                       const WideBounds *wb = nullptr, const WideStarts *ws = nullptr);
 tc_status launch_plan(const tc_plan *p, const float *x, float *y, cudaStream_t s);
 // Window plans (tc_window.cu): the planner (false when the matrix does not
@@ -295,8 +314,8 @@ tc_status window_prepare(DevPlan &dp);
 tc_status launch_window(const DevPlan &dp, const float *x, float *y, cudaStream_t s);
 // nnz_csr, max_row: the plan's CSR words and those of its longest row (they
 // pick the kernel).
-tc_status launch_spmm(const DevPlan &dp, int64_t nnz_csr, int max_row, const float *X, int ldx, int k, float *Y,
-                      int ldy, cudaStream_t s);
+tc_status launch_spmm(const DevPlan &dp, const PlanDiags &dg, int64_t nnz_csr, int max_row, const float *X, int ldx,
+                      int k, float *Y, int ldy, cudaStream_t s);
 // Multiprocessors of the current device (read once).
 int num_sms();
 

@@ -249,6 +249,7 @@ tc_status plan_upload(tc_plan *p, const int *csrRow, const int *csrCol, int64_t 
     const int M = p->M;
     const tc_params &prm = p->params;
     p->nnz_csr = nnz_csr;
+    p->set_diags();
     // shape table {xStart, xStop, yStart, Msub} and offset ranges
     std::vector<int4> shapes(p->dia_shapes);
     std::vector<int2> sd(p->dia_shapes);
@@ -346,7 +347,7 @@ tc_status plan_upload(tc_plan *p, const int *csrRow, const int *csrCol, int64_t 
     q.no_direct = (prm.flags & TC_FLAG_NO_DIRECT) != 0;
     TilePrm bq = q;                           // the tiles of batch and served launches
     bq.spread = kStreamNnz;
-    const bool second = prm.tile_mode == 2 && q.spread < kStreamNnz;
+    const bool second = M > 0 && prm.tile_mode == 2 && q.spread < kStreamNnz;
     if (M) {
         plan_strips<false><<<strips, 32, 0, stream>>>(csrRow, M, q, d_cnt, nullptr, nullptr, d_sum);
         if (second) plan_strips<false><<<strips, 32, 0, stream>>>(csrRow, M, bq, d_bcnt, nullptr, nullptr, d_sum + 1);
@@ -364,11 +365,13 @@ tc_status plan_upload(tc_plan *p, const int *csrRow, const int *csrCol, int64_t 
     TC_CUDA(cudaStreamSynchronize(stream));
     p->max_row = st.max_row;
     p->all_pos = !st.minus;                   // a hybrid plan with no holes: every word adds its term
-    // rows of at most one entry on average and none long: the whole matrix as
-    // wide direct tiles (a 1024-thread CTA each)
+    // rows of at most one entry on average and none long, at most one dense
+    // diagonal: the whole matrix as wide direct tiles (a 1024-thread CTA
+    // each).  Several diagonals make a thread's four rows a long chain and its
+    // loads of x four to a line; the rows kernel takes those plans.
     const bool wide = prm.tile_mode == 2 && prm.tile_rows >= kDirectRows &&
                       !(prm.flags & (TC_FLAG_NO_DIRECT | TC_FLAG_NO_WIDE | TC_FLAG_ROWS_STRIDED)) &&
-                      M >= kDirectWideRows && nnz_csr <= M && st.max_row <= kStreamRowMax;
+                      M >= kDirectWideRows && nnz_csr <= M && st.max_row <= kStreamRowMax && p->num_negs <= 1;
     p->wide_rows = wide ? wide_tile_rows(M, prm, num_sms()) : kDirectWideRows;
     p->ntiles = wide ? (M + p->wide_rows - 1) / p->wide_rows : made;
     const bool own = wide || !second;         // batches run the plan's own tiles
@@ -385,12 +388,12 @@ tc_status plan_upload(tc_plan *p, const int *csrRow, const int *csrCol, int64_t 
         const int *h = st.hist;
         const int mode = (int)(std::max_element(h + 1, h + kStreamRowMax + 1) - h);
         p->stream_skew = h[mode] > 0 && mode % 8 == 0;
-        // the rows kernel loads W words of a row together: the least of 4, 6, 8
-        // that holds 90 % of the rows whole
+        // the rows kernel loads W words of a row together: the least of 2, 4,
+        // 6, 8 that holds 90 % of the rows whole
         int64_t tot = 0, upto = 0;
         for (int L = 0; L <= kStreamRowMax; ++L) tot += h[L];
         p->rows_w = 8;
-        for (int L = 0, w = 4; L <= 8 && tot > 0; ++L) {
+        for (int L = 0, w = 2; L <= 8 && tot > 0; ++L) {
             upto += h[L];
             if (L == w) {
                 if (upto * 10 >= tot * 9) {

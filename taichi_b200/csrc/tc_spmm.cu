@@ -110,21 +110,18 @@ __device__ __forceinline__ void add_word(Cols<V, VEC> &acc, const Cols<V, VEC> &
 // The dense-diagonal terms of row r, added to acc in offset order, four loads
 // in flight; Xc: the lane's first column of X.
 template <int V, bool VEC>
-__device__ __forceinline__ void diag_cols(const DevPlan &p, const float *__restrict__ Xc, int ldx,
+__device__ __forceinline__ void diag_cols(const DevPlan &p, const PlanDiags &q, const float *__restrict__ Xc, int ldx,
                                           const Lane<V, VEC> &l, int r, Cols<V, VEC> &acc)
 {
-    if (p.dn > 0) {
-        // one shape of at most kPlanDiags offsets: each offset's rows and
-        // column shift come with the launch parameters
-#pragma unroll
-        for (int i = 0; i < kPlanDiags; i += 4) {
-            if (i >= p.dn) break;
+    if (q.n > 0) {                // offsets from the launch parameters
+#pragma unroll 1
+        for (int i = 0; i < q.n; i += 4) {
             Cols<V, VEC> d[4];
             bool in[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                in[u] = i + u < p.dn && r >= p.d_lo[i + u] && r < p.d_hi[i + u];
-                d[u].load(Xc + (long)(in[u] ? r + p.d_col[i + u] : 0) * ldx, l);
+                in[u] = i + u < q.n && r >= q.lo[i + u] && r < q.hi[i + u];
+                d[u].load(Xc + (long)(in[u] ? r + q.col[i + u] : 0) * ldx, l);
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u)
@@ -132,7 +129,7 @@ __device__ __forceinline__ void diag_cols(const DevPlan &p, const float *__restr
         }
         return;
     }
-    if (!p.dgen || r < p.row_start || r >= p.row_stop) return;
+    if (r < p.row_start || r >= p.row_stop) return;
     for (int s = 0; s < p.dia_shapes; ++s) {
         const int4 sh = __ldg(p.shapes + s);
         if (r < sh.x || r >= sh.y) continue;
@@ -195,8 +192,8 @@ __device__ __forceinline__ void sum_words(const DevPlan &p, const float *__restr
 // whole warp, whose groups sum every (32 >> lg)-th word each; a butterfly
 // joins the parts.
 template <bool SIGNED, int V, bool VEC, int W, bool MID>
-__device__ __forceinline__ void spmm_rows(const DevPlan &p, const float *__restrict__ Xc, int ldx,
-                                          const Lane<V, VEC> &l, int lg, int row0, int nrow,
+__device__ __forceinline__ void spmm_rows(const DevPlan &p, const typename DiagsOf<SIGNED>::type &q,
+                                          const float *__restrict__ Xc, int ldx, const Lane<V, VEC> &l, int lg, int row0, int nrow,
                                           float *__restrict__ Yc, int ldy)
 {
     const int group = threadIdx.x >> lg, r = row0 + group;
@@ -206,7 +203,7 @@ __device__ __forceinline__ void spmm_rows(const DevPlan &p, const float *__restr
         Cols<V, VEC> acc;
         acc.zero();
         sum_words<SIGNED, V, VEC, W>(p, Xc, ldx, l, b, e, 1, acc);
-        if (SIGNED) diag_cols(p, Xc, ldx, l, r, acc);
+        if constexpr (SIGNED) diag_cols(p, q, Xc, ldx, l, r, acc);
         acc.store(Yc + (long)r * ldy, l);
     }
     if (!MID) return;
@@ -224,7 +221,7 @@ __device__ __forceinline__ void spmm_rows(const DevPlan &p, const float *__restr
         for (int u = 0; u < V; ++u)
             for (int o = 1 << lg; o < 32; o <<= 1) acc.a[u] += __shfl_xor_sync(0xffffffffu, acc.a[u], o);
         if (wg == 0) {
-            if (SIGNED) diag_cols(p, Xc, ldx, l, mr, acc);
+            if constexpr (SIGNED) diag_cols(p, q, Xc, ldx, l, mr, acc);
             acc.store(Yc + (long)mr * ldy, l);
         }
     }
@@ -234,13 +231,13 @@ __device__ __forceinline__ void spmm_rows(const DevPlan &p, const float *__restr
 // CTA.
 template <bool SIGNED, int V, bool VEC, int W>
 __global__ void __launch_bounds__(kBlock, spmm_blocks(V, W))
-    spmm_rows_kernel(DevPlan p, const float *__restrict__ X, int ldx, int k, int lg, int ahead,
+    spmm_rows_kernel(DevPlan p, const __grid_constant__ typename DiagsOf<SIGNED>::type q, const float *__restrict__ X, int ldx, int k, int lg, int ahead,
                      float *__restrict__ Y, int ldy)
 {
     const int groups = kBlock >> lg, row0 = blockIdx.x * groups;
     const Lane<V, VEC> l(threadIdx.x & ((1 << lg) - 1), lg, k);
     if (threadIdx.x == 0) prefetch_later_rows(p, (long)row0 + (long)ahead * groups, groups);
-    spmm_rows<SIGNED, V, VEC, W, false>(p, X + l.at, ldx, l, lg, row0, min(groups, p.M - row0), Y + l.at, ldy);
+    spmm_rows<SIGNED, V, VEC, W, false>(p, q, X + l.at, ldx, l, lg, row0, min(groups, p.M - row0), Y + l.at, ldy);
 }
 
 // Other plans: a CTA per tile of the plan's tile list, whose words are
@@ -250,7 +247,7 @@ __global__ void __launch_bounds__(kBlock, spmm_blocks(V, W))
 // group joins the parts in group order.
 template <bool SIGNED, int V, bool VEC, int W>
 __global__ void __launch_bounds__(kBlock, spmm_blocks(V, W))
-    spmm_tiles_kernel(DevPlan p, const float *__restrict__ X, int ldx, int k, int lg, float *__restrict__ Y,
+    spmm_tiles_kernel(DevPlan p, const __grid_constant__ typename DiagsOf<SIGNED>::type q, const float *__restrict__ X, int ldx, int k, int lg, float *__restrict__ Y,
                       int ldy)
 {
     __shared__ float part[kBlock * V];
@@ -261,7 +258,7 @@ __global__ void __launch_bounds__(kBlock, spmm_blocks(V, W))
     const int nr = tile_nrows(t);
     if (nr > 1 || t.nnz <= kSpmmLongRow) {
         for (int i = 0; i < nr; i += groups)
-            spmm_rows<SIGNED, V, VEC, W, true>(p, Xc, ldx, l, lg, t.row0 + i, min(groups, nr - i), Y + l.at, ldy);
+            spmm_rows<SIGNED, V, VEC, W, true>(p, q, Xc, ldx, l, lg, t.row0 + i, min(groups, nr - i), Y + l.at, ldy);
         return;
     }
     Cols<V, VEC> acc;
@@ -274,7 +271,7 @@ __global__ void __launch_bounds__(kBlock, spmm_blocks(V, W))
         for (int g = 1; g < groups; ++g)
 #pragma unroll
             for (int u = 0; u < V; ++u) acc.a[u] += part[u * kBlock + (g << lg) + threadIdx.x];
-        if (SIGNED) diag_cols(p, Xc, ldx, l, t.row0, acc);
+        if constexpr (SIGNED) diag_cols(p, q, Xc, ldx, l, t.row0, acc);
         acc.store(Y + (long)t.row0 * ldy + l.at, l);
     }
 }
@@ -344,11 +341,13 @@ __global__ void __launch_bounds__(kBlock, kRunBlocks)
 }
 
 template <bool SIGNED, int V, bool VEC>
-tc_status launch(const DevPlan &dp, int64_t nnz_csr, int max_row, const float *X, int ldx, int k, float *Y,
+tc_status launch(const DevPlan &dp, const PlanDiags &dg, int64_t nnz_csr, int max_row, const float *X, int ldx, int k, float *Y,
                  int ldy, cudaStream_t s)
 {
     int lg = 0;
     while ((V << lg) < k) ++lg;
+    typename DiagsOf<SIGNED>::type q;
+    if constexpr (SIGNED) q = dg;
     // Runs: plain rows of at most two words on average, in groups of 8 lanes
     // or more (a run of 2^lg rows; smaller groups diverge more than they
     // save).  Longer rows keep a group's loads in flight by themselves.
@@ -356,7 +355,7 @@ tc_status launch(const DevPlan &dp, int64_t nnz_csr, int max_row, const float *X
         const unsigned grid = (unsigned)((dp.M + kBlock - 1) / kBlock);
         spmm_run_kernel<V, VEC, 4><<<grid, kBlock, 0, s>>>(dp, X, ldx, k, lg, kRunBlocks * num_sms(), Y, ldy);
     } else if (max_row > kSpmmMidRow) {
-        spmm_tiles_kernel<SIGNED, V, VEC, 4><<<dp.ntiles, kBlock, 0, s>>>(dp, X, ldx, k, lg, Y, ldy);
+        spmm_tiles_kernel<SIGNED, V, VEC, 4><<<dp.ntiles, kBlock, 0, s>>>(dp, q, X, ldx, k, lg, Y, ldy);
     } else {
         // Rows of at most 8 words on average: three words in flight and two
         // more CTAs per SM (mesh 1200^2, k = 8: 41 us in place of 47);
@@ -366,17 +365,17 @@ tc_status launch(const DevPlan &dp, int64_t nnz_csr, int max_row, const float *X
         const unsigned grid = (unsigned)((dp.M + (long)rows - 1) / rows);
         if (nnz_csr <= 8LL * dp.M)
             spmm_rows_kernel<SIGNED, V, VEC, W><<<grid, kBlock, 0, s>>>(
-                dp, X, ldx, k, lg, spmm_blocks(V, W) * num_sms(), Y, ldy);
+                dp, q, X, ldx, k, lg, spmm_blocks(V, W) * num_sms(), Y, ldy);
         else
             spmm_rows_kernel<SIGNED, V, VEC, 4><<<grid, kBlock, 0, s>>>(
-                dp, X, ldx, k, lg, spmm_blocks(V, 4) * num_sms(), Y, ldy);
+                dp, q, X, ldx, k, lg, spmm_blocks(V, 4) * num_sms(), Y, ldy);
     }
     TC_CUDA(cudaGetLastError());
     return TC_OK;
 }
 
 template <bool SIGNED>
-tc_status launch_cols(const DevPlan &dp, int64_t nnz_csr, int max_row, const float *X, int ldx, int k, float *Y,
+tc_status launch_cols(const DevPlan &dp, const PlanDiags &dg, int64_t nnz_csr, int max_row, const float *X, int ldx, int k, float *Y,
                       int ldy, cudaStream_t s)
 {
     const uintptr_t at = reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Y);
@@ -384,15 +383,15 @@ tc_status launch_cols(const DevPlan &dp, int64_t nnz_csr, int max_row, const flo
     // vectors of four or two columns where k, both leading dimensions and both
     // addresses allow them, else four single loads a lane 2^lg columns apart
     // (mesh 800^2, k = 13: 49 us in place of 100 with one column a lane)
-    if (!(all & 3) && !(at & 15)) return launch<SIGNED, 4, true>(dp, nnz_csr, max_row, X, ldx, k, Y, ldy, s);
-    if (!(all & 1) && !(at & 7)) return launch<SIGNED, 2, true>(dp, nnz_csr, max_row, X, ldx, k, Y, ldy, s);
-    if (k <= 2) return launch<SIGNED, 1, false>(dp, nnz_csr, max_row, X, ldx, k, Y, ldy, s);
-    return launch<SIGNED, 4, false>(dp, nnz_csr, max_row, X, ldx, k, Y, ldy, s);
+    if (!(all & 3) && !(at & 15)) return launch<SIGNED, 4, true>(dp, dg, nnz_csr, max_row, X, ldx, k, Y, ldy, s);
+    if (!(all & 1) && !(at & 7)) return launch<SIGNED, 2, true>(dp, dg, nnz_csr, max_row, X, ldx, k, Y, ldy, s);
+    if (k <= 2) return launch<SIGNED, 1, false>(dp, dg, nnz_csr, max_row, X, ldx, k, Y, ldy, s);
+    return launch<SIGNED, 4, false>(dp, dg, nnz_csr, max_row, X, ldx, k, Y, ldy, s);
 }
 
 }  // namespace
 
-tc_status launch_spmm(const DevPlan &dp, int64_t nnz_csr, int max_row, const float *X, int ldx, int k, float *Y,
+tc_status launch_spmm(const DevPlan &dp, const PlanDiags &dg, int64_t nnz_csr, int max_row, const float *X, int ldx, int k, float *Y,
                       int ldy, cudaStream_t s)
 {
     if (dp.M == 0) return TC_OK;
@@ -400,8 +399,8 @@ tc_status launch_spmm(const DevPlan &dp, int64_t nnz_csr, int max_row, const flo
         TC_CUDA(cudaMemset2DAsync(Y, sizeof(float) * (size_t)ldy, 0, sizeof(float) * (size_t)k, dp.M, s));
         return TC_OK;
     }
-    return dp.hybrid ? launch_cols<true>(dp, nnz_csr, max_row, X, ldx, k, Y, ldy, s)
-                     : launch_cols<false>(dp, nnz_csr, max_row, X, ldx, k, Y, ldy, s);
+    return dp.hybrid ? launch_cols<true>(dp, dg, nnz_csr, max_row, X, ldx, k, Y, ldy, s)
+                     : launch_cols<false>(dp, dg, nnz_csr, max_row, X, ldx, k, Y, ldy, s);
 }
 
 }  // namespace tc

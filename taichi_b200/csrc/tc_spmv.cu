@@ -189,7 +189,8 @@ __global__ void __launch_bounds__(kDirectWideBlock, 2)
 // instructions on parking terms in shared memory and no barrier waits.
 template <bool SIGNED, int W>
 __global__ void __launch_bounds__(kBlock, kRowsMinBlocks)
-    spmv_rows_kernel(DevPlan p, const float *__restrict__ x, float *__restrict__ y)
+    spmv_rows_kernel(DevPlan p, const __grid_constant__ typename DiagsOf<SIGNED>::type q,
+                     const float *__restrict__ x, float *__restrict__ y)
 {
     allow_next_grid();
     const int r = blockIdx.x * kBlock + threadIdx.x;
@@ -220,35 +221,20 @@ __global__ void __launch_bounds__(kBlock, kRowsMinBlocks)
 #pragma unroll
     for (int w = 0; w < W; ++w) v[w] = gather<SIGNED>(x, c[w]);
     float acc = 0.f;
-    if (SIGNED && p.dgen) {
-        acc = diag_row(p, x, r);
-    } else if (SIGNED && p.dn <= 4) {
-        // the plan's offsets in order, named by constant indices (operands
-        // straight from the parameter bank); a row outside an offset's range
-        // loads x[0] for it and does not add it
-        float d[4];
-        bool in[4];
+    if constexpr (SIGNED) {
+        if (p.dn > 0 && r >= p.d_in.x && r < p.d_in.y) {
+            // the plan's offsets in order, named by constant indices (operands
+            // straight from the parameter bank)
+            float d[kPlanDiags];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            in[u] = u < p.dn && r >= p.d_lo[u] && r < p.d_hi[u];
-            d[u] = ldx(x + (in[u] ? r + p.d_col[u] : 0));
-        }
+            for (int u = 0; u < kPlanDiags; ++u) d[u] = u < p.dn ? ldx(x + r + p.d_col[u]) : 0.f;
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (in[u]) acc += d[u];
-    } else if (SIGNED) {
-#pragma unroll 1
-        for (int i = 0; i < p.dn; i += 4) {                      // the plan's offsets in order
-            float d[4];
-            bool in[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                in[u] = i + u < p.dn && r >= p.d_lo[i + u] && r < p.d_hi[i + u];
-                d[u] = in[u] ? ldx(x + r + p.d_col[i + u]) : 0.f;
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (in[u]) acc += d[u];
+            for (int u = 0; u < kPlanDiags; ++u)
+                if (u < p.dn) acc += d[u];
+        } else if (q.n > 0) {
+            acc = diag_plan_row(q, x, r);
+        } else {
+            acc = diag_row(p, x, r);
         }
     }
 #pragma unroll
@@ -363,7 +349,7 @@ tc_status tiles_grid(const DevPlan &dp, int ctas_per_sm, int *grid)
 }
 
 template <bool SIGNED>
-static tc_status launch_tiles(const DevPlan &dp, const WideBounds *wb, const WideStarts *ws, const float *x,
+static tc_status launch_tiles(const DevPlan &dp, const PlanDiags &dg, const WideBounds *wb, const WideStarts *ws, const float *x,
                               float *y, cudaStream_t s)
 {
     if (dp.ntiles <= 0) return TC_OK;
@@ -391,11 +377,14 @@ static tc_status launch_tiles(const DevPlan &dp, const WideBounds *wb, const Wid
         TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_wide_kernel<SIGNED, true, true>, dp, x, y));
     else if (dp.per_tile == 3 && full) TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_wide_kernel<SIGNED, true>, dp, x, y));
     else if (dp.per_tile == 3) TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_wide_kernel<SIGNED, false>, dp, x, y));
-    else if (dp.per_tile == 4 && dp.rows) {
+    else if (dp.rows) {
         cfg.gridDim = dim3((unsigned)((dp.M + kBlock - 1) / kBlock));
-        if (dp.rows_w <= 4) TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_rows_kernel<SIGNED, 4>, dp, x, y));
-        else if (dp.rows_w <= 6) TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_rows_kernel<SIGNED, 6>, dp, x, y));
-        else TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_rows_kernel<SIGNED, 8>, dp, x, y));
+        typename DiagsOf<SIGNED>::type q;
+        if constexpr (SIGNED) q = dg;
+        if (dp.rows_w <= 2) TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_rows_kernel<SIGNED, 2>, dp, q, x, y));
+        else if (dp.rows_w <= 4) TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_rows_kernel<SIGNED, 4>, dp, q, x, y));
+        else if (dp.rows_w <= 6) TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_rows_kernel<SIGNED, 6>, dp, q, x, y));
+        else TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_rows_kernel<SIGNED, 8>, dp, q, x, y));
     }
     else if (dp.per_tile == 4 && dp.ntiles > kLeanMinBlocks * num_sms())
         TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_stream_kernel<SIGNED, true>, dp, x, y));
@@ -405,7 +394,7 @@ static tc_status launch_tiles(const DevPlan &dp, const WideBounds *wb, const Wid
     return TC_OK;
 }
 
-tc_status launch_spmv(const DevPlan &dp, const float *x, float *y, cudaStream_t s, const WideBounds *wb,
+tc_status launch_spmv(const DevPlan &dp, const PlanDiags &dg, const float *x, float *y, cudaStream_t s, const WideBounds *wb,
                       const WideStarts *ws)
 {
     if (dp.M == 0) return TC_OK;
@@ -416,7 +405,7 @@ tc_status launch_spmv(const DevPlan &dp, const float *x, float *y, cudaStream_t 
         return TC_OK;
     }
     if (dp.nwtiles > 0) return launch_window(dp, x, y, s);
-    return dp.hybrid ? launch_tiles<true>(dp, wb, ws, x, y, s) : launch_tiles<false>(dp, wb, ws, x, y, s);
+    return dp.hybrid ? launch_tiles<true>(dp, dg, wb, ws, x, y, s) : launch_tiles<false>(dp, dg, wb, ws, x, y, s);
 }
 
 tc_status launch_plan(const tc_plan *p, const float *x, float *y, cudaStream_t s)
@@ -424,14 +413,14 @@ tc_status launch_plan(const tc_plan *p, const float *x, float *y, cudaStream_t s
     if (!p->h_wide_nz.empty()) {
         WideBounds wb;
         memcpy(wb.nz, p->h_wide_nz.data(), sizeof(int) * p->h_wide_nz.size());
-        return launch_spmv(p->dev_plan(), x, y, s, &wb, nullptr);
+        return launch_spmv(p->dev_plan(), p->diags, x, y, s, &wb, nullptr);
     }
     if (!p->h_wide_z.empty()) {
         WideStarts ws;
         memcpy(ws.nz, p->h_wide_z.data(), sizeof(int) * p->h_wide_z.size());
-        return launch_spmv(p->dev_plan(), x, y, s, nullptr, &ws);
+        return launch_spmv(p->dev_plan(), p->diags, x, y, s, nullptr, &ws);
     }
-    return launch_spmv(p->dev_plan(), x, y, s, nullptr, nullptr);
+    return launch_spmv(p->dev_plan(), p->diags, x, y, s, nullptr, nullptr);
 }
 
 }  // namespace tc
@@ -466,23 +455,23 @@ tc::DevPlan tc_plan::dev_plan() const
     d.skew = stream_skew;
     d.dn = 0;
     d.dgen = 0;
-    if (dia_shapes == 1 && num_negs <= tc::kPlanDiags && (int)h_offsets.size() >= num_negs) {
-        // the rows where diag_row adds each offset's term (TaiChi.cu:1014-1023)
-        const int xs = h_xStart[0], xe = h_xStop[0];
-        d.dn = num_negs;
-        for (int i = 0; i < num_negs; ++i) {
-            const int off = h_offsets[i];
-            d.d_lo[i] = std::max(xs + std::max(0, -off), row_start);
-            d.d_hi[i] = std::min(xe - std::max(0, off), row_stop);
-            d.d_col[i] = h_yStart[0] - xs + off;
+    if (diags.n > 0 && diags.n <= tc::kPlanDiags) {
+        d.dn = diags.n;
+        d.d_in = diags.in;
+        for (int i = 0; i < diags.n; ++i) {
+            d.d_lo[i] = diags.lo[i];
+            d.d_hi[i] = diags.hi[i];
+            d.d_col[i] = diags.col[i];
         }
     } else if (dia_shapes > 0) {
         d.dgen = 1;
     }
     // the rows kernel: a stream plan (every row at most kStreamRowMax words)
-    // of short rows, or any stream plan on request
+    // of short rows, or any stream plan on request; hybrid plans that are not
+    // wide run it whatever their tiles (direct and four-row tiles among them)
+    const bool any_tiles = d.dia_shapes > 0 && d.per_tile == 2 && max_row <= tc::kStreamRowMax;
     d.rows = 0;
-    if (d.per_tile == 4 && !(params.flags & TC_FLAG_NO_ROWS))
+    if ((d.per_tile == 4 || any_tiles) && !(params.flags & TC_FLAG_NO_ROWS))
         d.rows = (params.flags & TC_FLAG_ROWS) || (M > 0 && nnz_csr <= (int64_t)tc::kRowsMeanMax * M && tc::kRowsByDefault);
     d.rows_w = params.rows_w ? params.rows_w : rows_w;
     d.pos = hybrid && all_pos ? 1 : 0;
@@ -501,6 +490,23 @@ tc::DevPlan tc_plan::dev_plan() const
     d.w_stages = w_stages;
     d.w_grid = w_grid;
     return d;
+}
+
+void tc_plan::set_diags()
+{
+    diags = tc::PlanDiags{};
+    if (dia_shapes != 1 || num_negs > tc::kMaxDiags || (int)h_offsets.size() < num_negs) return;
+    // the rows where diag_row adds each offset's term (TaiChi.cu:1014-1023)
+    const int xs = h_xStart[0], xe = h_xStop[0];
+    diags.n = num_negs;
+    diags.in = make_int2(std::max(xs, row_start), std::min(xe, row_stop));
+    for (int i = 0; i < num_negs; ++i) {
+        const int off = h_offsets[i];
+        diags.lo[i] = std::max(xs + std::max(0, -off), row_start);
+        diags.hi[i] = std::min(xe - std::max(0, off), row_stop);
+        diags.col[i] = h_yStart[0] - xs + off;
+        diags.in = make_int2(std::max(diags.in.x, diags.lo[i]), std::min(diags.in.y, diags.hi[i]));
+    }
 }
 
 int64_t tc_plan::spmv_bytes() const

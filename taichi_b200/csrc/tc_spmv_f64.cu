@@ -73,20 +73,19 @@ __device__ __forceinline__ void add_words(const double *__restrict__ x, int j, i
 
 // The dense-diagonal terms of row r that lane `lane` of `lanes` owns
 // (offsets lane, lane + lanes, ... of each shape holding the row).
-__device__ __forceinline__ double diag_terms64(const DevPlan &p, const double *__restrict__ x, int r, int lane,
-                                               int lanes)
+__device__ __forceinline__ double diag_terms64(const DevPlan &p, const PlanDiags &q, const double *__restrict__ x,
+                                               int r, int lane, int lanes)
 {
     double acc = 0.0;
-    if (p.dn > 0) {               // one shape of few offsets: from the launch parameters
-#pragma unroll
-        for (int i = 0; i < kPlanDiags; i += 4) {
-            if (i >= p.dn) break;
+    if (q.n > 0) {                // offsets from the launch parameters
+#pragma unroll 1
+        for (int i = 0; i < q.n; i += 4) {
             double d[4];
             bool in[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                in[u] = i + u < p.dn && r >= p.d_lo[i + u] && r < p.d_hi[i + u] && ((i + u) & (lanes - 1)) == lane;
-                d[u] = ldx64(x + (in[u] ? r + p.d_col[i + u] : 0));
+                in[u] = i + u < q.n && r >= q.lo[i + u] && r < q.hi[i + u] && ((i + u) & (lanes - 1)) == lane;
+                d[u] = ldx64(x + (in[u] ? r + q.col[i + u] : 0));
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u)
@@ -94,7 +93,7 @@ __device__ __forceinline__ double diag_terms64(const DevPlan &p, const double *_
         }
         return acc;
     }
-    if (!p.dgen || r < p.row_start || r >= p.row_stop) return acc;
+    if (r < p.row_start || r >= p.row_stop) return acc;
     for (int s = 0; s < p.dia_shapes; ++s) {
         const int4 sh = __ldg(p.shapes + s);
         if (r < sh.x || r >= sh.y) continue;
@@ -127,7 +126,7 @@ __device__ __forceinline__ double group_sum(double v, int lanes)
 // Short rows: kBlock >> LG rows a CTA.
 template <bool SIGNED, int LG>
 __global__ void __launch_bounds__(kBlock, kF64Blocks)
-    f64_rows_kernel(DevPlan p, int ahead, const double *__restrict__ x, double *__restrict__ y)
+    f64_rows_kernel(DevPlan p, const __grid_constant__ typename DiagsOf<SIGNED>::type q, int ahead, const double *__restrict__ x, double *__restrict__ y)
 {
     constexpr int G = 1 << LG, R = kBlock >> LG, W = LG ? 4 : 3;
     allow_next_grid();
@@ -143,7 +142,10 @@ __global__ void __launch_bounds__(kBlock, kF64Blocks)
     int c[W];
     load_words(p, b, e, G, c);
     wait_prior64(x, y);
-    double acc = SIGNED && ok ? diag_terms64(p, x, r, lane, G) : 0.0;
+    double acc = 0.0;
+    if constexpr (SIGNED) {
+        if (ok) acc = diag_terms64(p, q, x, r, lane, G);
+    }
     add_words<SIGNED>(x, b, e, G, c, acc);
     for (int j = b + W * G; j < e; j += W * G) {
         load_words(p, j, e, G, c);
@@ -168,7 +170,7 @@ __device__ __forceinline__ void sum_words64(const DevPlan &p, const double *__re
 // Any plan: a CTA per tile.
 template <bool SIGNED>
 __global__ void __launch_bounds__(kBlock, kF64Blocks)
-    f64_tiles_kernel(DevPlan p, const double *__restrict__ x, double *__restrict__ y)
+    f64_tiles_kernel(DevPlan p, const __grid_constant__ typename DiagsOf<SIGNED>::type q, const double *__restrict__ x, double *__restrict__ y)
 {
     __shared__ double red[kBlock / 32];
     allow_next_grid();
@@ -176,7 +178,10 @@ __global__ void __launch_bounds__(kBlock, kF64Blocks)
     const int nr = tile_nrows(t), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     wait_prior64(x, y);
     if (nr == 1 && t.nnz > kLongTile) {
-        double acc = SIGNED ? diag_terms64(p, x, t.row0, threadIdx.x, kBlock) : 0.0;
+        double acc = 0.0;
+        if constexpr (SIGNED) {
+            acc = diag_terms64(p, q, x, t.row0, threadIdx.x, kBlock);
+        }
         sum_words64<SIGNED>(p, x, t.nz0 + threadIdx.x, t.nz0 + t.nnz, kBlock, acc);
         acc = group_sum(acc, 32);
         if (lane == 0) red[warp] = acc;
@@ -195,7 +200,10 @@ __global__ void __launch_bounds__(kBlock, kF64Blocks)
         const bool ok = rl < nr;
         const int b = ok ? __ldg(p.rowptr + r) : 0, e = ok ? __ldg(p.rowptr + r + 1) : 0;
         const bool own = e - b <= kLaneMost << lg;
-        double acc = SIGNED && ok && own ? diag_terms64(p, x, r, gl, G) : 0.0;
+        double acc = 0.0;
+        if constexpr (SIGNED) {
+            if (ok && own) acc = diag_terms64(p, q, x, r, gl, G);
+        }
         if (own) sum_words64<SIGNED>(p, x, b + gl, e, G, acc);
         acc = group_sum(acc, G);
         if (ok && own && gl == 0) y[r] = acc;
@@ -203,7 +211,10 @@ __global__ void __launch_bounds__(kBlock, kF64Blocks)
             const int src = __ffs(mid) - 1;       // a row for the whole warp
             const int mr = __shfl_sync(0xffffffffu, r, src);
             const int mb = __shfl_sync(0xffffffffu, b, src), me = __shfl_sync(0xffffffffu, e, src);
-            double a = SIGNED ? diag_terms64(p, x, mr, lane, 32) : 0.0;
+            double a = 0.0;
+            if constexpr (SIGNED) {
+                a = diag_terms64(p, q, x, mr, lane, 32);
+            }
             sum_words64<SIGNED>(p, x, mb + lane, me, 32, a);
             a = group_sum(a, 32);
             if (lane == 0) y[mr] = a;
@@ -212,8 +223,10 @@ __global__ void __launch_bounds__(kBlock, kF64Blocks)
 }
 
 template <bool SIGNED>
-tc_status launch_f64(const DevPlan &dp, int64_t nnz_csr, int max_row, const double *x, double *y, cudaStream_t s)
+tc_status launch_f64(const DevPlan &dp, const PlanDiags &dg, int64_t nnz_csr, int max_row, const double *x, double *y, cudaStream_t s)
 {
+    typename DiagsOf<SIGNED>::type q;
+    if constexpr (SIGNED) q = dg;
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(kBlock);
     cfg.stream = s;
@@ -226,19 +239,19 @@ tc_status launch_f64(const DevPlan &dp, int64_t nnz_csr, int max_row, const doub
     auto grid = [&](int lg) { return dim3((unsigned)(((long)dp.M + (kBlock >> lg) - 1) / (kBlock >> lg))); };
     if (max_row > kShortRow) {
         cfg.gridDim = dim3(dp.ntiles);
-        TC_CUDA(cudaLaunchKernelEx(&cfg, f64_tiles_kernel<SIGNED>, dp, x, y));
+        TC_CUDA(cudaLaunchKernelEx(&cfg, f64_tiles_kernel<SIGNED>, dp, q, x, y));
     } else if (nnz_csr <= 8LL * dp.M) {
         // a thread a row while a warp's words of consecutive rows share lines;
         // above, lanes enough for 4 words or fewer each (18 words: 4.9 us at 8
         // lanes in place of 8.3 at one; 32 words: 36 in place of 107)
         cfg.gridDim = grid(0);
-        TC_CUDA(cudaLaunchKernelEx(&cfg, f64_rows_kernel<SIGNED, 0>, dp, ahead, x, y));
+        TC_CUDA(cudaLaunchKernelEx(&cfg, f64_rows_kernel<SIGNED, 0>, dp, q, ahead, x, y));
     } else if (nnz_csr <= 16LL * dp.M) {
         cfg.gridDim = grid(2);
-        TC_CUDA(cudaLaunchKernelEx(&cfg, f64_rows_kernel<SIGNED, 2>, dp, ahead, x, y));
+        TC_CUDA(cudaLaunchKernelEx(&cfg, f64_rows_kernel<SIGNED, 2>, dp, q, ahead, x, y));
     } else {
         cfg.gridDim = grid(3);
-        TC_CUDA(cudaLaunchKernelEx(&cfg, f64_rows_kernel<SIGNED, 3>, dp, ahead, x, y));
+        TC_CUDA(cudaLaunchKernelEx(&cfg, f64_rows_kernel<SIGNED, 3>, dp, q, ahead, x, y));
     }
     return TC_OK;
 }
@@ -257,6 +270,6 @@ tc_status tc_spmv_f64(const tc_plan *p, const double *d_x, double *d_y, void *st
         TC_CUDA(cudaMemsetAsync(d_y, 0, sizeof(double) * (size_t)dp.M, s));
         return TC_OK;
     }
-    return dp.hybrid ? launch_f64<true>(dp, p->nnz_csr, p->max_row, d_x, d_y, s)
-                     : launch_f64<false>(dp, p->nnz_csr, p->max_row, d_x, d_y, s);
+    return dp.hybrid ? launch_f64<true>(dp, p->diags, p->nnz_csr, p->max_row, d_x, d_y, s)
+                     : launch_f64<false>(dp, p->diags, p->nnz_csr, p->max_row, d_x, d_y, s);
 }

@@ -311,6 +311,46 @@ __device__ __forceinline__ int merge_split(const Src &src, int nr, int nz, int d
 // issued before their adds (a wide band's terms do not wait on each other).
 constexpr int kDiagU = 4;
 
+// The same for a plan whose offsets come with its launch parameters, for a
+// row that every offset reaches (q.in): no range checks (15 offsets a row,
+// 900,000 rows: 12.2 us from the shape arrays, 14.1 with a check per offset).
+__device__ __forceinline__ float diag_plan_inner(const PlanDiags &q, const float *__restrict__ x, int r)
+{
+    const float *__restrict__ xr = x + r;
+    float acc = 0.f;
+#pragma unroll 1
+    for (int i = 0; i < q.n; i += kDiagU) {
+        float v[kDiagU];
+#pragma unroll
+        for (int u = 0; u < kDiagU; ++u) v[u] = i + u < q.n ? ldx(xr + q.col[i + u]) : 0.f;
+#pragma unroll
+        for (int u = 0; u < kDiagU; ++u)
+            if (i + u < q.n) acc += v[u];
+    }
+    return acc;
+}
+
+// The same for any row.
+__device__ __forceinline__ float diag_plan_row(const PlanDiags &q, const float *__restrict__ x, int r)
+{
+    if (r >= q.in.x && r < q.in.y) return diag_plan_inner(q, x, r);
+    float acc = 0.f;
+#pragma unroll 1
+    for (int i = 0; i < q.n; i += kDiagU) {
+        float v[kDiagU];
+        bool in[kDiagU];
+#pragma unroll
+        for (int u = 0; u < kDiagU; ++u) {
+            in[u] = i + u < q.n && r >= q.lo[i + u] && r < q.hi[i + u];
+            v[u] = ldx(x + (in[u] ? r + q.col[i + u] : 0));      // x[0] past the shape, not added
+        }
+#pragma unroll
+        for (int u = 0; u < kDiagU; ++u)
+            if (in[u]) acc += v[u];
+    }
+    return acc;
+}
+
 __device__ __forceinline__ float diag_row(const DevPlan &p, const float *__restrict__ x, int r)
 {
     float acc = 0.f;
@@ -521,7 +561,7 @@ __device__ __forceinline__ float diag_tile_row(const DevPlan &p, const float *__
 {
     if (dc == kDiagNone) return 0.f;
     if (dc == kDiagGeneral) return diag_row(p, x, r);
-    if (p.dn > 0 && p.dn <= 4) {
+    if (p.dn > 0) {
         // the plan's one shape, every offset inside it for this tile's rows:
         // the columns' shifts come with the plan descriptor (no shape or
         // offset reads), offsets in order
