@@ -151,13 +151,16 @@ constexpr double kWinCover = 0.95;    // share of the in-halo accesses the windo
 // The dense diagonals of a plan with one shape of at most kMaxDiags offsets
 // (n of them, in offset order; otherwise n = 0), for the kernels that walk
 // whole rows: a second launch parameter, so that the others' stays small.
-// Offset i adds x[r + col[i]] to the rows r of [lo[i], hi[i]); every offset
-// reaches the rows of [in.x, in.y).
-constexpr int kMaxDiags = 32;
+// Offset i adds x[r + col[i]] to the rows r of [rows.x, rows.y) for which the
+// column lies in [cols.x, cols.y); every offset reaches the rows of
+// [in.x, in.y).
+constexpr int kMaxDiags = 64;
 struct PlanDiags {
     int n;
-    int2 in;
-    int lo[kMaxDiags], hi[kMaxDiags], col[kMaxDiags];
+    int2 in, rows, cols;
+    int col[kMaxDiags];
+    // whether offset i reaches row r, for a row of [rows.x, rows.y)
+    __host__ __device__ bool has(int i, int r) const { return r + col[i] >= cols.x && r + col[i] < cols.y; }
 };
 struct NoDiags {};                    // plain plans
 template <bool SIGNED>
@@ -184,7 +187,8 @@ struct DevPlan {
     int *err;               // device error word (1: a bounded wait gave up)
     int wide_rows;          // rows of each wide direct tile (the last may have fewer)
     // plans whose dense part is one shape of at most kPlanDiags offsets
-    // (dn of them; see PlanDiags, whose first kPlanDiags they are).  dn = 0:
+    // (dn of them, in offset order): offset i adds x[r + d_col[i]] to the rows
+    // r of [d_lo[i], d_hi[i]) and no other row has a diagonal term.  dn = 0:
     // no dense part, or more than one shape / more offsets (dgen = 1: the
     // per-row shape search, diag_row)
     int dn, dgen;

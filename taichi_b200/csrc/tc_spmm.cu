@@ -18,7 +18,7 @@
 //   9-point mesh 1200^2, k = 8 (hybrid, 6 words a row)  505 -> 41
 //   9-point mesh 800^2, k = 13 (no vector loads)        231 -> 49
 //   banded 300,000 x 22, k = 32                         181 -> 55
-//   15 diagonals of 400,000 rows with holes, k = 24     185 -> 63
+//   15 diagonals of 400,000 rows with holes, k = 24     185 -> 49
 //   power-law R-MAT scale 18, k = 16                   5800 -> 129
 
 #include <cuda_runtime.h>
@@ -114,14 +114,28 @@ __device__ __forceinline__ void diag_cols(const DevPlan &p, const PlanDiags &q, 
                                           const Lane<V, VEC> &l, int r, Cols<V, VEC> &acc)
 {
     if (q.n > 0) {                // offsets from the launch parameters
+        if (r < q.rows.x || r >= q.rows.y) return;
+        if (r >= q.in.x && r < q.in.y) {                       // every offset reaches the row
+#pragma unroll 1
+            for (int i = 0; i < q.n; i += 4) {
+                Cols<V, VEC> d[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (i + u < q.n) d[u].load(Xc + (long)(r + q.col[i + u]) * ldx, l);
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (i + u < q.n) acc.add(d[u]);
+            }
+            return;
+        }
 #pragma unroll 1
         for (int i = 0; i < q.n; i += 4) {
             Cols<V, VEC> d[4];
             bool in[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                in[u] = i + u < q.n && r >= q.lo[i + u] && r < q.hi[i + u];
-                d[u].load(Xc + (long)(in[u] ? r + q.col[i + u] : 0) * ldx, l);
+                in[u] = i + u < q.n && q.has(i + u, r);
+                if (in[u]) d[u].load(Xc + (long)(r + q.col[i + u]) * ldx, l);
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u)

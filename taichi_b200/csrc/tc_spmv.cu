@@ -459,9 +459,9 @@ tc::DevPlan tc_plan::dev_plan() const
         d.dn = diags.n;
         d.d_in = diags.in;
         for (int i = 0; i < diags.n; ++i) {
-            d.d_lo[i] = diags.lo[i];
-            d.d_hi[i] = diags.hi[i];
             d.d_col[i] = diags.col[i];
+            d.d_lo[i] = std::max(diags.rows.x, diags.cols.x - diags.col[i]);
+            d.d_hi[i] = std::min(diags.rows.y, diags.cols.y - diags.col[i]);
         }
     } else if (dia_shapes > 0) {
         d.dgen = 1;
@@ -497,15 +497,14 @@ void tc_plan::set_diags()
     diags = tc::PlanDiags{};
     if (dia_shapes != 1 || num_negs > tc::kMaxDiags || (int)h_offsets.size() < num_negs) return;
     // the rows where diag_row adds each offset's term (TaiChi.cu:1014-1023)
-    const int xs = h_xStart[0], xe = h_xStop[0];
+    const int xs = h_xStart[0], xe = h_xStop[0], ys = h_yStart[0];
     diags.n = num_negs;
-    diags.in = make_int2(std::max(xs, row_start), std::min(xe, row_stop));
+    diags.rows = make_int2(std::max(xs, row_start), std::min(xe, row_stop));
+    diags.cols = make_int2(ys, ys + xe - xs);
+    diags.in = diags.rows;
     for (int i = 0; i < num_negs; ++i) {
-        const int off = h_offsets[i];
-        diags.lo[i] = std::max(xs + std::max(0, -off), row_start);
-        diags.hi[i] = std::min(xe - std::max(0, off), row_stop);
-        diags.col[i] = h_yStart[0] - xs + off;
-        diags.in = make_int2(std::max(diags.in.x, diags.lo[i]), std::min(diags.in.y, diags.hi[i]));
+        const int c = diags.col[i] = ys - xs + h_offsets[i];
+        diags.in = make_int2(std::max(diags.in.x, diags.cols.x - c), std::min(diags.in.y, diags.cols.y - c));
     }
 }
 

@@ -21,7 +21,7 @@
 //   banded 700,001 x 32                             107.5 -> 35.9
 //   banded 65,536 x 18                                8.3 -> 5.8
 //   R-MAT scale 20 (0.6 words a row)                 22.9 -> 7.1
-//   15 diagonals of 900,000 rows with holes          31.5 -> 17.2
+//   15 diagonals of 900,000 rows with holes          31.5 -> 15.0
 //   power-law R-MAT scale 20 / 18 / 16          82 / 30 / 17 -> 73 / 23 / 12
 
 #include <cuda_runtime.h>
@@ -78,13 +78,16 @@ __device__ __forceinline__ double diag_terms64(const DevPlan &p, const PlanDiags
 {
     double acc = 0.0;
     if (q.n > 0) {                // offsets from the launch parameters
+        if (r < q.rows.x || r >= q.rows.y) return acc;
+        const bool inner = r >= q.in.x && r < q.in.y;          // every offset reaches the row
 #pragma unroll 1
         for (int i = 0; i < q.n; i += 4) {
             double d[4];
             bool in[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                in[u] = i + u < q.n && r >= q.lo[i + u] && r < q.hi[i + u] && ((i + u) & (lanes - 1)) == lane;
+                in[u] = i + u < q.n && (lanes == 1 || ((i + u) & (lanes - 1)) == lane);
+                if (!inner) in[u] = in[u] && q.has(i + u, r);
                 d[u] = ldx64(x + (in[u] ? r + q.col[i + u] : 0));
             }
 #pragma unroll

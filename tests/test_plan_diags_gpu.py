@@ -1,0 +1,73 @@
+"""Hybrid plans whose diagonals come with the launch parameters, at the edges
+of that: 1, 4, 5, 8, 9, 33, 64 and 65 offsets (the last from the shape
+arrays), shapes that end inside the matrix, off the main diagonal, and cut by
+the format's row range: FP32, FP64 and four right-hand sides against numpy
+for integer x, batched launch bit-identical."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+
+pytestmark = pytest.mark.gpu
+
+
+def hybrid(M, N, x0, x1, y0, offs, seed, cut=(0, 0)):
+    """A format with one shape (rows [x0, x1), columns from y0) and a random
+    remainder of holes and left-overs, and its dense meaning as a CSR."""
+    rng = np.random.default_rng(seed)
+    words, rp = [], np.zeros(M + 1, np.int32)
+    for r in range(M):
+        n = int(rng.integers(0, 4))
+        words += ((rng.integers(0, N, n) << 1) | (rng.random(n) < 0.7)).tolist()
+        rp[r + 1] = len(words)
+    return dict(dia_shapes=1, num_negs=len(offs), dense_nnz=1, zero_elements=0, sparse_nnz=len(words),
+                row_start=x0 + cut[0], row_stop=x1 - cut[1], xStart=[x0], yStart=[y0], xStop=[x1],
+                nDiasPtr=[0, len(offs)], neg_offsets=offs, csrRow=rp, csrCol=np.array(words + [0], np.int32)[:len(words)])
+
+
+def dense_multiply(f, M, x):
+    y = np.zeros((M,) + x.shape[1:])
+    rows = np.repeat(np.arange(M), np.diff(f["csrRow"]))
+    w = f["csrCol"]
+    np.add.at(y, rows, np.where(w & 1, 1.0, -1.0).reshape((-1,) + (1,) * (x.ndim - 1)) * x[w >> 1])
+    x0, x1, y0 = f["xStart"][0], f["xStop"][0], f["yStart"][0]
+    for off in f["neg_offsets"]:
+        r = np.arange(x0, x1)
+        r = r[(r - x0 + off >= 0) & (r - x0 + off < x1 - x0) & (r >= f["row_start"]) & (r < f["row_stop"])]
+        y[r] += x[r - x0 + y0 + off]
+    return y
+
+
+@pytest.mark.parametrize("noffs", [1, 4, 5, 8, 9, 33, 64, 65])
+@pytest.mark.parametrize("box", ["whole", "inside", "cut"])
+def test_offsets(tc, dev, noffs, box):
+    import torch
+    M, N = 3001, 3300
+    x0, x1, y0, cut = {"whole": (0, 3001, 0, (0, 0)), "inside": (700, 2500, 1100, (0, 0)),
+                       "cut": (700, 2500, 300, (40, 77))}[box]
+    offs = sorted(np.random.default_rng(noffs).choice(np.arange(-90, 90), noffs, replace=False).tolist())
+    f = hybrid(M, N, x0, x1, y0, offs, noffs, cut)
+    plan = tc.Plan.from_format(M, N, f)
+    x = np.random.default_rng(2).integers(-8, 9, (N, 4)).astype(np.float64)
+    want = dense_multiply(f, M, x)
+    xd = torch.from_numpy(x[:, 0].astype(np.float32)).to(dev)
+    y = torch.full((M,), float("nan"), device=dev)
+    plan.spmv(xd, y)
+    y64 = torch.full((M,), float("nan"), dtype=torch.float64, device=dev)
+    plan.spmv_f64(torch.from_numpy(x[:, 0].copy()).to(dev), y64)
+    Y = torch.full((M, 4), float("nan"), device=dev)
+    plan.spmm(torch.from_numpy(x.astype(np.float32)).to(dev), Y)
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(y.cpu().numpy().astype(np.float64), want[:, 0])
+    np.testing.assert_array_equal(y64.cpu().numpy(), want[:, 0])
+    np.testing.assert_array_equal(Y.cpu().numpy().astype(np.float64), want)
+    xf = torch.from_numpy(np.random.default_rng(3).uniform(-1, 1, N).astype(np.float32)).to(dev)
+    plan.spmv(xf, y)
+    yb = torch.full((M,), float("nan"), device=dev)
+    b, one = C.c_void_p(), C.c_void_p * 1
+    tc.check(tc.lib().tc_batch_create(1, one(plan.handle.value), one(xf.data_ptr()), one(yb.data_ptr()), C.byref(b)))
+    tc.check(tc.lib().tc_batch_run(b, None))
+    torch.cuda.synchronize()
+    tc.check(tc.lib().tc_batch_destroy(b))
+    assert torch.equal(y, yb)
