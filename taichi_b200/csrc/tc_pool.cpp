@@ -6,8 +6,8 @@
 // pool that still holds the memory of the last build costs 2 us.  So scratch
 // comes from a memory pool of the library's own (not the device's default
 // pool, whose settings belong to the program), one per device.  It keeps at
-// most kPoolKeep bytes between builds and gives them back when the process's
-// last plan is destroyed.  The pool is found by the CUDA context it was made
+// most kPoolKeep bytes between builds and gives all but kPoolIdle of them back
+// when the process's last plan is destroyed.  The pool is found by the CUDA context it was made
 // in, so a device reset starts a new one.  Allocations and frees are ordered
 // on the build's own stream; pools are safe across threads and streams.
 
@@ -25,6 +25,10 @@ namespace tc {
 namespace {
 
 constexpr size_t kPoolKeep = 256u << 20;
+// What stays after the last plan: a program that makes and drops one plan at
+// a time does not pay for unmapping (0.3 ms, and hundreds at times when other
+// processes use the machine's driver) and mapping with every plan.
+constexpr size_t kPoolIdle = 64u << 20;
 
 ContextAddressCache<> g_pools;
 std::atomic<long> g_live_plans{0};
@@ -120,7 +124,7 @@ void plan_born() { g_live_plans.fetch_add(1, std::memory_order_relaxed); }
 void plan_gone()
 {
     if (g_live_plans.fetch_sub(1, std::memory_order_relaxed) != 1) return;
-    if (cudaMemPool_t pool = current_pool(false)) cudaMemPoolTrimTo(pool, 0);
+    if (cudaMemPool_t pool = current_pool(false)) cudaMemPoolTrimTo(pool, kPoolIdle);
     (void)cudaGetLastError();
 }
 

@@ -44,6 +44,17 @@ __device__ __forceinline__ float ldx(const float *p)
     return v;
 }
 
+// The same for a gather whose neighbours are unlikely to be gathered again by
+// this SM: its line is the first to leave L1 (wide tiles; R-MAT scale 20:
+// 4.27 -> 4.13 us per multiply.  Not for banded rows, whose neighbours share
+// lines: 93 -> 161 us).
+__device__ __forceinline__ float ldx_once(const float *p)
+{
+    float v;
+    asm("ld.global.L1::evict_first.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+
 template <bool SIGNED>
 __device__ __forceinline__ float gather(const float *__restrict__ x, int c)
 {
@@ -54,13 +65,14 @@ __device__ __forceinline__ float gather(const float *__restrict__ x, int c)
     return ldx(x + c);
 }
 
-// gather() of a signed word known to be an addition (c & 1 set: a plan
-// with no holes in its dense diagonals), without the sign select.
+// gather() of a wide tile's word (ldx_once); POS: a signed word known to be an
+// addition (c & 1 set: a plan with no holes in its dense diagonals), without
+// the sign select.
 template <bool SIGNED, bool POS>
-__device__ __forceinline__ float gather_pos(const float *__restrict__ x, int c)
+__device__ __forceinline__ float gather_once(const float *__restrict__ x, int c)
 {
-    if (SIGNED && POS) return ldx(x + (c >> 1));
-    return gather<SIGNED>(x, c);
+    const float v = ldx_once(x + (SIGNED ? c >> 1 : c));
+    return SIGNED && !POS && !(c & 1) ? -v : v;
 }
 
 // Programmatic dependent launch: a kernel reads only immutable plan data
@@ -482,6 +494,23 @@ __device__ void tile_merge(const DevPlan &p, const Tile &t, const Src &src,
 // before wait_prior_grid().
 constexpr int kStreamQ = 2;   // int4 CSR words per thread per round
 
+// The words pass L1 by: the lines they would take hold x and its misses in
+// flight, of which eight tiles' shared memory leaves room for 92 KB (tiles of
+// 6,144 words, which leave 28 KB, ran the banded matrix of 2,279,375 x 32 at
+// 157 us in place of 93).  Past it by ld.global.cg in tiles of short rows
+// (93.4 -> 92.0 us, 256 matrices in a batch 149.4 -> 148.1), without
+// allocation in mixed ones (power-law R-MAT scale 20: 69.4 -> 66.4; each form
+// loses 1 % in the other's place).
+template <bool MIXED>
+__device__ __forceinline__ int4 load_words4(const int4 *p)
+{
+    if (!MIXED) return __ldcg(p);
+    int4 v;
+    asm("ld.global.nc.L1::no_allocate.v4.s32 {%0, %1, %2, %3}, [%4];"
+        : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
 struct StreamWords {
     const int4 *cq;   // aligned-down start of the tile's CSR words
     int lead;         // words before nz0 in the first int4
@@ -489,6 +518,7 @@ struct StreamWords {
     int4 w[kStreamQ]; // this thread's first-round words
 };
 
+template <bool MIXED>
 __device__ __forceinline__ void stream_words_first(const DevPlan &p, const Tile &t, StreamWords &sw)
 {
     sw.lead = t.nz0 & 3;
@@ -497,7 +527,7 @@ __device__ __forceinline__ void stream_words_first(const DevPlan &p, const Tile 
 #pragma unroll
     for (int q = 0; q < kStreamQ; ++q) {
         const int i = threadIdx.x + q * kBlock;
-        sw.w[q] = i < sw.nq ? __ldg(sw.cq + i) : make_int4(0, 0, 0, 0);
+        sw.w[q] = i < sw.nq ? load_words4<MIXED>(sw.cq + i) : make_int4(0, 0, 0, 0);
     }
 }
 
@@ -512,7 +542,7 @@ __device__ __forceinline__ int vslot(int j) { return j + (j >> 5); }
 
 // vals[slot(lead + j)] = signed x term of entry j of the tile; ends with a
 // barrier.
-template <bool SIGNED>
+template <bool SIGNED, bool MIXED>
 __device__ __forceinline__ void stream_gather(const float *__restrict__ x, float *vals, StreamWords &sw, bool skew)
 {
     const int tid = threadIdx.x;
@@ -521,7 +551,7 @@ __device__ __forceinline__ void stream_gather(const float *__restrict__ x, float
 #pragma unroll
             for (int q = 0; q < kStreamQ; ++q) {
                 const int i = base + tid + q * kBlock;
-                sw.w[q] = i < sw.nq ? __ldg(sw.cq + i) : make_int4(0, 0, 0, 0);
+                sw.w[q] = i < sw.nq ? load_words4<MIXED>(sw.cq + i) : make_int4(0, 0, 0, 0);
             }
         }
         // signed words: every slot is gathered -- a slot past the window
@@ -619,12 +649,12 @@ __device__ void tile_stream(const DevPlan &p, const Tile &t, const float *__rest
     static_assert(kStreamRows == kBlock, "one row per thread");
     const int rl = threadIdx.x, nr = tile_nrows(t), row0 = t.row0, dc = tile_dclass(t);
     StreamWords sw;
-    stream_words_first(p, t, sw);
+    stream_words_first<MIXED>(p, t, sw);
     const int base = t.nz0 - sw.lead;                           // rowptr value of vals[0]
     const int b = rl < nr ? __ldg(p.rowptr + row0 + rl) - base : 0;
     const int e = rl < nr ? __ldg(p.rowptr + row0 + rl + 1) - base : 0;
     if (wait) wait_prior_grid(x, y);
-    stream_gather<SIGNED>(x, vals, sw, p.skew);
+    stream_gather<SIGNED, MIXED>(x, vals, sw, p.skew);
     // (Loading the rows' diagonal terms while the gathers are in flight
     // measured slower on the mesh: into registers 69.5 against 65.6 us; as
     // the tile's x segment staged in shared memory 58.3 against 52.5 us.)
@@ -664,7 +694,7 @@ __device__ void tile_stream4(const DevPlan &p, const Tile &t, const float *__res
     constexpr int GQ = kStream4Rows / (4 * kBlock);             // row groups per thread
     const int tid = threadIdx.x, nr = tile_nrows(t), row0 = t.row0, dc = tile_dclass(t);
     StreamWords sw;
-    stream_words_first(p, t, sw);
+    stream_words_first<false>(p, t, sw);
     const int base = t.nz0 - sw.lead;
     int4 rp[GQ];
     int rp4[GQ];
@@ -676,7 +706,7 @@ __device__ void tile_stream4(const DevPlan &p, const Tile &t, const float *__res
         rp4[k] = ok ? __ldg(p.rowptr + row0 + min(g + 4, nr)) : 0;
     }
     if (wait) wait_prior_grid(x, y);
-    stream_gather<SIGNED>(x, vals, sw, p.skew);
+    stream_gather<SIGNED, false>(x, vals, sw, p.skew);
 #pragma unroll
     for (int k = 0; k < GQ; ++k) {
         const int g = 4 * (tid + k * kBlock);
@@ -827,7 +857,7 @@ __device__ __forceinline__ void direct_run_full(const DevPlan &p, int dc, const 
     wait_prior_grid(x, y);
     float v[kDirectWFull];
 #pragma unroll
-    for (int w = 0; w < kDirectWFull; ++w) v[w] = gather_pos<SIGNED, POS>(x, c[w]);   // past the run: x[0], not added
+    for (int w = 0; w < kDirectWFull; ++w) v[w] = gather_once<SIGNED, POS>(x, c[w]);   // past the run: x[0], not added
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
     if (SIGNED && p.dn == 1) {
         // one dense diagonal: which rows have its term comes from the launch
@@ -858,7 +888,7 @@ __device__ __forceinline__ void direct_run_full(const DevPlan &p, int dc, const 
         for (int u = 0; u < 4; ++u)
             if (b[0] + w >= b[u] && b[0] + w < b[u + 1]) acc[u] += v[w];
     for (int j = b[0] + kDirectWFull; j < e4; ++j) {
-        const float z = gather_pos<SIGNED, POS>(x, __ldg(p.cols + j));
+        const float z = gather_once<SIGNED, POS>(x, __ldg(p.cols + j));
 #pragma unroll
         for (int u = 0; u < 4; ++u)
             if (j >= b[u] && j < b[u + 1]) acc[u] += z;
