@@ -189,15 +189,16 @@ __device__ __forceinline__ void sum_words(const DevPlan &p, const float *__restr
                                           const Lane<V, VEC> &l, int b, int e, int by, Cols<V, VEC> &acc)
 {
     for (int j = b; j < e; j += W * by) {
+        const int left = e - j;
         int c[W];
         Cols<V, VEC> v[W];
 #pragma unroll
-        for (int w = 0; w < W; ++w) c[w] = j + w * by < e ? __ldg(p.cols + j + w * by) : 0;
+        for (int w = 0; w < W; ++w) c[w] = w * by < left ? __ldg(p.cols + j + w * by) : 0;
 #pragma unroll
         for (int w = 0; w < W; ++w) v[w].load(Xc + (long)word_col<SIGNED>(c[w]) * ldx, l);
 #pragma unroll
         for (int w = 0; w < W; ++w)
-            if (j + w * by < e) add_word<SIGNED>(acc, v[w], c[w]);
+            if (w * by < left) add_word<SIGNED>(acc, v[w], c[w]);
     }
 }
 

@@ -207,9 +207,10 @@ __global__ void __launch_bounds__(kBlock, kRowsMinBlocks)
         za = __ldg(p.rowptr + ra);
         zb = __ldg(p.rowptr + min(ra + kBlock, p.M));
     }
+    const int n = e - b;
     int c[W];
 #pragma unroll
-    for (int w = 0; w < W; ++w) c[w] = b + w < e ? __ldg(p.cols + b + w) : 0;
+    for (int w = 0; w < W; ++w) c[w] = w < n ? __ldg(p.cols + b + w) : 0;
     if (ahead && threadIdx.x == 0) {
         const int ra = (blockIdx.x + p.ahead) * kBlock;
         prefetch_rows_ahead(p, ra, min(ra + kBlock, p.M), za, zb);
@@ -239,18 +240,19 @@ __global__ void __launch_bounds__(kBlock, kRowsMinBlocks)
     }
 #pragma unroll
     for (int w = 0; w < W; ++w)
-        if (b + w < e) acc += v[w];
+        if (w < n) acc += v[w];
 #pragma unroll 1
     for (int j = b + W; j < e; j += W) {                            // longer rows, W words at a time
+        const int left = e - j;
         int cc[W];
         float vv[W];
 #pragma unroll
-        for (int u = 0; u < W; ++u) cc[u] = j + u < e ? __ldg(p.cols + j + u) : 0;
+        for (int u = 0; u < W; ++u) cc[u] = u < left ? __ldg(p.cols + j + u) : 0;
 #pragma unroll
         for (int u = 0; u < W; ++u) vv[u] = gather<SIGNED>(x, cc[u]);
 #pragma unroll
         for (int u = 0; u < W; ++u)
-            if (j + u < e) acc += vv[u];
+            if (u < left) acc += vv[u];
     }
     if (r < p.M) y[r] = acc;
 }

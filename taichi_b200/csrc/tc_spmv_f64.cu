@@ -51,12 +51,18 @@ __device__ __forceinline__ void wait_prior64(const double *__restrict__ &x, doub
     asm volatile("griddepcontrol.wait;" : "+l"(x), "+l"(y)::"memory");
 }
 
+// v of an addition word (c & 1), -v of a hole's.
+__device__ __forceinline__ double signed_term64(double v, int c)
+{
+    return __hiloint2double(__double2hiint(v) ^ (int)((unsigned)~c << 31), __double2loint(v));
+}
+
 // Words j, j + by, ... (W of them, before e), and their terms added to acc.
 template <int W>
 __device__ __forceinline__ void load_words(const DevPlan &p, int j, int e, int by, int (&c)[W])
 {
 #pragma unroll
-    for (int w = 0; w < W; ++w) c[w] = j + w * by < e ? __ldg(p.cols + j + w * by) : 0;
+    for (int w = 0; w < W; ++w) c[w] = w * by < e - j ? __ldg(p.cols + j + w * by) : 0;
 }
 
 template <bool SIGNED, int W>
@@ -68,7 +74,7 @@ __device__ __forceinline__ void add_words(const double *__restrict__ x, int j, i
     for (int w = 0; w < W; ++w) v[w] = ldx64(x + (SIGNED ? c[w] >> 1 : c[w]));
 #pragma unroll
     for (int w = 0; w < W; ++w)
-        if (j + w * by < e) acc += SIGNED && !(c[w] & 1) ? -v[w] : v[w];
+        if (w * by < e - j) acc += SIGNED ? signed_term64(v[w], c[w]) : v[w];
 }
 
 // The dense-diagonal terms of row r that lane `lane` of `lanes` owns
