@@ -45,33 +45,8 @@ template <bool LEAN, int B>
 __global__ void __launch_bounds__(kBlock, B)
     batch_kernel(const DevPlan *__restrict__ plans, const BatchItem *__restrict__ items)
 {
-    union {
-        BatchItem it;
-        int4 q[4];
-    } u;
-    const int4 *src = reinterpret_cast<const int4 *>(items + blockIdx.x);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) u.q[k] = __ldg(src + k);
-    const BatchItem &it = u.it;
-    DevPlan p;                     // the fields the tile code reads
-    p.rowptr = it.rowptr;
-    p.cols = it.cols;
-    p.N = it.N;
-    p.skew = it.hybrid_skew >> 1;
-    p.dia_shapes = 0;
-    if (!(it.hybrid_skew & 1)) {
-        run_tile_part<false, LEAN>(p, it.tile, it.part, it.x, it.y, true);
-        return;
-    }
-    const DevPlan *g = plans + it.plan;
-    p.shapes = g->shapes;
-    p.shape_dias = g->shape_dias;
-    p.offsets = g->offsets;
-    p.dia_shapes = g->dia_shapes;
-    p.row_start = g->row_start;
-    p.row_stop = g->row_stop;
-    p.dn = 0;                      // offsets from the shape arrays (the descriptor's would be indexed in local memory)
-    run_tile_part<true, LEAN>(p, it.tile, it.part, it.x, it.y, true);
+    const BatchItem it = load64(items + blockIdx.x);
+    run_item<LEAN>(it.rowptr, it.cols, it.N, it.hybrid_skew, plans + it.plan, it.tile, it.part, it.x, it.y, true);
 }
 
 }  // namespace

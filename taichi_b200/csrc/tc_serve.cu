@@ -38,7 +38,7 @@ namespace tc {
 namespace {
 
 struct ReqDesc {
-    int plan;          // index into the server's device plan table
+    int plan;          // index into the server's device plan tables
     int tile_begin;    // first work item of this request in its launch
     const float *x;
     float *y;
@@ -53,35 +53,33 @@ struct BatchArgs {
     ReqDesc r[kMaxBatch];
 };
 
-// One CTA per work item (tile, or quarter of a wide direct tile) of the
-// batch's requests; request i owns items [r[i].tile_begin, r[i + 1].tile_begin).
-// Thread 0 finds the CTA's request by binary search and parks its plan
-// descriptor in shared memory; the CTA then runs the tile code of its plan's
-// word kind (plain or hybrid), so one launch serves every request of the
-// batch.  LEAN: every admitted plan holds only stream, direct and long tiles.
+// One CTA per work item (tile, or part of a wide direct tile) of the batch's
+// requests; request i owns items [r[i].tile_begin, r[i + 1].tile_begin).  Every
+// thread finds the CTA's request by binary search in the launch parameters and
+// reads what the item needs of its plan with uniform loads -- no shared-memory
+// descriptor and no barrier before the tile's words -- and the CTA runs the
+// tile code of its plan's word kind, so one launch serves every request of the
+// batch.  `large`: the items are the plans' tiles for large launches.  LEAN:
+// every admitted plan holds only stream, direct and long tiles.
 template <bool LEAN>
 __global__ void __launch_bounds__(kBlock, LEAN ? kItemManyBlocks : 1)
-    serve_kernel(const DevPlan *__restrict__ plans, const __grid_constant__ BatchArgs b)
+    serve_kernel(const DevPlan *__restrict__ plans, const ItemPlan *__restrict__ cores, int large,
+                 const __grid_constant__ BatchArgs b)
 {
-    __shared__ DevPlan sp;
-    __shared__ ReqDesc sr;
-    __shared__ int sitem;
     const int g = blockIdx.x;
-    if (threadIdx.x == 0) {
-        int lo = 0, hi = b.n;                      // r[lo].tile_begin <= g < r[hi].tile_begin
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (b.r[mid].tile_begin <= g) lo = mid; else hi = mid;
-        }
-        sr = b.r[lo];
-        sp = plans[sr.plan];
-        sitem = g - sr.tile_begin;
+    int lo = 0, hi = b.n;                          // r[lo].tile_begin <= g < r[hi].tile_begin
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (b.r[mid].tile_begin <= g) lo = mid; else hi = mid;
     }
-    __syncthreads();
-    const int parts = tile_parts(sp.per_tile, sp.wide_rows);
-    const Tile t = sp.tiles[sitem / parts];
-    if (sp.hybrid) run_tile_part<true, LEAN>(sp, t, sitem % parts, sr.x, sr.y, false);
-    else run_tile_part<false, LEAN>(sp, t, sitem % parts, sr.x, sr.y, false);
+    const int plan = b.r[lo].plan, item = g - b.r[lo].tile_begin;
+    const ItemPlan c = load64(cores + plan);
+    const int parts = tile_parts(c.per_tile, c.wide_rows);
+    const int at = parts > 1 ? item / parts : item;
+    const int4 q = __ldg(reinterpret_cast<const int4 *>((large ? c.btiles : c.tiles) + at));
+    const Tile t{q.x, q.y, q.z, q.w};
+    run_item<LEAN>(c.rowptr, c.cols, c.N, c.hybrid_skew, plans + plan, t, item - at * parts, b.r[lo].x, b.r[lo].y,
+                   false);
 }
 
 double now_s()
@@ -114,6 +112,7 @@ struct tc_server {
     std::vector<int> inflight;             // queued or running requests per plan
     int64_t used = 0;
     tc::DevPlan *d_plans = nullptr;
+    tc::ItemPlan *d_cores = nullptr;       // per plan, what a served item starts from
     int max_plans = 0;
     int nonlean = 0;                       // admitted plans with lane or merge tiles
     std::mutex admit_mu;                   // plan table vs. the dispatcher
@@ -180,7 +179,6 @@ tc_status launch_batch(tc_server *sv, tc_server::Ctx &c, std::deque<uint64_t> &p
     const bool dv = sv->mode_device_vectors != 0;
     tc::BatchArgs args;
     args.n = 0;
-    int tiles = 0;
     int64_t used = 0;
     std::vector<std::pair<uint64_t, int>> order;    // ticket, 0: shared launch, 1: its own
     std::vector<tc::ReqDesc> solo;
@@ -206,10 +204,7 @@ tc_status launch_batch(tc_server *sv, tc_server::Ctx &c, std::deque<uint64_t> &p
             solo.push_back(tc::ReqDesc{s.matrix, 0, dx, dy});
             order.emplace_back(tk, 1);
         } else {
-            args.r[args.n] = tc::ReqDesc{s.matrix, tiles, dx, dy};
-            const tc::DevPlan dp = p->dev_plan();
-            tiles += p->ntiles * tc::tile_parts(dp.per_tile, dp.wide_rows);
-            ++args.n;
+            args.r[args.n++] = tc::ReqDesc{s.matrix, 0, dx, dy};
             order.emplace_back(tk, 0);
         }
         s.state.store(tc::kRunning, std::memory_order_relaxed);
@@ -224,9 +219,21 @@ tc_status launch_batch(tc_server *sv, tc_server::Ctx &c, std::deque<uint64_t> &p
         TC_CUDA(cudaEventRecord(c.join, c.s2));
     }
     const bool lean = sv->nonlean == 0;
+    // the requests' items: the plans' own tiles while they fill at most one
+    // wave of CTAs, else the tiles for large launches
+    int tiles = 0, large = 0;
+    for (; large < 2; ++large) {
+        tiles = 0;
+        for (int i = 0; i < args.n; ++i) {
+            const tc_plan *p = sv->plans[args.r[i].plan];
+            args.r[i].tile_begin = tiles;
+            tiles += (large ? p->nbtiles : p->ntiles) * (p->ntiles_wide ? tc::tile_parts(3, p->wide_rows) : 1);
+        }
+        if (large || tiles <= tc::kItemManyBlocks * tc::num_sms()) break;
+    }
     if (tiles > 0) {
-        if (lean) tc::serve_kernel<true><<<tiles, tc::kBlock, 0, c.s>>>(sv->d_plans, args);
-        else tc::serve_kernel<false><<<tiles, tc::kBlock, 0, c.s>>>(sv->d_plans, args);
+        if (lean) tc::serve_kernel<true><<<tiles, tc::kBlock, 0, c.s>>>(sv->d_plans, sv->d_cores, large, args);
+        else tc::serve_kernel<false><<<tiles, tc::kBlock, 0, c.s>>>(sv->d_plans, sv->d_cores, large, args);
     }
     TC_CUDA(cudaGetLastError());
     if (!solo.empty()) TC_CUDA(cudaStreamWaitEvent(c.s, c.join, 0));
@@ -372,6 +379,7 @@ tc_status tc_server_create(const tc_serve_config *cfg, tc_server **out)
         return fail(TC_ERR_ALLOC, "host allocation of %llu request slots", (unsigned long long)ring);
     }
     cudaError_t e = cudaMalloc(&sv->d_plans, sizeof(tc::DevPlan) * (size_t)c.max_plans);
+    if (e == cudaSuccess) e = cudaMalloc(&sv->d_cores, sizeof(tc::ItemPlan) * (size_t)c.max_plans);
     sv->ctx.resize(c.contexts);
     for (auto &x : sv->ctx) {
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&x.s, cudaStreamNonBlocking);
@@ -415,7 +423,9 @@ tc_status tc_server_admit(tc_server *sv, tc_plan *plan, int *id)
         sv->inflight.push_back(0);
     }
     const tc::DevPlan dp = plan->dev_plan();
+    const tc::ItemPlan core = tc::item_plan(dp, plan->d_btiles);
     TC_CUDA(cudaMemcpy(sv->d_plans + slot, &dp, sizeof dp, cudaMemcpyHostToDevice));
+    TC_CUDA(cudaMemcpy(sv->d_cores + slot, &core, sizeof core, cudaMemcpyHostToDevice));
     sv->plans[slot] = plan;
     sv->footprint[slot] = fp;
     sv->nonlean += lean_plan(plan) ? 0 : 1;
@@ -682,6 +692,7 @@ tc_status tc_server_destroy(tc_server *sv)
         if (c.s) cudaStreamDestroy(c.s);
     }
     if (sv->d_plans) cudaFree(sv->d_plans);
+    if (sv->d_cores) cudaFree(sv->d_cores);
     delete[] sv->slots;
     delete sv;
     return TC_OK;

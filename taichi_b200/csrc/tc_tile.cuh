@@ -1072,4 +1072,66 @@ __device__ __forceinline__ void run_tile_part(const DevPlan &p, const Tile &t, i
     else run_tile<SIGNED>(p, t, x, y, wait);
 }
 
+// What an item of a batch or served launch needs of its plan to start: the
+// fields the tile code reads, in 64 bytes, so that every thread of the CTA
+// takes them with four loads.  The rest (dense diagonals) is read from the
+// plan's descriptor, by hybrid plans only.
+struct alignas(64) ItemPlan {
+    const int *rowptr, *cols;
+    const Tile *tiles;     // the plan's own tiles
+    const Tile *btiles;    // the tiles for large launches
+    int N;
+    int wide_rows;
+    int per_tile;
+    int hybrid_skew;       // bit 0: hybrid plan, bit 1: skewed slots
+    long unused[2];
+};
+static_assert(sizeof(ItemPlan) == 64, "read as four int4s");
+
+inline ItemPlan item_plan(const DevPlan &d, const Tile *btiles)
+{
+    return ItemPlan{d.rowptr, d.cols, d.tiles, btiles, d.N, d.wide_rows, d.per_tile,
+                    (d.hybrid ? 1 : 0) | (d.skew ? 2 : 0), {0, 0}};
+}
+
+// 64 bytes of plan or item data by uniform loads.
+template <class T>
+__device__ __forceinline__ T load64(const T *src)
+{
+    static_assert(sizeof(T) == 64, "four int4s");
+    union {
+        T v;
+        int4 q[4];
+    } u;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) u.q[k] = __ldg(reinterpret_cast<const int4 *>(src) + k);
+    return u.v;
+}
+
+// Runs one item of a plan.  d: the plan's descriptor in device memory.
+template <bool LEAN>
+__device__ __forceinline__ void run_item(const int *rowptr, const int *cols, int N, int hybrid_skew,
+                                         const DevPlan *__restrict__ d, const Tile &t, int part,
+                                         const float *__restrict__ x, float *__restrict__ y, bool wait)
+{
+    DevPlan p;                     // the fields the tile code reads
+    p.rowptr = rowptr;
+    p.cols = cols;
+    p.N = N;
+    p.skew = hybrid_skew >> 1;
+    p.dia_shapes = 0;
+    if (!(hybrid_skew & 1)) {
+        run_tile_part<false, LEAN>(p, t, part, x, y, wait);
+        return;
+    }
+    p.shapes = d->shapes;
+    p.shape_dias = d->shape_dias;
+    p.offsets = d->offsets;
+    p.dia_shapes = d->dia_shapes;
+    p.row_start = d->row_start;
+    p.row_stop = d->row_stop;
+    p.dn = 0;                      // offsets from the shape arrays (the descriptor's would be indexed in local memory)
+    run_tile_part<true, LEAN>(p, t, part, x, y, wait);
+}
+
 }  // namespace tc
