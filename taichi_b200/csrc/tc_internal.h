@@ -288,12 +288,14 @@ int wide_tile_rows(int M, const tc_params &prm, int sms);
 // Resident CTAs per SM the lean one-CTA-per-tile kernel is compiled for
 // (40 registers: the stream tiles' words, terms and row pointers fit
 // without spills).
-constexpr int kLeanMinBlocks = 6, kLeanMinBlocksSigned = 6;
-// The stream-only kernel for plans of more tiles than one wave at that
-// occupancy: 8 CTAs per SM at 32 registers (no spills).  Many waves of tiles
-// gain from the extra resident loads (9-point mesh on 2048^2: 63.2 -> 52.5
-// µs); a single wave loses from the thinner threads (n = 65,536 random
-// matrix: 5.6 -> 6.7 µs), so a plan takes it only above one wave.
+constexpr int kLeanMinBlocks = 6;
+// The stream-only kernel: 5 CTAs per SM (48 registers) for plans that fit one
+// wave of them, where each CTA's chain counts (65,536 rows of 18 words, 60,000
+// of 39 and 100,000 of 29, iterated: 5.3 -> 4.9, 5.1 -> 4.6 and 5.6 -> 5.2 us
+// against 6 CTAs; 6.4 at 7 or 8); 8 CTAs at 32 registers (no spills) for plans
+// of more tiles, which gain from the extra resident loads (9-point mesh on
+// 2048^2: 63.2 -> 52.5 us).
+constexpr int kStreamFewMinBlocks = 5;
 constexpr int kStreamManyMinBlocks = 8;
 // The rows kernel: 8 CTAs per SM (32 registers) with one strip of rows per
 // CTA, 4 with two.

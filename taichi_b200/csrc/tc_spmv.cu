@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(kBlock, kRowsMinBlocks)
 // shared-memory stages (stream tiles read their CSR words as coalesced int4s;
 // direct and long tiles read global memory directly).
 template <bool SIGNED>
-__global__ void __launch_bounds__(kBlock, SIGNED ? kLeanMinBlocksSigned : kLeanMinBlocks)
+__global__ void __launch_bounds__(kBlock, kLeanMinBlocks)
     spmv_grid_kernel(DevPlan p, const float *__restrict__ x, float *__restrict__ y)
 {
     allow_next_grid();
@@ -302,8 +302,7 @@ __global__ void __launch_bounds__(kDirectWideBlock, 2)
 // matrices of short, even rows): the grid kernel with no code for the other
 // tile kinds.  MANY: more tiles than one wave, compiled for 8 CTAs per SM.
 template <bool SIGNED, bool MANY>
-__global__ void __launch_bounds__(kBlock, MANY ? kStreamManyMinBlocks
-                                               : (SIGNED ? kLeanMinBlocksSigned : kLeanMinBlocks))
+__global__ void __launch_bounds__(kBlock, MANY ? kStreamManyMinBlocks : kStreamFewMinBlocks)
     spmv_stream_kernel(DevPlan p, const float *__restrict__ x, float *__restrict__ y)
 {
     allow_next_grid();
@@ -388,7 +387,7 @@ static tc_status launch_tiles(const DevPlan &dp, const PlanDiags &dg, const Wide
         else if (dp.rows_w <= 6) TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_rows_kernel<SIGNED, 6>, dp, q, x, y));
         else TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_rows_kernel<SIGNED, 8>, dp, q, x, y));
     }
-    else if (dp.per_tile == 4 && dp.ntiles > kLeanMinBlocks * num_sms())
+    else if (dp.per_tile == 4 && dp.ntiles > kStreamFewMinBlocks * num_sms())
         TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_stream_kernel<SIGNED, true>, dp, x, y));
     else if (dp.per_tile == 4) TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_stream_kernel<SIGNED, false>, dp, x, y));
     else if (dp.per_tile) TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_grid_kernel<SIGNED>, dp, x, y));
