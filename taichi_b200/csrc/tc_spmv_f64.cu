@@ -17,11 +17,11 @@
 // -> word -> x.  Rows of a few words strided over a tile's CTA, one dependent
 // word and gather after the other, which this replaces, ran at 35 % of the
 // copy rate.  Measured per multiply (us, before -> now):
-//   9-point mesh 1531^2 (hybrid, 6 words a row)      45.1 -> 30.0
+//   9-point mesh 1531^2 (hybrid, 6 words a row)      45.1 -> 27.8
 //   banded 700,001 x 32                             107.5 -> 35.9
-//   banded 65,536 x 18                                8.3 -> 5.8
-//   R-MAT scale 20 (0.6 words a row)                 22.9 -> 7.1
-//   15 diagonals of 900,000 rows with holes          31.5 -> 15.0
+//   banded 65,536 x 18                                8.3 -> 4.9
+//   R-MAT scale 20 (0.6 words a row)                 22.9 -> 6.9
+//   15 diagonals of 900,000 rows with holes          31.5 -> 14.4
 //   power-law R-MAT scale 20 / 18 / 16          82 / 30 / 17 -> 73 / 23 / 12
 
 #include <cuda_runtime.h>
@@ -142,6 +142,11 @@ __global__ void __launch_bounds__(kBlock, kF64Blocks)
     const int row0 = blockIdx.x * R, group = threadIdx.x >> LG, lane = threadIdx.x & (G - 1);
     const bool ok = group < p.M - row0;
     const int r = row0 + group;
+    // one lane a row: most words are near the row, so the CTA's x goes to L2
+    // while its row pointers and words are on the way (mesh 29.3 -> 27.8 us);
+    // with lane groups the rows are few and their words far: 35.9 -> 37.5 on
+    // the banded 700,001
+    if (LG == 0 && threadIdx.x == 0) prefetch_x_window(x, p.N, row0, R);
     if (threadIdx.x == 0 && (long)row0 + (long)ahead * R < p.M) {
         const int ra = row0 + ahead * R, rb = ra + min(R, p.M - ra);
         const int za = __ldg(p.rowptr + ra), zb = __ldg(p.rowptr + rb);

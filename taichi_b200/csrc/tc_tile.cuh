@@ -117,7 +117,8 @@ __device__ __forceinline__ void after_wait(const float *__restrict__ &x, float *
 // is only a hint and L2 is where every SM's writes land, so it may be issued
 // before wait_prior_grid(): a later write of x by an earlier grid still
 // reaches the loads that follow the wait.
-__device__ __forceinline__ void prefetch_x_window(const float *x, int N, int r0, int n)
+template <typename V>
+__device__ __forceinline__ void prefetch_x_window(const V *x, int N, int r0, int n)
 {
     const int a = max(r0, 0), b = min(r0 + n, N);
     if (b <= a) return;
