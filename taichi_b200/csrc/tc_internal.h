@@ -57,6 +57,9 @@ struct Scratch {
     void release();
     template <class T> T *as() const { return static_cast<T *>(p); }
 };
+// cudaMalloc that gives the pool's unused memory back and tries again before
+// it fails (waits for `stream` then).
+tc_status device_alloc(void **p, size_t bytes, cudaStream_t stream);
 // Plans alive in the process (the pool is trimmed when the last one goes).
 void plan_born();
 void plan_gone();
@@ -244,7 +247,7 @@ struct tc_plan {
     int *d_err = nullptr;
     int wide_rows = 0;                   // rows of each wide direct tile
     int stream_skew = 0;                 // the plan's usual row length is a multiple of 8
-    int rows_w = 8;                      // the rows kernel's words in flight (the usual row length, 4 / 6 / 8)
+    int rows_w = 8;                      // the rows kernel's words in flight (the usual row length, 2 / 4 / 6 / 8)
     int all_pos = 0;                     // hybrid plan with no holes (every word an addition)
     // window plan (tc_window.cu); nwtiles == 0 when the plan has none
     tc::Tile *d_wtiles = nullptr;
@@ -287,7 +290,8 @@ tc_status tiles_grid(const DevPlan &dp, int ctas_per_sm, int *grid);
 int wide_tile_rows(int M, const tc_params &prm, int sms);
 // Resident CTAs per SM the lean one-CTA-per-tile kernel is compiled for
 // (40 registers: the stream tiles' words, terms and row pointers fit
-// without spills).
+// without spills; power-law R-MAT scale 20 at 5 / 6 / 7 / 8: 70.2 / 66.7 / 72.3
+// / 72.3 us).
 constexpr int kLeanMinBlocks = 6;
 // The stream-only kernel: 5 CTAs per SM (48 registers) for plans that fit one
 // wave of them, where each CTA's chain counts (65,536 rows of 18 words, 60,000
@@ -297,8 +301,7 @@ constexpr int kLeanMinBlocks = 6;
 // 2048^2: 63.2 -> 52.5 us).
 constexpr int kStreamFewMinBlocks = 5;
 constexpr int kStreamManyMinBlocks = 8;
-// The rows kernel: 8 CTAs per SM (32 registers) with one strip of rows per
-// CTA, 4 with two.
+// The rows kernel: 8 CTAs per SM (32 registers).
 constexpr int kRowsMinBlocks = 8;
 // The same for the batch and served kernels: 6 CTAs per SM for a batch of one
 // or two waves, 8 (32 registers) for more, and for served launches.  Batches

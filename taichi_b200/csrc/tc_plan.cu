@@ -3,12 +3,12 @@
 //
 // Replaces the upload part of taichi_SpMV (TaiChi.cu:1357-1385).  The format
 // comes from host arrays or, after a partition, from device arrays; either
-// way the row statistics and the tile list are computed on the GPU, so a partitioned matrix never crosses
-// the host link.  What bounds a build is then the copies of the format (read
-// and written once) and a few round trips of counts to the host.  Measured on
-// the 9-point mesh 2048^2 (25.7 M words): 1 ms from device arrays in place of
-// 85 ms for the copy to the host, the host's passes over the words and rows,
-// and the copy back.
+// way the row statistics and the tile list are computed on the GPU, so a
+// partitioned matrix never crosses the host link.  What bounds a build is then
+// the copies of the format (read and written once) and a few round trips of
+// counts to the host.  Measured on the 9-point mesh 2048^2 (25.7 M words): 1 ms
+// from device arrays in place of 85 ms for the copy to the host, the host's
+// passes over the words and rows, and the copy back.
 
 #include <cuda_runtime.h>
 
@@ -418,11 +418,8 @@ tc_status plan_upload(tc_plan *p, const int *csrRow, const int *csrCol, int64_t 
     const size_t o_bt = align256(o_tiles + sizeof(Tile) * (size_t)p->ntiles);
     const size_t o_wt = align256(o_bt + sizeof(Tile) * (size_t)(own ? 0 : p->nbtiles));
     const size_t total = align256(o_wt + sizeof(Tile) * wtiles.size());
-    char *base = nullptr;
-    const cudaError_t e = cudaMalloc(&base, total);
-    if (e != cudaSuccess)
-        return fail(TC_ERR_ALLOC, "cudaMalloc(%zu) for the plan: %s", total, cudaGetErrorString(e));
-    p->dev = base;
+    TC_CHECK(device_alloc(&p->dev, total, stream));
+    char *const base = static_cast<char *>(p->dev);
     p->dev_bytes = total;
     p->d_rowptr = reinterpret_cast<int *>(base);
     p->d_cols = reinterpret_cast<int *>(base + o_cols);

@@ -7,7 +7,8 @@
 // comes from a memory pool of the library's own (not the device's default
 // pool, whose settings belong to the program), one per device.  It keeps at
 // most kPoolKeep bytes between builds and gives all but kPoolIdle of them back
-// when the process's last plan is destroyed.  The pool is found by the CUDA context it was made
+// when the process's last plan is destroyed; a plan that finds no room takes
+// all of them back first.  The pool is found by the CUDA context it was made
 // in, so a device reset starts a new one.  Allocations and frees are ordered
 // on the build's own stream; pools are safe across threads and streams.
 
@@ -112,10 +113,22 @@ tc_status Scratch::alloc(size_t bytes, cudaStream_t stream)
     pooled = pool && cudaMallocFromPoolAsync(&p, bytes, pool, stream) == cudaSuccess;
     if (pooled) return TC_OK;
     (void)cudaGetLastError();
-    const cudaError_t e = cudaMalloc(&p, bytes);
+    return device_alloc(&p, bytes, stream);
+}
+
+tc_status device_alloc(void **p, size_t bytes, cudaStream_t stream)
+{
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) {               // once more without what the pool holds unused
+        (void)cudaGetLastError();
+        if (cudaMemPool_t pool = current_pool(false)) {
+            if (cudaStreamSynchronize(stream) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
+            e = cudaMalloc(p, bytes);
+        }
+    }
     if (e == cudaSuccess) return TC_OK;
     (void)cudaGetLastError();
-    p = nullptr;
+    *p = nullptr;
     return fail(TC_ERR_ALLOC, "cudaMalloc(%zu): %s", bytes, cudaGetErrorString(e));
 }
 
