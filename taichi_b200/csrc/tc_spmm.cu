@@ -19,7 +19,7 @@
 //   9-point mesh 800^2, k = 13 (no vector loads)        231 -> 49
 //   banded 300,000 x 22, k = 32                         181 -> 55
 //   15 diagonals of 400,000 rows with holes, k = 24     185 -> 49
-//   power-law R-MAT scale 18, k = 16                   5800 -> 129
+//   power-law R-MAT scale 18, k = 16                   5800 -> 112
 
 #include <cuda_runtime.h>
 
@@ -208,7 +208,8 @@ __device__ __forceinline__ void sum_words(const DevPlan &p, const float *__restr
 // joins the parts.
 template <bool SIGNED, int V, bool VEC, int W, bool MID>
 __device__ __forceinline__ void spmm_rows(const DevPlan &p, const typename DiagsOf<SIGNED>::type &q,
-                                          const float *__restrict__ Xc, int ldx, const Lane<V, VEC> &l, int lg, int row0, int nrow,
+                                          const float *__restrict__ Xc, int ldx, const Lane<V, VEC> &l, int lg,
+                                           int row0, int nrow,
                                           float *__restrict__ Yc, int ldy)
 {
     const int group = threadIdx.x >> lg, r = row0 + group;
@@ -246,7 +247,8 @@ __device__ __forceinline__ void spmm_rows(const DevPlan &p, const typename Diags
 // CTA.
 template <bool SIGNED, int V, bool VEC, int W>
 __global__ void __launch_bounds__(kBlock, spmm_blocks(V, W))
-    spmm_rows_kernel(DevPlan p, const __grid_constant__ typename DiagsOf<SIGNED>::type q, const float *__restrict__ X, int ldx, int k, int lg, int ahead,
+    spmm_rows_kernel(DevPlan p, const __grid_constant__ typename DiagsOf<SIGNED>::type q,
+                     const float *__restrict__ X, int ldx, int k, int lg, int ahead,
                      float *__restrict__ Y, int ldy)
 {
     const int groups = kBlock >> lg, row0 = blockIdx.x * groups;
@@ -262,7 +264,8 @@ __global__ void __launch_bounds__(kBlock, spmm_blocks(V, W))
 // group joins the parts in group order.
 template <bool SIGNED, int V, bool VEC, int W>
 __global__ void __launch_bounds__(kBlock, spmm_blocks(V, W))
-    spmm_tiles_kernel(DevPlan p, const __grid_constant__ typename DiagsOf<SIGNED>::type q, const float *__restrict__ X, int ldx, int k, int lg, float *__restrict__ Y,
+    spmm_tiles_kernel(DevPlan p, const __grid_constant__ typename DiagsOf<SIGNED>::type q,
+                      const float *__restrict__ X, int ldx, int k, int lg, float *__restrict__ Y,
                       int ldy)
 {
     __shared__ float part[kBlock * V];
@@ -356,8 +359,8 @@ __global__ void __launch_bounds__(kBlock, kRunBlocks)
 }
 
 template <bool SIGNED, int V, bool VEC>
-tc_status launch(const DevPlan &dp, const PlanDiags &dg, int64_t nnz_csr, int max_row, const float *X, int ldx, int k, float *Y,
-                 int ldy, cudaStream_t s)
+tc_status launch(const DevPlan &dp, const PlanDiags &dg, int64_t nnz_csr, int max_row, const float *X, int ldx, int k,
+                 float *Y, int ldy, cudaStream_t s)
 {
     int lg = 0;
     while ((V << lg) < k) ++lg;
@@ -367,7 +370,7 @@ tc_status launch(const DevPlan &dp, const PlanDiags &dg, int64_t nnz_csr, int ma
     // or more (a run of 2^lg rows; smaller groups diverge more than they
     // save).  Longer rows keep a group's loads in flight by themselves.
     if (!SIGNED && lg >= 3 && max_row <= kSpmmMidRow && nnz_csr <= 2LL * dp.M) {
-        const unsigned grid = (unsigned)((dp.M + kBlock - 1) / kBlock);
+        const unsigned grid = (unsigned)((dp.M + (long)kBlock - 1) / kBlock);
         spmm_run_kernel<V, VEC, 4><<<grid, kBlock, 0, s>>>(dp, X, ldx, k, lg, kRunBlocks * num_sms(), Y, ldy);
     } else if (max_row > kSpmmMidRow) {
         spmm_tiles_kernel<SIGNED, V, VEC, 4><<<dp.ntiles, kBlock, 0, s>>>(dp, q, X, ldx, k, lg, Y, ldy);
@@ -390,8 +393,8 @@ tc_status launch(const DevPlan &dp, const PlanDiags &dg, int64_t nnz_csr, int ma
 }
 
 template <bool SIGNED>
-tc_status launch_cols(const DevPlan &dp, const PlanDiags &dg, int64_t nnz_csr, int max_row, const float *X, int ldx, int k, float *Y,
-                      int ldy, cudaStream_t s)
+tc_status launch_cols(const DevPlan &dp, const PlanDiags &dg, int64_t nnz_csr, int max_row, const float *X, int ldx,
+                      int k, float *Y, int ldy, cudaStream_t s)
 {
     const uintptr_t at = reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Y);
     const int all = ldx | ldy | k;
@@ -406,8 +409,8 @@ tc_status launch_cols(const DevPlan &dp, const PlanDiags &dg, int64_t nnz_csr, i
 
 }  // namespace
 
-tc_status launch_spmm(const DevPlan &dp, const PlanDiags &dg, int64_t nnz_csr, int max_row, const float *X, int ldx, int k, float *Y,
-                      int ldy, cudaStream_t s)
+tc_status launch_spmm(const DevPlan &dp, const PlanDiags &dg, int64_t nnz_csr, int max_row, const float *X, int ldx,
+                      int k, float *Y, int ldy, cudaStream_t s)
 {
     if (dp.M == 0) return TC_OK;
     if (dp.N == 0) {      // no terms, and no X for the lanes' unconditional loads

@@ -350,8 +350,8 @@ tc_status tiles_grid(const DevPlan &dp, int ctas_per_sm, int *grid)
 }
 
 template <bool SIGNED>
-static tc_status launch_tiles(const DevPlan &dp, const PlanDiags &dg, const WideBounds *wb, const WideStarts *ws, const float *x,
-                              float *y, cudaStream_t s)
+static tc_status launch_tiles(const DevPlan &dp, const PlanDiags &dg, const WideBounds *wb, const WideStarts *ws,
+                              const float *x, float *y, cudaStream_t s)
 {
     if (dp.ntiles <= 0) return TC_OK;
     const size_t smem = dp.per_tile ? 0 : stream_smem_bytes(dp);
@@ -395,8 +395,8 @@ static tc_status launch_tiles(const DevPlan &dp, const PlanDiags &dg, const Wide
     return TC_OK;
 }
 
-tc_status launch_spmv(const DevPlan &dp, const PlanDiags &dg, const float *x, float *y, cudaStream_t s, const WideBounds *wb,
-                      const WideStarts *ws)
+tc_status launch_spmv(const DevPlan &dp, const PlanDiags &dg, const float *x, float *y, cudaStream_t s,
+                      const WideBounds *wb, const WideStarts *ws)
 {
     if (dp.M == 0) return TC_OK;
     // no columns: no terms, and the kernels' unconditional loads of x[0]

@@ -9,9 +9,9 @@
 // butterfly.  Plans of short rows run kBlock >> lg consecutive rows a CTA
 // straight from the row pointers; plans with rows of more than kShortRow words
 // run a CTA per tile of the plan's list (whose words are bounded), leaving a
-// row that is long for its tile to a warp and a one-row tile to the whole CTA.  The launch may overlap the end of
-// the kernel before it, as in FP32: x is read and y written after
-// griddepcontrol.wait only, with coherent loads.
+// row that is long for its tile to a warp and a one-row tile to the whole CTA.
+// The launch may overlap the end of the kernel before it, as in FP32: x is
+// read and y written after griddepcontrol.wait only, with coherent loads.
 //
 // What bounds it: bytes (8 per x and y value), and the latency of row pointer
 // -> word -> x.  Rows of a few words strided over a tile's CTA, one dependent
@@ -135,7 +135,8 @@ __device__ __forceinline__ double group_sum(double v, int lanes)
 // Short rows: kBlock >> LG rows a CTA.
 template <bool SIGNED, int LG>
 __global__ void __launch_bounds__(kBlock, kF64Blocks)
-    f64_rows_kernel(DevPlan p, const __grid_constant__ typename DiagsOf<SIGNED>::type q, int ahead, const double *__restrict__ x, double *__restrict__ y)
+    f64_rows_kernel(DevPlan p, const __grid_constant__ typename DiagsOf<SIGNED>::type q, int ahead,
+                    const double *__restrict__ x, double *__restrict__ y)
 {
     constexpr int G = 1 << LG, R = kBlock >> LG, W = LG ? 4 : 3;
     allow_next_grid();
@@ -184,7 +185,8 @@ __device__ __forceinline__ void sum_words64(const DevPlan &p, const double *__re
 // Any plan: a CTA per tile.
 template <bool SIGNED>
 __global__ void __launch_bounds__(kBlock, kF64Blocks)
-    f64_tiles_kernel(DevPlan p, const __grid_constant__ typename DiagsOf<SIGNED>::type q, const double *__restrict__ x, double *__restrict__ y)
+    f64_tiles_kernel(DevPlan p, const __grid_constant__ typename DiagsOf<SIGNED>::type q,
+                     const double *__restrict__ x, double *__restrict__ y)
 {
     __shared__ double red[kBlock / 32];
     allow_next_grid();
@@ -237,7 +239,8 @@ __global__ void __launch_bounds__(kBlock, kF64Blocks)
 }
 
 template <bool SIGNED>
-tc_status launch_f64(const DevPlan &dp, const PlanDiags &dg, int64_t nnz_csr, int max_row, const double *x, double *y, cudaStream_t s)
+tc_status launch_f64(const DevPlan &dp, const PlanDiags &dg, int64_t nnz_csr, int max_row, const double *x, double *y,
+                     cudaStream_t s)
 {
     typename DiagsOf<SIGNED>::type q;
     if constexpr (SIGNED) q = dg;
