@@ -8,7 +8,7 @@
 //                  thumbnail row, bits in shared memory.
 //  2. morphology   hole fill (imfill) by union-find over runs of zeros; 30x1
 //                  and 1x30 openings, subtraction and the eye(5) opening on
-//                  bit-packed rows in one CTA, with OpenCV's conventions
+//                  bit-packed rows, with OpenCV's conventions
 //                  (non-reflected element, anchor at the centre, erosion sees
 //                  1 and dilation 0 outside the image).
 //  3. contours     findContours(RETR_CCOMP, CHAIN_APPROX_NONE): union-find
@@ -245,10 +245,11 @@ __global__ void fill_holes(Img B, int *L, Img F)
 }
 
 // --------------------------------------------------------------- morphology
-// The openings in one CTA (65 us for a 512 x 512 thumbnail, most of it the
-// vertical lines' 30 shared-memory reads a word; the horizontal ones take 5
-// steps in registers); images live wherever the pointers say (shared
-// memory for thumbnails up to 50 KB per image, else global memory).
+// The openings on bit-packed rows, a launch for each step that needs its
+// neighbours' results: the 30x1 opening stays inside a row, the 1x30 one inside
+// a column of words, so each is one launch with a barrier between its erosion
+// and dilation; the eye crosses both and takes two.  Bound by launch latency
+// on a 512 x 512 thumbnail: 17 us in four launches, 65 in one CTA.
 
 // AND (erode) or OR over the L pixels x - a .. x - a + L - 1 of a row for the
 // 32 pixels x of word k, a = L / 2; outside the image the neutral value.
@@ -278,61 +279,58 @@ __device__ __forceinline__ unsigned line_h(const Img &src, int y, int k, int L, 
     return erode ? v : ~v;
 }
 
-__device__ void erode_dilate_h(const Img &src, Img &tmp, Img &dst, int L)
+// Opening by L x 1: blockDim.x / WW whole rows a CTA (at least one).
+__global__ void open_rows(Img src, Img tmp, Img dst, int L)
 {
-    const int n = src.H * src.WW;
+    const int WW = src.WW, per = max(1, (int)blockDim.x / WW), y0 = blockIdx.x * per;
+    const int n = min(per, src.H - y0) * WW;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const int y = i / src.WW, k = i % src.WW;
-        tmp.w[i] = line_h(src, y, k, L, true) & word_mask(src, k);
+        const int y = y0 + i / WW, k = i % WW;
+        tmp.w[y * WW + k] = line_h(src, y, k, L, true) & word_mask(src, k);
     }
     __syncthreads();
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const int y = i / src.WW, k = i % src.WW;
-        dst.w[i] = line_h(tmp, y, k, L, false) & word_mask(src, k);
+        const int y = y0 + i / WW, k = i % WW;
+        dst.w[y * WW + k] = line_h(tmp, y, k, L, false) & word_mask(src, k);
     }
-    __syncthreads();
 }
 
-__device__ void erode_dilate_v(const Img &src, Img &tmp, Img &dst, int L)
+// O = opening of src by 1 x L, D = B - O (saturating): a CTA per column of
+// words, in shared memory (2 H words).
+__global__ void open_cols(Img src, Img B, Img O, Img D, int L)
 {
-    const int a = L / 2;
-    const int n = src.H * src.WW;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const int y = i / src.WW;
+    extern __shared__ unsigned col[];
+    const int k = blockIdx.x, H = src.H, WW = src.WW, a = L / 2;
+    unsigned *const er = col + H;
+    for (int y = threadIdx.x; y < H; y += blockDim.x) col[y] = src.w[y * WW + k];
+    __syncthreads();
+    for (int y = threadIdx.x; y < H; y += blockDim.x) {
         unsigned v = 0xffffffffu;
-        for (int r = max(y - a, 0); r < min(y + L - a, src.H); ++r) v &= src.w[i + (r - y) * src.WW];
-        tmp.w[i] = v;
+        for (int r = max(y - a, 0); r < min(y + L - a, H); ++r) v &= col[r];
+        er[y] = v;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const int y = i / src.WW;
+    for (int y = threadIdx.x; y < H; y += blockDim.x) {
         unsigned v = 0;
-        for (int r = max(y - a, 0); r < min(y + L - a, src.H); ++r) v |= tmp.w[i + (r - y) * src.WW];
-        dst.w[i] = v;
+        for (int r = max(y - a, 0); r < min(y + L - a, H); ++r) v |= er[r];
+        O.w[y * WW + k] = v;
+        D.w[y * WW + k] = B.w[y * WW + k] & ~v;
     }
-    __syncthreads();
 }
 
-__device__ void erode_dilate_eye(const Img &src, Img &tmp, Img &dst, int K)
+// Erosion or dilation by the K x K eye (diagonal line).
+template <bool ERODE>
+__global__ void eye_pass(Img src, Img dst, int K)
 {
-    const int a = K / 2;
-    const int n = src.H * src.WW;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const int y = i / src.WW, k = i % src.WW;
-        unsigned v = 0xffffffffu;
-        for (int t = 0; t < K; ++t) v &= src.shifted(y + t - a, k, t - a, 0xffffffffu);
-        if (k == src.WW - 1) v &= src.lastmask();
-        tmp.w[i] = v;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, WW = src.WW;
+    if (i >= src.H * WW) return;
+    const int y = i / WW, k = i % WW, a = K / 2;
+    unsigned v = ERODE ? 0xffffffffu : 0u;
+    for (int t = 0; t < K; ++t) {
+        const unsigned u = src.shifted(y + t - a, k, t - a, ERODE ? 0xffffffffu : 0u);
+        v = ERODE ? v & u : v | u;
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const int y = i / src.WW, k = i % src.WW;
-        unsigned v = 0;
-        for (int t = 0; t < K; ++t) v |= tmp.shifted(y + t - a, k, t - a, 0u);
-        if (k == src.WW - 1) v &= src.lastmask();
-        dst.w[i] = v;
-    }
-    __syncthreads();
+    dst.w[i] = v & word_mask(src, k);
 }
 
 struct MorphArgs {
@@ -340,34 +338,7 @@ struct MorphArgs {
     Img O2, D, E;             // open-open, subtracted, eye-opened
     Img T1, T2;               // scratch
     int open_len, eye;
-    int use_smem;
 };
-
-__global__ void __launch_bounds__(1024) morph_kernel(MorphArgs a)
-{
-    extern __shared__ unsigned sm[];
-    const int n = a.B.H * a.B.WW;
-    Img F = a.F, O2 = a.O2, E = a.E, T1 = a.T1, T2 = a.T2;
-    if (a.use_smem) {   // work on shared copies; results are written back
-        F.w = sm; T1.w = sm + n; T2.w = sm + 2 * n; O2.w = E.w = sm + 3 * n;
-        for (int i = threadIdx.x; i < n; i += blockDim.x) F.w[i] = a.F.w[i];
-        __syncthreads();
-    }
-    // O1 = open 30x1 (F) -> T1 ; O2 = open 1x30 (O1)
-    erode_dilate_h(F, T2, T1, a.open_len);
-    erode_dilate_v(T1, T2, O2, a.open_len);
-    // D = B - O2 (saturating) -> T1
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const unsigned o = O2.w[i], d = a.B.w[i] & ~o;
-        if (a.use_smem) a.O2.w[i] = o;
-        T1.w[i] = d;
-        a.D.w[i] = d;
-    }
-    __syncthreads();
-    // E = open eye(5) (D)
-    erode_dilate_eye(T1, T2, E, a.eye);
-    if (a.use_smem) for (int i = threadIdx.x; i < n; i += blockDim.x) a.E.w[i] = E.w[i];
-}
 
 // Raster of the CSR to the five stage images in `a` (a.B .. a.E), with L
 // (H * W + 1 ints) and *flag as scratch of the hole filling; *flag stays 0
@@ -380,16 +351,12 @@ tc_status thumbnail_stages(const int *d_rowptr, const int *d_col, int M, int pM,
     regions_init<false><<<(n + T - 1) / T, T, 0, s>>>(a.B, L);
     regions_join<false><<<(n + T - 1) / T, T, 0, s>>>(a.B, L, flag);
     fill_holes<<<(n + T - 1) / T, T, 0, s>>>(a.B, L, a.F);
-    TC_CUDA(cudaGetLastError());
-    const size_t smem = sizeof(unsigned) * (size_t)n * 4;
-    a.use_smem = smem <= 200 * 1024;
-    if (a.use_smem) {   // raise (never lower) the kernel's shared-memory limit
-        cudaFuncAttributes fa;
-        TC_CUDA(cudaFuncGetAttributes(&fa, morph_kernel));
-        if ((size_t)fa.maxDynamicSharedSizeBytes < smem)
-            TC_CUDA(cudaFuncSetAttribute(morph_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    }
-    morph_kernel<<<1, 1024, a.use_smem ? smem : 0, s>>>(a);
+    const int per = std::max(1, 256 / WW);
+    open_rows<<<(H + per - 1) / per, 256, 0, s>>>(a.F, a.T2, a.T1, a.open_len);
+    open_cols<<<WW, std::min(1024, (H + 31) & ~31), 2 * sizeof(unsigned) * (size_t)H, s>>>(a.T1, a.B, a.O2, a.D,
+                                                                                         a.open_len);
+    eye_pass<true><<<(n + T - 1) / T, T, 0, s>>>(a.D, a.T2, a.eye);
+    eye_pass<false><<<(n + T - 1) / T, T, 0, s>>>(a.T2, a.E, a.eye);
     TC_CUDA(cudaGetLastError());
     return TC_OK;
 }
