@@ -609,15 +609,28 @@ struct ShapeBox {
     int nd;           // 2w - 1 candidate diagonals
 };
 
-// Per-diagonal counts of unclaimed entries inside the box and the band
+// The boxes of a launch of band_hist: row blockIdx.y of the grid counts b[y]
+// into cnt[at[y]] on.
+constexpr int kHistBoxes = 32;
+struct HistBoxes {
+    ShapeBox b[kHistBoxes];
+    int at[kHistBoxes];
+};
+
+// Per-diagonal counts of unclaimed entries inside each box and its band
 // (TaiChi.cu:723-734); one thread per row of the box, four of its entries in
-// flight (9-point mesh 2048^2: 78 -> 57 us).
+// flight (9-point mesh 2048^2: 78 -> 57 us), all boxes in one launch (15 of
+// R-MAT scale 20 with self loops: 86 us in a launch each, 38 in one).
+constexpr int kHistLocal = 8192;     // most diagonals counted in shared memory
 __global__ void band_hist(const int *__restrict__ rowptr, const int *__restrict__ col,
-                          const unsigned char *__restrict__ claimed, ShapeBox sb,
-                          unsigned *__restrict__ cnt)
+                          const unsigned char *__restrict__ claimed, const __grid_constant__ HistBoxes boxes,
+                          unsigned *__restrict__ cnt_all)
 {
     extern __shared__ unsigned sh[];
-    const bool local = sb.nd <= 8192;
+    const ShapeBox sb = boxes.b[blockIdx.y];
+    unsigned *const cnt = cnt_all + boxes.at[blockIdx.y];
+    if ((long)blockIdx.x * blockDim.x >= sb.b) return;
+    const bool local = sb.nd <= kHistLocal;
     if (local) {
         for (int i = threadIdx.x; i < sb.nd; i += blockDim.x) sh[i] = 0;
         __syncthreads();
@@ -1136,19 +1149,28 @@ static tc_status settle_duplicates(const int *d_rowptr, const int *d_col, const 
     return TC_OK;
 }
 
+// The counts of shapes [i, stop), at most kHistBoxes of them.
 static tc_status launch_hist(const int *d_rowptr, const int *d_col, const unsigned char *d_claim,
-                             const ShapeBox &sb, unsigned *cnt, cudaStream_t s)
+                             const std::vector<ShapeResult> &shapes, size_t i, size_t stop, unsigned *cnt,
+                             cudaStream_t s)
 {
-    const size_t hsm = sb.nd <= 8192 ? sizeof(unsigned) * sb.nd : 0;
-    band_hist<<<box_grid(sb), 256, hsm, s>>>(d_rowptr, d_col, d_claim, sb, cnt);
+    HistBoxes h{};
+    int grid = 1, most = 0;
+    for (size_t k = i; k < stop; ++k) {
+        h.b[k - i] = shapes[k].box;
+        h.at[k - i] = shapes[k].cnt0;
+        grid = std::max(grid, box_grid(shapes[k].box));
+        if (shapes[k].box.nd <= kHistLocal) most = std::max(most, shapes[k].box.nd);
+    }
+    band_hist<<<dim3((unsigned)grid, (unsigned)(stop - i)), 256, sizeof(unsigned) * (size_t)most, s>>>(
+        d_rowptr, d_col, d_claim, h, cnt);
     TC_CUDA(cudaGetLastError());
     return TC_OK;
 }
 
 // The shapes in order (TaiChi.cu:361-421).  A shape's counts see the claims
-// of the shapes before it, so they are taken for up to kHistAhead shapes at
+// of the shapes before it, so they are taken for up to kHistBoxes shapes at
 // once and taken again for the rest after a shape that claims.
-constexpr int kHistAhead = 32;
 constexpr int kMarks = 250;          // marks 2 .. 251; 1: claimed earlier
 
 static tc_status process_shapes(const int *d_rowptr, const int *d_col, unsigned char *d_claim, int64_t nnz,
@@ -1165,7 +1187,7 @@ static tc_status process_shapes(const int *d_rowptr, const int *d_col, unsigned 
         return TC_OK;
     };
     for (size_t i = 0; i < n;) {
-        const size_t stop = std::min(n, i + kHistAhead);
+        const size_t stop = std::min(n, i + kHistBoxes);
         int total = 0;
         for (size_t k = i; k < stop; ++k) {
             shapes[k].cnt0 = total;
@@ -1173,8 +1195,7 @@ static tc_status process_shapes(const int *d_rowptr, const int *d_col, unsigned 
         }
         TC_CHECK(cnt.alloc(sizeof(unsigned) * (size_t)total, s));
         TC_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(unsigned) * (size_t)total, s));
-        for (size_t k = i; k < stop; ++k)
-            TC_CHECK(launch_hist(d_rowptr, d_col, d_claim, shapes[k].box, cnt.as<unsigned>() + shapes[k].cnt0, s));
+        TC_CHECK(launch_hist(d_rowptr, d_col, d_claim, shapes, i, stop, cnt.as<unsigned>(), s));
         hc.resize(total);
         TC_CUDA(cudaMemcpyAsync(hc.data(), cnt.p, sizeof(unsigned) * (size_t)total, cudaMemcpyDeviceToHost, s));
         TC_CUDA(cudaStreamSynchronize(s));
