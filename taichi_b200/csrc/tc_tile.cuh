@@ -44,17 +44,6 @@ __device__ __forceinline__ float ldx(const float *p)
     return v;
 }
 
-// The same for a gather whose neighbours are unlikely to be gathered again by
-// this SM: its line is the first to leave L1 (wide tiles; R-MAT scale 20:
-// 4.27 -> 4.13 us per multiply.  Not for banded rows, whose neighbours share
-// lines: 93 -> 161 us).
-__device__ __forceinline__ float ldx_once(const float *p)
-{
-    float v;
-    asm("ld.global.L1::evict_first.f32 %0, [%1];" : "=f"(v) : "l"(p));
-    return v;
-}
-
 // v of an addition word (c & 1), -v of a hole's.
 __device__ __forceinline__ float signed_term(float v, int c)
 {
@@ -72,13 +61,15 @@ __device__ __forceinline__ float gather(const float *__restrict__ x, int c)
     return ldx(x + c);
 }
 
-// gather() of a wide tile's word (ldx_once); POS: a signed word known to be an
-// addition (c & 1 set: a plan with no holes in its dense diagonals), without
-// the sign select.
+// gather() of a wide tile's word; POS: a signed word known to be an addition
+// (c & 1 set: a plan with no holes in its dense diagonals), without the sign
+// select.  (A load whose line leaves L1 first: 8 chained R-MAT scale 20
+// multiplies 34.4 -> 33.0 us from a warm L2, but 4.49 -> 5.30 us a multiply
+// over matrices that come from HBM; without allocation in L1 13 us.)
 template <bool SIGNED, bool POS>
-__device__ __forceinline__ float gather_once(const float *__restrict__ x, int c)
+__device__ __forceinline__ float gather_wide(const float *__restrict__ x, int c)
 {
-    const float v = ldx_once(x + (SIGNED ? c >> 1 : c));
+    const float v = ldx(x + (SIGNED ? c >> 1 : c));
     return SIGNED && !POS ? signed_term(v, c) : v;
 }
 
@@ -865,7 +856,7 @@ __device__ __forceinline__ void direct_run_full(const DevPlan &p, int dc, const 
     wait_prior_grid(x, y);
     float v[kDirectWFull];
 #pragma unroll
-    for (int w = 0; w < kDirectWFull; ++w) v[w] = gather_once<SIGNED, POS>(x, c[w]);   // past the run: x[0], not added
+    for (int w = 0; w < kDirectWFull; ++w) v[w] = gather_wide<SIGNED, POS>(x, c[w]);   // past the run: x[0], not added
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
     if (SIGNED && p.dn == 1) {
         // one dense diagonal: which rows have its term comes from the launch
@@ -896,7 +887,7 @@ __device__ __forceinline__ void direct_run_full(const DevPlan &p, int dc, const 
         for (int u = 0; u < 4; ++u)
             if (b[0] + w >= b[u] && b[0] + w < b[u + 1]) acc[u] += v[w];
     for (int j = b[0] + kDirectWFull; j < e4; ++j) {
-        const float z = gather_once<SIGNED, POS>(x, __ldg(p.cols + j));
+        const float z = gather_wide<SIGNED, POS>(x, __ldg(p.cols + j));
 #pragma unroll
         for (int u = 0; u < 4; ++u)
             if (j >= b[u] && j < b[u + 1]) acc[u] += z;
