@@ -103,13 +103,13 @@ tc_status tc_batch_create(int n, tc_plan *const *plans, const float *const *d_x,
     b->dev = base;
     b->d_plans = reinterpret_cast<tc::DevPlan *>(base);
     b->d_items = reinterpret_cast<tc::BatchItem *>(base + o_it);
-    cudaError_t e = cudaMemcpy(b->d_plans, dps.data(), sizeof(tc::DevPlan) * n, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && !items.empty())
-        e = cudaMemcpy(b->d_items, items.data(), sizeof(tc::BatchItem) * items.size(), cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) {
+    tc_status st = tc::upload(b->d_plans, dps.data(), sizeof(tc::DevPlan) * n);    // run on any stream
+    if (st == TC_OK && !items.empty())
+        st = tc::upload(b->d_items, items.data(), sizeof(tc::BatchItem) * items.size());
+    if (st != TC_OK) {
         cudaFree(base);
         delete b;
-        return fail(TC_ERR_CUDA, "tc_batch_create: %s", cudaGetErrorString(e));
+        return st;
     }
     *out = b;
     return TC_OK;

@@ -60,6 +60,11 @@ struct Scratch {
 // cudaMalloc that gives the pool's unused memory back and tries again before
 // it fails (waits for `stream` then).
 tc_status device_alloc(void **p, size_t bytes, cudaStream_t stream);
+// Copies host data to device memory and waits until it has arrived: kernels of
+// any stream may read it after the return.  (cudaMemcpy alone returns once
+// pageable data is staged, and a non-blocking stream does not wait for the
+// legacy stream that carries the copy.)
+tc_status upload(void *dst, const void *src, size_t bytes);
 // Plans alive in the process (the pool is trimmed when the last one goes).
 void plan_born();
 void plan_gone();

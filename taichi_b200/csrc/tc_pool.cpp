@@ -132,6 +132,13 @@ tc_status device_alloc(void **p, size_t bytes, cudaStream_t stream)
     return fail(TC_ERR_ALLOC, "cudaMalloc(%zu): %s", bytes, cudaGetErrorString(e));
 }
 
+tc_status upload(void *dst, const void *src, size_t bytes)
+{
+    TC_CUDA(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice));
+    TC_CUDA(cudaStreamSynchronize(nullptr));
+    return TC_OK;
+}
+
 void plan_born() { g_live_plans.fetch_add(1, std::memory_order_relaxed); }
 
 void plan_gone()

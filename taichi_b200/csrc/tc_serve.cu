@@ -424,8 +424,8 @@ tc_status tc_server_admit(tc_server *sv, tc_plan *plan, int *id)
     }
     const tc::DevPlan dp = plan->dev_plan();
     const tc::ItemPlan core = tc::item_plan(dp, plan->d_btiles);
-    TC_CUDA(cudaMemcpy(sv->d_plans + slot, &dp, sizeof dp, cudaMemcpyHostToDevice));
-    TC_CUDA(cudaMemcpy(sv->d_cores + slot, &core, sizeof core, cudaMemcpyHostToDevice));
+    TC_CHECK(tc::upload(sv->d_plans + slot, &dp, sizeof dp));     // read on the contexts' own streams
+    TC_CHECK(tc::upload(sv->d_cores + slot, &core, sizeof core));
     sv->plans[slot] = plan;
     sv->footprint[slot] = fp;
     sv->nonlean += lean_plan(plan) ? 0 : 1;
