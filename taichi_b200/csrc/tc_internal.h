@@ -120,6 +120,7 @@ constexpr int kStreamRows = 256;      // most rows of a TILE_STREAM tile (1 per 
 constexpr int kStreamRowMax = 128;    // longer rows of a stream tile are summed by a warp (TILE_MIXED)
 constexpr int kStream4Rows = 1024;    // most rows of a TILE_STREAM4 tile (a run of 4 per thread)
 constexpr int kDirectRows = 1024;     // most rows of a direct tile (TILE_DIRECT4)
+constexpr int kDirectMaxWords = 0x7fffffff - 64;   // most words of a plan with direct tiles
 constexpr int kDirectWideBlock = 1024; // threads of the direct kernel's CTAs
 constexpr int kPlanDiags = 4;         // dense diagonals a plan's descriptor carries
 // The rows kernel by default: stream plans whose rows average at most this

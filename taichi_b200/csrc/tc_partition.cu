@@ -37,6 +37,7 @@
 #include "tc_ctxcache.h"
 #include "tc_internal.h"
 #include "tc_scan.cuh"
+#include "tc_words.h"
 
 namespace tc {
 namespace {
@@ -88,10 +89,9 @@ __global__ void raster_kernel(const int *__restrict__ rowptr, const int *__restr
     const long r0 = (long)px * pM;
     const long r1 = r0 + pM < (long)M ? r0 + pM : (long)M;   // rows >= H*pM are never drawn
     if (r0 < M) {
-        const int b = __ldg(rowptr + r0), e = __ldg(rowptr + r1);
         unsigned cur_w = 0xffffffffu, cur_bits = 0;
-        for (int j = b + threadIdx.x; j < e; j += blockDim.x) {
-            const int py = __ldg(col + j) / pN;
+        for (Words a(__ldg(rowptr + r0), __ldg(rowptr + r1), threadIdx.x); a.left > 0; a.skip(blockDim.x)) {
+            const int py = __ldg(col + a.at) / pN;
             if (py < img.W) {
                 const unsigned wi = (unsigned)py >> 5, bit = 1u << (py & 31);
                 if (wi != cur_w) {
@@ -640,13 +640,13 @@ __global__ void band_hist(const int *__restrict__ rowptr, const int *__restrict_
          r += (long)gridDim.x * blockDim.x) {
         const int b = __ldg(rowptr + r), e = __ldg(rowptr + r + 1);
         const long lo = r + dof - sb.w + 1, hi = r + dof + sb.w - 1;
-        for (int j = b; j < e; j += 4) {
+        for (Words a(b, e); a.left > 0; a.skip(4)) {
             int c[4];
             unsigned char k[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                c[u] = j + u < e ? __ldg(col + j + u) : -1;
-                k[u] = j + u < e ? claimed[j + u] : 1;
+                c[u] = u < a.left ? __ldg(col + a.at + u) : -1;
+                k[u] = u < a.left ? claimed[a.at + u] : 1;
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
@@ -688,19 +688,19 @@ __global__ void band_claim(const int *__restrict__ rowptr, const int *__restrict
             *f = old | bits;
             bits = 0;
         };
-        for (int j = b; j < e; j += 4) {
+        for (Words a(b, e); a.left > 0; a.skip(4)) {
             int dd[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                const int c = j + u < e ? __ldg(col + j + u) : -1;
-                const bool in = c >= sb.y && c < sb.y + sb.a && c >= lo && c <= hi && !claimed[j + u];
+                const int c = u < a.left ? __ldg(col + a.at + u) : -1;
+                const bool in = c >= sb.y && c < sb.y + sb.a && c >= lo && c <= hi && !claimed[a.at + u];
                 dd[u] = in ? __ldg(dense_idx + (c - r - dof + sb.w - 1)) : -1;
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const int d = dd[u];
                 if (d < 0) continue;
-                claimed[j + u] = mark;
+                claimed[a.at + u] = mark;
                 if (d >> 5 != at) {
                     flush();
                     at = d >> 5;

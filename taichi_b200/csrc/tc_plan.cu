@@ -344,7 +344,8 @@ tc_status plan_upload(tc_plan *p, const int *csrRow, const int *csrCol, int64_t 
     q.spread = (int)std::min<int64_t>(kStreamNnz, std::max<int64_t>(512, nnz_csr / std::max(1, min_tiles)));
     q.max_lanes = prm.max_lanes;
     q.strided = (prm.flags & TC_FLAG_ROWS_STRIDED) != 0;
-    q.no_direct = (prm.flags & TC_FLAG_NO_DIRECT) != 0;
+    const bool no_direct = (prm.flags & TC_FLAG_NO_DIRECT) || nnz_csr > kDirectMaxWords;
+    q.no_direct = no_direct;
     TilePrm bq = q;                           // the tiles of batch and served launches
     bq.spread = kStreamNnz;
     const bool second = M > 0 && prm.tile_mode == 2 && q.spread < kStreamNnz;
@@ -370,10 +371,10 @@ tc_status plan_upload(tc_plan *p, const int *csrRow, const int *csrCol, int64_t 
     // each).  Several diagonals make a thread's four rows a long chain and its
     // loads of x four to a line; the rows kernel takes those plans.
     const bool wide = prm.tile_mode == 2 && prm.tile_rows >= kDirectRows &&
-                      !(prm.flags & (TC_FLAG_NO_DIRECT | TC_FLAG_NO_WIDE | TC_FLAG_ROWS_STRIDED)) &&
+                      !no_direct && !(prm.flags & (TC_FLAG_NO_WIDE | TC_FLAG_ROWS_STRIDED)) &&
                       M >= kDirectWideRows && nnz_csr <= M && st.max_row <= kStreamRowMax && p->num_negs <= 1;
     p->wide_rows = wide ? wide_tile_rows(M, prm, num_sms()) : kDirectWideRows;
-    p->ntiles = wide ? (M + p->wide_rows - 1) / p->wide_rows : made;
+    p->ntiles = wide ? (int)(((long)M + p->wide_rows - 1) / p->wide_rows) : made;
     const bool own = wide || !second;         // batches run the plan's own tiles
     p->nbtiles = own ? p->ntiles : bmade;
     p->ntiles_wide = wide ? p->ntiles : 0;

@@ -177,28 +177,27 @@ constexpr int spmm_blocks(int V, int W) { return V < 4 || W < 4 ? 8 : 6; }
 __device__ __forceinline__ void prefetch_later_rows(const DevPlan &p, long r0, int rows)
 {
     if (r0 >= p.M) return;
-    const int ra = (int)r0, rb = min(ra + rows, p.M);
+    const int ra = (int)r0, rb = ra + min(rows, p.M - ra);
     const int za = __ldg(p.rowptr + ra), zb = __ldg(p.rowptr + rb);
-    prefetch_rows_ahead(p, ra, rb, za, min(zb, za + kAheadWords));
+    prefetch_rows_ahead(p, ra, rb, za, words_upto(za, zb, kAheadWords));
 }
 
-// Adds to acc the terms of words b, b + by, b + 2 by, ... before e, W of them
-// in flight together (a slot past the end loads X's row 0 and is not added).
+// Adds to acc the terms of every by-th of the words `a`, W of them in flight
+// together (a slot past the end loads X's row 0 and is not added).
 template <bool SIGNED, int V, bool VEC, int W>
 __device__ __forceinline__ void sum_words(const DevPlan &p, const float *__restrict__ Xc, int ldx,
-                                          const Lane<V, VEC> &l, int b, int e, int by, Cols<V, VEC> &acc)
+                                          const Lane<V, VEC> &l, Words a, int by, Cols<V, VEC> &acc)
 {
-    for (int j = b; j < e; j += W * by) {
-        const int left = e - j;
+    for (; a.left > 0; a.skip(W * by)) {
         int c[W];
         Cols<V, VEC> v[W];
 #pragma unroll
-        for (int w = 0; w < W; ++w) c[w] = w * by < left ? __ldg(p.cols + j + w * by) : 0;
+        for (int w = 0; w < W; ++w) c[w] = w * by < a.left ? __ldg(p.cols + a.at + w * by) : 0;
 #pragma unroll
         for (int w = 0; w < W; ++w) v[w].load(Xc + (long)word_col<SIGNED>(c[w]) * ldx, l);
 #pragma unroll
         for (int w = 0; w < W; ++w)
-            if (w * by < left) add_word<SIGNED>(acc, v[w], c[w]);
+            if (w * by < a.left) add_word<SIGNED>(acc, v[w], c[w]);
     }
 }
 
@@ -218,7 +217,7 @@ __device__ __forceinline__ void spmm_rows(const DevPlan &p, const typename Diags
     if (group < nrow && (!MID || e - b <= kSpmmMidRow)) {
         Cols<V, VEC> acc;
         acc.zero();
-        sum_words<SIGNED, V, VEC, W>(p, Xc, ldx, l, b, e, 1, acc);
+        sum_words<SIGNED, V, VEC, W>(p, Xc, ldx, l, Words(b, e), 1, acc);
         if constexpr (SIGNED) diag_cols(p, q, Xc, ldx, l, r, acc);
         acc.store(Yc + (long)r * ldy, l);
     }
@@ -232,7 +231,7 @@ __device__ __forceinline__ void spmm_rows(const DevPlan &p, const typename Diags
         const int re = __shfl_sync(0xffffffffu, e, src);
         Cols<V, VEC> acc;
         acc.zero();
-        sum_words<SIGNED, V, VEC, W>(p, Xc, ldx, l, rb + wg, re, gw, acc);
+        sum_words<SIGNED, V, VEC, W>(p, Xc, ldx, l, Words(rb, re, wg), gw, acc);
 #pragma unroll
         for (int u = 0; u < V; ++u)
             for (int o = 1 << lg; o < 32; o <<= 1) acc.a[u] += __shfl_xor_sync(0xffffffffu, acc.a[u], o);
@@ -281,7 +280,7 @@ __global__ void __launch_bounds__(kBlock, spmm_blocks(V, W))
     }
     Cols<V, VEC> acc;
     acc.zero();
-    sum_words<SIGNED, V, VEC, W>(p, Xc, ldx, l, t.nz0 + group, t.nz0 + t.nnz, groups, acc);
+    sum_words<SIGNED, V, VEC, W>(p, Xc, ldx, l, Words(t.nz0, t.nz0 + t.nnz, group), groups, acc);
 #pragma unroll
     for (int u = 0; u < V; ++u) part[u * kBlock + threadIdx.x] = acc.a[u];
     __syncthreads();
@@ -319,17 +318,18 @@ __global__ void __launch_bounds__(kBlock, kRunBlocks)
     const int z = __shfl_up_sync(0xffffffffu, end, 1);
     const int begin = lane ? z : __ldg(p.rowptr + r0);
     const unsigned mask = (lg == 5 ? 0xffffffffu : ((1u << (1 << lg)) - 1u)) << first;
-    const int jb = __shfl_sync(mask, begin, first), je = __shfl_sync(mask, end, first + (1 << lg) - 1);
+    // positions of words: unsigned, as a step past the run's end may leave 2^31 - 1 behind
+    const unsigned jb = __shfl_sync(mask, begin, first), je = __shfl_sync(mask, end, first + (1 << lg) - 1);
     int row = 0;                                                  // current row of the group
-    int re = __shfl_sync(mask, end, first);
+    unsigned re = __shfl_sync(mask, end, first);
     const int nrow = min(1 << lg, p.M - r0 - first);              // <= 0: no rows
     float *yr = Y + (long)(r0 + first) * ldy + l.at;
     Cols<V, VEC> acc;
     acc.zero();
-    for (int j0 = jb; j0 < je; j0 += 1 << lg) {
+    for (unsigned j0 = jb; j0 < je; j0 += 1 << lg) {
         // the next 2^lg words, one per lane of the group
         const int word = j0 + gl < je ? __ldg(p.cols + j0 + gl) : 0;
-        const int n = min(1 << lg, je - j0);
+        const int n = min(1 << lg, (int)(je - j0));
         for (int t = 0; t < n; t += U) {
             int c[U];
             Cols<V, VEC> v[U];

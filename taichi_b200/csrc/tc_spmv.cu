@@ -193,19 +193,20 @@ __global__ void __launch_bounds__(kBlock, kRowsMinBlocks)
                      const float *__restrict__ x, float *__restrict__ y)
 {
     allow_next_grid();
-    const int r = blockIdx.x * kBlock + threadIdx.x;
+    const int row0 = blockIdx.x * kBlock, r = row0 + (int)threadIdx.x;
+    const bool own = (int)threadIdx.x < p.M - row0;
     // warp 0 also brings into L2 the x window of the strip and the operands
     // of the strip a wave later (thread 0; the other warps skip it whole)
     const bool lead = threadIdx.x < 32;
     const bool ahead = lead && blockIdx.x + p.ahead < gridDim.x;
     int za = 0, zb = 0;
     if (lead && threadIdx.x == 0) prefetch_x_window(x, p.N, r, kBlock);
-    const int b = r < p.M ? __ldg(p.rowptr + r) : 0;
-    const int e = r < p.M ? __ldg(p.rowptr + r + 1) : 0;
+    const int b = own ? __ldg(p.rowptr + r) : 0;
+    const int e = own ? __ldg(p.rowptr + r + 1) : 0;
     if (ahead) {
         const int ra = (blockIdx.x + p.ahead) * kBlock;
         za = __ldg(p.rowptr + ra);
-        zb = __ldg(p.rowptr + min(ra + kBlock, p.M));
+        zb = __ldg(p.rowptr + ra + min(kBlock, p.M - ra));
     }
     const int n = e - b;
     int c[W];
@@ -213,7 +214,7 @@ __global__ void __launch_bounds__(kBlock, kRowsMinBlocks)
     for (int w = 0; w < W; ++w) c[w] = w < n ? __ldg(p.cols + b + w) : 0;
     if (ahead && threadIdx.x == 0) {
         const int ra = (blockIdx.x + p.ahead) * kBlock;
-        prefetch_rows_ahead(p, ra, min(ra + kBlock, p.M), za, zb);
+        prefetch_rows_ahead(p, ra, ra + min(kBlock, p.M - ra), za, zb);
     }
     wait_prior_grid(x, y);
     // every slot is loaded (a slot past the row holds word 0, a load of x[0]
@@ -242,19 +243,18 @@ __global__ void __launch_bounds__(kBlock, kRowsMinBlocks)
     for (int w = 0; w < W; ++w)
         if (w < n) acc += v[w];
 #pragma unroll 1
-    for (int j = b + W; j < e; j += W) {                            // longer rows, W words at a time
-        const int left = e - j;
+    for (Words a(b, e, W); a.left > 0; a.skip(W)) {                 // longer rows, W words at a time
         int cc[W];
         float vv[W];
 #pragma unroll
-        for (int u = 0; u < W; ++u) cc[u] = u < left ? __ldg(p.cols + j + u) : 0;
+        for (int u = 0; u < W; ++u) cc[u] = u < a.left ? __ldg(p.cols + a.at + u) : 0;
 #pragma unroll
         for (int u = 0; u < W; ++u) vv[u] = gather<SIGNED>(x, cc[u]);
 #pragma unroll
         for (int u = 0; u < W; ++u)
-            if (u < left) acc += vv[u];
+            if (u < a.left) acc += vv[u];
     }
-    if (r < p.M) y[r] = acc;
+    if (own) y[r] = acc;
 }
 
 // The multiply of a stream plan (any of its tile kinds): one CTA per tile, no
@@ -379,7 +379,7 @@ static tc_status launch_tiles(const DevPlan &dp, const PlanDiags &dg, const Wide
     else if (dp.per_tile == 3 && full) TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_wide_kernel<SIGNED, true>, dp, x, y));
     else if (dp.per_tile == 3) TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_wide_kernel<SIGNED, false>, dp, x, y));
     else if (dp.rows) {
-        cfg.gridDim = dim3((unsigned)((dp.M + kBlock - 1) / kBlock));
+        cfg.gridDim = dim3((unsigned)(((long)dp.M + kBlock - 1) / kBlock));
         typename DiagsOf<SIGNED>::type q;
         if constexpr (SIGNED) q = dg;
         if (dp.rows_w <= 2) TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_rows_kernel<SIGNED, 2>, dp, q, x, y));

@@ -22,6 +22,7 @@
 #include <cstdint>
 
 #include "tc_internal.h"
+#include "tc_words.h"
 
 namespace tc {
 
@@ -111,7 +112,7 @@ __device__ __forceinline__ void after_wait(const float *__restrict__ &x, float *
 template <typename V>
 __device__ __forceinline__ void prefetch_x_window(const V *x, int N, int r0, int n)
 {
-    const int a = max(r0, 0), b = min(r0 + n, N);
+    const int a = max(r0, 0), b = (int)min((long)r0 + n, (long)N);
     if (b <= a) return;
     const uintptr_t lo = (reinterpret_cast<uintptr_t>(x + a) + 15) & ~uintptr_t(15);
     const uintptr_t hi = reinterpret_cast<uintptr_t>(x + b) & ~uintptr_t(15);
@@ -792,7 +793,10 @@ template <bool SIGNED>
 constexpr int direct_w_full() { return SIGNED ? 8 : 6; }
 
 // The run of rows [row0 + g, row0 + g + 4) of a direct tile of nr rows from
-// row0 and diagonal class dc, g a multiple of 4.
+// row0 and diagonal class dc, g a multiple of 4.  (Positions of words are ints
+// here, also a few past the end of a run: the planner makes direct tiles of no
+// plan with more than kDirectMaxWords words.  Unsigned positions, or positions
+// from the run's start, cost the wide kernel 1 to 7 %.)
 template <bool SIGNED>
 __device__ __forceinline__ void direct_run(const DevPlan &p, int row0, int nr, int dc, const float *__restrict__ x,
                                            float *__restrict__ y, bool wait, int g)
@@ -972,13 +976,10 @@ __device__ void long_row(const DevPlan &p, const Tile &t, const float *__restric
                 if (c >= sh.z && c < sh.z + sh.w) acc += ldx(x + c);
             }
         }
-    for (int base = 0; base < t.nnz; base += kBlock * U) {
+    for (Words a(0, t.nnz, tid); a.left > 0; a.skip(kBlock * U)) {
         int c[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int i = base + u * kBlock + tid;
-            c[u] = i < t.nnz ? __ldg(cols + i) : -1;
-        }
+        for (int u = 0; u < U; ++u) c[u] = u * kBlock < a.left ? __ldg(cols + a.at + u * kBlock) : -1;
 #pragma unroll
         for (int u = 0; u < U; ++u)
             if (c[u] >= 0) acc += gather<SIGNED>(x, c[u]);
