@@ -168,6 +168,7 @@ tc_status tc_plan_from_format(int M, int N, const tc_format *f, const tc_params 
     tc_plan *p = nullptr;
     TC_CHECK(plan_of_shapes(M, N, f, prm, &p));
     p->nnz_input = (int64_t)f->dense_nnz + f->sparse_nnz;
+    tc::ScratchEnd end((cudaStream_t)stream);
     tc_status st = tc::plan_upload(p, rp, f->csrCol, nnz_csr, false, (cudaStream_t)stream);
     if (st != TC_OK) { tc_plan_destroy(p); return st; }
     *out = p;
@@ -379,6 +380,7 @@ tc_status tc_plan_create(int M, int N, int64_t nnz, const int *rowptr, const int
 
     // GPU partition from a device copy of the input; the plan is built from
     // its device arrays (the input's own when nothing was extracted)
+    tc::ScratchEnd end(s);
     tc::Scratch own_rp, own_col, own_val;
     const int *d_rp = rowptr, *d_col = col;
     const float *d_val = val;

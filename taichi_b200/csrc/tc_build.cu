@@ -153,6 +153,7 @@ tc_status coo_to_csr_device(int M, int N, bool symmetric, const MtxEntry *h_entr
                             int **d_rowptr, int **d_col, float **d_val, int64_t *nnz_out)
 {
     (void)N;
+    ScratchEnd end(s);
     Scratch ent, keyA, keyB, idxA, idxB, hist, tmp;
     Buf rp, cl, vl;                                  // handed to the caller
     const long nrec = 2 * n;

@@ -228,6 +228,7 @@ void partition_shapes(char *sdf_name, int M, int N, int nnz, int *&csrRow, int *
         cudaMemcpy(d_col, csrCol, sizeof(int) * nz, cudaMemcpyHostToDevice);
         cudaMemcpy(d_val, csrVal, sizeof(float) * nz, cudaMemcpyHostToDevice);
     }
+    tc::ScratchEnd end(nullptr);
     tc::PartitionOut po;
     double t0 = now_ms();
     tc_status st = tc::gpu_partition(M, N, nnz, d_rp, d_col, d_val, prm, false, true, 0, po);

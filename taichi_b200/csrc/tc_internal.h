@@ -57,6 +57,17 @@ struct Scratch {
     void release();
     template <class T> T *as() const { return static_cast<T *>(p); }
 };
+// Declared before the Scratch of a call: waits for `s` once they are freed.
+// The pool gives back what it holds beyond its bound at such a wait only, so
+// without it a call would return with all of its scratch still held.
+struct ScratchEnd {
+    cudaStream_t s;
+    bool on;
+    explicit ScratchEnd(cudaStream_t stream, bool used = true) : s(stream), on(used) {}
+    ScratchEnd(const ScratchEnd &) = delete;
+    ScratchEnd &operator=(const ScratchEnd &) = delete;
+    ~ScratchEnd();
+};
 // cudaMalloc that gives the pool's unused memory back and tries again before
 // it fails (waits for `stream` then).
 tc_status device_alloc(void **p, size_t bytes, cudaStream_t stream);

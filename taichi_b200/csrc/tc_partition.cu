@@ -1333,6 +1333,7 @@ tc_status gpu_one_shape(int M, int64_t nnz, const int *h_rowptr, const int *h_co
                         int x, int y, int a, int b, double density, OneShape &o)
 {
     cudaStream_t s = 0;
+    ScratchEnd end(s);
     Scratch rp, cl, va, claim;
     TC_CHECK(rp.alloc(sizeof(int) * ((size_t)M + 1), s));
     TC_CHECK(cl.alloc(sizeof(int) * (size_t)std::max<int64_t>(nnz, 1), s));
@@ -1381,6 +1382,7 @@ extern "C" tc_status tc_getsdf(int M, int N, const int *d_rowptr, const int *d_c
     tc_params_default(&prm);
     if (p) prm = *p;
     TC_CHECK(tc::check_params(prm));
+    tc::ScratchEnd end((cudaStream_t)stream, M > prm.thumb_height);
     tc::SdfOut o;
     TC_CHECK(tc::getsdf_device(M, N, d_rowptr, d_col, prm, stages != nullptr, (cudaStream_t)stream, o));
     *mF = o.mF;
@@ -1399,6 +1401,7 @@ extern "C" tc_status tc_trace_contours(const unsigned char *img, int H, int W, i
     if ((long)H * W > (1L << 26)) return fail(TC_ERR_UNSUPPORTED, "image too large");
     const int WW = (W + 31) / 32;
     cudaStream_t s = nullptr;
+    tc::ScratchEnd end(s);
     tc::Scratch bytes, bits;
     TC_CHECK(bytes.alloc((size_t)H * W, s));
     TC_CHECK(bits.alloc(sizeof(unsigned) * (size_t)H * WW, s));
@@ -1549,6 +1552,7 @@ void getSdf(std::string path, int M, int N, int nnz, int *&csrRowIndexHostPtr, i
         report(tc::fail(TC_ERR_INVALID, "bad arguments"));
         return;
     }
+    tc::ScratchEnd end(nullptr);
     tc::Scratch drp, dcol;
     tc_status st = drp.alloc(sizeof(int) * ((size_t)M + 1), nullptr);
     if (st == TC_OK) st = dcol.alloc(sizeof(int) * (size_t)std::max(nnz, 1), nullptr);

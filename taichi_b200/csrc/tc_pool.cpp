@@ -6,9 +6,11 @@
 // pool that still holds the memory of the last build costs 2 us.  So scratch
 // comes from a memory pool of the library's own (not the device's default
 // pool, whose settings belong to the program), one per device.  It keeps at
-// most kPoolKeep bytes between builds and gives all but kPoolIdle of them back
-// when the process's last plan is destroyed; a plan that finds no room takes
-// all of them back first.  The pool is found by the CUDA context it was made
+// most kPoolKeep bytes between builds: it lets go of more at the wait that
+// ends a call, after the call's scratch is freed (ScratchEnd).  It gives all
+// but kPoolIdle of them back when the process's last plan is destroyed (in
+// the device that is current then); a plan that finds no room takes all of
+// them back first.  The pool is found by the CUDA context it was made
 // in, so a device reset starts a new one.  Allocations and frees are ordered
 // on the build's own stream; pools are safe across threads and streams.
 
@@ -95,6 +97,11 @@ unsigned long long current_context_id()
 }
 
 Scratch::~Scratch() { release(); }
+
+ScratchEnd::~ScratchEnd()
+{
+    if (on) cudaStreamSynchronize(s);
+}
 
 void Scratch::release()
 {
