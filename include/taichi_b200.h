@@ -88,10 +88,11 @@ typedef struct tc_params {
 #define TC_FLAG_WIDE_FIXED   0x200 /* wide plans: tiles of 4096 rows
                                      instead of two equal tiles per SM     */
 #define TC_FLAG_ROWS         0x400 /* plans of stream tiles only, and hybrid
-                                     plans without rows of more than 128
-                                     words: run the rows kernel (one row per
-                                     thread, words straight from global
-                                     memory) whatever the rows' mean length */
+                                     plans without rows of more than 128 or
+                                     tile_nnz words: run the rows kernel (one
+                                     row per thread, words straight from
+                                     global memory) whatever the rows' mean
+                                     length                                 */
 #define TC_FLAG_NO_ROWS      0x800 /* the same plans: never run the rows
                                      kernel                                 */
 #define TC_FLAG_NO_PREFETCH  0x2000 /* stream and rows kernels: no L2

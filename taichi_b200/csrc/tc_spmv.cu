@@ -469,8 +469,10 @@ tc::DevPlan tc_plan::dev_plan() const
     }
     // the rows kernel: a stream plan (every row at most kStreamRowMax words)
     // of short rows, or any stream plan on request; hybrid plans that are not
-    // wide run it whatever their tiles (direct and four-row tiles among them)
-    const bool any_tiles = d.dia_shapes > 0 && d.per_tile == 2 && max_row <= tc::kStreamRowMax;
+    // wide run it whatever their tiles (direct and four-row tiles among them),
+    // unless a row is a CTA's: the CTA adds its words in another order, and a
+    // plan gives the same y alone, in a batch and served
+    const bool any_tiles = d.dia_shapes > 0 && d.per_tile == 2 && max_row <= tc::kStreamRowMax && ntiles_long == 0;
     d.rows = 0;
     if ((d.per_tile == 4 || any_tiles) && !(params.flags & TC_FLAG_NO_ROWS))
         d.rows = (params.flags & TC_FLAG_ROWS) || (M > 0 && nnz_csr <= (int64_t)tc::kRowsMeanMax * M && tc::kRowsByDefault);

@@ -71,3 +71,30 @@ def test_offsets(tc, dev, noffs, box):
     torch.cuda.synchronize()
     tc.check(tc.lib().tc_batch_destroy(b))
     assert torch.equal(y, yb)
+
+
+@pytest.mark.parametrize("tile_nnz", [16, 100, 128])
+def test_rows_of_a_cta(tc, dev, tile_nnz):
+    """Rows of more than tile_nnz words get a CTA each, which adds them in
+    another order than one thread: the same y alone and in a batch."""
+    import torch
+    M, rng = 30000, np.random.default_rng(tile_nnz)
+    lens = rng.poisson(1.5, M)
+    lens[rng.choice(M, 300, replace=False)] = rng.integers(10, 129, 300)
+    rp = np.zeros(M + 1, np.int32)
+    np.cumsum(lens, out=rp[1:])
+    words = ((rng.integers(0, M, rp[-1]) << 1) | (rng.random(rp[-1]) < 0.7)).astype(np.int32)
+    f = dict(dia_shapes=1, num_negs=3, dense_nnz=1, zero_elements=0, sparse_nnz=len(words), row_start=0, row_stop=M,
+             xStart=[0], yStart=[0], xStop=[M], nDiasPtr=[0, 3], neg_offsets=[-1, 0, 1], csrRow=rp, csrCol=words)
+    plan = tc.Plan.from_format(M, M, f, prm=tc.params(tile_nnz=tile_nnz))
+    x = rng.uniform(-1, 1, M).astype(np.float32)
+    xd, y, yb = torch.from_numpy(x).to(dev), torch.empty(M, device=dev), torch.empty(M, device=dev)
+    plan.spmv(xd, y)
+    b, one = C.c_void_p(), C.c_void_p * 1
+    tc.check(tc.lib().tc_batch_create(1, one(plan.handle.value), one(xd.data_ptr()), one(yb.data_ptr()), C.byref(b)))
+    tc.check(tc.lib().tc_batch_run(b, None))
+    torch.cuda.synchronize()
+    tc.check(tc.lib().tc_batch_destroy(b))
+    assert torch.equal(y, yb)
+    want = dense_multiply(f, M, x.astype(np.float64))
+    assert np.abs(y.cpu().numpy() - want).max() <= 131 * 131 * 2.0 ** -24   # 131 terms of at most 1, one rounding each
