@@ -264,6 +264,7 @@ struct tc_plan {
     int *d_err = nullptr;
     int wide_rows = 0;                   // rows of each wide direct tile
     int stream_skew = 0;                 // the plan's usual row length is a multiple of 8
+    bool rows_any = false;               // the rows kernel may take direct and four-row tiles too
     int rows_w = 8;                      // the rows kernel's words in flight (the usual row length, 2 / 4 / 6 / 8)
     int all_pos = 0;                     // hybrid plan with no holes (every word an addition)
     // window plan (tc_window.cu); nwtiles == 0 when the plan has none

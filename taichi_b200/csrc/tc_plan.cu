@@ -390,20 +390,43 @@ tc_status plan_upload(tc_plan *p, const int *csrRow, const int *csrCol, int64_t 
         const int mode = (int)(std::max_element(h + 1, h + kStreamRowMax + 1) - h);
         p->stream_skew = h[mode] > 0 && mode % 8 == 0;
         // the rows kernel loads W words of a row together: the least of 2, 4,
-        // 6, 8 that holds 90 % of the rows whole
-        int64_t tot = 0, upto = 0;
+        // 6, 8 that holds 90 % of the rows whole, 2 only where the longest
+        // row takes four rounds (3 diagonals of 100,000 rows, 0.3 words each
+        // and one row of 32: 4.8 us at 2, 3.2 at 4; of 1,000,000 rows and 1 %
+        // of 16 words: 9.8 and 8.7; without the long ones 6.2 and 6.5)
+        int64_t tot = 0, upto = 0, many = 0;
         for (int L = 0; L <= kStreamRowMax; ++L) tot += h[L];
         p->rows_w = 8;
         for (int L = 0, w = 2; L <= 8 && tot > 0; ++L) {
             upto += h[L];
             if (L == w) {
-                if (upto * 10 >= tot * 9) {
+                if (upto * 10 >= tot * 9 && (w > 2 || st.max_row <= 8)) {
                     p->rows_w = w;
                     break;
                 }
                 w += 2;
             }
         }
+        // whether the rows kernel also takes the plan's direct and four-row
+        // tiles (hybrid plans).  A long row is one thread's there, and its
+        // warp waits.  Up to a word a row it is in those tiles too, in runs of
+        // four rows, and what counts is the number of rows: with few, a thread
+        // a row keeps more loads in flight; over several waves of CTAs the
+        // runs' wide accesses win (3 diagonals, 0.3 words a row, us in rows
+        // and in tiles: 100,000 rows 1.9 and 3.3; 650,000 4.5 and 4.6;
+        // 2,500,000 13.6 and 10.5; 7 diagonals 6.1 and 6.5 at 650,000, 8.5 and
+        // 8.1 at 1,000,000; 2 diagonals 6.1 and 5.4 there).  Above a word a
+        // row the tiles gather the words side by side, and the rows kernel is
+        // the faster one while no row takes more than 8 rounds and at most
+        // 0.5 % take more than 4 (300,000 rows of 1.3 words, 3 diagonals: 3.0
+        // and 5.4; with 0.1 % of 64 words 7.6 and 4.8, with one row of 128
+        // 11.0 and 5.2; 1,000,000 rows with 1 % of 32 words 12.6 and 11.5,
+        // with 0.1 % of 16 8.2 and 10.0)
+        const int W = prm.rows_w ? prm.rows_w : p->rows_w;
+        for (int L = std::min(4 * W, kStreamRowMax) + 1; L <= kStreamRowMax; ++L) many += h[L];
+        const int64_t wave = (int64_t)kRowsMinBlocks * num_sms() * kBlock;
+        p->rows_any = nnz_csr <= M ? M <= (p->num_negs <= 2 ? 3 : 4) * wave
+                                   : st.max_row <= 8 * W && many * 200 <= tot;
     }
 
     // the format: row pointers and words, each followed by at least 16 zero

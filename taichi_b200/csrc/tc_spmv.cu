@@ -473,9 +473,10 @@ tc::DevPlan tc_plan::dev_plan() const
     // unless a row is a CTA's: the CTA adds its words in another order, and a
     // plan gives the same y alone, in a batch and served
     const bool any_tiles = d.dia_shapes > 0 && d.per_tile == 2 && max_row <= tc::kStreamRowMax && ntiles_long == 0;
+    const bool short_rows = M > 0 && nnz_csr <= (int64_t)tc::kRowsMeanMax * M && (d.per_tile == 4 || rows_any);
     d.rows = 0;
     if ((d.per_tile == 4 || any_tiles) && !(params.flags & TC_FLAG_NO_ROWS))
-        d.rows = (params.flags & TC_FLAG_ROWS) || (M > 0 && nnz_csr <= (int64_t)tc::kRowsMeanMax * M && tc::kRowsByDefault);
+        d.rows = (params.flags & TC_FLAG_ROWS) || (short_rows && tc::kRowsByDefault);
     d.rows_w = params.rows_w ? params.rows_w : rows_w;
     d.pos = hybrid && all_pos ? 1 : 0;
     // CTAs resident at once (the stream kernel's many-tile build, the rows

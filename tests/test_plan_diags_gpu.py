@@ -98,3 +98,35 @@ def test_rows_of_a_cta(tc, dev, tile_nnz):
     assert torch.equal(y, yb)
     want = dense_multiply(f, M, x.astype(np.float64))
     assert np.abs(y.cpu().numpy() - want).max() <= 131 * 131 * 2.0 ** -24   # 131 terms of at most 1, one rounding each
+
+
+@pytest.mark.parametrize("M,mean,long,share,kernel", [
+    (60001, 0.4, 8, 0.01, 5), (60001, 0.4, 9, 0.01, 5), (60001, 0.4, 128, 0.002, 5),    # up to a word a row
+    (1212417, 0.3, 16, 0.001, 2), (1200001, 0.3, 16, 0.001, 5),                        # about four waves of rows
+    (400001, 1.3, 32, 0.004, 5), (400001, 1.3, 33, 0.004, 2), (400001, 1.3, 20, 0.02, 2), (400001, 1.3, 128, 1e-5, 2)])
+def test_spread_rows(tc, dev, M, mean, long, share, kernel):
+    """Hybrid plans of three diagonals on both sides of the rules that give
+    them to the rows kernel (5) or to their tiles (2), which lie at 148
+    multiprocessors: y against numpy, alone and in a batch."""
+    import torch
+    rng = np.random.default_rng(M + long)
+    lens = np.minimum(rng.poisson(mean, M), 6)
+    lens[rng.choice(M, max(1, int(M * share)), replace=False)] = long
+    rp = np.zeros(M + 1, np.int32)
+    np.cumsum(lens, out=rp[1:])
+    words = ((rng.integers(0, M, rp[-1]) << 1) | (rng.random(rp[-1]) < 0.7)).astype(np.int32)
+    f = dict(dia_shapes=1, num_negs=3, dense_nnz=1, zero_elements=0, sparse_nnz=len(words), row_start=0, row_stop=M,
+             xStart=[0], yStart=[0], xStop=[M], nDiasPtr=[0, 3], neg_offsets=[-1, 0, 2], csrRow=rp, csrCol=words)
+    plan = tc.Plan.from_format(M, M, f)
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert plan.info()["kernel"] == kernel
+    x = rng.integers(-8, 9, M).astype(np.float64)
+    xd, y, yb = torch.from_numpy(x.astype(np.float32)).to(dev), torch.empty(M, device=dev), torch.empty(M, device=dev)
+    plan.spmv(xd, y)
+    b, one = C.c_void_p(), C.c_void_p * 1
+    tc.check(tc.lib().tc_batch_create(1, one(plan.handle.value), one(xd.data_ptr()), one(yb.data_ptr()), C.byref(b)))
+    tc.check(tc.lib().tc_batch_run(b, None))
+    torch.cuda.synchronize()
+    tc.check(tc.lib().tc_batch_destroy(b))
+    np.testing.assert_array_equal(y.cpu().numpy().astype(np.float64), dense_multiply(f, M, x))
+    assert torch.equal(y, yb)
