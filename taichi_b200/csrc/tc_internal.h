@@ -314,10 +314,13 @@ constexpr int kLeanMinBlocks = 6;
 // The stream-only kernel: 5 CTAs per SM (48 registers) for plans that fit one
 // wave of them, where each CTA's chain counts (65,536 rows of 18 words, 60,000
 // of 39 and 100,000 of 29, iterated: 5.3 -> 4.9, 5.1 -> 4.6 and 5.6 -> 5.2 us
-// against 6 CTAs; 6.4 at 7 or 8); 8 CTAs at 32 registers (no spills) for plans
-// of more tiles, which gain from the extra resident loads (9-point mesh on
-// 2048^2: 63.2 -> 52.5 us).
+// against 6 CTAs; 6.4 at 7 or 8); 6 CTAs (40 registers) for plans that fit one
+// wave of those; 8 CTAs at 32 registers (no spills) for plans of more tiles,
+// which gain from the extra resident loads (9-point mesh on 2048^2: 63.2 ->
+// 52.5 us).  Without the 6-CTA build plans of 741 to 888 tiles ran the last
+// one: 200,000 rows of 12 words 12.0 -> 16.4 us, of 18 15.1 -> 20.3.
 constexpr int kStreamFewMinBlocks = 5;
+constexpr int kStreamWaveMinBlocks = 6;
 constexpr int kStreamManyMinBlocks = 8;
 // The rows kernel: 8 CTAs per SM (32 registers).
 constexpr int kRowsMinBlocks = 8;

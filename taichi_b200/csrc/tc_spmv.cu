@@ -300,16 +300,16 @@ __global__ void __launch_bounds__(kDirectWideBlock, 2)
 
 // The multiply of a plan of stream tiles only (meshes, banded and other
 // matrices of short, even rows): the grid kernel with no code for the other
-// tile kinds.  MANY: more tiles than one wave, compiled for 8 CTAs per SM.
-template <bool SIGNED, bool MANY>
-__global__ void __launch_bounds__(kBlock, MANY ? kStreamManyMinBlocks : kStreamFewMinBlocks)
+// tile kinds, compiled for B CTAs per SM (see kStreamFewMinBlocks).
+template <bool SIGNED, int B>
+__global__ void __launch_bounds__(kBlock, B)
     spmv_stream_kernel(DevPlan p, const float *__restrict__ x, float *__restrict__ y)
 {
     allow_next_grid();
     const Tile t = p.tiles[blockIdx.x];
     if (threadIdx.x == 0) {
         prefetch_x_window(x, p.N, t.row0, tile_nrows(t));
-        if (MANY && blockIdx.x + p.ahead < p.ntiles) {   // the tile a wave later
+        if (B == kStreamManyMinBlocks && blockIdx.x + p.ahead < p.ntiles) {   // the tile a wave later
             const Tile a = p.tiles[blockIdx.x + p.ahead];
             prefetch_rows_ahead(p, a.row0, a.row0 + tile_nrows(a), a.nz0, a.nz0 + a.nnz);
         }
@@ -387,9 +387,12 @@ static tc_status launch_tiles(const DevPlan &dp, const PlanDiags &dg, const Wide
         else if (dp.rows_w <= 6) TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_rows_kernel<SIGNED, 6>, dp, q, x, y));
         else TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_rows_kernel<SIGNED, 8>, dp, q, x, y));
     }
-    else if (dp.per_tile == 4 && dp.ntiles > kStreamFewMinBlocks * num_sms())
-        TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_stream_kernel<SIGNED, true>, dp, x, y));
-    else if (dp.per_tile == 4) TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_stream_kernel<SIGNED, false>, dp, x, y));
+    else if (dp.per_tile == 4 && dp.ntiles <= kStreamFewMinBlocks * num_sms())
+        TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_stream_kernel<SIGNED, kStreamFewMinBlocks>, dp, x, y));
+    else if (dp.per_tile == 4 && dp.ntiles <= kStreamWaveMinBlocks * num_sms())
+        TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_stream_kernel<SIGNED, kStreamWaveMinBlocks>, dp, x, y));
+    else if (dp.per_tile == 4)
+        TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_stream_kernel<SIGNED, kStreamManyMinBlocks>, dp, x, y));
     else if (dp.per_tile) TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_grid_kernel<SIGNED>, dp, x, y));
     else TC_CUDA(cudaLaunchKernelEx(&cfg, spmv_tiles_kernel<SIGNED>, dp, x, y));
     return TC_OK;
