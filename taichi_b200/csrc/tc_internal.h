@@ -126,6 +126,7 @@ __host__ __device__ inline int tile_word(int nrows, int kind) { return nrows | (
 constexpr int kBlock = 256;           // threads per CTA of the multiply kernels
 constexpr int kMaxTileRows = 1 << 20; // planner limit on rows per tile
 constexpr int kStageNnz = 8192;       // CSR words of a tile staged in shared memory
+constexpr int kMergeRows = 2048;      // most rows in one merge tile
 constexpr int kStreamNnz = 4096;      // most entries of a TILE_STREAM tile
 constexpr int kStreamRows = 256;      // most rows of a TILE_STREAM tile (1 per thread)
 constexpr int kStreamRowMax = 128;    // longer rows of a stream tile are summed by a warp (TILE_MIXED)

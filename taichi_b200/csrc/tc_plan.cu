@@ -30,10 +30,13 @@ int wide_tile_rows(int M, const tc_params &prm, int sms)
 
 namespace {
 
-// Rows are planned in strips of kStripRows, one warp each; a tile never
-// crosses a strip.  (A strip holds whole multiples of every kind's largest
-// tile, so short rows lose no tile to the cut.)
-constexpr int kStripRows = 2048;
+// Rows are planned in strips of kStripRows, a CTA each; a tile never crosses a
+// strip.  The last tile of a strip is what is left of it, so short strips make
+// small tiles: strips of 2,048 rows gave banded plans of 17 to 30 words a row,
+// whose tiles hold 136 to 240 rows, 5 to 10 % more tiles (220,000 rows of 24
+// words: 1,397 in place of 1,298 and 24.9 us in place of 22.4).
+constexpr int kStripRows = 16384;
+constexpr int kPlanBlock = 1024;
 
 struct RowStats {
     int max_row;                     // CSR words of the longest row
@@ -89,107 +92,183 @@ __device__ __forceinline__ int lanes_for(double mean, int max_lanes)
     return l;
 }
 
-// The number of leading i in [0, limit) for which ok(i) holds (a warp).
-template <class Ok>
-__device__ __forceinline__ int run_of(int limit, Ok ok)
+// A strip in shared memory: its row pointers, and a bit per row for the rows
+// of more than kStreamRowMax words and for those that get a CTA each.
+struct Strip {
+    const int *rp;
+    const unsigned *mid, *lng;
+    int n;                          // rows
+    bool any_mid, any_long;         // in the whole matrix
+};
+
+// The first i in [0, limit) for which row r + i is marked, else limit; rows
+// [r, r + limit) inside the strip.
+__device__ __forceinline__ int first_marked(const unsigned *mask, int r, int limit)
 {
-    const int lane = threadIdx.x & 31;
-    for (int i = 0; i < limit; i += 32) {
-        const unsigned bad = __ballot_sync(0xffffffffu, !(i + lane < limit && ok(i + lane)));
-        if (bad) return i + __ffs(bad) - 1;
+    for (int w = r >> 5; 32 * w < r + limit; ++w) {
+        unsigned v = mask[w];
+        if (w == r >> 5) v &= ~0u << (r & 31);
+        if (v) return min(limit, 32 * w + __ffs(v) - 1 - r);
     }
     return limit;
 }
 
-// The tiles of one strip per warp (a CTA of 32 threads): counted, and with
-// WRITE written from tiles[first[strip]] on.
-template <bool WRITE>
-__global__ void __launch_bounds__(32) plan_strips(const int *__restrict__ rowptr, int M, TilePrm q,
-                                                  int *__restrict__ count, const int *__restrict__ first,
-                                                  Tile *__restrict__ tiles, TileCounts *__restrict__ sum)
+// The tile that starts at row r of a strip (tile_mode 2): its rows, and its
+// kind from bit kTileRowBits on.
+constexpr int kTileRowBits = 12;
+static_assert(kMergeRows < 1 << kTileRowBits && TILE_MIXED < 1 << (16 - kTileRowBits), "packed in 16 bits");
+__device__ __forceinline__ int tile_at(const Strip &s, const TilePrm &q, int r)
 {
-    __shared__ int rp[kStripRows + 1];
-    const long row0 = (long)blockIdx.x * kStripRows;
-    const int n = (int)min((long)kStripRows, (long)M - row0), lane = threadIdx.x;
-    for (int i = lane; i <= n; i += 32) rp[i] = __ldg(rowptr + row0 + i);
-    __syncwarp();
-    TileCounts c{0, 0, 0, 1, 0};
-    int made = 0;
-    Tile *const out = WRITE ? tiles + first[blockIdx.x] : nullptr;
-    auto len = [&](int r) { return rp[r + 1] - rp[r]; };
-    auto put = [&](int r, int rows, int kind) {
-        const int nz = rp[r + rows] - rp[r];
-        if (WRITE && lane == 0) out[made] = Tile{(int)(row0 + r), rp[r], nz, tile_word(rows, kind)};
-        ++made;
-        c.stream += kind == TILE_STREAM;
-        c.lng += kind == TILE_LONG;
-        if (kind <= TILE_L32 || kind == TILE_MERGE) {
-            c.max_rows = max(c.max_rows, rows);
-            c.max_nnz = max(c.max_nnz, nz);
-        }
-    };
-    for (int r = 0; r < n;) {
-        if (len(r) > q.long_len) {
-            put(r, 1, TILE_LONG);
-            ++r;
-            continue;
-        }
-        if (q.mode == 2) {
-            // stream tile: rows up to the row and entry caps.  A run that
-            // starts on a multiple of 4 rows and holds many rows runs 4
-            // consecutive rows per thread: read directly from global memory
-            // when they average at most one entry (TILE_DIRECT4), through
-            // shared memory when at most two (TILE_STREAM4); otherwise one
-            // row per thread (TILE_STREAM; TILE_MIXED when it holds a row of
-            // more than kStreamRowMax entries)
-            const bool a4 = (r & 3) == 0 && !q.strided;
-            const int cap_rows = min(q.rows_cap, a4 ? kDirectRows : kStreamRows);
-            const int cap_nnz = max(1, min(2 * min(q.tile_nnz, 1 << 24), q.spread));
-            int m = run_of(min(cap_rows, n - r), [&](int i) {
-                return len(r + i) <= q.long_len && rp[r + i + 1] - rp[r] <= cap_nnz;
-            });
-            if (m == 0) m = 1;        // a single row longer than cap_nnz
-            const int small = run_of(m, [&](int i) { return len(r + i) <= kStreamRowMax; });
-            if (small >= 2 * kBlock) m = small;       // direct and four-row tiles hold short rows only
-            const int ent = rp[r + m] - rp[r];
-            const bool direct = a4 && small >= 2 * kBlock && ent <= m && !q.no_direct;
-            const bool four = !direct && a4 && small >= 2 * kBlock && ent <= 2 * m;
-            if (!direct) m = min(m, four ? kStream4Rows : kStreamRows);
-            if (r + m < n) {          // end on a multiple of 256 rows (whole row sweeps), else of 4
-                const int cut = (r + m) & ~255;
-                if (cut - r >= 256) m = cut - r;
-                else if (m > 4) m -= (r + m) & 3;
-            }
-            put(r, m, direct ? TILE_DIRECT4 : four ? TILE_STREAM4 : small < m ? TILE_MIXED : TILE_STREAM);
-            r += m;
-            continue;
-        }
-        // candidate run: up to 1024 rows (merge tiles: tile_rows), stopping
-        // before a long row
-        const int run_cap = q.mode == 0 ? min(q.rows_cap, kStripRows) : 1024;
-        const int m = run_of(min(run_cap, n - r), [&](int i) { return len(r + i) <= q.long_len; });
-        if (q.mode == 0) {            // merge tile: rows + entries split evenly
-            int rows = m;
-            while (rows > 1 && rp[r + rows] - rp[r] > kStageNnz) rows = (rows + 1) / 2;
-            put(r, rows, TILE_MERGE);
-            r += rows;
-            continue;
-        }
-        int lanes = lanes_for((double)(rp[r + m] - rp[r]) / m, q.max_lanes);
-        int rows = min(min(m, kBlock / lanes * 4), q.rows_cap);
-        while (rows > 1 && rp[r + rows] - rp[r] > kStageNnz) rows = (rows + 1) / 2;   // fits a stage
-        lanes = lanes_for((double)(rp[r + rows] - rp[r]) / rows, q.max_lanes);
-        c.vector += lanes > 1;
-        put(r, rows, 31 - __clz(lanes));
-        r += rows;
+    if (s.any_long && (s.lng[r >> 5] >> (r & 31) & 1u)) return 1 | TILE_LONG << kTileRowBits;
+    // stream tile: rows up to the row and entry caps.  A run that starts on a
+    // multiple of 4 rows and holds many rows runs 4 consecutive rows per
+    // thread: read directly from global memory when they average at most one
+    // entry (TILE_DIRECT4), through shared memory when at most two
+    // (TILE_STREAM4); otherwise one row per thread (TILE_STREAM; TILE_MIXED
+    // when it holds a row of more than kStreamRowMax entries)
+    const bool a4 = (r & 3) == 0 && !q.strided;
+    const int cap_nnz = max(1, min(2 * min(q.tile_nnz, 1 << 24), q.spread));
+    const int z = s.rp[r];
+    int m = 0;                    // most rows of at most cap_nnz words together
+    for (int hi = min(min(q.rows_cap, a4 ? kDirectRows : kStreamRows), s.n - r); m < hi;) {
+        const int half = (m + hi + 1) >> 1;
+        if (s.rp[r + half] - z <= cap_nnz) m = half;
+        else hi = half - 1;
     }
-    if (WRITE || lane) return;
-    count[blockIdx.x] = made;
-    if (c.vector) atomicAdd(&sum->vector, c.vector);
-    if (c.lng) atomicAdd(&sum->lng, c.lng);
-    if (c.stream) atomicAdd(&sum->stream, c.stream);
-    atomicMax(&sum->max_rows, c.max_rows);
-    atomicMax(&sum->max_nnz, c.max_nnz);
+    if (s.any_long) m = first_marked(s.lng, r, m);
+    if (m == 0) m = 1;            // a single row longer than cap_nnz
+    const int small = s.any_mid ? first_marked(s.mid, r, m) : m;
+    if (small >= 2 * kBlock) m = small;       // direct and four-row tiles hold short rows only
+    const int ent = s.rp[r + m] - z;
+    const bool direct = a4 && small >= 2 * kBlock && ent <= m && !q.no_direct;
+    const bool four = !direct && a4 && small >= 2 * kBlock && ent <= 2 * m;
+    if (!direct) m = min(m, four ? kStream4Rows : kStreamRows);
+    if (r + m < s.n) {            // end on a multiple of 256 rows (whole row sweeps), else of 4
+        const int cut = (r + m) & ~255;
+        if (cut - r >= 256) m = cut - r;
+        else if (m > 4) m -= (r + m) & 3;
+    }
+    return m | (direct ? TILE_DIRECT4 : four ? TILE_STREAM4 : small < m ? TILE_MIXED : TILE_STREAM) << kTileRowBits;
+}
+
+// The tile that starts at row r of a strip in tile_mode 0 or 1.
+__device__ __forceinline__ int tile_at_lanes(const Strip &s, const TilePrm &q, int r)
+{
+    if (s.any_long && (s.lng[r >> 5] >> (r & 31) & 1u)) return 1 | TILE_LONG << kTileRowBits;
+    // candidate run: up to 1024 rows (merge tiles: tile_rows), stopping
+    // before a long row
+    int m = min(q.mode == 0 ? min(q.rows_cap, kMergeRows) : 1024, s.n - r);
+    if (s.any_long) m = first_marked(s.lng, r, m);
+    const int z = s.rp[r];
+    if (q.mode == 0) {            // merge tile: rows + entries split evenly
+        while (m > 1 && s.rp[r + m] - z > kStageNnz) m = (m + 1) / 2;
+        return m | TILE_MERGE << kTileRowBits;
+    }
+    int lanes = lanes_for((double)(s.rp[r + m] - z) / m, q.max_lanes);
+    m = min(min(m, kBlock / lanes * 4), q.rows_cap);
+    while (m > 1 && s.rp[r + m] - z > kStageNnz) m = (m + 1) / 2;   // fits a stage
+    lanes = lanes_for((double)(s.rp[r + m] - z) / m, q.max_lanes);
+    return m | (31 - __clz(lanes)) << kTileRowBits;
+}
+
+// Rows between the starts whose tiles are found ahead of the walk: tiles of
+// stream plans start on multiples of 4 rows, but for a few.
+constexpr int kAheadStep = 4;
+
+size_t strip_smem(int rows)
+{
+    const size_t words = ((size_t)rows + 31) / 32;
+    return sizeof(int) * ((size_t)rows + 1 + 2 * words) + sizeof(unsigned short) * (words * 32 / kAheadStep);
+}
+
+// The planner's parameters of a plan's own tiles and of those for batches
+// (blockIdx.y).
+struct PlanLists {
+    TilePrm q[2];
+};
+
+// The tiles of one strip of one list: counted, and with WRITE written from
+// tiles[first[strip]] on.  Which tile starts at a row depends on the rows
+// alone, so the threads find the tile of every fourth row side by side, one
+// thread follows the chain of starts (a shared-memory read a tile), and all
+// write the tiles.  (A warp that looks through the rows tile by tile takes
+// 20 us for such a strip.)
+template <bool WRITE>
+__global__ void __launch_bounds__(kPlanBlock)
+    plan_strips(const int *__restrict__ rowptr, int M, const __grid_constant__ PlanLists lists,
+                const RowStats *__restrict__ st, int *__restrict__ count, const int *__restrict__ first,
+                Tile *__restrict__ tiles0, Tile *__restrict__ tiles1, TileCounts *__restrict__ sum)
+{
+    extern __shared__ int rp[];
+    __shared__ int made_s;
+    const TilePrm q = lists.q[blockIdx.y];
+    const long row0 = (long)blockIdx.x * kStripRows;
+    const int n = (int)min((long)kStripRows, (long)M - row0), words = (n + 31) >> 5;
+    unsigned *const mid = reinterpret_cast<unsigned *>(rp + n + 1), *const lng = mid + words;
+    unsigned short *const ahead = reinterpret_cast<unsigned short *>(lng + words);
+#pragma unroll 4
+    for (int i = threadIdx.x; i <= n; i += kPlanBlock) rp[i] = __ldg(rowptr + row0 + i);
+    const Strip s{rp, mid, lng, n, st->max_row > kStreamRowMax, st->max_row > q.long_len};
+    __syncthreads();
+    if (s.any_mid || s.any_long) {
+        for (int r = threadIdx.x; r < 32 * words; r += kPlanBlock) {        // whole warps
+            const int len = r < n ? rp[r + 1] - rp[r] : 0;
+            const unsigned m = __ballot_sync(0xffffffffu, len > kStreamRowMax);
+            const unsigned l = __ballot_sync(0xffffffffu, len > q.long_len);
+            if ((r & 31) == 0) {
+                mid[r >> 5] = m;
+                lng[r >> 5] = l;
+            }
+        }
+        __syncthreads();
+    }
+    if (q.mode == 2) {
+        for (int r = kAheadStep * threadIdx.x; r < n; r += kAheadStep * kPlanBlock)
+            ahead[r / kAheadStep] = (unsigned short)tile_at(s, q, r);
+        __syncthreads();
+    }
+    auto tile = [&](int r) {
+        if (q.mode != 2) return tile_at_lanes(s, q, r);
+        return r % kAheadStep ? tile_at(s, q, r) : (int)ahead[r / kAheadStep];
+    };
+    constexpr int kRows = (1 << kTileRowBits) - 1;
+    const int at = (int)blockIdx.y * ((int)gridDim.x + 1) + (int)blockIdx.x;     // of the list's counts
+    Tile *const out = WRITE ? (blockIdx.y ? tiles1 : tiles0) + first[at] : nullptr;
+    if (threadIdx.x == 0) {
+        TileCounts c{0, 0, 0, 1, 0};
+        int made = 0;
+        for (int r = 0; r < n; ++made) {
+            const int t = tile(r), rows = t & kRows, kind = t >> kTileRowBits;
+            if (WRITE) {
+                out[made].row0 = r;
+            } else {
+                c.stream += kind == TILE_STREAM;
+                c.lng += kind == TILE_LONG;
+                c.vector += kind > TILE_L1 && kind <= TILE_L32;
+                if (kind <= TILE_L32 || kind == TILE_MERGE) {
+                    c.max_rows = max(c.max_rows, rows);
+                    c.max_nnz = max(c.max_nnz, rp[r + rows] - rp[r]);
+                }
+            }
+            r += rows;
+        }
+        made_s = made;
+        if (!WRITE) {
+            TileCounts *const total = sum + blockIdx.y;
+            count[at] = made;
+            if (c.vector) atomicAdd(&total->vector, c.vector);
+            if (c.lng) atomicAdd(&total->lng, c.lng);
+            if (c.stream) atomicAdd(&total->stream, c.stream);
+            atomicMax(&total->max_rows, c.max_rows);
+            atomicMax(&total->max_nnz, c.max_nnz);
+        }
+    }
+    if (!WRITE) return;
+    __syncthreads();
+    for (int k = threadIdx.x; k < made_s; k += kPlanBlock) {
+        const int r = out[k].row0, t = tile(r), rows = t & kRows;
+        out[k] = Tile{(int)(row0 + r), rp[r], rp[r + rows] - rp[r], tile_word(rows, t >> kTileRowBits)};
+    }
 }
 
 // Wide direct tiles: `rows` rows each, in row order.
@@ -349,9 +428,13 @@ tc_status plan_upload(tc_plan *p, const int *csrRow, const int *csrCol, int64_t 
     TilePrm bq = q;                           // the tiles of batch and served launches
     bq.spread = kStreamNnz;
     const bool second = M > 0 && prm.tile_mode == 2 && q.spread < kStreamNnz;
+    const size_t smem = strip_smem(std::min(M, kStripRows));
+    const PlanLists lists{{q, bq}};
     if (M) {
-        plan_strips<false><<<strips, 32, 0, stream>>>(csrRow, M, q, d_cnt, nullptr, nullptr, d_sum);
-        if (second) plan_strips<false><<<strips, 32, 0, stream>>>(csrRow, M, bq, d_bcnt, nullptr, nullptr, d_sum + 1);
+        TC_CHECK(ensure_smem((const void *)plan_strips<false>, smem));
+        TC_CHECK(ensure_smem((const void *)plan_strips<true>, smem));
+        plan_strips<false><<<dim3(strips, second ? 2 : 1), kPlanBlock, smem, stream>>>(csrRow, M, lists, d_st, d_cnt, nullptr,
+                                                                                     nullptr, nullptr, d_sum);
         TC_CUDA(cudaGetLastError());
         TC_CHECK(exclusive_scan(d_cnt, d_first, strips, d_tmp, stream));
         if (second) TC_CHECK(exclusive_scan(d_bcnt, d_bfirst, strips, d_tmp, stream));
@@ -476,8 +559,8 @@ tc_status plan_upload(tc_plan *p, const int *csrRow, const int *csrCol, int64_t 
         wide_tiles<<<(unsigned)((p->ntiles + 255) / 256), 256, 0, stream>>>(p->d_rowptr, M, p->wide_rows, p->ntiles,
                                                                           p->d_tiles);
     else if (M)
-        plan_strips<true><<<strips, 32, 0, stream>>>(p->d_rowptr, M, q, nullptr, d_first, p->d_tiles, nullptr);
-    if (!own) plan_strips<true><<<strips, 32, 0, stream>>>(p->d_rowptr, M, bq, nullptr, d_bfirst, p->d_btiles, nullptr);
+        plan_strips<true><<<dim3(strips, own ? 1 : 2), kPlanBlock, smem, stream>>>(p->d_rowptr, M, lists, d_st, nullptr, d_first,
+                                                                                 p->d_tiles, p->d_btiles, nullptr);
     for (int k = 0; k < 3; ++k) {
         Tile *list = k == 0 ? p->d_tiles : k == 1 ? p->d_wtiles : p->d_btiles;
         const int n = k == 0 ? p->ntiles : k == 1 ? p->nwtiles : own ? 0 : p->nbtiles;

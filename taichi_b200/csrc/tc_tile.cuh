@@ -303,7 +303,6 @@ __device__ __forceinline__ void tile_rows_seq(const DevPlan &p, const Tile &t, c
 // leaves a carry there; the thread that closes the row adds the carries of
 // the runs before it in thread order, so the sum order is fixed by the tile
 // alone.  Then each row gets its dense-diagonal terms and y is stored once.
-constexpr int kMergeRows = 2048;          // most rows in one merge tile
 constexpr int kMergeBatch = 8;            // gathers in flight per thread
 
 // Largest i in [0, nr] whose first CSR entry plus i does not pass item d.
