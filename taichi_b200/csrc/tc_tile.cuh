@@ -71,7 +71,7 @@ template <bool SIGNED, bool POS>
 __device__ __forceinline__ float gather_wide(const float *__restrict__ x, int c)
 {
     const float v = ldx(x + (SIGNED ? c >> 1 : c));
-    return SIGNED && !POS ? signed_term(v, c) : v;
+    return !SIGNED || POS || (c & 1) ? v : -v;
 }
 
 // Programmatic dependent launch: a kernel reads only immutable plan data
