@@ -368,8 +368,11 @@ tc_status launch(const DevPlan &dp, const PlanDiags &dg, int64_t nnz_csr, int ma
     if constexpr (SIGNED) q = dg;
     // Runs: plain rows of at most two words on average, in groups of 8 lanes
     // or more (a run of 2^lg rows; smaller groups diverge more than they
-    // save).  Longer rows keep a group's loads in flight by themselves.
-    if (!SIGNED && lg >= 3 && max_row <= kSpmmMidRow && nnz_csr <= 2LL * dp.M) {
+    // save), and rows for two CTAs per SM, as a warp's 32 rows are a chain (k =
+    // 64, R-MAT, us as runs and row by row: 8,192 rows 4.5 and 2.5, 32,768 5.0
+    // and 3.8, 65,536 5.8 and 5.9, 131,072 8.2 and 9.9).  Longer rows keep a
+    // group's loads in flight by themselves.
+    if (!SIGNED && lg >= 3 && max_row <= kSpmmMidRow && nnz_csr <= 2LL * dp.M && dp.M >= 2 * kBlock * num_sms()) {
         const unsigned grid = (unsigned)((dp.M + (long)kBlock - 1) / kBlock);
         spmm_run_kernel<V, VEC, 4><<<grid, kBlock, 0, s>>>(dp, X, ldx, k, lg, kRunBlocks * num_sms(), Y, ldy);
     } else if (max_row > kSpmmMidRow) {

@@ -83,6 +83,29 @@ def test_layouts(tc, dev, name):
         assert bool(torch.isnan(yb).all()), (k, pad, off)
 
 
+@pytest.mark.parametrize("more", [-1, 0, 1, 31, 255])
+def test_runs(tc, dev, more):
+    """Short plain rows about the number from which they run as runs (two CTAs
+    of 256 rows per multiprocessor)."""
+    import torch
+    M = 512 * torch.cuda.get_device_properties(0).multi_processor_count + more
+    rng = np.random.default_rng(M)
+    lens = rng.choice([0, 0, 1, 1, 2, 5], M)
+    lens[[0, 31, 32, M - 1]] = [64, 0, 64, 40]
+    rp = np.zeros(M + 1, np.int32)
+    np.cumsum(lens, out=rp[1:])
+    col = rng.integers(0, 3000, rp[-1]).astype(np.int32)
+    plan = tc.Plan.from_csr(M, 3000, rp, col, partition=False)
+    for k in (5, 16, 29, 32, 64):
+        X = rng.integers(-8, 9, (3000, k)).astype(np.float32)
+        Y = torch.full((M, k), float("nan"), device=dev)
+        plan.spmm(torch.from_numpy(X).to(dev), Y)
+        torch.cuda.synchronize()
+        sums = np.zeros((rp[-1] + 1, k))
+        np.cumsum(X[col], axis=0, out=sums[1:], dtype=np.float64)
+        np.testing.assert_array_equal(Y.cpu().numpy().astype(np.float64), sums[rp[1:]] - sums[rp[:-1]], err_msg=str(k))
+
+
 def test_non_finite_rows_stay_apart(tc, dev):
     """Slots past a row's words load X's row 0 and must not add it."""
     import torch
