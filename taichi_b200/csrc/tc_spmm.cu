@@ -258,10 +258,11 @@ __global__ void __launch_bounds__(kBlock, spmm_blocks(V, W))
 
 // Other plans: a CTA per tile of the plan's tile list, whose words are
 // bounded, so that rows of many words do not gather in a few CTAs (they are
-// neighbours in a power-law graph).  A row that is a tile of its own is
-// summed by the whole CTA: each group adds every groups-th word, the first
-// group joins the parts in group order.
-template <bool SIGNED, int V, bool VEC, int W>
+// neighbours in a power-law graph).  Tiles of short rows hold up to 4,096 of
+// them, kBlock >> lg a pass; SPLIT deals the passes out to gridDim.y CTAs.  A
+// row that is a tile of its own is summed by the whole CTA: each group adds
+// every groups-th word, the first group joins the parts in group order.
+template <bool SIGNED, int V, bool VEC, int W, bool SPLIT>
 __global__ void __launch_bounds__(kBlock, spmm_blocks(V, W))
     spmm_tiles_kernel(DevPlan p, const __grid_constant__ typename DiagsOf<SIGNED>::type q,
                       const float *__restrict__ X, int ldx, int k, int lg, float *__restrict__ Y,
@@ -274,10 +275,11 @@ __global__ void __launch_bounds__(kBlock, spmm_blocks(V, W))
     const Tile t = p.tiles[blockIdx.x];
     const int nr = tile_nrows(t);
     if (nr > 1 || t.nnz <= kSpmmLongRow) {
-        for (int i = 0; i < nr; i += groups)
+        for (int i = SPLIT ? blockIdx.y * groups : 0; i < nr; i += SPLIT ? gridDim.y * groups : groups)
             spmm_rows<SIGNED, V, VEC, W, true>(p, q, Xc, ldx, l, lg, t.row0 + i, min(groups, nr - i), Y + l.at, ldy);
         return;
     }
+    if (SPLIT && blockIdx.y) return;
     Cols<V, VEC> acc;
     acc.zero();
     sum_words<SIGNED, V, VEC, W>(p, Xc, ldx, l, Words(t.nz0, t.nz0 + t.nnz, group), groups, acc);
@@ -376,7 +378,19 @@ tc_status launch(const DevPlan &dp, const PlanDiags &dg, int64_t nnz_csr, int ma
         const unsigned grid = (unsigned)((dp.M + (long)kBlock - 1) / kBlock);
         spmm_run_kernel<V, VEC, 4><<<grid, kBlock, 0, s>>>(dp, X, ldx, k, lg, kRunBlocks * num_sms(), Y, ldy);
     } else if (max_row > kSpmmMidRow) {
-        spmm_tiles_kernel<SIGNED, V, VEC, 4><<<dp.ntiles, kBlock, 0, s>>>(dp, q, X, ldx, k, lg, Y, ldy);
+        // Two passes a CTA where the tiles hold more rows than stream tiles do
+        // and more than four passes, on average (k = 64, one row of 65 words,
+        // us with a CTA per tile and now: 65,536 rows of 0.6 words 33.0 and
+        // 8.9, 1,048,576 190 and 119, 200,000 of one word and three diagonals
+        // 78 and 58).  (Row by row whenever no row takes a CTA: the same for
+        // these, but 400 neighbouring rows of 400 words 5 -> 76 at k = 2.)
+        const int rows = dp.M / dp.ntiles, pass = kBlock >> lg;
+        if (rows > std::max(kStreamRows, 4 * pass)) {
+            const dim3 grid(dp.ntiles, (rows + 2 * pass - 1) / (2 * pass));
+            spmm_tiles_kernel<SIGNED, V, VEC, 4, true><<<grid, kBlock, 0, s>>>(dp, q, X, ldx, k, lg, Y, ldy);
+        } else {
+            spmm_tiles_kernel<SIGNED, V, VEC, 4, false><<<dp.ntiles, kBlock, 0, s>>>(dp, q, X, ldx, k, lg, Y, ldy);
+        }
     } else {
         // Rows of at most 8 words on average: three words in flight and two
         // more CTAs per SM (mesh 1200^2, k = 8: 41 us in place of 47);

@@ -106,6 +106,45 @@ def test_runs(tc, dev, more):
         np.testing.assert_array_equal(Y.cpu().numpy().astype(np.float64), sums[rp[1:]] - sums[rp[:-1]], err_msg=str(k))
 
 
+@pytest.mark.parametrize("name", ["wide", "direct", "hybrid"])
+def test_large_tiles(tc, dev, name):
+    """Plans with rows of more than 64 words whose tiles hold hundreds of short
+    rows, dealt out to several CTAs: row counts off every boundary."""
+    import torch
+    M, N = {"wide": 40003, "direct": 9001, "hybrid": 30011}[name], 3000 if name != "hybrid" else 30011
+    rng = np.random.default_rng(M)
+    lens = rng.choice([0, 0, 1, 1, 2], M)
+    lens[[0, 1, M // 2, M - 1]] = [65, 128, 100, 70]
+    if name == "direct":
+        lens[[5000, 5001]] = [1500, 5000]
+    rp = np.zeros(M + 1, np.int32)
+    np.cumsum(lens, out=rp[1:])
+    col = rng.integers(0, N, rp[-1]).astype(np.int32)
+    sign = np.ones(rp[-1])
+    if name == "hybrid":
+        sign = np.where(rng.random(rp[-1]) < 0.7, 1.0, -1.0)
+        f = dict(dia_shapes=1, num_negs=3, dense_nnz=1, zero_elements=0, sparse_nnz=rp[-1], row_start=0, row_stop=M,
+                 xStart=[0], yStart=[0], xStop=[M], nDiasPtr=[0, 3], neg_offsets=[-2, 0, 1], csrRow=rp,
+                 csrCol=(col << 1) | (sign > 0))
+        plan = tc.Plan.from_format(M, N, f)
+    else:
+        plan = tc.Plan.from_csr(M, N, rp, col, partition=False)
+    assert M // plan.info()["ntiles"] > 256 and (plan.info()["kernel"] == 3) == (name == "wide")
+    for k in (1, 2, 5, 16, 29, 64):
+        X = rng.integers(-8, 9, (N, k)).astype(np.float32)
+        Y = torch.full((M, k), float("nan"), device=dev)
+        plan.spmm(torch.from_numpy(X).to(dev), Y)
+        torch.cuda.synchronize()
+        sums = np.zeros((rp[-1] + 1, k))
+        np.cumsum(X[col] * sign[:, None], axis=0, out=sums[1:])
+        want = sums[rp[1:]] - sums[rp[:-1]]
+        if name == "hybrid":
+            want += X
+            want[2:] += X[:-2]
+            want[:-1] += X[1:]
+        np.testing.assert_array_equal(Y.cpu().numpy().astype(np.float64), want, err_msg=str(k))
+
+
 def test_non_finite_rows_stay_apart(tc, dev):
     """Slots past a row's words load X's row 0 and must not add it."""
     import torch
