@@ -20,6 +20,7 @@
 //   9-point mesh 1531^2 (hybrid, 6 words a row)      45.1 -> 27.8
 //   banded 700,001 x 32                             107.5 -> 35.9
 //   banded 65,536 x 18                                8.3 -> 4.9
+//   banded 1,003,602 x 19                            39.7 -> 36.7
 //   R-MAT scale 20 (0.6 words a row)                 22.9 -> 6.9
 //   15 diagonals of 900,000 rows with holes          31.5 -> 14.4
 //   power-law R-MAT scale 20 / 18 / 16          82 / 30 / 17 -> 73 / 23 / 12
@@ -259,11 +260,18 @@ tc_status launch_f64(const DevPlan &dp, const PlanDiags &dg, int64_t nnz_csr, in
         TC_CUDA(cudaLaunchKernelEx(&cfg, f64_tiles_kernel<SIGNED>, dp, q, x, y));
     } else if (nnz_csr <= 8LL * dp.M) {
         // a thread a row while a warp's words of consecutive rows share lines;
-        // above, lanes enough for 4 words or fewer each (18 words: 4.9 us at 8
-        // lanes in place of 8.3 at one; 32 words: 36 in place of 107)
+        // above, more lanes the longer the rows (banded matrices, us at 1 / 2 /
+        // 4 / 8 lanes: 2,000,000 x 9 43.5 / 42.2 / 48.8 / 77.2, 600,000 x 17
+        // 14.8 / 13.7 / 16.4 / 20.8, 1,003,602 x 19 42.3 / 37.9 / 36.6 / 43.6,
+        // 831,425 x 30 61.2 / 50.2 / 45.1 / 46.0, 363,335 x 32 62.5 / 32.4 /
+        // 21.3 / 18.3), and four in place of two where two would not fill the
+        // GPU (60,000 x 9 4.4 / 4.0 / 2.6 / 3.5)
         cfg.gridDim = grid(0);
         TC_CUDA(cudaLaunchKernelEx(&cfg, f64_rows_kernel<SIGNED, 0>, dp, q, ahead, x, y));
-    } else if (nnz_csr <= 16LL * dp.M) {
+    } else if (nnz_csr <= 17LL * dp.M && dp.M >= kF64Blocks * (kBlock >> 1) * num_sms()) {
+        cfg.gridDim = grid(1);
+        TC_CUDA(cudaLaunchKernelEx(&cfg, f64_rows_kernel<SIGNED, 1>, dp, q, ahead, x, y));
+    } else if (nnz_csr <= 28LL * dp.M) {
         cfg.gridDim = grid(2);
         TC_CUDA(cudaLaunchKernelEx(&cfg, f64_rows_kernel<SIGNED, 2>, dp, q, ahead, x, y));
     } else {

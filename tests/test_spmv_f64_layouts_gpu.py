@@ -42,6 +42,28 @@ def test_layouts(tc, dev, name):
     np.testing.assert_array_equal(y.cpu().numpy(), want)
 
 
+@pytest.mark.parametrize("more", [-1, 0, 1, 127])
+@pytest.mark.parametrize("mean", [9, 17, 18, 29])
+def test_lanes(tc, dev, mean, more):
+    """Rows about the lengths and the number from which two, four or eight
+    lanes share one (8 CTAs of 128 rows per multiprocessor)."""
+    import torch
+    M = 1024 * torch.cuda.get_device_properties(0).multi_processor_count + more
+    rng = np.random.default_rng(mean)
+    lens = np.full(M, mean)
+    lens[[1, M - 1]] = [mean - 9, mean + 9]          # the mean as it is, not every row the same
+    rp = np.zeros(M + 1, np.int32)
+    np.cumsum(lens, out=rp[1:])
+    col = rng.integers(0, M, rp[-1]).astype(np.int32)
+    plan = tc.Plan.from_csr(M, M, rp, col, partition=False)
+    x = rng.integers(-8, 9, M)
+    y = torch.full((M,), float("nan"), dtype=torch.float64, device=dev)
+    plan.spmv_f64(torch.from_numpy(x.astype(np.float64)).to(dev), y)
+    torch.cuda.synchronize()
+    sums = np.concatenate([[0], np.cumsum(x[col])])
+    np.testing.assert_array_equal(y.cpu().numpy().astype(np.int64), sums[rp[1:]] - sums[rp[:-1]])
+
+
 def test_no_columns(tc, dev):
     import torch
     plan = tc.Plan.from_csr(40, 0, np.zeros(41, np.int32), np.zeros(0, np.int32), partition=False)
