@@ -68,3 +68,34 @@ def test_mixed_tiles(tc, dev, name):
         server.run([0.0], [mid], [xd], [ys], mode=tc.SERVE_DEVICE_VECTORS)
         server.close()
         assert torch.equal(y, ys)
+
+
+def test_served_in_large_launches(tc, dev):
+    """Requests whose plans' own tiles come to more than a wave of CTAs (8 per
+    multiprocessor) run the plans' tiles for large launches, also in one launch
+    with smaller plans: each y as its plan alone gives it."""
+    import torch
+    rng = np.random.default_rng(4)
+    names = ["edges", "eights", "sparse", "hybrid"]
+    plans = [tc.Plan.from_csr(*matrix(n)) for n in names]
+    M = 60000                                        # tiles of 512 words alone, of up to 4,096 in large launches
+    plans.append(tc.Plan.from_csr(M, M, np.arange(0, 5 * M + 1, 5, dtype=np.int32),
+                                  rng.integers(0, M, 5 * M).astype(np.int32), partition=False))
+    sizes = [p.info() for p in plans]
+    order = [4, 0, 4, 1, 4, 2, 4, 3] * 6
+    wave = 8 * torch.cuda.get_device_properties(0).multi_processor_count
+    for at in range(len(order) - 4):                 # any five requests together are a large launch
+        assert sum(sizes[i]["ntiles"] for i in order[at:at + 5]) > wave > sizes[4]["ntiles"]
+    xs = [torch.from_numpy(rng.uniform(-1, 1, sizes[i]["N"]).astype(np.float32)).to(dev) for i in order]
+    want = [torch.empty(sizes[i]["M"], device=dev) for i in order]
+    for i, x, y in zip(order, xs, want):
+        plans[i].spmv(x, y)
+    server = tc.Server(solo_bytes=0, contexts=1, max_inflight=1)     # requests wait while a launch runs
+    ids = [server.admit(p) for p in plans]
+    ys = [torch.full_like(y, float("nan")) for y in want]
+    torch.cuda.synchronize()
+    stats, _ = server.run([0.0] * len(order), [ids[i] for i in order], xs, ys, mode=tc.SERVE_DEVICE_VECTORS)
+    server.close()
+    assert stats["mean_batch"] > 4
+    for i, y, w in zip(order, ys, want):
+        assert torch.equal(y, w), i

@@ -81,3 +81,39 @@ def test_hole_bits(tc, dev, kind, segs, many):
         assert got[k] == want[k], k
     for k in ("xStart", "yStart", "xStop", "nDiasPtr", "neg_offsets", "csrRow", "csrCol"):
         np.testing.assert_array_equal(got[k], want[k], err_msg=k)
+
+
+def blocks(nb, side, gap, dup, seed):
+    """nb diagonal blocks of seven diagonals with holes, some with entries twice."""
+    rng = np.random.default_rng(seed)
+    rows, cols = [], []
+    for b in range(nb):
+        o = b * (side + gap)
+        i = np.arange(o, o + side)
+        for d in range(-3, 4):
+            ok = (i + d >= o) & (i + d < o + side) & (rng.random(side) >= 0.05)
+            rows.append(i[ok])
+            cols.append(i[ok] + d)
+        if b in dup:
+            k = o + rng.integers(0, side, 6)
+            rows.append(k)
+            cols.append(k)
+    rows, cols = np.concatenate(rows), np.concatenate(cols)
+    order = np.lexsort((cols, rows))
+    M = nb * (side + gap)
+    return (M,) + rebuild(M, rows[order], cols[order])
+
+
+@pytest.mark.parametrize("nb,height,more_than", [(40, 1024, 32), (270, 4096, 250)])
+def test_many_shapes(tc, dev, nb, height, more_than):
+    """More shapes than one histogram launch counts, and more claiming shapes
+    than there are marks, with duplicate entries in shapes before and after."""
+    M, rp, col = blocks(nb, 100, 12, {2, nb // 3, nb - 3}, 1)
+    over = dict(thumb_height=height, min_contour=10, min_shape_side=20)
+    want, _ = oracle.partition(M, M, rp, col, params=oracle.default_params(**over))
+    assert want["dia_shapes"] > more_than and want["zero_elements"] > 0
+    got = tc.Plan.from_csr(M, M, rp, col, prm=tc.params(**over)).export()
+    for k in oracle.FORMAT_KEYS:
+        assert got[k] == want[k], k
+    for k in ("xStart", "yStart", "xStop", "nDiasPtr", "neg_offsets", "csrRow", "csrCol"):
+        np.testing.assert_array_equal(got[k], want[k], err_msg=k)
