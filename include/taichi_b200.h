@@ -95,10 +95,11 @@ typedef struct tc_params {
                                      length                                 */
 #define TC_FLAG_NO_ROWS      0x800 /* the same plans: never run the rows
                                      kernel                                 */
-#define TC_FLAG_NO_PREFETCH  0x2000 /* stream and rows kernels: no L2
-                                     prefetch of the operands of the CTA a
-                                     wave ahead; wide kernel: no L2 prefetch
-                                     of a tile's CSR words                  */
+#define TC_FLAG_NO_PREFETCH  0x2000 /* stream and rows kernels, tc_spmm and
+                                     tc_spmv_f64: no L2 prefetch of the
+                                     operands of the CTA a wave ahead; wide
+                                     kernel: no L2 prefetch of a tile's CSR
+                                     words                                  */
 #define TC_FLAG_NO_PARAM_STARTS 0x4000 /* wide plans: each tile's word
                                      range from its tile record, not from
                                      the launch parameters                  */

@@ -368,6 +368,8 @@ tc_status launch(const DevPlan &dp, const PlanDiags &dg, int64_t nnz_csr, int ma
     while ((V << lg) < k) ++lg;
     typename DiagsOf<SIGNED>::type q;
     if constexpr (SIGNED) q = dg;
+    // CTAs resident at once, whose operands later CTAs' prefetches run ahead by
+    auto ahead = [&](int blocks) { return dp.prefetch ? blocks * num_sms() : 1 << 30; };
     // Runs: plain rows of at most two words on average, in groups of 8 lanes
     // or more (a run of 2^lg rows; smaller groups diverge more than they
     // save), and rows for two CTAs per SM, as a warp's 32 rows are a chain (k =
@@ -376,7 +378,7 @@ tc_status launch(const DevPlan &dp, const PlanDiags &dg, int64_t nnz_csr, int ma
     // group's loads in flight by themselves.
     if (!SIGNED && lg >= 3 && max_row <= kSpmmMidRow && nnz_csr <= 2LL * dp.M && dp.M >= 2 * kBlock * num_sms()) {
         const unsigned grid = (unsigned)((dp.M + (long)kBlock - 1) / kBlock);
-        spmm_run_kernel<V, VEC, 4><<<grid, kBlock, 0, s>>>(dp, X, ldx, k, lg, kRunBlocks * num_sms(), Y, ldy);
+        spmm_run_kernel<V, VEC, 4><<<grid, kBlock, 0, s>>>(dp, X, ldx, k, lg, ahead(kRunBlocks), Y, ldy);
     } else if (max_row > kSpmmMidRow) {
         // Two passes a CTA where the tiles hold more rows than stream tiles do
         // and more than four passes, on average (k = 64, one row of 65 words,
@@ -400,10 +402,10 @@ tc_status launch(const DevPlan &dp, const PlanDiags &dg, int64_t nnz_csr, int ma
         const unsigned grid = (unsigned)((dp.M + (long)rows - 1) / rows);
         if (nnz_csr <= 8LL * dp.M)
             spmm_rows_kernel<SIGNED, V, VEC, W><<<grid, kBlock, 0, s>>>(
-                dp, q, X, ldx, k, lg, spmm_blocks(V, W) * num_sms(), Y, ldy);
+                dp, q, X, ldx, k, lg, ahead(spmm_blocks(V, W)), Y, ldy);
         else
             spmm_rows_kernel<SIGNED, V, VEC, 4><<<grid, kBlock, 0, s>>>(
-                dp, q, X, ldx, k, lg, spmm_blocks(V, 4) * num_sms(), Y, ldy);
+                dp, q, X, ldx, k, lg, ahead(spmm_blocks(V, 4)), Y, ldy);
     }
     TC_CUDA(cudaGetLastError());
     return TC_OK;

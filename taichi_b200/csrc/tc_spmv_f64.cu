@@ -253,7 +253,7 @@ tc_status launch_f64(const DevPlan &dp, const PlanDiags &dg, int64_t nnz_csr, in
     attr[0].val.programmaticStreamSerializationAllowed = dp.pdl ? 1 : 0;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const int ahead = kF64Blocks * num_sms();
+    const int ahead = dp.prefetch ? kF64Blocks * num_sms() : 1 << 30;
     auto grid = [&](int lg) { return dim3((unsigned)(((long)dp.M + (kBlock >> lg) - 1) / (kBlock >> lg))); };
     if (max_row > kShortRow) {
         cfg.gridDim = dim3(dp.ntiles);

@@ -130,3 +130,31 @@ def test_spread_rows(tc, dev, M, mean, long, share, kernel):
     tc.check(tc.lib().tc_batch_destroy(b))
     np.testing.assert_array_equal(y.cpu().numpy().astype(np.float64), dense_multiply(f, M, x))
     assert torch.equal(y, yb)
+
+
+@pytest.mark.parametrize("diags", [0, 3])
+@pytest.mark.parametrize("mean", [1, 6, 12, 30])
+def test_no_prefetch(tc, dev, diags, mean):
+    """TC_FLAG_NO_PREFETCH changes no result of any multiply."""
+    import torch
+    M, rng = 310001, np.random.default_rng(mean)
+    lens = rng.poisson(mean, M)
+    rp = np.zeros(M + 1, np.int32)
+    np.cumsum(lens, out=rp[1:])
+    col = rng.integers(0, M, rp[-1]).astype(np.int32)
+    f = dict(dia_shapes=int(diags > 0), num_negs=diags, dense_nnz=diags, zero_elements=0, sparse_nnz=rp[-1], row_start=0,
+             row_stop=M if diags else 0, xStart=[0], yStart=[0], xStop=[M], nDiasPtr=[0, diags], neg_offsets=[-1, 0, 1],
+             csrRow=rp, csrCol=(col << 1) | 1 if diags else col)
+    x = torch.rand(M, 16, device=dev)
+    got = []
+    for flags in (0, 0x2000):
+        plan = tc.Plan.from_format(M, M, f, prm=tc.params(flags=flags))
+        y, Y = torch.empty(M, device=dev), torch.empty(M, 16, device=dev)
+        y64 = torch.empty(M, dtype=torch.float64, device=dev)
+        plan.spmv(x[:, 0].contiguous(), y)
+        plan.spmv_f64(x[:, 1].double(), y64)
+        plan.spmm(x, Y)
+        torch.cuda.synchronize()
+        got.append((y, y64, Y))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
