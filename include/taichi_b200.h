@@ -52,7 +52,8 @@ typedef struct tc_params {
     double density;       /* a diagonal is dense if nnz/len >= density (0.6)   */
     int tile_rows;        /* max rows per multiply tile (1024)                 */
     int tile_nnz;         /* rows with more CSR entries get a CTA each (2048)  */
-    int max_lanes;        /* most lanes the planner gives one row: 1..32 (32)  */
+    int max_lanes;        /* tile_mode 1: most lanes the planner gives one row,
+                             1..32 (32)                                        */
     int ctas_per_sm;      /* resident CTAs per SM of the multiply grid (4)     */
     int tile_mode;        /* 0: rows and entries split evenly over a CTA's
                              threads (merge path); 1: lanes per row chosen
@@ -61,7 +62,8 @@ typedef struct tc_params {
                              row sums), one CTA per tile (2)                   */
     int flags;            /* TC_FLAG_*                                         */
     int rows_w;           /* rows kernel: words of a row loaded together, 4, 6
-                             or 8 (0: the least that holds 90 % of the rows)   */
+                             or 8 (0: the least that holds 90 % of the rows,
+                             2 too where no row has more than 8)               */
 } tc_params;
 
 #define TC_FLAG_NO_PARTITION 0x1  /* skip the morphology: plain CSR plan      */
@@ -150,6 +152,10 @@ TC_API tc_status tc_plan_create(int M, int N, int64_t nnz, const int *rowptr, co
 TC_API tc_status tc_plan_from_format(int M, int N, const tc_format *fmt, const tc_params *params,
                               void *stream, tc_plan **out);
 
+/* Builds take their scratch memory from a pool of the library, which keeps up
+ * to 256 MB of it between calls while plans exist and 64 MB after the last one
+ * is destroyed (of the device that is current then); more is given back before
+ * the call that took it returns. */
 TC_API tc_status tc_plan_destroy(tc_plan *plan);
 
 typedef struct tc_plan_info {

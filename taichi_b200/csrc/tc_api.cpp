@@ -96,10 +96,6 @@ tc_status tc::check_params(const tc_params &p)
 
 using tc::check_params;
 
-extern "C" {
-
-}  // extern "C"
-
 // A plan with the format's scalars and shape arrays (host arrays, checked
 // against M x N); the CSR remainder is still to be uploaded.
 static tc_status plan_of_shapes(int M, int N, const tc_format *f, const tc_params &prm, tc_plan **out)

@@ -137,7 +137,7 @@ constexpr int kDirectWideBlock = 1024; // threads of the direct kernel's CTAs
 constexpr int kPlanDiags = 4;         // dense diagonals a plan's descriptor carries
 // The rows kernel by default: stream plans whose rows average at most this
 // many CSR words.  Measured per multiply against stream tiles: mesh (6.1
-// words, hybrid) 39.4 against 45.7 µs; banded plain matrices of 9 words
+// words, hybrid) 37.2 against 45.7 µs; banded plain matrices of 9 words
 // 12.6 / 12.7 µs, of 11 words 81.4 / 71.5 µs, of 12 words 5.4 / 5.1 µs.
 constexpr int kRowsMeanMax = 8;
 constexpr bool kRowsByDefault = true;
@@ -198,7 +198,6 @@ struct DevPlan {
     const int2 *shape_dias; // dia_shapes: {first offset, end offset}
     const int *offsets;     // num_negs
     int M, N, ntiles, dia_shapes, row_start, row_stop, hybrid;
-    int max_span;           // widest offset span of any shape (max-min)
     int pdl;                // launch with programmatic stream serialization
     int stage_rp, stage_cw; // ints per shared-memory stage (row pointers, CSR words)
     int grid;               // persistent grid size
@@ -210,9 +209,9 @@ struct DevPlan {
     // plans whose dense part is one shape of at most kPlanDiags offsets
     // (dn of them, in offset order): offset i adds x[r + d_col[i]] to the rows
     // r of [d_lo[i], d_hi[i]) and no other row has a diagonal term.  dn = 0:
-    // no dense part, or more than one shape / more offsets (dgen = 1: the
+    // no dense part, or more than one shape / more offsets (PlanDiags, or the
     // per-row shape search, diag_row)
-    int dn, dgen;
+    int dn;
     int d_lo[kPlanDiags], d_hi[kPlanDiags], d_col[kPlanDiags];
     int2 d_in;              // the rows that every offset reaches
     int rows;               // stream plan run by the rows kernel (one row per thread)
@@ -228,8 +227,6 @@ struct DevPlan {
     int w_rp, w_cw, w_xw;   // ints per stage: row pointers, CSR words, x window
     int w_stages, w_grid;   // pipeline depth, persistent grid
 };
-
-struct tc_plan_impl;
 
 }  // namespace tc
 
@@ -260,7 +257,6 @@ struct tc_plan {
     // own tiles are as large as they get)
     tc::Tile *d_btiles = nullptr;
     int nbtiles = 0;
-    int max_span = 0;
     int stage_rp = 8, stage_cw = 8, grid = 1;
     int *d_err = nullptr;
     int wide_rows = 0;                   // rows of each wide direct tile

@@ -390,7 +390,6 @@ struct Border {
     int parent;     // hole: start pixel of the enclosing outer border
     int len;        // points of the traced contour
     int mid;        // pixel index of point len/2
-    int unused;
     long long area2;   // twice the signed area of the contour polygon (shoelace sum)
 };
 
@@ -449,7 +448,6 @@ __global__ void border_write(Img img, int *L, const int *__restrict__ at, Border
         }
         b.len = 0;
         b.mid = b.start;
-        b.unused = 0;
         b.area2 = 0;
         out[slot++] = b;
     }
@@ -1054,19 +1052,7 @@ struct ShapeResult {
     Scratch bits;                    // hole bits (see hole_bits)
 };
 
-static int g_sms = 0;
-static int sm_count()
-{
-    if (!g_sms) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev);
-        if (g_sms <= 0) g_sms = 148;
-    }
-    return g_sms;
-}
-
-static int box_grid(const ShapeBox &sb) { return std::max(1, std::min(cdiv(sb.b, 256), sm_count() * 8)); }
+static int box_grid(const ShapeBox &sb) { return std::max(1, std::min(cdiv(sb.b, 256), num_sms() * 8)); }
 
 // The box of a shape; nd <= 0 or b <= 0: no diagonal can be dense.
 static ShapeBox shape_box(int x, int y, int a, int b)
@@ -1227,7 +1213,7 @@ tc_status gpu_partition(int M, int N, int64_t nnz, const int *d_rowptr, const in
     TC_CHECK(bad.alloc(sizeof(int), s));
     const int T = 256;
     TC_CUDA(cudaMemsetAsync(bad.p, 0, sizeof(int), s));
-    validate_csr<<<std::max(1, std::min(cdiv(std::max<long>(nnz, M), T), sm_count() * 16)), T, 0, s>>>(
+    validate_csr<<<std::max(1, std::min(cdiv(std::max<long>(nnz, M), T), num_sms() * 16)), T, 0, s>>>(
         d_rowptr, d_col, M, N, nnz, bad.as<int>());
     int hbad = 0;
     TC_CUDA(cudaMemcpyAsync(&hbad, bad.p, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -1303,7 +1289,7 @@ tc_status gpu_partition(int M, int N, int64_t nnz, const int *d_rowptr, const in
         TC_CUDA(cudaMemcpyAsync(tab.as<char>() + o_off, out.offsets.data(), sizeof(int) * out.offsets.size(),
                                 cudaMemcpyHostToDevice, s));
         int *const rp_out = out.d_rowptr.as<int>();
-        const int grid = std::max(1, std::min(cdiv(M, T), sm_count() * 8));
+        const int grid = std::max(1, std::min(cdiv(M, T), num_sms() * 8));
         TC_CUDA(cudaMemsetAsync(cnt.as<int>() + M, 0, sizeof(int), s));          // the scan's trailing 0
         remainder_counts<<<grid, T, 0, s>>>(d_rowptr, claim.as<unsigned char>(), d_hs, (int)hs.size(), M,
                                             cnt.as<int>());

@@ -332,7 +332,6 @@ tc_status plan_upload(tc_plan *p, const int *csrRow, const int *csrCol, int64_t 
     // shape table {xStart, xStop, yStart, Msub} and offset ranges
     std::vector<int4> shapes(p->dia_shapes);
     std::vector<int2> sd(p->dia_shapes);
-    p->max_span = 0;
     for (int s = 0; s < p->dia_shapes; ++s) {
         shapes[s] = make_int4(p->h_xStart[s], p->h_xStop[s], p->h_yStart[s],
                               p->h_xStop[s] - p->h_xStart[s]);
@@ -341,7 +340,6 @@ tc_status plan_upload(tc_plan *p, const int *csrRow, const int *csrCol, int64_t 
         for (int n = sd[s].x + 1; n < sd[s].y; ++n)
             if (p->h_offsets[n] <= p->h_offsets[n - 1])
                 return fail(TC_ERR_FORMAT, "offsets of shape %d are not increasing", s);
-        p->max_span = std::max(p->max_span, p->h_offsets[sd[s].y - 1] - p->h_offsets[sd[s].x]);
     }
 
     // window plan: a second tile list for the window kernel (the batch and

@@ -445,7 +445,6 @@ tc::DevPlan tc_plan::dev_plan() const
     d.row_start = row_start;
     d.row_stop = row_stop;
     d.hybrid = hybrid;
-    d.max_span = max_span;
     d.pdl = (params.flags & TC_FLAG_NO_PDL) ? 0 : 1;
     d.stage_rp = stage_rp;
     d.stage_cw = stage_cw;
@@ -458,7 +457,6 @@ tc::DevPlan tc_plan::dev_plan() const
     d.wide_rows = wide_rows;
     d.skew = stream_skew;
     d.dn = 0;
-    d.dgen = 0;
     if (diags.n > 0 && diags.n <= tc::kPlanDiags) {
         d.dn = diags.n;
         d.d_in = diags.in;
@@ -467,8 +465,6 @@ tc::DevPlan tc_plan::dev_plan() const
             d.d_lo[i] = std::max(diags.rows.x, diags.cols.x - diags.col[i]);
             d.d_hi[i] = std::min(diags.rows.y, diags.cols.y - diags.col[i]);
         }
-    } else if (dia_shapes > 0) {
-        d.dgen = 1;
     }
     // the rows kernel: a stream plan (every row at most kStreamRowMax words)
     // of short rows, or any stream plan on request; hybrid plans that are not

@@ -2,8 +2,8 @@
 // kernel (single plan, batch, served) so that a matrix gets bit-identical y
 // whichever kernel runs it.
 //
-// A tile is a run of rows.  Its kind, chosen by the host planner from the
-// tile's row lengths, fixes how many lanes share a row (1, 2, 4, ..., 32); a
+// A tile is a run of rows.  Its kind, chosen by the planner (tc_plan.cu) from
+// the tile's row lengths, fixes how many lanes share a row (1, 2, 4, ..., 32); a
 // row longer than the planner's limit gets a whole CTA (TILE_LONG).  A lane
 // group handles kRPT rows per pass and keeps their loads in flight together.
 // Per row (FP32), each lane accumulates: the dense-diagonal terms of the
@@ -508,9 +508,10 @@ constexpr int kStreamQ = 2;   // int4 CSR words per thread per round
 // flight, of which eight tiles' shared memory leaves room for 92 KB (tiles of
 // 6,144 words, which leave 28 KB, ran the banded matrix of 2,279,375 x 32 at
 // 157 us in place of 93).  Past it by ld.global.cg in tiles of short rows
-// (93.4 -> 92.0 us, 256 matrices in a batch 149.4 -> 148.1), without
-// allocation in mixed ones (power-law R-MAT scale 20: 69.4 -> 66.4; each form
-// loses 1 % in the other's place).
+// (hybrid, 1.3 words a row: 1,000,000 rows 9.90 -> 9.72 us, 650,000 7.73 ->
+// 7.56, runs alike to 0.02; 65,536 x 18 7.13 -> 7.03), without allocation in
+// mixed ones (power-law R-MAT scale 20: 69.4 -> 66.4; each form loses 1 % in
+// the other's place).
 template <bool MIXED>
 __device__ __forceinline__ int4 load_words4(const int4 *p)
 {

@@ -214,18 +214,6 @@ __global__ void __launch_bounds__(kWinBlock, 1)
     }
 }
 
-int g_sms = 0;
-int sms()
-{
-    if (g_sms == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev);
-        if (g_sms <= 0) g_sms = 148;
-    }
-    return g_sms;
-}
-
 }  // namespace
 
 size_t window_smem_bytes(const DevPlan &dp)
