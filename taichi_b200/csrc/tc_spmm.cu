@@ -182,23 +182,25 @@ __device__ __forceinline__ void prefetch_later_rows(const DevPlan &p, long r0, i
     prefetch_rows_ahead(p, ra, rb, za, words_upto(za, zb, kAheadWords));
 }
 
-// Adds to acc the terms of every by-th of the words `a`, W of them in flight
-// together (a slot past the end loads X's row 0 and is not added).
+// Adds to acc the terms of every by-th of the words [b, e) from word b +
+// skipped on, W of them in flight together (a slot past the end loads X's row
+// 0 and is not added).
 template <bool SIGNED, int V, bool VEC, int W>
 __device__ __forceinline__ void sum_words(const DevPlan &p, const float *__restrict__ Xc, int ldx,
-                                          const Lane<V, VEC> &l, Words a, int by, Cols<V, VEC> &acc)
+                                          const Lane<V, VEC> &l, int b, int e, int skipped, int by,
+                                          Cols<V, VEC> &acc)
 {
-    for (; a.left > 0; a.skip(W * by)) {
+    each_step(b, e, skipped, W * by, [&](int j, int left) {
         int c[W];
         Cols<V, VEC> v[W];
 #pragma unroll
-        for (int w = 0; w < W; ++w) c[w] = w * by < a.left ? __ldg(p.cols + a.at + w * by) : 0;
+        for (int w = 0; w < W; ++w) c[w] = w * by < left ? __ldg(p.cols + j + w * by) : 0;
 #pragma unroll
         for (int w = 0; w < W; ++w) v[w].load(Xc + (long)word_col<SIGNED>(c[w]) * ldx, l);
 #pragma unroll
         for (int w = 0; w < W; ++w)
-            if (w * by < a.left) add_word<SIGNED>(acc, v[w], c[w]);
-    }
+            if (w * by < left) add_word<SIGNED>(acc, v[w], c[w]);
+    });
 }
 
 // Rows [row0, row0 + nrow) of a CTA, nrow <= kBlock >> lg: one row per group
@@ -217,7 +219,7 @@ __device__ __forceinline__ void spmm_rows(const DevPlan &p, const typename Diags
     if (group < nrow && (!MID || e - b <= kSpmmMidRow)) {
         Cols<V, VEC> acc;
         acc.zero();
-        sum_words<SIGNED, V, VEC, W>(p, Xc, ldx, l, Words(b, e), 1, acc);
+        sum_words<SIGNED, V, VEC, W>(p, Xc, ldx, l, b, e, 0, 1, acc);
         if constexpr (SIGNED) diag_cols(p, q, Xc, ldx, l, r, acc);
         acc.store(Yc + (long)r * ldy, l);
     }
@@ -231,7 +233,7 @@ __device__ __forceinline__ void spmm_rows(const DevPlan &p, const typename Diags
         const int re = __shfl_sync(0xffffffffu, e, src);
         Cols<V, VEC> acc;
         acc.zero();
-        sum_words<SIGNED, V, VEC, W>(p, Xc, ldx, l, Words(rb, re, wg), gw, acc);
+        sum_words<SIGNED, V, VEC, W>(p, Xc, ldx, l, rb, re, wg, gw, acc);
 #pragma unroll
         for (int u = 0; u < V; ++u)
             for (int o = 1 << lg; o < 32; o <<= 1) acc.a[u] += __shfl_xor_sync(0xffffffffu, acc.a[u], o);
@@ -282,7 +284,7 @@ __global__ void __launch_bounds__(kBlock, spmm_blocks(V, W))
     if (SPLIT && blockIdx.y) return;
     Cols<V, VEC> acc;
     acc.zero();
-    sum_words<SIGNED, V, VEC, W>(p, Xc, ldx, l, Words(t.nz0, t.nz0 + t.nnz, group), groups, acc);
+    sum_words<SIGNED, V, VEC, W>(p, Xc, ldx, l, t.nz0, t.nz0 + t.nnz, group, groups, acc);
 #pragma unroll
     for (int u = 0; u < V; ++u) part[u * kBlock + threadIdx.x] = acc.a[u];
     __syncthreads();

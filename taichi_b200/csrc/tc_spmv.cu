@@ -193,8 +193,8 @@ __global__ void __launch_bounds__(kBlock, kRowsMinBlocks)
                      const float *__restrict__ x, float *__restrict__ y)
 {
     allow_next_grid();
-    const int row0 = blockIdx.x * kBlock, r = row0 + (int)threadIdx.x;
-    const bool own = (int)threadIdx.x < p.M - row0;
+    const int r = blockIdx.x * kBlock + threadIdx.x;
+    const bool own = (unsigned)r < (unsigned)p.M;     // a last CTA's rows may lie past 2^31 - 1
     // warp 0 also brings into L2 the x window of the strip and the operands
     // of the strip a wave later (thread 0; the other warps skip it whole)
     const bool lead = threadIdx.x < 32;

@@ -112,7 +112,7 @@ __device__ __forceinline__ void after_wait(const float *__restrict__ &x, float *
 template <typename V>
 __device__ __forceinline__ void prefetch_x_window(const V *x, int N, int r0, int n)
 {
-    const int a = max(r0, 0), b = (int)min((long)r0 + n, (long)N);
+    const int a = max(r0, 0), b = r0 < N - n ? r0 + n : N;
     if (b <= a) return;
     const uintptr_t lo = (reinterpret_cast<uintptr_t>(x + a) + 15) & ~uintptr_t(15);
     const uintptr_t hi = reinterpret_cast<uintptr_t>(x + b) & ~uintptr_t(15);

@@ -29,6 +29,20 @@ static long walk(int b, int e, int lane, int by, int round)
     return bad + (want < end);                                  // a word left out
 }
 
+// The same with each_step.
+static long steps(int b, int e, int lane, int by, int round)
+{
+    long want = (long)b + lane, bad = 0;
+    tc::each_step(b, e, lane, round * by, [&](int j, int left) {
+        bad += j < b || j >= e || left != (long)e - j;
+        for (int w = 0; w < round && w * by < left; ++w) {
+            bad += (long)j + w * by != want;
+            want += by;
+        }
+    });
+    return bad + (want < e);
+}
+
 int main()
 {
     const int top = 2147483647;
@@ -40,7 +54,7 @@ int main()
             for (int by : bys)
                 for (int r : rounds)
                     for (int lane : {0, 1, by / 2, by - 1})
-                        if (lane < by && walk(end - n, end, lane, by, r)) ++bad;
+                        if (lane < by && (walk(end - n, end, lane, by, r) || steps(end - n, end, lane, by, r))) ++bad;
     for (int b : {0, 77, top - 100, top - 16384, top - 16385})
         for (int e : {b, b + 1, top - (top - b) / 2, top}) {
             const long want = (long)e - b > 16384 ? (long)b + 16384 : (long)e;
