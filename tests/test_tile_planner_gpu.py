@@ -7,7 +7,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-STRIP, BLOCK = 16384, 256
+STRIP, SPAN, BLOCK = 16384, 2048, 256
 
 
 def lanes_for(mean, most):
@@ -38,7 +38,8 @@ def plan(lens, sms, mode=2, tile_rows=1024, tile_nnz=2048, strided=False, no_dir
             stop = over[np.searchsorted(over, r)]
             if mode == 2:
                 a4 = r % 4 == 0 and not strided
-                m = min(np.searchsorted(rp, rp[r] + cap_nnz, "right") - 1 - r, min(tile_rows, 1024 if a4 else 256), stop - r)
+                end = min(n, r // SPAN * SPAN + SPAN) if lens.max() > 128 else n
+                m = min(np.searchsorted(rp, rp[r] + cap_nnz, "right") - 1 - r, min(tile_rows, 1024 if a4 else 256), stop - r, end - r)
                 m = max(int(m), 1)
                 small = min(m, mids[np.searchsorted(mids, r)] - r)
                 if small >= 2 * BLOCK:
@@ -48,7 +49,7 @@ def plan(lens, sms, mode=2, tile_rows=1024, tile_nnz=2048, strided=False, no_dir
                 four = not direct and a4 and small >= 2 * BLOCK and ent <= 2 * m
                 if not direct:
                     m = min(m, 1024 if four else 256)
-                if r + m < n:
+                if r + m < end:
                     cut = (r + m) // 256 * 256
                     m = cut - r if cut - r >= 256 else m - (r + m) % 4 if m > 4 else m
             else:
