@@ -255,6 +255,7 @@ tc_status launch_f64(const DevPlan &dp, const PlanDiags &dg, int64_t nnz_csr, in
     cfg.numAttrs = 1;
     const int ahead = dp.prefetch ? kF64Blocks * num_sms() : 1 << 30;
     auto grid = [&](int lg) { return dim3((unsigned)(((long)dp.M + (kBlock >> lg) - 1) / (kBlock >> lg))); };
+    auto full = [&](int lg) { return kF64Blocks * (kBlock >> lg) * num_sms(); };    // rows of a wave
     if (max_row > kShortRow) {
         cfg.gridDim = dim3(dp.ntiles);
         TC_CUDA(cudaLaunchKernelEx(&cfg, f64_tiles_kernel<SIGNED>, dp, q, x, y));
@@ -264,14 +265,14 @@ tc_status launch_f64(const DevPlan &dp, const PlanDiags &dg, int64_t nnz_csr, in
         // 4 / 8 lanes: 2,000,000 x 9 43.5 / 42.2 / 48.8 / 77.2, 600,000 x 17
         // 14.8 / 13.7 / 16.4 / 20.8, 1,003,602 x 19 42.3 / 37.9 / 36.6 / 43.6,
         // 831,425 x 30 61.2 / 50.2 / 45.1 / 46.0, 363,335 x 32 62.5 / 32.4 /
-        // 21.3 / 18.3), and four in place of two where two would not fill the
-        // GPU (60,000 x 9 4.4 / 4.0 / 2.6 / 3.5)
+        // 21.3 / 18.3), and more of them where these would not fill the GPU
+        // (60,000 x 9 4.4 / 4.0 / 2.6 / 3.5, 31,935 x 18 4.0 at 4 and 2.6 at 8)
         cfg.gridDim = grid(0);
         TC_CUDA(cudaLaunchKernelEx(&cfg, f64_rows_kernel<SIGNED, 0>, dp, q, ahead, x, y));
-    } else if (nnz_csr <= 17LL * dp.M && dp.M >= kF64Blocks * (kBlock >> 1) * num_sms()) {
+    } else if (nnz_csr <= 17LL * dp.M && dp.M >= full(1)) {
         cfg.gridDim = grid(1);
         TC_CUDA(cudaLaunchKernelEx(&cfg, f64_rows_kernel<SIGNED, 1>, dp, q, ahead, x, y));
-    } else if (nnz_csr <= 28LL * dp.M) {
+    } else if (nnz_csr <= 16LL * dp.M || (nnz_csr <= 28LL * dp.M && dp.M >= full(2))) {
         cfg.gridDim = grid(2);
         TC_CUDA(cudaLaunchKernelEx(&cfg, f64_rows_kernel<SIGNED, 2>, dp, q, ahead, x, y));
     } else {

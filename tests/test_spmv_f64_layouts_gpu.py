@@ -44,11 +44,12 @@ def test_layouts(tc, dev, name):
 
 @pytest.mark.parametrize("more", [-1, 0, 1, 127])
 @pytest.mark.parametrize("mean", [9, 17, 18, 29])
-def test_lanes(tc, dev, mean, more):
-    """Rows about the lengths and the number from which two, four or eight
-    lanes share one (8 CTAs of 128 rows per multiprocessor)."""
+@pytest.mark.parametrize("wave", [512, 1024])
+def test_lanes(tc, dev, wave, mean, more):
+    """Rows about the lengths and the numbers from which two, four or eight
+    lanes share one (8 CTAs of 128 and of 64 rows per multiprocessor)."""
     import torch
-    M = 1024 * torch.cuda.get_device_properties(0).multi_processor_count + more
+    M = wave * torch.cuda.get_device_properties(0).multi_processor_count + more
     rng = np.random.default_rng(mean)
     lens = np.full(M, mean)
     lens[[1, M - 1]] = [mean - 9, mean + 9]          # the mean as it is, not every row the same
