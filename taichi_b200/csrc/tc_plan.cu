@@ -43,24 +43,30 @@ struct RowStats {
     int max_row;                     // CSR words of the longest row
     int minus;                       // a word without the addition bit exists
     int hist[kStreamRowMax + 1];     // sampled rows by length
+    int whist[kStreamRowMax + 1];    // groups of 32 rows by their longest row (at most kStreamRowMax words)
 };
 
 __global__ void row_stats(const int *__restrict__ rowptr, int M, int step, RowStats *__restrict__ st)
 {
-    __shared__ int hist[kStreamRowMax + 1];
-    for (int i = threadIdx.x; i <= kStreamRowMax; i += blockDim.x) hist[i] = 0;
+    __shared__ int hist[kStreamRowMax + 1], whist[kStreamRowMax + 1];
+    for (int i = threadIdx.x; i <= kStreamRowMax; i += blockDim.x) hist[i] = whist[i] = 0;
     __syncthreads();
+    const int lane = threadIdx.x & 31;
     int most = 0;
-    for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < M; r += (long)gridDim.x * blockDim.x) {
-        const int n = __ldg(rowptr + r + 1) - __ldg(rowptr + r);
-        most = max(most, n);
-        if (n <= kStreamRowMax && r % step == 0) atomicAdd(hist + n, 1);
+    for (long r0 = (long)blockIdx.x * blockDim.x + threadIdx.x - lane; r0 < M; r0 += (long)gridDim.x * blockDim.x) {
+        const long r = r0 + lane;                    // whole warps: 32 consecutive rows
+        const int n = r < M ? __ldg(rowptr + r + 1) - __ldg(rowptr + r) : 0;
+        if (r < M && n <= kStreamRowMax && r % step == 0) atomicAdd(hist + n, 1);
+        const int longest = __reduce_max_sync(0xffffffffu, n);
+        most = max(most, longest);
+        if (lane == 0 && longest <= kStreamRowMax) atomicAdd(whist + longest, 1);
     }
-    most = __reduce_max_sync(0xffffffffu, most);
-    if ((threadIdx.x & 31) == 0) atomicMax(&st->max_row, most);
+    if (lane == 0) atomicMax(&st->max_row, most);
     __syncthreads();
-    for (int i = threadIdx.x; i <= kStreamRowMax; i += blockDim.x)
+    for (int i = threadIdx.x; i <= kStreamRowMax; i += blockDim.x) {
         if (hist[i]) atomicAdd(st->hist + i, hist[i]);
+        if (whist[i]) atomicAdd(st->whist + i, whist[i]);
+    }
 }
 
 __global__ void word_signs(const int *__restrict__ cols, long nnz, RowStats *__restrict__ st)
@@ -504,16 +510,18 @@ tc_status plan_upload(tc_plan *p, const int *csrRow, const int *csrCol, int64_t 
         // 2,500,000 13.6 and 10.5; 7 diagonals 6.1 and 6.5 at 650,000, 8.5 and
         // 8.1 at 1,000,000; 2 diagonals 6.1 and 5.4 there).  Above a word a
         // row the tiles gather the words side by side, and the rows kernel is
-        // the faster one while no row takes more than 8 rounds and at most
-        // 0.5 % take more than 4 (300,000 rows of 1.3 words, 3 diagonals: 3.0
-        // and 5.4; with 0.1 % of 64 words 7.6 and 4.8, with one row of 128
-        // 11.0 and 5.2; 1,000,000 rows with 1 % of 32 words 12.6 and 11.5,
-        // with 0.1 % of 16 8.2 and 10.0)
+        // the faster one while no row takes more than 8 rounds and at most a
+        // seventh of the warps hold one of more than 4 (300,000 rows of 1.3
+        // words, 3 diagonals: 3.0 and 5.4; with 0.1 % of 64 words 7.6 and 4.8,
+        // with one row of 128 11.0 and 5.2; 1,000,000 rows with 1 % of 32 words
+        // anywhere, 27 % of the warps, 12.6 and 11.5, with 0.1 % of 16 8.2 and
+        // 10.0; 697,228 rows of 19 diagonals with 0.8 % of 19 words, all at the
+        // end, 12.5 and 14.8)
         const int W = prm.rows_w ? prm.rows_w : p->rows_w;
-        for (int L = std::min(4 * W, kStreamRowMax) + 1; L <= kStreamRowMax; ++L) many += h[L];
+        for (int L = std::min(4 * W, kStreamRowMax) + 1; L <= kStreamRowMax; ++L) many += st.whist[L];
         const int64_t wave = (int64_t)kRowsMinBlocks * num_sms() * kBlock;
         p->rows_any = nnz_csr <= M ? M <= (p->num_negs <= 2 ? 3 : 4) * wave
-                                   : st.max_row <= 8 * W && many * 200 <= tot;
+                                   : st.max_row <= 8 * W && many * 7 <= (M + 31L) / 32;
     }
 
     // the format: row pointers and words, each followed by at least 16 zero

@@ -103,7 +103,8 @@ def test_rows_of_a_cta(tc, dev, tile_nnz):
 @pytest.mark.parametrize("M,mean,long,share,kernel", [
     (60001, 0.4, 8, 0.01, 5), (60001, 0.4, 9, 0.01, 5), (60001, 0.4, 128, 0.002, 5),    # up to a word a row
     (1212417, 0.3, 16, 0.001, 2), (1200001, 0.3, 16, 0.001, 5),                        # about four waves of rows
-    (400001, 1.3, 32, 0.004, 5), (400001, 1.3, 33, 0.004, 2), (400001, 1.3, 20, 0.02, 2), (400001, 1.3, 128, 1e-5, 2)])
+    (400001, 1.3, 32, 0.004, 5), (400001, 1.3, 33, 0.004, 2), (400001, 1.3, 20, 0.02, 2), (400001, 1.3, 128, 1e-5, 2),
+    (400001, 1.3, 20, -0.08, 5)])                   # negative share: neighbours
 def test_spread_rows(tc, dev, M, mean, long, share, kernel):
     """Hybrid plans of three diagonals on both sides of the rules that give
     them to the rows kernel (5) or to their tiles (2), which lie at 148
@@ -111,7 +112,10 @@ def test_spread_rows(tc, dev, M, mean, long, share, kernel):
     import torch
     rng = np.random.default_rng(M + long)
     lens = np.minimum(rng.poisson(mean, M), 6)
-    lens[rng.choice(M, max(1, int(M * share)), replace=False)] = long
+    if share < 0:
+        lens[M // 3:M // 3 - int(M * share)] = long
+    else:
+        lens[rng.choice(M, max(1, int(M * share)), replace=False)] = long
     rp = np.zeros(M + 1, np.int32)
     np.cumsum(lens, out=rp[1:])
     words = ((rng.integers(0, M, rp[-1]) << 1) | (rng.random(rp[-1]) < 0.7)).astype(np.int32)
