@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 
 #include "tc_internal.h"
 #include "tc_words.h"
@@ -327,9 +328,11 @@ constexpr int kDiagU = 4;
 __device__ __forceinline__ float diag_plan_inner(const PlanDiags &q, const float *__restrict__ x, int r)
 {
     // U loads of a thread in flight, as each round waits for L2; whole rounds
-    // without a test per offset (25 offsets, 201,369 rows: 7.2 -> 5.6 us; 15,
-    // 900,000 rows: 11.7 -> 10.4; from the shape arrays 6.9 and 17.5)
-    constexpr int U = 8, R = 4;
+    // without a test per offset, the rest in one round as short as it fits (25
+    // offsets, 201,369 rows: 7.2 -> 5.4 us, 5.7 with a last round of 8; 15,
+    // 900,000 rows: 11.7 -> 10.4; from the shape arrays 6.9 and 17.5; 7,
+    // 264,226 rows: 2.8, 3.1 with two rounds of 4)
+    constexpr int U = 8;
     const float *__restrict__ xr = x + r;
     float acc = 0.f;
     int i = 0;
@@ -341,15 +344,16 @@ __device__ __forceinline__ float diag_plan_inner(const PlanDiags &q, const float
 #pragma unroll
         for (int u = 0; u < U; ++u) acc += v[u];
     }
-#pragma unroll 1
-    for (; i < q.n; i += R) {
-        float v[R];
+    auto rest = [&](auto most) {
+        float v[most];
 #pragma unroll
-        for (int u = 0; u < R; ++u) v[u] = i + u < q.n ? ldx(xr + q.col[i + u]) : 0.f;
+        for (int u = 0; u < most; ++u) v[u] = i + u < q.n ? ldx(xr + q.col[i + u]) : 0.f;
 #pragma unroll
-        for (int u = 0; u < R; ++u)
+        for (int u = 0; u < most; ++u)
             if (i + u < q.n) acc += v[u];
-    }
+    };
+    if (q.n - i > U / 2) rest(std::integral_constant<int, U - 1>{});
+    else if (q.n > i) rest(std::integral_constant<int, U / 2>{});
     return acc;
 }
 
