@@ -58,16 +58,16 @@ __device__ __forceinline__ double signed_term64(double v, int c)
     return __hiloint2double(__double2hiint(v) ^ (int)((unsigned)~c << 31), __double2loint(v));
 }
 
-// Every by-th of the words `a` (W of them), and their terms added to acc.
+// Words j, j + by, ... (W of them, before e), and their terms added to acc.
 template <int W>
-__device__ __forceinline__ void load_words(const DevPlan &p, const Words &a, int by, int (&c)[W])
+__device__ __forceinline__ void load_words(const DevPlan &p, int j, int e, int by, int (&c)[W])
 {
 #pragma unroll
-    for (int w = 0; w < W; ++w) c[w] = w * by < a.left ? __ldg(p.cols + a.at + w * by) : 0;
+    for (int w = 0; w < W; ++w) c[w] = w * by < words_left(j, e) ? __ldg(p.cols + j + w * by) : 0;
 }
 
 template <bool SIGNED, int W>
-__device__ __forceinline__ void add_words(const double *__restrict__ x, const Words &a, int by, const int (&c)[W],
+__device__ __forceinline__ void add_words(const double *__restrict__ x, int j, int e, int by, const int (&c)[W],
                                           double &acc)
 {
     double v[W];                  // a slot past the row loads x[0] and is not added
@@ -75,7 +75,7 @@ __device__ __forceinline__ void add_words(const double *__restrict__ x, const Wo
     for (int w = 0; w < W; ++w) v[w] = ldx64(x + (SIGNED ? c[w] >> 1 : c[w]));
 #pragma unroll
     for (int w = 0; w < W; ++w)
-        if (w * by < a.left) acc += SIGNED ? signed_term64(v[w], c[w]) : v[w];
+        if (w * by < words_left(j, e)) acc += SIGNED ? signed_term64(v[w], c[w]) : v[w];
 }
 
 // The dense-diagonal terms of row r that lane `lane` of `lanes` owns
@@ -154,33 +154,35 @@ __global__ void __launch_bounds__(kBlock, kF64Blocks)
         const int za = __ldg(p.rowptr + ra), zb = __ldg(p.rowptr + rb);
         prefetch_rows_ahead(p, ra, rb, za, words_upto(za, zb, kAheadWords));
     }
-    Words a(ok ? __ldg(p.rowptr + r) : 0, ok ? __ldg(p.rowptr + r + 1) : 0, lane);
+    int j = words_from(ok ? __ldg(p.rowptr + r) : 0, lane);
+    const int e = ok ? __ldg(p.rowptr + r + 1) : 0;
     int c[W];
-    load_words(p, a, G, c);
+    load_words(p, j, e, G, c);
     wait_prior64(x, y);
     double acc = 0.0;
     if constexpr (SIGNED) {
         if (ok) acc = diag_terms64(p, q, x, r, lane, G);
     }
-    add_words<SIGNED>(x, a, G, c, acc);
-    for (a.skip(W * G); a.left > 0; a.skip(W * G)) {
-        load_words(p, a, G, c);
-        add_words<SIGNED>(x, a, G, c, acc);
+    add_words<SIGNED>(x, j, e, G, c, acc);
+    while (words_left(j, e) > W * G) {
+        j += W * G;
+        load_words(p, j, e, G, c);
+        add_words<SIGNED>(x, j, e, G, c, acc);
     }
     acc = group_sum(acc, G);
     if (ok && lane == 0) y[r] = acc;
 }
 
-// A lane's share of the words `a`: every by-th of them.
+// A lane's share of the words [b, e): every by-th from word b + skipped on.
 template <bool SIGNED>
-__device__ __forceinline__ void sum_words64(const DevPlan &p, const double *__restrict__ x, Words a, int by,
-                                            double &acc)
+__device__ __forceinline__ void sum_words64(const DevPlan &p, const double *__restrict__ x, int b, int e, int skipped,
+                                            int by, double &acc)
 {
-    for (; a.left > 0; a.skip(4 * by)) {
+    each_step(b, e, skipped, 4 * by, [&](int j, int) {
         int c[4];
-        load_words(p, a, by, c);
-        add_words<SIGNED>(x, a, by, c, acc);
-    }
+        load_words(p, j, e, by, c);
+        add_words<SIGNED>(x, j, e, by, c, acc);
+    });
 }
 
 // Any plan: a CTA per tile.
@@ -199,7 +201,7 @@ __global__ void __launch_bounds__(kBlock, kF64Blocks)
         if constexpr (SIGNED) {
             acc = diag_terms64(p, q, x, t.row0, threadIdx.x, kBlock);
         }
-        sum_words64<SIGNED>(p, x, Words(t.nz0, t.nz0 + t.nnz, threadIdx.x), kBlock, acc);
+        sum_words64<SIGNED>(p, x, t.nz0, t.nz0 + t.nnz, threadIdx.x, kBlock, acc);
         acc = group_sum(acc, 32);
         if (lane == 0) red[warp] = acc;
         __syncthreads();
@@ -221,7 +223,7 @@ __global__ void __launch_bounds__(kBlock, kF64Blocks)
         if constexpr (SIGNED) {
             if (ok && own) acc = diag_terms64(p, q, x, r, gl, G);
         }
-        if (own) sum_words64<SIGNED>(p, x, Words(b, e, gl), G, acc);
+        if (own) sum_words64<SIGNED>(p, x, b, e, gl, G, acc);
         acc = group_sum(acc, G);
         if (ok && own && gl == 0) y[r] = acc;
         for (unsigned mid = __ballot_sync(0xffffffffu, !own && gl == 0); mid; mid &= mid - 1) {
@@ -232,7 +234,7 @@ __global__ void __launch_bounds__(kBlock, kF64Blocks)
             if constexpr (SIGNED) {
                 a = diag_terms64(p, q, x, mr, lane, 32);
             }
-            sum_words64<SIGNED>(p, x, Words(mb, me, lane), 32, a);
+            sum_words64<SIGNED>(p, x, mb, me, lane, 32, a);
             a = group_sum(a, 32);
             if (lane == 0) y[mr] = a;
         }

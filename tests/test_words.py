@@ -43,6 +43,22 @@ static long steps(int b, int e, int lane, int by, int round)
     return bad + (want < e);
 }
 
+// The same by hand.
+static long by_hand(int b, int e, int lane, int by, int round)
+{
+    long want = (long)b + lane, bad = 0;
+    int j = tc::words_from(b, lane);
+    for (;;) {
+        for (int w = 0; w < round && w * by < tc::words_left(j, e); ++w) {
+            bad += (long)j + w * by != want || want >= e;
+            want += by;
+        }
+        if (tc::words_left(j, e) <= round * by) break;
+        j += round * by;
+    }
+    return bad + (want < e);
+}
+
 int main()
 {
     const int top = 2147483647;
@@ -54,7 +70,8 @@ int main()
             for (int by : bys)
                 for (int r : rounds)
                     for (int lane : {0, 1, by / 2, by - 1})
-                        if (lane < by && (walk(end - n, end, lane, by, r) || steps(end - n, end, lane, by, r))) ++bad;
+                        if (lane < by && (walk(end - n, end, lane, by, r) || steps(end - n, end, lane, by, r) ||
+                                           by_hand(end - n, end, lane, by, r))) ++bad;
     for (int b : {0, 77, top - 100, top - 16384, top - 16385})
         for (int e : {b, b + 1, top - (top - b) / 2, top}) {
             const long want = (long)e - b > 16384 ? (long)b + 16384 : (long)e;
