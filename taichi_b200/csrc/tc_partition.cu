@@ -1253,7 +1253,13 @@ tc_status gpu_partition(int M, int N, int64_t nnz, const int *d_rowptr, const in
         }
     out.dense_nnz = (int)dense;
     out.sparse_nnz = (int)(nnz - dense);
-    long zeros = 0;
+    long zeros = 0, holes = 0;
+    for (const ShapeResult &S : shapes)
+        if (S.nnz > 0)
+            for (int z : S.nzero) holes += std::max(z, 0);
+    // a low density threshold can make more holes than a row pointer counts
+    if (holes + out.sparse_nnz > 0x7fffffffL)
+        return fail(TC_ERR_UNSUPPORTED, "%ld holes and %d entries left: more than 2^31 - 1 CSR words", holes, out.sparse_nnz);
     out.nDiasPtr.push_back(0);
     std::vector<HoleShape> hs;
     for (const ShapeResult &S : shapes) {

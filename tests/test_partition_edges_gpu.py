@@ -117,3 +117,28 @@ def test_many_shapes(tc, dev, nb, height, more_than):
         assert got[k] == want[k], k
     for k in ("xStart", "yStart", "xStop", "nDiasPtr", "neg_offsets", "csrRow", "csrCol"):
         np.testing.assert_array_equal(got[k], want[k], err_msg=k)
+
+
+def test_more_holes_than_words(tc, dev):
+    """Two wide bands of few entries under a density threshold near zero: their
+    holes are more than 2^31, which no row pointer holds; refused, and the same
+    matrix is partitioned under the usual threshold."""
+    import torch
+    side, gap, half = 990_000, 60_000, 980
+    M = 2 * (side + gap)
+    g = torch.Generator(dev).manual_seed(3)
+    rows = torch.arange(M, device=dev)
+    rows = rows[(rows % (side + gap)) < side].repeat_interleave(4)
+    block = torch.div(rows, side + gap, rounding_mode="floor") * (side + gap)
+    cols = rows + torch.randint(-half, half + 1, rows.shape, device=dev, generator=g)
+    ok = (cols >= block) & (cols < block + side)
+    keys = torch.unique(rows[ok] * M + cols[ok])
+    rows = torch.div(keys, M, rounding_mode="floor")
+    rp = torch.zeros(M + 1, dtype=torch.int64, device=dev)
+    rp[1:] = torch.cumsum(torch.bincount(rows, minlength=M), 0)
+    rp, col = rp.int(), (keys - rows * M).int()
+    with pytest.raises(tc.TcError) as e:
+        tc.Plan.from_csr(M, M, rp, col, prm=tc.params(density=1e-6), on_device=True)
+    assert e.value.status == 8 and "2^31" in str(e.value)          # TC_ERR_UNSUPPORTED
+    plan = tc.Plan.from_csr(M, M, rp, col, on_device=True)
+    assert plan.info()["dia_shapes"] == 0 and plan.info()["nnz_csr"] == col.numel()
